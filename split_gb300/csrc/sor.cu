@@ -22,9 +22,11 @@
 // null space, and the relaxation order decides that component of the
 // converged normals.  The order here (red, then black, within a sweep) is the
 // one the FP64 restatement in the oracle follows.  The residual test runs
-// before every sweep as in the reference's monitor; its sums are FP64
-// per-block partials added in block order by every block, so every block
-// takes the same decision and the result does not depend on timing.
+// before every sweep as in the reference's monitor; its sums are per-block
+// partials added in one fixed order by every block, so every block takes the
+// same decision and the result does not depend on timing.
+#include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "common.cuh"
@@ -32,13 +34,21 @@
 namespace sg {
 namespace sor {
 
-constexpr int kThreads = 256;
-constexpr int kMaxBlocks = 4096;
+constexpr int kThreads = 1024;
+constexpr int kWarps = kThreads / 32;
+constexpr int kMaxBlocks = 1024;   // a thread holds one block's partial
 
+// The unknowns are kept per colour (red: row + column even), one float4 per
+// pixel (x0, x1, x2, shading intensity), row r of a colour holding its pixels
+// in column order at [r * wh, r * wh + wh), wh = (W + 1) / 2: pixel k of row r
+// and colour p is column 2 k + ((r + p) & 1).  A pixel's four neighbours are
+// all of the other colour: k in the rows above and below, k and one of k - 1,
+// k + 1 in its own row.
 struct Args {
   const float* s;      // shading intensity, H x W
-  float* x;            // normals, planar 3 x N (in/out)
-  int W, H;
+  float* normals;      // planar 3 x N
+  float4 *red, *red_next, *black, *black_next;   // two iterates of each colour
+  int W, H, wh;
   float L0, L1, L2;    // normalised light direction
   float lam2;          // 2 * smoothness weight
   int max_iter;
@@ -52,143 +62,296 @@ __device__ __forceinline__ int valence(int r, int c, int H, int W) {
   return 4 - ((r == 0 || r == H - 1) ? 1 : 0) - ((c == 0 || c == W - 1) ? 1 : 0);
 }
 
-// sum of the in-grid 4-neighbours' unknowns
-__device__ __forceinline__ void neighbour_sum(const float* x, long long n, int r, int c, int H,
-                                              int W, float (&S)[3]) {
+// A sum of squares in two floats (about 48 bits): each square's product is
+// exact as p + pe, and so is each sum's rounding error, so only the small
+// word rounds.  FP64 on this part runs at two lanes per clock and SM: summing
+// the three squares of a pixel and the warp trees in FP64 took 5.6 us of a
+// VGA sweep, more than everything else in it.
+struct Sum2 {
+  float hi = 0.0f, lo = 0.0f;
+  __device__ __forceinline__ void add(float v, float small) {
+    const float s = __fadd_rn(hi, v);
+    const float b = __fsub_rn(s, hi);
+    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(v, b));
+    lo = __fadd_rn(lo, __fadd_rn(e, small));
+    hi = s;
+  }
+  __device__ __forceinline__ void add_square(float e) {
+    const float p = __fmul_rn(e, e);
+    add(p, __fmaf_rn(e, e, -p));
+  }
+};
+
+struct Problem {
+  float L[3], LL, lam2;
+  int W, H, wh;
+};
+
+// sum of the in-grid 4-neighbours' unknowns of pixel k of row r, column c:
+// `y` holds the other colour
+__device__ __forceinline__ void neighbour_sum(const Problem& P, const float4* y, int r, int k,
+                                              int c, float (&S)[3]) {
+  const long long i = (long long)r * P.wh + k;
+  const int odd = c & 1;
+  // up, left, right, down
+  const long long at[4] = {i - P.wh, odd ? i : i - 1, odd ? i + 1 : i, i + P.wh};
+  const bool in[4] = {r > 0, c > 0, c + 1 < P.W, r + 1 < P.H};
+  float4 v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = in[q] ? y[at[q]] : make_float4(0.f, 0.f, 0.f, 0.f);
   S[0] = S[1] = S[2] = 0.0f;
-  const long long i = (long long)r * W + c;
-  const long long nb[4] = {i - W, i - 1, i + 1, i + W};
-  const bool in[4] = {r > 0, c > 0, c + 1 < W, r + 1 < H};
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (!in[k]) continue;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) S[d] = __fadd_rn(S[d], __ldcg(x + d * n + nb[k]));
+  for (int q = 0; q < 4; ++q) {
+    if (!in[q]) continue;
+    S[0] = __fadd_rn(S[0], v[q].x);
+    S[1] = __fadd_rn(S[1], v[q].y);
+    S[2] = __fadd_rn(S[2], v[q].z);
   }
 }
 
-// FP64 block sum in a fixed order (warp trees, then warps in order)
-__device__ double block_sum(double v) {
-  __shared__ double w[kThreads / 32];
+// adds the squared residual of a pixel (scaled by the power of two `scale`)
+// whose unknowns are x and whose neighbours sum to S
+__device__ __forceinline__ void residual(const Problem& P, const float (&x)[3], float si, float v,
+                                         const float (&S)[3], float scale, Sum2& sum,
+                                         bool& nonzero) {
+  const float lx = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], x[0]), __fmul_rn(P.L[1], x[1])),
+                             __fmul_rn(P.L[2], x[2]));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < kThreads / 32; ++k) t += w[k];
-  __syncthreads();
-  return t;   // valid in thread 0
+  for (int d = 0; d < 3; ++d) {
+    const float lap = __fsub_rn(__fmul_rn(v, x[d]), S[d]);
+    const float ax = __fadd_rn(__fmul_rn(P.L[d], lx), __fmul_rn(P.lam2, lap));
+    const float e = __fsub_rn(__fmul_rn(si, P.L[d]), ax);
+    nonzero |= e != 0.0f;
+    sum.add_square(__fmul_rn(e, scale));
+  }
 }
 
-// every block adds the partials of all blocks in block order
-__device__ double grid_total(const double* partial) {
+// the block solve of a pixel from its neighbours' sum
+__device__ __forceinline__ void solve(const Problem& P, float si, float v, const float (&S)[3],
+                                      float (&x)[3]) {
+  float rv[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) rv[d] = __fadd_rn(__fmul_rn(si, P.L[d]), __fmul_rn(P.lam2, S[d]));
+  const float cc = __fmul_rn(P.lam2, v);
+  const float lr = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], rv[0]), __fmul_rn(P.L[1], rv[1])),
+                             __fmul_rn(P.L[2], rv[2]));
+  const float q = __fdiv_rn(lr, __fadd_rn(cc, P.LL));
+#pragma unroll
+  for (int d = 0; d < 3; ++d) x[d] = __fdiv_rn(__fsub_rn(rv[d], __fmul_rn(P.L[d], q)), cc);
+}
+
+// FP64 sum of the block's lanes in a fixed order: two-float warp trees, then
+// the warps' values in FP64 by the first warp (valid in thread 0)
+__device__ double block_sum(Sum2 v) {
+  __shared__ double w[kWarps];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float h = __shfl_down_sync(0xffffffffu, v.hi, o);
+    const float l = __shfl_down_sync(0xffffffffu, v.lo, o);
+    v.add(h, l);
+  }
+  __syncthreads();   // the last call's words have been read
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = (double)v.hi + (double)v.lo;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 32) {
+    t = w[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  }
+  return t;
+}
+
+// FP64 sum of one value per thread, every thread's result the same; warps
+// whose lanes hold no value skip their tree
+__device__ double block_total(double v, int nvalues) {
+  __shared__ double w[kWarps];
   __shared__ double tot;
+  const int warp = threadIdx.x >> 5;
+  __syncthreads();
+  if (warp * 32 < nvalues) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) w[warp] = v;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (unsigned b = 0; b < gridDim.x; ++b) t += __ldcg(partial + b);
+    for (int i = 0; i * 32 < nvalues; ++i) t += w[i];
     tot = t;
   }
   __syncthreads();
   return tot;
 }
 
-__global__ void __launch_bounds__(kThreads) sor_kernel(Args a) {
-  const long long n = (long long)a.W * a.H;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const float L[3] = {a.L0, a.L1, a.L2};
-  const float LL = __fadd_rn(__fadd_rn(__fmul_rn(L[0], L[0]), __fmul_rn(L[1], L[1])),
-                             __fmul_rn(L[2], L[2]));
+// The pixels of one colour that a thread owns: packed indices first + j *
+// kThreads below `end`, row and place stepped without divisions.
+struct Walk {
+  int i, r, k, dr, dk, end, wh;
+  __device__ __forceinline__ Walk(const Problem& P, int chunk) : wh(P.wh) {
+    const int n = P.H * P.wh;
+    const int b = (int)blockIdx.x * chunk;
+    end = min(n, b + chunk);
+    i = b + (int)threadIdx.x;
+    r = i / wh;
+    k = i - r * wh;
+    dr = kThreads / wh;
+    dk = kThreads - dr * wh;
+  }
+  __device__ __forceinline__ bool more() const { return i < end; }
+  __device__ __forceinline__ void next() {
+    i += kThreads;
+    r += dr;
+    k += dk;
+    if (k >= wh) {
+      k -= wh;
+      ++r;
+    }
+  }
+};
+
+// One persistent cooperative launch, one block per SM at most, every block
+// owning the same contiguous packed pixels of both colours.
+//
+// What bounds it: at VGA a thread holds one pixel per colour, so a pass is
+// the latency of one round of L2 loads and of a grid barrier; larger images
+// are bound by L2 bandwidth.  So a sweep is two passes and two barriers, with
+// no residual pass: the red pass reads the neighbours that the residual of
+// the iterate before it needs as well, and a black pixel's neighbours do not
+// change after its update, so the black pass adds the residuals of the next
+// iterate.  The test's total is known after the barrier that ends the red
+// pass and is added up beside the black pass, so both passes write a second
+// buffer and the iterate before them is the result when the test holds.
+// VGA: 8.2 us a sweep; with a separate residual pass over planar unknowns,
+// FP64 sums, one thread adding all blocks' partials and 760 blocks it took
+// 94 us.
+__global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
+  Problem P;
+  P.L[0] = a.L0;
+  P.L[1] = a.L1;
+  P.L[2] = a.L2;
+  P.LL = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], P.L[0]), __fmul_rn(P.L[1], P.L[1])),
+                   __fmul_rn(P.L[2], P.L[2]));
+  P.lam2 = a.lam2;
+  P.W = a.W;
+  P.H = a.H;
+  P.wh = a.wh;
+  unsigned nbar = 0;
+  float4 *red = a.red, *red_next = a.red_next, *blk = a.black, *blk_next = a.black_next;
   // x0 = (0, 0, 1) and |b|^2 = sum s_i^2 |L|^2
   double acc = 0.0;
-  for (long long i = tid; i < n; i += stride) {
-    __stcg(a.x + i, 0.0f);
-    __stcg(a.x + n + i, 0.0f);
-    __stcg(a.x + 2 * n + i, 1.0f);
-    const double si = (double)__ldg(a.s + i);
-    acc += si * si;
+  for (int colour = 0; colour < 2; ++colour)
+    for (Walk w(P, chunk); w.more(); w.next()) {
+      const int c = 2 * w.k + ((w.r + colour) & 1);
+      if (c >= P.W) continue;
+      const float si = __ldg(a.s + (long long)w.r * P.W + c);
+      (colour ? blk : red)[w.i] = make_float4(0.0f, 0.0f, 1.0f, si);
+      acc += (double)si * (double)si;
+    }
+  acc = block_total(acc, kThreads);
+  if (threadIdx.x == 0) __stcg(a.partial + kMaxBlocks + blockIdx.x, acc);
+  if (!grid_barrier_counted(a.hdr, ++nbar)) return;
+  const bool has = threadIdx.x < gridDim.x;
+  const double bnorm2 =
+      block_total(has ? __ldcg(a.partial + kMaxBlocks + threadIdx.x) : 0.0, (int)gridDim.x) *
+      (double)P.LL;
+  // the residual is summed scaled by a power of two near 1 / |b|, so that its
+  // squares neither overflow nor vanish in FP32 at any intensity
+  int ex = 0;
+  if (bnorm2 > 0.0 && bnorm2 < INFINITY) ex = -(ilogb(bnorm2) / 2);
+  ex = max(-120, min(120, ex));
+  const float scale = ldexpf(1.0f, ex);
+  const double limit2 = (double)a.tol * (double)a.tol * bnorm2 * ldexp(1.0, 2 * ex);
+  // the black pixels' residual at x0
+  Sum2 black;
+  bool black_nz = false;
+  for (Walk w(P, chunk); w.more(); w.next()) {
+    const int c = 2 * w.k + ((w.r + 1) & 1);
+    if (c >= P.W) continue;
+    const float4 o = blk[w.i];
+    const float x[3] = {o.x, o.y, o.z};
+    float S[3];
+    neighbour_sum(P, red, w.r, w.k, c, S);
+    residual(P, x, o.w, (float)valence(w.r, c, P.H, P.W), S, scale, black, black_nz);
   }
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) __stcg(a.partial + blockIdx.x, acc);
-  if (!grid_barrier(a.hdr)) return;
-  const double bnorm2 = grid_total(a.partial) * (double)LL;
-  const double limit2 = (double)a.tol * (double)a.tol * bnorm2;
-  const int Wh = (a.W + 1) / 2;
-  const long long nh = (long long)a.H * Wh;
   int it = 0;
-  for (;; ++it) {
-    // residual of the current iterate
-    double* part = a.partial + (size_t)((it + 1) & 1) * kMaxBlocks;
-    double r2 = 0.0;
-    for (long long i = tid; i < n; i += stride) {
-      const int r = (int)(i / a.W), c = (int)(i - (long long)r * a.W);
-      float S[3];
-      neighbour_sum(a.x, n, r, c, a.H, a.W, S);
-      const float xi[3] = {__ldcg(a.x + i), __ldcg(a.x + n + i), __ldcg(a.x + 2 * n + i)};
-      const float lx = __fadd_rn(__fadd_rn(__fmul_rn(L[0], xi[0]), __fmul_rn(L[1], xi[1])),
-                                 __fmul_rn(L[2], xi[2]));
-      const float v = (float)valence(r, c, a.H, a.W);
-      const float si = __ldg(a.s + i);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float lap = __fsub_rn(__fmul_rn(v, xi[d]), S[d]);
-        const float ax = __fadd_rn(__fmul_rn(L[d], lx), __fmul_rn(a.lam2, lap));
-        const double e = (double)__fsub_rn(__fmul_rn(si, L[d]), ax);
-        r2 += e * e;
-      }
+  for (; it < a.max_iter; ++it) {
+    double* part = a.partial + (size_t)(it & 1) * kMaxBlocks;
+    // red: the residual of the current iterate and the next one's values
+    Sum2 sum = black;
+    bool nz = black_nz;
+    for (Walk w(P, chunk); w.more(); w.next()) {
+      const int c = 2 * w.k + (w.r & 1);
+      if (c >= P.W) continue;
+      const float4 o = red[w.i];
+      float x[3] = {o.x, o.y, o.z}, S[3];
+      const float v = (float)valence(w.r, c, P.H, P.W);
+      neighbour_sum(P, blk, w.r, w.k, c, S);
+      residual(P, x, o.w, v, S, scale, sum, nz);
+      solve(P, o.w, v, S, x);
+      red_next[w.i] = make_float4(x[0], x[1], x[2], o.w);
     }
-    r2 = block_sum(r2);
+    // a residual too small to square in FP32 still is not zero
+    if (nz) sum.hi = fmaxf(sum.hi, FLT_MIN);
+    const double r2 = block_sum(sum);
     if (threadIdx.x == 0) __stcg(part + blockIdx.x, r2);
-    if (!grid_barrier(a.hdr)) return;
-    if (grid_total(part) <= limit2 || it >= a.max_iter) break;
-    // one red-black sweep
-    for (int colour = 0; colour < 2; ++colour) {
-      for (long long k = tid; k < nh; k += stride) {
-        const int r = (int)(k / Wh);
-        const int c = 2 * (int)(k - (long long)r * Wh) + ((r + colour) & 1);
-        if (c >= a.W) continue;
-        const long long i = (long long)r * a.W + c;
-        float S[3];
-        neighbour_sum(a.x, n, r, c, a.H, a.W, S);
-        const float si = __ldg(a.s + i);
-        float rv[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) rv[d] = __fadd_rn(__fmul_rn(si, L[d]), __fmul_rn(a.lam2, S[d]));
-        const float cc = __fmul_rn(a.lam2, (float)valence(r, c, a.H, a.W));
-        const float lr = __fadd_rn(__fadd_rn(__fmul_rn(L[0], rv[0]), __fmul_rn(L[1], rv[1])),
-                                   __fmul_rn(L[2], rv[2]));
-        const float q = __fdiv_rn(lr, __fadd_rn(cc, LL));
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          __stcg(a.x + d * n + i, __fdiv_rn(__fsub_rn(rv[d], __fmul_rn(L[d], q)), cc));
-      }
-      if (!grid_barrier(a.hdr)) return;
+    if (!grid_barrier_counted(a.hdr, ++nbar)) return;
+    const double mine = has ? __ldcg(part + threadIdx.x) : 0.0;
+    // black: the next iterate's values and their residual
+    black = Sum2();
+    black_nz = false;
+    for (Walk w(P, chunk); w.more(); w.next()) {
+      const int c = 2 * w.k + ((w.r + 1) & 1);
+      if (c >= P.W) continue;
+      const float si = blk[w.i].w;
+      float x[3], S[3];
+      const float v = (float)valence(w.r, c, P.H, P.W);
+      neighbour_sum(P, red_next, w.r, w.k, c, S);
+      solve(P, si, v, S, x);
+      residual(P, x, si, v, S, scale, black, black_nz);
+      blk_next[w.i] = make_float4(x[0], x[1], x[2], si);
     }
+    if (block_total(mine, (int)gridDim.x) <= limit2) break;   // iterate `it` is the result
+    if (!grid_barrier_counted(a.hdr, ++nbar)) return;
+    float4* r = red;
+    red = red_next;
+    red_next = r;
+    r = blk;
+    blk = blk_next;
+    blk_next = r;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && a.d_iters) *a.d_iters = it;
-  // unit normals with z >= 0
-  for (long long i = tid; i < n; i += stride) {
-    const float x0 = __ldcg(a.x + i), x1 = __ldcg(a.x + n + i), x2 = __ldcg(a.x + 2 * n + i);
-    const float m = __fadd_rn(__fadd_rn(__fmul_rn(x0, x0), __fmul_rn(x1, x1)), __fmul_rn(x2, x2));
-    const float rmag = __fdiv_rn(1.0f, __fsqrt_rn(m));
-    a.x[i] = __fmul_rn(x0, rmag);
-    a.x[n + i] = __fmul_rn(x1, rmag);
-    a.x[2 * n + i] = __fmul_rn(fabsf(x2), rmag);
-  }
+  // unit normals with z >= 0, each thread from the pixels it wrote itself
+  const long long n = (long long)P.W * P.H;
+  for (int colour = 0; colour < 2; ++colour)
+    for (Walk w(P, chunk); w.more(); w.next()) {
+      const int c = 2 * w.k + ((w.r + colour) & 1);
+      if (c >= P.W) continue;
+      const long long i = (long long)w.r * P.W + c;
+      const float4 x = (colour ? blk : red)[w.i];
+      const float m =
+          __fadd_rn(__fadd_rn(__fmul_rn(x.x, x.x), __fmul_rn(x.y, x.y)), __fmul_rn(x.z, x.z));
+      const float rmag = __fdiv_rn(1.0f, __fsqrt_rn(m));
+      a.normals[i] = __fmul_rn(x.x, rmag);
+      a.normals[n + i] = __fmul_rn(x.y, rmag);
+      a.normals[2 * n + i] = __fmul_rn(fabsf(x.z), rmag);
+    }
 }
 
 struct Layout {
   WsHeader* hdr;
   double* partial;
+  float4* x[2][2];
   size_t bytes;
 };
 
-inline Layout carve(void* ws) {
+inline Layout carve(void* ws, int W, int H) {
   Carver c(ws);
   Layout l;
   l.hdr = c.take<WsHeader>(1);
   l.partial = c.take<double>((size_t)2 * kMaxBlocks);
+  for (int colour = 0; colour < 2; ++colour)
+    for (int i = 0; i < 2; ++i) l.x[colour][i] = c.take<float4>((size_t)H * ((W + 1) / 2));
   l.bytes = c.size();
   return l;
 }
@@ -200,7 +363,7 @@ using namespace sg;
 
 extern "C" size_t split_estimate_normals_workspace_size(int width, int height) {
   if (width < 1 || height < 1) return 0;
-  return sor::carve(nullptr).bytes;
+  return sor::carve(nullptr, width, height).bytes;
 }
 
 extern "C" int split_estimate_normals(const float* intensity, int width, int height, float lx,
@@ -214,26 +377,28 @@ extern "C" int split_estimate_normals(const float* intensity, int width, int hei
   if ((int64_t)width * height > 0x7fffffffLL / 3) return SPLIT_ERR_INVALID;
   const float mag2 = lx * lx + ly * ly + lz * lz;
   if (!(mag2 > 0.0f)) return SPLIT_ERR_INVALID;
-  Layout l = carve(nullptr);
+  Layout l = carve(nullptr, width, height);
   if (!workspace || workspace_bytes < l.bytes || (reinterpret_cast<uintptr_t>(workspace) & 255))
     return SPLIT_ERR_WORKSPACE;
-  l = carve(workspace);
+  l = carve(workspace, width, height);
   cudaStream_t st = as_stream(stream);
   SG_CUDA_TRY(cudaMemsetAsync(l.hdr, 0, sizeof(WsHeader), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
-  int per_sm = 0;
-  SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sor_kernel, kThreads, 0));
-  if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-  int grid = di.sm_count * per_sm;
-  if (grid > kMaxBlocks) grid = kMaxBlocks;
-  const int64_t need = ((int64_t)width * height + kThreads - 1) / kThreads;
-  if (grid > need) grid = (int)need;
+  // One block per SM at most, and one pixel of a colour per thread at least:
+  // the barriers slow with the block count.
+  const int wh = (width + 1) / 2;
+  const int64_t packed = (int64_t)height * wh;
+  int grid = std::min(di.sm_count, kMaxBlocks);
+  grid = (int)std::min<int64_t>(grid, (packed + kThreads - 1) / kThreads);
+  const int64_t chunk64 = (packed + grid - 1) / grid;
+  int chunk = (int)chunk64;
   // the light direction normalised as the reference does (estimate_normals.cu:258-265)
   const float rmag = 1.0f / std::sqrt(mag2);
-  Args a{intensity, normals, width, height, lx * rmag, ly * rmag, lz * rmag, 2.0f * smoothness,
-         max_iter, tol, l.partial, d_iterations, l.hdr};
-  void* args[] = {&a};
+  Args a{intensity, normals, l.x[0][0], l.x[0][1], l.x[1][0], l.x[1][1], width, height, wh,
+         lx * rmag, ly * rmag, lz * rmag, 2.0f * smoothness, max_iter, tol, l.partial,
+         d_iterations, l.hdr};
+  void* args[] = {&a, &chunk};
   SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)sor_kernel, dim3(grid), dim3(kThreads),
                                           args, 0, st));
   return launch_status();
