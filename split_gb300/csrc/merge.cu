@@ -10,14 +10,16 @@
 // for its segment with one 64-bit atomicMax:
 //   MOST_BOUNDARY: (edge count << 32) | ~neighbour      (most edges, lowest id)
 //   REF_CHROMA   : ~((bits(d2) << 32) | neighbour)       (least d2, lowest id)
-// and the winning pair writes the segment's map entry.
+// and the winning pair writes the segment's map entry.  A small segment that
+// lies wholly inside one tile has all its pairs in that tile's table: it is
+// decided there and never enters the global table.
 //
 // Workspace state (kept clean between calls):
 //   table keys / counts / slot list   zero outside a call
 //   best[n]                            zero outside a call
 // Per-call arrays: size[n] (unless the caller passes component sizes),
 // map[n], fin[n] (final target of every small segment), sum[n] (chroma),
-// dec[n] (segments decided by the overflow path).
+// dec[n] (the decided segments).
 //
 // The table holds at most half its capacity (2^ceil(log2 n) slots) of pairs.
 // An image cut into very many small segments can have more distinct pairs
@@ -169,74 +171,253 @@ size_kernel(const int32_t* __restrict__ lab, int64_t n, Layout L, bool count_siz
   }
 }
 
-// boundary histogram of the small segments (of class (lev, cls) when CLASSES)
-// in one 32 x 64 tile, by the block
+__device__ __forceinline__ float seg_mean(const Layout& L, const int32_t* sizes, int s) {
+  return (float)L.sum[s] / (float)__ldg(sizes + s);
+}
+
+// what pair (s, t) with `count` edges bids for its segment s
+__device__ __forceinline__ unsigned long long bid_of(const Layout& L, const int32_t* sizes,
+                                                     int policy, int s, int t, unsigned count) {
+  if (policy == SPLIT_MERGE_MOST_BOUNDARY)
+    return ((unsigned long long)count << 32) | (unsigned)(0xffffffffu - (unsigned)t);
+  const float x = seg_mean(L, sizes, s) - seg_mean(L, sizes, t);
+  const float d2 = __fadd_rn(__fmul_rn(x, x), __fmul_rn(x, x));
+  return ~(((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)t);
+}
+
+__device__ __forceinline__ int bid_target(unsigned long long b, int policy) {
+  if (policy == SPLIT_MERGE_MOST_BOUNDARY) return (int)(0xffffffffu - (unsigned)(b & 0xffffffffull));
+  return (int)(unsigned)((~b) & 0xffffffffull);
+}
+
+// Appends s of the calling lanes to the decided list, one atomic per group of
+// lanes that arrive together.
+__device__ __forceinline__ void list_decided(const Layout& L, int s) {
+  const unsigned am = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(am) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(&L.state->dec_count, (unsigned)__popc(am));
+  base = __shfl_sync(am, base, leader);
+  L.dec[base + __popc(am & ((1u << lane) - 1u))] = s;
+}
+
+// The distinct neighbour segments of the pixel at `c` (row pitch `pitch`) of
+// small segment s, each once with its number of edges: f(t, m) returns
+// whether to go on.
+template <class F>
+__device__ __forceinline__ void for_neighbours(const int* c, int pitch, int s, long long n,
+                                               int* status, F&& f) {
+  int v[8] = {c[-pitch - 1], c[-pitch], c[-pitch + 1], c[-1],
+              c[1],          c[pitch - 1], c[pitch],   c[pitch + 1]};
+  bool any = false;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    if (v[a] >= n) {
+      set_status(status, SPLIT_ERR_INVALID);
+      v[a] = -1;
+    }
+    if (v[a] < 0) v[a] = s;
+    any |= v[a] != s;
+  }
+  if (!any) return;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    bool first = v[a] != s;
+    unsigned m = 1;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      if (b < a) first &= v[b] != v[a];
+      if (b > a) m += v[b] == v[a];
+    }
+    if (first && !f(v[a], m)) return;
+  }
+}
+
+// One tile's tables: its small segments (pixels in the tile, best bid) and
+// their pairs.  Sized for four blocks per SM; a tile of speckle that does not
+// fit inserts into the global table pixel by pixel.
+constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 2;
+constexpr int kSegSlots = 1024, kSegBits = 10;
+constexpr int kPairSlots = 2048, kPairBits = 11;
+constexpr int kTileProbes = 64;
+struct TileTables {
+  union {
+    int lab[kHaloH * kHaloW];              // until the pairs are counted
+    unsigned long long best[kSegSlots];    // after
+  };
+  int seg[kSegSlots];                      // -1: free
+  int pixels[kSegSlots];
+  unsigned long long pair[kPairSlots];     // (segment slot + 1, t); 0: free
+  unsigned edges[kPairSlots];
+  int full;
+};
+
+__device__ __forceinline__ int tile_seg_slot(TileTables& T, int s) {
+  unsigned h = ((unsigned)s * 2654435761u) >> (32 - kSegBits);
+  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (kSegSlots - 1)) {
+    int k = *(volatile int*)&T.seg[h];
+    if (k == -1) k = atomicCAS(&T.seg[h], -1, s);
+    if (k == -1 || k == s) return (int)h;
+  }
+  return -1;
+}
+
+__device__ __forceinline__ bool tile_add_pair(TileTables& T, int slot, int t, unsigned m) {
+  const unsigned long long key = ((unsigned long long)(slot + 1) << 32) | (unsigned)t;
+  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kPairBits));
+  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (kPairSlots - 1)) {
+    unsigned long long k = *(volatile unsigned long long*)&T.pair[h];
+    if (k == 0ull) k = atomicCAS(&T.pair[h], 0ull, key);
+    if (k == 0ull || k == key) {
+      atomicAdd(&T.edges[h], m);
+      return true;
+    }
+  }
+  return false;
+}
+
+// Boundary histogram of the small segments (of class (lev, cls) when CLASSES)
+// in one 32 x 64 tile, by the block.
+//
+// What bounds it: the latency of global atomics where segments are small and
+// many.  Inserting pixel by pixel, up to eight dependent rounds of a table
+// probe, a compare-and-swap and two adds, took 237 us for a 512 x 512 frame
+// of 128 tiles and 4.2 ms for an 8192 x 8192 maze with 1.4 M segments.
+// The shared tables take one round per distinct pair and tile, and segments
+// inside the tile (most segments below a few dozen pixels) none at all: the
+// maze's labelling and merge 6.68 to 3.70 ms, the 512 x 512 frame (which took
+// the decision twice) 418 to 293 us.
 template <bool CLASSES>
 __device__ __forceinline__ void pair_tile(const int32_t* __restrict__ lab, const Geoms& gs,
-                                          const Layout& L, const int32_t* sizes, int P, int tile,
-                                          int lev, unsigned cls, int* status) {
+                                          const Layout& L, const int32_t* sizes, int P, int policy,
+                                          TileTables& T, int tile, int lev, unsigned cls,
+                                          int* status) {
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, tile);
   const int W = tr.W, H = tr.H;
   // an overflow flagged before the tile starts: nothing more to insert
-  __shared__ int stopped;
-  if (threadIdx.x == 0) stopped = *(volatile int*)&L.state->overflow;
-  __syncthreads();
-  bool go = stopped == 0;
-  // all label loads, then all size gathers, before any pixel is examined:
-  // the eight pixels' dependent load pairs overlap instead of serialising
-  constexpr int kPer = kTileH * kTileW / kThreads;
-  int seg[kPer], sz[kPer];
+  if (threadIdx.x == 0) T.full = *(volatile int*)&L.state->overflow ? 2 : 0;
+  // every label load, then every size gather, before any pixel is examined
+  constexpr int kLoads = (kHaloH * kHaloW + kThreads - 1) / kThreads;
+  int v[kLoads];
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) {
+  for (int j = 0; j < kLoads; ++j) {
     const int q = threadIdx.x + j * kThreads;
-    const int x = tr.tx0 + q % kTileW, y = tr.ty0 + q / kTileW;
-    seg[j] = (x < W && y < H) ? __ldg(lab + tr.off + (long long)y * W + x) : -1;
+    const int y = tr.ty0 - 1 + q / kHaloW, x = tr.tx0 - 1 + q % kHaloW;
+    v[j] = (q < kHaloH * kHaloW && x >= 0 && y >= 0 && x < W && y < H)
+               ? __ldg(lab + tr.off + (long long)y * W + x)
+               : -1;
   }
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) sz[j] = (seg[j] >= 0 && seg[j] < n) ? __ldg(sizes + seg[j]) : P;
-  for (int j = 0; j < kPer; ++j) {
-    if (sz[j] >= P || (CLASSES && seg_class(seg[j], lev) != cls)) continue;
+  for (int j = 0; j < kLoads; ++j) {
     const int q = threadIdx.x + j * kThreads;
-    const int x = tr.tx0 + q % kTileW, y = tr.ty0 + q / kTileW;
-    const int s = seg[j];
-    L.fin[s] = s;
-    int t[8];
-    int nt = 0;
+    if (q < kHaloH * kHaloW) T.lab[q] = v[j];
+  }
+  __syncthreads();
+  constexpr int kPer = kTileH * kTileW / kThreads;
+  int seg[kPer];
+  bool any = false;
 #pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const int dx = (d == 0 || d == 3 || d == 5) ? -1 : (d == 2 || d == 4 || d == 7) ? 1 : 0;
-      const int dy = d < 3 ? -1 : d > 4 ? 1 : 0;
-      const int nx = x + dx, ny = y + dy;
-      int v = -1;
-      if (nx >= 0 && ny >= 0 && nx < W && ny < H) v = __ldg(lab + tr.off + (long long)ny * W + nx);
-      if (v >= n) {
-        set_status(status, SPLIT_ERR_INVALID);
-        v = -1;
-      }
-      if (v != s && v >= 0) t[nt++] = v;
+  for (int j = 0; j < kPer; ++j) {
+    const int q = threadIdx.x + j * kThreads;
+    seg[j] = T.lab[(q / kTileW + 1) * kHaloW + q % kTileW + 1];
+  }
+  unsigned small = 0;   // bit j: pixel j belongs to a small segment of the class
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const bool ok = seg[j] >= 0 && seg[j] < n && __ldg(sizes + seg[j]) < P &&
+                    !(CLASSES && seg_class(seg[j], lev) != cls);
+    if (ok) small |= 1u << j;
+    any |= ok;
+  }
+  const bool stopped = T.full == 2;
+  if (!__syncthreads_or(any && !stopped)) return;   // (T.full is read before it changes)
+  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
+    T.seg[i] = -1;
+    T.pixels[i] = 0;
+  }
+  for (int i = threadIdx.x; i < kPairSlots; i += kThreads) {
+    T.pair[i] = 0ull;
+    T.edges[i] = 0u;
+  }
+  __syncthreads();
+  for (int j = 0; j < kPer; ++j) {
+    if (!((small >> j) & 1u)) continue;
+    if (*(volatile int*)&T.full) break;
+    const int q = threadIdx.x + j * kThreads;
+    const int* c = T.lab + (q / kTileW + 1) * kHaloW + q % kTileW + 1;
+    const int s = *c;
+    const int slot = tile_seg_slot(T, s);
+    if (slot < 0) {
+      *(volatile int*)&T.full = 1;
+      break;
     }
-    for (int a = 0; a < nt; ++a) {
-      bool first = true;
-      unsigned m = 1;
-      for (int b = 0; b < a; ++b) first &= (t[b] != t[a]);
-      if (!first) continue;
-      for (int b = a + 1; b < nt; ++b) m += (t[b] == t[a]);
-      if (go && insert(L, s, t[a], m)) go = false;
+    atomicAdd(&T.pixels[slot], 1);
+    for_neighbours(c, kHaloW, s, n, status, [&](int t, unsigned m) {
+      const bool ok = tile_add_pair(T, slot, t, m);
+      if (!ok) *(volatile int*)&T.full = 1;
+      return ok;
+    });
+  }
+  __syncthreads();
+  if (T.full) {
+    // more segments or pairs than the tables hold: straight into the global one
+    for (int j = 0; j < kPer; ++j) {
+      if (!((small >> j) & 1u)) continue;
+      const int q = threadIdx.x + j * kThreads;
+      const int* c = T.lab + (q / kTileW + 1) * kHaloW + q % kTileW + 1;
+      const int s = *c;
+      L.fin[s] = s;
+      bool go = true;
+      for_neighbours(c, kHaloW, s, n, status, [&](int t, unsigned m) {
+        go = !insert(L, s, t, m);
+        return go;
+      });
+      if (!go) break;
     }
+    if (CLASSES) __syncthreads();   // the tables are reused by the block's next tile
+    return;
+  }
+  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
+    T.best[i] = 0ull;
+    const int s = T.seg[i];
+    if (s < 0) continue;
+    L.fin[s] = s;
+    // only a segment wholly inside the tile keeps its count
+    if (CLASSES || T.pixels[i] != __ldg(sizes + s)) T.pixels[i] = 0;
+  }
+  __syncthreads();
+  bool go = true;
+  for (int i = threadIdx.x; i < kPairSlots; i += kThreads) {
+    const unsigned long long k = T.pair[i];
+    if (k == 0ull) continue;
+    const int slot = (int)(k >> 32) - 1, t = (int)(unsigned)(k & 0xffffffffull);
+    const int s = T.seg[slot];
+    if (T.pixels[slot]) {
+      atomicMax(&T.best[slot], bid_of(L, sizes, policy, s, t, T.edges[i]));
+    } else if (go) {
+      go = !insert(L, s, t, T.edges[i]);
+    }
+  }
+  __syncthreads();
+  if (CLASSES) return;
+  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
+    const unsigned long long b = T.best[i];
+    if (b == 0ull) continue;
+    const int s = T.seg[i];
+    L.best[s] = b;
+    L.map[s] = bid_target(b, policy);
+    list_decided(L, s);
   }
 }
 
 // boundary histogram of small segments, one block per 32 x 64 tile
 __global__ void __launch_bounds__(kThreads, 4)
 pair_kernel(const int32_t* __restrict__ lab, Geoms gs, Layout L, const int32_t* sizes, int P,
-            int* status) {
+            int policy, int* status) {
+  __shared__ TileTables T;
   pdl_wait();
-  pair_tile<false>(lab, gs, L, sizes, P, blockIdx.x, 0, 0u, status);
-}
-
-__device__ __forceinline__ float seg_mean(const Layout& L, const int32_t* sizes, int s) {
-  return (float)L.sum[s] / (float)__ldg(sizes + s);
+  pair_tile<false>(lab, gs, L, sizes, P, policy, T, blockIdx.x, 0, 0u, status);
 }
 
 __device__ void bid_phase(const Layout& L, const int32_t* sizes, int policy) {
@@ -245,29 +426,8 @@ __device__ void bid_phase(const Layout& L, const int32_t* sizes, int policy) {
     const int h = L.list[j];
     const unsigned long long k = L.keys[h];
     const int s = key_s(k), t = key_t(k);
-    unsigned long long bid;
-    if (policy == SPLIT_MERGE_MOST_BOUNDARY) {
-      bid = ((unsigned long long)L.counts[h] << 32) | (unsigned)(0xffffffffu - (unsigned)t);
-    } else {
-      const float x = seg_mean(L, sizes, s) - seg_mean(L, sizes, t);
-      const float d2 = __fadd_rn(__fmul_rn(x, x), __fmul_rn(x, x));
-      bid = ~(((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)t);
-    }
+    const unsigned long long bid = bid_of(L, sizes, policy, s, t, L.counts[h]);
     atomicMax(L.best + s, bid);
-  }
-}
-
-__device__ __forceinline__ int bid_target(unsigned long long b, int policy) {
-  if (policy == SPLIT_MERGE_MOST_BOUNDARY) return (int)(0xffffffffu - (unsigned)(b & 0xffffffffull));
-  return (int)(unsigned)((~b) & 0xffffffffull);
-}
-
-__device__ void decide_phase(const Layout& L, int policy) {
-  const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    if (bid_target(L.best[s], policy) == t) L.map[s] = t;
   }
 }
 
@@ -285,52 +445,6 @@ __device__ __forceinline__ int next_of(const Layout& L, const int32_t* sizes, in
   return nx;
 }
 
-// mutual pairs: the larger id keeps itself (fix_map_cycles.cuh:28-43)
-__device__ void cycle_phase(const Layout& L, const int32_t* sizes, int P, int policy) {
-  const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    if (bid_target(L.best[s], policy) != t) continue;
-    if (next_of(L, sizes, P, t) == s && s > t) *(volatile int*)(L.map + s) = s;
-  }
-}
-
-__device__ void resolve_phase(const Layout& L, const int32_t* sizes, int P, int policy,
-                              int* status) {
-  const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    if (bid_target(L.best[s], policy) != t) continue;
-    int r = s;
-    unsigned steps = 0;
-    for (;;) {
-      const int nx = next_of(L, sizes, P, r);
-      if (nx == r) break;
-      r = nx;
-      if (++steps > kChainCap) {
-        set_status(status, SPLIT_ERR_NOT_CONVERGED);
-        break;
-      }
-    }
-    L.fin[s] = r;
-  }
-}
-
-// return the table and the bids to zero
-__device__ void cleanup_phase(const Layout& L) {
-  const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const int h = L.list[j];
-    const unsigned long long k = L.keys[h];
-    L.best[key_s(k)] = 0ull;
-    L.keys[h] = 0ull;
-    L.counts[h] = 0u;
-  }
-}
-
-// ---- overflow path -----------------------------------------------------
 // empties the table slots listed in the claimed-slot list
 __device__ void clear_table(const Layout& L) {
   const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
@@ -341,38 +455,36 @@ __device__ void clear_table(const Layout& L) {
   }
 }
 
-// decisions of one round, also listing the decided segments
-__device__ void decide_list_phase(const Layout& L, int policy) {
+// the winning pairs of the global table: map entries and the decided list
+__device__ void decide_phase(const Layout& L, int policy) {
   const unsigned cnt = *(volatile unsigned*)&L.state->list_count;
   for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
     const unsigned long long k = L.keys[L.list[j]];
     const int s = key_s(k), t = key_t(k);
     if (bid_target(L.best[s], policy) == t) {
       L.map[s] = t;
-      L.dec[atomicAdd(&L.state->dec_count, 1u)] = s;
+      list_decided(L, s);
     }
   }
 }
 
-__device__ void cycle_dec_phase(const Layout& L, const int32_t* sizes, int P) {
+// The end of every decided segment's chain.  Of a mutual pair the larger id
+// keeps itself (fix_map_cycles.cuh:28-43): a chain that meets one ends at the
+// larger id, so the map itself need not be changed first.
+__device__ void resolve_phase(const Layout& L, const int32_t* sizes, int P, int* status) {
   const unsigned cnt = *(volatile unsigned*)&L.state->dec_count;
   for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
     const int s = L.dec[j];
-    const int t = *(volatile int*)(L.map + s);
-    if (next_of(L, sizes, P, t) == s && s > t) *(volatile int*)(L.map + s) = s;
-  }
-}
-
-__device__ void resolve_dec_phase(const Layout& L, const int32_t* sizes, int P, int* status) {
-  const unsigned cnt = *(volatile unsigned*)&L.state->dec_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const int s = L.dec[j];
-    int r = s;
+    int r = s, nx = next_of(L, sizes, P, r);
     unsigned steps = 0;
-    for (;;) {
-      const int nx = next_of(L, sizes, P, r);
-      if (nx == r) break;
+    while (nx != r) {
+      const int nn = next_of(L, sizes, P, nx);
+      if (nn == r) {
+        r = max(r, nx);
+        break;
+      }
       r = nx;
+      nx = nn;
       if (++steps > kChainCap) {
         set_status(status, SPLIT_ERR_NOT_CONVERGED);
         break;
@@ -382,9 +494,18 @@ __device__ void resolve_dec_phase(const Layout& L, const int32_t* sizes, int P, 
   }
 }
 
+// returns the bids of the decided segments to zero
+__device__ void clear_bids(const Layout& L) {
+  const unsigned cnt = *(volatile unsigned*)&L.state->dec_count;
+  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x)
+    L.best[L.dec[j]] = 0ull;
+}
+
+// ---- overflow path -----------------------------------------------------
 // The pair pass overflowed: decide class by class (see the top of the file).
 // Runs inside the cooperative decision launch; every phase sits behind a
-// bounded grid barrier and the round count is bounded.
+// bounded grid barrier and the round count is bounded.  Segments the pair pass
+// decided inside their tiles are decided again, to the same end.
 __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& gs,
                               const int32_t* sizes, int P, int policy,
                               unsigned long long stamp, unsigned& nbar) {
@@ -402,6 +523,7 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
     L.stack[3] = 1, L.stack[4] = 0;
   }
   if (!grid_barrier_counted(h, ++nbar)) return;
+  __shared__ TileTables T;
   __shared__ int lev, cls;
   for (unsigned round = 0;; ++round) {
     if (threadIdx.x == 0) {
@@ -412,13 +534,13 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
     __syncthreads();
     if (lev < 0) break;   // the same decision in every block
     for (int t = blockIdx.x; t < gs.total_tiles; t += gridDim.x)
-      pair_tile<true>(lab, gs, L, sizes, P, t, lev, (unsigned)cls, &h->status);
+      pair_tile<true>(lab, gs, L, sizes, P, policy, T, t, lev, (unsigned)cls, &h->status);
     if (!grid_barrier_counted(h, ++nbar)) return;
     const bool split = *(volatile int*)&st->overflow != 0;
     if (!split) {
       bid_phase(L, sizes, policy);
       if (!grid_barrier_counted(h, ++nbar)) return;
-      decide_list_phase(L, policy);
+      decide_phase(L, policy);
       if (!grid_barrier_counted(h, ++nbar)) return;
     }
     clear_table(L);
@@ -442,20 +564,17 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
     }
     if (!grid_barrier_counted(h, ++nbar)) return;
   }
-  cycle_dec_phase(L, sizes, P);
+  resolve_phase(L, sizes, P, &h->status);
   if (!grid_barrier_counted(h, ++nbar)) return;
-  resolve_dec_phase(L, sizes, P, &h->status);
-  if (!grid_barrier_counted(h, ++nbar)) return;
-  const unsigned cnt = *(volatile unsigned*)&st->dec_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x)
-    L.best[L.dec[j]] = 0ull;
+  clear_bids(L);
   if (lead) h->stamp = stamp;
 }
 
-// The decision over the pair list, one cooperative launch (one block per
-// SM): bids, decisions, mutual-pair fix, chains, cleanup, each phase behind a
-// bounded grid barrier.  The last step records the layout the guard cleared for.
-// When the pair pass overflowed, the overflow path decides instead.
+// The decision, one cooperative launch (at most one block per SM, see
+// merge_run): bids and decisions over the global pair list (skipped when the
+// tiles decided everything), chains, cleanup, each phase behind a bounded grid
+// barrier.  The last step records the layout the guard cleared for.  When the
+// pair pass overflowed, the overflow path decides instead.
 __global__ void __launch_bounds__(kThreads)
 list_kernel(Layout L, const int32_t* lab, Geoms gs, const int32_t* sizes, int P, int policy,
             unsigned long long stamp) {
@@ -466,15 +585,16 @@ list_kernel(Layout L, const int32_t* lab, Geoms gs, const int32_t* sizes, int P,
     overflow_path(L, lab, gs, sizes, P, policy, stamp, nbar);
     return;
   }
-  bid_phase(L, sizes, policy);
+  if (*(volatile unsigned*)&L.state->list_count) {   // likewise
+    bid_phase(L, sizes, policy);
+    if (!grid_barrier_counted(h, ++nbar)) return;
+    decide_phase(L, policy);
+    if (!grid_barrier_counted(h, ++nbar)) return;
+  }
+  resolve_phase(L, sizes, P, &h->status);
   if (!grid_barrier_counted(h, ++nbar)) return;
-  decide_phase(L, policy);
-  if (!grid_barrier_counted(h, ++nbar)) return;
-  cycle_phase(L, sizes, P, policy);
-  if (!grid_barrier_counted(h, ++nbar)) return;
-  resolve_phase(L, sizes, P, policy, &h->status);
-  if (!grid_barrier_counted(h, ++nbar)) return;
-  cleanup_phase(L);
+  clear_table(L);
+  clear_bids(L);
   if (blockIdx.x == 0 && threadIdx.x == 0) h->stamp = stamp;
 }
 
@@ -580,19 +700,23 @@ static int merge_run(int32_t* labels, const Geoms& gs, int P, int policy, const 
     SG_TRY(launch_status());
   }
   launch_pdl(mrg::pair_kernel, dim3(gs.total_tiles), dim3(mrg::kThreads), 0, st, labels, gs, l,
-             sizes, P, &l.hdr->status);
+             sizes, P, policy, &l.hdr->status);
   SG_TRY(launch_status());
   {
-    // One co-resident block per SM: the lists of most images are short and
-    // the decision is bound by its grid barriers, which slow with the block
-    // count.  Images and arenas of 2^24 pixels and more can hold lists of
-    // millions of pairs, walked with a dependent load or two per entry:
-    // there as many blocks as fit, up to 4 per SM.
+    // At most one co-resident block per SM and one per 4096 pixels: the lists
+    // of most images are short and the decision is bound by its grid
+    // barriers, which slow with the block count.  Images and arenas of 2^24
+    // pixels and more can hold lists of millions of entries, walked with a
+    // dependent load or two per entry: there as many blocks as fit, up to 4
+    // per SM.
     int per_sm = 0;
     SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrg::list_kernel,
                                                               mrg::kThreads, 0));
     if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-    const int list_blocks = di.sm_count * (n >= ((int64_t)1 << 24) ? std::min(per_sm, 4) : 1);
+    const int list_blocks =
+        n >= ((int64_t)1 << 24)
+            ? di.sm_count * std::min(per_sm, 4)
+            : (int)std::max<int64_t>(1, std::min<int64_t>(di.sm_count, n / 4096));
     unsigned long long stamp_arg = stamp;
     int P_arg = P, policy_arg = policy;
     const int32_t* sizes_arg = sizes;

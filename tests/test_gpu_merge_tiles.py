@@ -1,0 +1,39 @@
+"""Small-segment merge at the edges of its per-tile tables: segments inside a
+tile (decided there), across tiles (global table), more segments or pairs than
+a tile's tables hold, and workspaces used twice; bit-exact against the
+oracle."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("policy", [0, 1])
+@pytest.mark.parametrize("shape,block,values,P", [
+    ((32, 64), 1, 3, 50),       # one tile of speckle
+    ((32, 64), 1, 1000, 2),     # more single-pixel segments than the tile's table holds
+    ((33, 65), 2, 40, 6),       # the last tiles are one pixel wide or high
+    ((200, 330), 3, 5, 30),     # mixed sizes, many inside their tiles
+    ((200, 330), 1, 60, 9),     # pair tables nearly full
+    ((256, 320), 40, 9, 2000),  # every segment crosses tiles
+    ((1, 500), 1, 4, 3), ((500, 1), 1, 4, 3)])
+def test_merge_tile_tables(cuda, policy, shape, block, values, P):
+    import torch
+    from split_gb300 import ccl
+    h, w = shape
+    rng = np.random.default_rng(h * 7 + w + block)
+    ws = None
+    for k in range(2):   # the second call finds the workspace as the first left it
+        lab = rng.integers(0, values, size=(h // block + 1, w // block + 1))
+        lab = np.ascontiguousarray(lab.repeat(block, 0).repeat(block, 1)[:h, :w]).astype(np.int32)
+        lab[:, : w // 3] = 0 if k else lab[:, : w // 3]   # a large segment beside the speckle
+        seg = oracle.ccl(lab, 8 if k else 4, k)
+        chroma = (rng.integers(0, 256, size=(2, h * w)) / 256.0).astype(np.float32)
+        want = oracle.merge_small(seg, P, policy, chroma)
+        g = torch.from_numpy(seg).to(cuda)
+        ws = ccl.merge_small_segments(torch.from_numpy(chroma).to(cuda), g, ws, P, policy=policy)
+        torch.cuda.synchronize()
+        ws.check("merge")
+        assert np.array_equal(g.cpu().numpy(), want), k
