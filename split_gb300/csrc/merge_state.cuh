@@ -47,5 +47,8 @@ size_t merge_workspace_bytes(int64_t n);
 int merge_decide_only(const int32_t* labels, int width, int height, int P, int policy,
                       const float* chroma, const int32_t* d_sizes, void* workspace,
                       size_t workspace_bytes, cudaStream_t st);
+// out = in with the merged segments' labels, after merge_decide_only.
+int merge_relabel(const int32_t* in, int32_t* out, int width, int height, const void* workspace,
+                  cudaStream_t st);
 
 }  // namespace sg

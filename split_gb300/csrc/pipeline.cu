@@ -143,7 +143,8 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
   SG_TRY(split_ccl(cluster_labels, width, height, p.connectivity, p.convention, l.seg,
                    p.merge_P > 0 ? l.sizes : nullptr, l.ccl_ws, l.ccl_bytes, stream));
   SG_TRY(mark(5));
-  // 3: merge decision (the relabel is fused into the erosion below)
+  // 3: merge decision (the relabel is fused into the erosion below, or runs
+  // alone into the output)
   SG_TRY(mark(6));
   // the reference rule compares mean chroma: the sample's r / intensity
   // plane (row 1 of rgb_to_ic, main.cu:176-193)
@@ -161,12 +162,11 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
                                 stream));
     else
       SG_TRY(split_erode(l.seg, segment_labels, width, height, p.erode_radius, stream));
+  } else if (p.merge_P > 0) {
+    SG_TRY(merge_relabel(l.seg, segment_labels, width, height, l.mrg_ws, st));
   } else {
     SG_CUDA_TRY(cudaMemcpyAsync(segment_labels, l.seg, sizeof(int32_t) * (size_t)n,
                                 cudaMemcpyDeviceToDevice, st));
-    if (p.merge_P > 0)
-      SG_TRY(split_merge_small(segment_labels, width, height, p.merge_P, p.merge_policy, chroma,
-                               l.sizes, l.mrg_ws, l.mrg_bytes, stream));
   }
   SG_TRY(mark(9));
   // 5: normals of the luminance plane, straight from the bytes
