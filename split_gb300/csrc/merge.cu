@@ -32,6 +32,7 @@
 // disjoint classes decide exactly what one pass over a large enough table
 // would.  The chains then resolve over the decided segments.
 #include <algorithm>
+#include <mutex>
 
 #include "geom.cuh"
 #include "merge_state.cuh"
@@ -40,7 +41,10 @@ namespace sg {
 namespace mrg {
 
 constexpr int kThreads = 256;
-static_assert(kTileH * kTileW % kThreads == 0, "whole pixels per thread in a tile");
+// the pair pass: six blocks of 256 threads per SM (three of 512 take 8% more
+// on the maze's 32768 tiles, 5% less on a 512 x 512 frame of 128)
+constexpr int kPairThreads = 256, kPairBlocks = 6;
+constexpr int kListThreads = 512;   // the decision launch (1024: the 4K frame 4 us more)
 constexpr int kProbeCap = 1 << 16;
 constexpr unsigned kChainCap = 1u << 24;
 // overflow path: pending classes (level, class) on a stack, and a bound on rounds
@@ -97,45 +101,59 @@ __device__ __forceinline__ unsigned long long pair_key(int s, int t) {
 __device__ __forceinline__ int key_s(unsigned long long k) { return (int)((k - 1ull) >> 32); }
 __device__ __forceinline__ int key_t(unsigned long long k) { return (int)(unsigned)((k - 1ull) & 0xffffffffull); }
 
-// Inserts (s, t) with multiplicity m.  A new pair that takes the table past
-// half its capacity (or a probe sequence that runs out) flags the overflow
-// and returns true: the caller then stops inserting (the pass decides class
-// by class instead), and so does every tile that starts after the flag is
-// set, so the table never grows past half by more than the lanes running at
-// once.  Every claimed slot is listed (the list holds as many entries as the
-// table), so the table can always be cleared through the list.  The list
-// counter is one word that every new pair increments: the lanes of a warp
-// that claim slots in the same step take their list places with one atomic,
-// and nothing else reads that word during the pass.
-__device__ bool insert(const Layout& L, int s, int t, unsigned m) {
+// Adds m edges to pair (s, t) of the global table.  Returns the slot of a
+// pair not seen before (which the caller lists), -1 for one already there,
+// -2 (and flags the overflow) when a probe sequence runs out.
+__device__ __forceinline__ int claim(const Layout& L, int s, int t, unsigned m) {
   const unsigned long long key = pair_key(s, t);
   const unsigned mask = (1u << L.cap_log2) - 1u;
-  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - L.cap_log2));
+  // a segment's pairs start within eight slots of each other: its claims,
+  // counts and bids share a cache line or two
+  unsigned h = (((unsigned)s * 0x9E3779B9u) >> (32 - L.cap_log2)) +
+               (((unsigned)t * 0x9E3779B9u) >> 29);
+  h &= mask;
   for (int probe = 0; probe < kProbeCap; ++probe, h = (h + 1) & mask) {
     unsigned long long k = *(volatile unsigned long long*)(L.keys + h);
     if (k == 0ull) {
       k = atomicCAS(L.keys + h, 0ull, key);
       if (k == 0ull) {
         atomicAdd(L.counts + h, m);
-        const unsigned am = __activemask();
-        const int lane = threadIdx.x & 31, leader = __ffs(am) - 1;
-        unsigned base = 0;
-        if (lane == leader) base = atomicAdd(&L.state->list_count, (unsigned)__popc(am));
-        base = __shfl_sync(am, base, leader);
-        const unsigned idx = base + __popc(am & ((1u << lane) - 1u));
-        L.list[idx] = (int)h;
-        if (idx < (mask >> 1)) return false;
-        *(volatile int*)&L.state->overflow = 1;
-        return true;
+        return (int)h;
       }
     }
     if (k == key) {
       atomicAdd(L.counts + h, m);
-      return false;
+      return -1;
     }
   }
   *(volatile int*)&L.state->overflow = 1;
-  return true;
+  return -2;
+}
+
+// Lists claimed slot h at place idx.  A pair past half the table's capacity
+// flags the overflow and returns false: the caller then stops inserting (the
+// pass decides class by class instead), and so does every tile that starts
+// after the flag is set, so the table never grows past half by more than the
+// lanes running at once.  Every claimed slot is listed (the list holds as
+// many entries as the table), so the table can always be cleared through it.
+__device__ __forceinline__ bool list_slot(const Layout& L, unsigned idx, int h) {
+  L.list[idx] = h;
+  if (idx < (((1u << L.cap_log2) - 1u) >> 1)) return true;
+  *(volatile int*)&L.state->overflow = 1;
+  return false;
+}
+
+// claim, listing a new pair with one atomic for the lanes that arrive
+// together; returns whether to go on inserting
+__device__ bool insert(const Layout& L, int s, int t, unsigned m) {
+  const int h = claim(L, s, t, m);
+  if (h < 0) return h == -1;
+  const unsigned am = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(am) - 1;
+  unsigned base = 0;
+  if (lane == leader) base = atomicAdd(&L.state->list_count, (unsigned)__popc(am));
+  base = __shfl_sync(am, base, leader);
+  return list_slot(L, base + __popc(am & ((1u << lane) - 1u)), h);
 }
 
 // Class of segment s at split level `lev`: the top lev bits of a hash of s
@@ -296,43 +314,57 @@ __device__ __forceinline__ void for_neighbours(const int* c, int pitch, int s, l
   }
 }
 
-// One tile's tables: its small segments (pixels in the tile, best bid) and
-// their pairs.  Sized for four blocks per SM; a tile of speckle that does not
-// fit inserts into the global table pixel by pixel.
+// One tile's tables: its small segments of several pixels (pixels in the
+// tile, best bid) and their pairs.
 constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 2;
-constexpr int kSegSlots = 1024, kSegBits = 10;
-constexpr int kPairSlots = 2048, kPairBits = 11;
-constexpr int kTileProbes = 64;
+// a table this long into a probe sequence is called full: near capacity the
+// sequences of every pixel grow long (a dense tile took 100 us to fill up)
+constexpr int kTileProbes = 16;
+template <int THREADS, int SEG_BITS, int PAIR_BITS>
 struct TileTables {
+  static constexpr int kThreads = THREADS, kSegBits = SEG_BITS, kPairBits = PAIR_BITS;
+  static constexpr int kSegs = 1 << SEG_BITS, kPairs = 1 << PAIR_BITS;
   union {
-    int lab[kHaloH * kHaloW];              // until the pairs are counted
-    unsigned long long best[kSegSlots];    // after
+    int lab[kHaloH * kHaloW];            // until the pairs are counted
+    unsigned long long best[kSegs];      // after
   };
-  int seg[kSegSlots];                      // -1: free
-  int pixels[kSegSlots];
-  unsigned long long pair[kPairSlots];     // (segment slot + 1, t); 0: free
-  unsigned edges[kPairSlots];
-  int full;
+  unsigned long long pair[kPairs];       // (segment slot + 1, t); 0: free
+  unsigned edges[kPairs];
+  int seg[kSegs];                        // -1: free
+  int pixels[kSegs];
+  unsigned short out[kPairs];            // pairs for the global table
+  int nout, nclaim, full;
+  unsigned base;
+  int scan[THREADS / 32];
 };
+// The pair pass: 28 KB, six blocks per SM.  Ordinary tiles hold up to a few
+// hundred pairs (the maze's at most 250); a tile of dense speckle has
+// thousands and is left to the decision launch's tables (146 KB, one block per
+// SM), which hold any realistic tile; past that, pairs go into the global
+// table pixel by pixel.
+using PassTables = TileTables<kPairThreads, 9, 10>;
+using DenseTables = TileTables<kListThreads, 11, 13>;
 
-__device__ __forceinline__ int tile_seg_slot(TileTables& T, int s) {
-  unsigned h = ((unsigned)s * 2654435761u) >> (32 - kSegBits);
-  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (kSegSlots - 1)) {
-    int k = *(volatile int*)&T.seg[h];
-    if (k == -1) k = atomicCAS(&T.seg[h], -1, s);
+template <class T>
+__device__ __forceinline__ int tile_seg_slot(T& tab, int s) {
+  unsigned h = ((unsigned)s * 2654435761u) >> (32 - T::kSegBits);
+  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (T::kSegs - 1)) {
+    int k = *(volatile int*)&tab.seg[h];
+    if (k == -1) k = atomicCAS(&tab.seg[h], -1, s);
     if (k == -1 || k == s) return (int)h;
   }
   return -1;
 }
 
-__device__ __forceinline__ bool tile_add_pair(TileTables& T, int slot, int t, unsigned m) {
+template <class T>
+__device__ __forceinline__ bool tile_add_pair(T& tab, int slot, int t, unsigned m) {
   const unsigned long long key = ((unsigned long long)(slot + 1) << 32) | (unsigned)t;
-  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kPairBits));
-  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (kPairSlots - 1)) {
-    unsigned long long k = *(volatile unsigned long long*)&T.pair[h];
-    if (k == 0ull) k = atomicCAS(&T.pair[h], 0ull, key);
+  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - T::kPairBits));
+  for (int probe = 0; probe < kTileProbes; ++probe, h = (h + 1) & (T::kPairs - 1)) {
+    unsigned long long k = *(volatile unsigned long long*)&tab.pair[h];
+    if (k == 0ull) k = atomicCAS(&tab.pair[h], 0ull, key);
     if (k == 0ull || k == key) {
-      atomicAdd(&T.edges[h], m);
+      atomicAdd(&tab.edges[h], m);
       return true;
     }
   }
@@ -340,147 +372,232 @@ __device__ __forceinline__ bool tile_add_pair(TileTables& T, int slot, int t, un
 }
 
 // Boundary histogram of the small segments (of class (lev, cls) when CLASSES)
-// in one 32 x 64 tile, by the block.
+// in one 32 x 64 tile, by the block.  DEFER: a tile that does not fit the
+// tables is listed for the decision launch instead (at the end of dec, which
+// never meets its front: every such tile has segments of several pixels, so
+// more pixels than decided segments).
 //
 // What bounds it: the latency of global atomics where segments are small and
 // many.  Inserting pixel by pixel, up to eight dependent rounds of a table
 // probe, a compare-and-swap and two adds, took 237 us for a 512 x 512 frame
 // of 128 tiles and 4.2 ms for an 8192 x 8192 maze with 1.4 M segments.
-// The shared tables take one round per distinct pair and tile, and segments
-// inside the tile (most segments below a few dozen pixels) none at all: the
-// maze's labelling and merge 6.68 to 3.70 ms, the 512 x 512 frame (which took
-// the decision twice) 418 to 293 us.
-template <bool CLASSES>
+// The shared tables take one round per distinct pair and tile, segments inside
+// the tile (most segments below a few dozen pixels) none at all, and segments
+// of one pixel are decided from registers; list places are taken with one
+// atomic per block.  Maze: this pass 4.2 to 1.15 ms, with the labelling 6.67
+// to 2.61 ms; 512 x 512 speckle (which took the decision twice) 496 to 252 us
+// a frame.
+template <bool CLASSES, bool DEFER, class T>
 __device__ __forceinline__ void pair_tile(const int32_t* __restrict__ lab, const Geoms& gs,
                                           const Layout& L, const int32_t* sizes, int P, int policy,
-                                          TileTables& T, int tile, int lev, unsigned cls,
-                                          int* status) {
+                                          T& tab, int tile, int lev, unsigned cls, int* status) {
+  constexpr int NT = T::kThreads;
+  constexpr int kPer = kTileH * kTileW / NT;
+  static_assert(kTileH * kTileW % NT == 0, "whole pixels per thread in a tile");
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, tile);
   const int W = tr.W, H = tr.H;
-  // an overflow flagged before the tile starts: nothing more to insert
-  if (threadIdx.x == 0) T.full = *(volatile int*)&L.state->overflow ? 2 : 0;
   // every label load, then every size gather, before any pixel is examined
-  constexpr int kLoads = (kHaloH * kHaloW + kThreads - 1) / kThreads;
-  int v[kLoads];
+  int seg[kPer], sz[kPer];
 #pragma unroll
-  for (int j = 0; j < kLoads; ++j) {
-    const int q = threadIdx.x + j * kThreads;
+  for (int j = 0; j < kPer; ++j) {
+    const int q = threadIdx.x + j * NT;
+    const int x = tr.tx0 + q % kTileW, y = tr.ty0 + q / kTileW;
+    seg[j] = (x < W && y < H) ? __ldg(lab + tr.off + (long long)y * W + x) : -1;
+  }
+  // an overflow flagged before the tile starts: nothing more to insert
+  const bool stopped = *(volatile int*)&L.state->overflow != 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) sz[j] = (seg[j] >= 0 && seg[j] < n) ? __ldg(sizes + seg[j]) : P;
+  // bit j: pixel j belongs to a small segment (of the class) of several
+  // pixels / is one by itself
+  unsigned small = 0, single = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (sz[j] >= P || (CLASSES && seg_class(seg[j], lev) != cls)) continue;
+    if (!CLASSES && sz[j] == 1)
+      single |= 1u << j;
+    else
+      small |= 1u << j;
+  }
+  if (!__syncthreads_or((small | single) != 0u)) return;
+  for (int q = threadIdx.x; q < kHaloH * kHaloW; q += NT) {
     const int y = tr.ty0 - 1 + q / kHaloW, x = tr.tx0 - 1 + q % kHaloW;
-    v[j] = (q < kHaloH * kHaloW && x >= 0 && y >= 0 && x < W && y < H)
-               ? __ldg(lab + tr.off + (long long)y * W + x)
-               : -1;
+    tab.lab[q] = (x >= 0 && y >= 0 && x < W && y < H)
+                     ? __ldg(lab + tr.off + (long long)y * W + x)
+                     : -1;
   }
+  if (threadIdx.x == 0) {
+    tab.nout = 0;
+    tab.nclaim = 0;
+    tab.full = 0;
+  }
+  // (one thread's view of the overflow flag decides for the block)
+  if (__syncthreads_or(threadIdx.x == 0 && stopped)) return;
+  auto at = [&](int j) {
+    const int q = threadIdx.x + j * NT;
+    return tab.lab + (q / kTileW + 1) * kHaloW + q % kTileW + 1;
+  };
+  unsigned decided = 0;   // bit j: the single pixel j has a target
+  if (!CLASSES) {
+    // a segment of one pixel: its eight neighbours are all there is to know
 #pragma unroll
-  for (int j = 0; j < kLoads; ++j) {
-    const int q = threadIdx.x + j * kThreads;
-    if (q < kHaloH * kHaloW) T.lab[q] = v[j];
-  }
-  __syncthreads();
-  constexpr int kPer = kTileH * kTileW / kThreads;
-  int seg[kPer];
-  bool any = false;
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int q = threadIdx.x + j * kThreads;
-    seg[j] = T.lab[(q / kTileW + 1) * kHaloW + q % kTileW + 1];
-  }
-  unsigned small = 0;   // bit j: pixel j belongs to a small segment of the class
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const bool ok = seg[j] >= 0 && seg[j] < n && __ldg(sizes + seg[j]) < P &&
-                    !(CLASSES && seg_class(seg[j], lev) != cls);
-    if (ok) small |= 1u << j;
-    any |= ok;
-  }
-  const bool stopped = T.full == 2;
-  if (!__syncthreads_or(any && !stopped)) return;   // (T.full is read before it changes)
-  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
-    T.seg[i] = -1;
-    T.pixels[i] = 0;
-  }
-  for (int i = threadIdx.x; i < kPairSlots; i += kThreads) {
-    T.pair[i] = 0ull;
-    T.edges[i] = 0u;
-  }
-  __syncthreads();
-  for (int j = 0; j < kPer; ++j) {
-    if (!((small >> j) & 1u)) continue;
-    if (*(volatile int*)&T.full) break;
-    const int q = threadIdx.x + j * kThreads;
-    const int* c = T.lab + (q / kTileW + 1) * kHaloW + q % kTileW + 1;
-    const int s = *c;
-    const int slot = tile_seg_slot(T, s);
-    if (slot < 0) {
-      *(volatile int*)&T.full = 1;
-      break;
+    for (int j = 0; j < kPer; ++j) {
+      if (!((single >> j) & 1u)) continue;
+      const int s = seg[j];
+      unsigned long long best = 0ull;
+      for_neighbours(at(j), kHaloW, s, n, status, [&](int t, unsigned m) {
+        best = max(best, bid_of(L, sizes, policy, s, t, m));
+        return true;
+      });
+      L.fin[s] = s;
+      if (best == 0ull) continue;
+      L.best[s] = best;
+      L.map[s] = bid_target(best, policy);
+      decided |= 1u << j;
     }
-    atomicAdd(&T.pixels[slot], 1);
-    for_neighbours(c, kHaloW, s, n, status, [&](int t, unsigned m) {
-      const bool ok = tile_add_pair(T, slot, t, m);
-      if (!ok) *(volatile int*)&T.full = 1;
-      return ok;
-    });
   }
-  __syncthreads();
-  if (T.full) {
+  const bool tables = __syncthreads_or(small != 0u);
+  if (tables) {
+    for (int i = threadIdx.x; i < T::kSegs; i += NT) {
+      tab.seg[i] = -1;
+      tab.pixels[i] = 0;
+    }
+    for (int i = threadIdx.x; i < T::kPairs; i += NT) {
+      tab.pair[i] = 0ull;
+      tab.edges[i] = 0u;
+    }
+    __syncthreads();
+    for (int j = 0; j < kPer; ++j) {
+      if (!((small >> j) & 1u)) continue;
+      if (*(volatile int*)&tab.full) break;
+      const int* c = at(j);
+      const int s = *c;
+      const int slot = tile_seg_slot(tab, s);
+      if (slot < 0) {
+        *(volatile int*)&tab.full = 1;
+        break;
+      }
+      atomicAdd(&tab.pixels[slot], 1);
+      for_neighbours(c, kHaloW, s, n, status, [&](int t, unsigned m) {
+        const bool ok = tile_add_pair(tab, slot, t, m);
+        if (!ok) *(volatile int*)&tab.full = 1;
+        return ok;
+      });
+    }
+    __syncthreads();
+  }
+  const bool full = tables && tab.full;
+  if (DEFER && full) {
+    if (threadIdx.x == 0) L.dec[n - 1 - atomicAdd(&L.state->dense_count, 1u)] = tile;
+    return;
+  }
+  if (full) {
     // more segments or pairs than the tables hold: straight into the global one
     for (int j = 0; j < kPer; ++j) {
       if (!((small >> j) & 1u)) continue;
-      const int q = threadIdx.x + j * kThreads;
-      const int* c = T.lab + (q / kTileW + 1) * kHaloW + q % kTileW + 1;
+      const int* c = at(j);
       const int s = *c;
       L.fin[s] = s;
       bool go = true;
       for_neighbours(c, kHaloW, s, n, status, [&](int t, unsigned m) {
-        go = !insert(L, s, t, m);
+        go = insert(L, s, t, m);
         return go;
       });
       if (!go) break;
     }
-    if (CLASSES) __syncthreads();   // the tables are reused by the block's next tile
-    return;
-  }
-  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
-    T.best[i] = 0ull;
-    const int s = T.seg[i];
-    if (s < 0) continue;
-    L.fin[s] = s;
-    // only a segment wholly inside the tile keeps its count
-    if (CLASSES || T.pixels[i] != __ldg(sizes + s)) T.pixels[i] = 0;
-  }
-  __syncthreads();
-  bool go = true;
-  for (int i = threadIdx.x; i < kPairSlots; i += kThreads) {
-    const unsigned long long k = T.pair[i];
-    if (k == 0ull) continue;
-    const int slot = (int)(k >> 32) - 1, t = (int)(unsigned)(k & 0xffffffffull);
-    const int s = T.seg[slot];
-    if (T.pixels[slot]) {
-      atomicMax(&T.best[slot], bid_of(L, sizes, policy, s, t, T.edges[i]));
-    } else if (go) {
-      go = !insert(L, s, t, T.edges[i]);
+  } else if (tables) {
+    for (int i = threadIdx.x; i < T::kSegs; i += NT) {
+      tab.best[i] = 0ull;
+      const int s = tab.seg[i];
+      if (s < 0) continue;
+      L.fin[s] = s;
+      // only a segment wholly inside the tile keeps its count
+      if (CLASSES || tab.pixels[i] != __ldg(sizes + s)) tab.pixels[i] = 0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < T::kPairs; i += NT) {
+      const unsigned long long k = tab.pair[i];
+      if (k == 0ull) continue;
+      const int slot = (int)(k >> 32) - 1, t = (int)(unsigned)(k & 0xffffffffull);
+      if (tab.pixels[slot])
+        atomicMax(&tab.best[slot], bid_of(L, sizes, policy, tab.seg[slot], t, tab.edges[i]));
+      else
+        tab.out[atomicAdd(&tab.nout, 1)] = (unsigned short)i;
+    }
+    __syncthreads();
+    const int nout = tab.nout;
+    bool go = true;
+    for (int o0 = 0; o0 < nout; o0 += NT) {
+      const int o = o0 + threadIdx.x;
+      int h = -1;
+      if (o < nout && go) {
+        const int i = tab.out[o];
+        const unsigned long long k = tab.pair[i];
+        h = claim(L, tab.seg[(int)(k >> 32) - 1], (int)(unsigned)(k & 0xffffffffull),
+                  tab.edges[i]);
+        go = h != -2;
+      }
+      const int place = h >= 0 ? atomicAdd(&tab.nclaim, 1) : 0;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        tab.base = tab.nclaim ? atomicAdd(&L.state->list_count, (unsigned)tab.nclaim) : 0u;
+        tab.nclaim = 0;
+      }
+      __syncthreads();
+      if (h >= 0) go = list_slot(L, tab.base + (unsigned)place, h) && go;
     }
   }
-  __syncthreads();
-  if (CLASSES) return;
-  for (int i = threadIdx.x; i < kSegSlots; i += kThreads) {
-    const unsigned long long b = T.best[i];
-    if (b == 0ull) continue;
-    const int s = T.seg[i];
-    L.best[s] = b;
-    L.map[s] = bid_target(b, policy);
-    list_decided(L, s);
+  if (CLASSES) {
+    __syncthreads();   // the tables are reused by the block's next tile
+    return;
   }
+  // the tile's decided segments, listed with one atomic
+  int mine = __popc(decided);
+  if (tables && !full)
+    for (int i = threadIdx.x; i < T::kSegs; i += NT) mine += tab.best[i] != 0ull;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) tab.scan[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < NT / 32; ++w) {
+      const int c = tab.scan[w];
+      tab.scan[w] = sum;
+      sum += c;
+    }
+    tab.base = sum ? atomicAdd(&L.state->dec_count, (unsigned)sum) : 0u;
+  }
+  __syncthreads();
+  unsigned place = tab.base + (unsigned)(tab.scan[warp] + incl - mine);
+#pragma unroll
+  for (int j = 0; j < kPer; ++j)
+    if ((decided >> j) & 1u) L.dec[place++] = seg[j];
+  if (tables && !full)
+    for (int i = threadIdx.x; i < T::kSegs; i += NT) {
+      const unsigned long long b = tab.best[i];
+      if (b == 0ull) continue;
+      const int s = tab.seg[i];
+      L.best[s] = b;
+      L.map[s] = bid_target(b, policy);
+      L.dec[place++] = s;
+    }
+  if (!DEFER) __syncthreads();   // the tables are reused by the block's next tile
 }
 
 // boundary histogram of small segments, one block per 32 x 64 tile
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kPairThreads, kPairBlocks)
 pair_kernel(const int32_t* __restrict__ lab, Geoms gs, Layout L, const int32_t* sizes, int P,
             int policy, int* status) {
-  __shared__ TileTables T;
+  __shared__ PassTables tab;
   pdl_wait();
-  pair_tile<false>(lab, gs, L, sizes, P, policy, T, blockIdx.x, 0, 0u, status);
+  pair_tile<false, true>(lab, gs, L, sizes, P, policy, tab, blockIdx.x, 0, 0u, status);
 }
 
 __device__ void bid_phase(const Layout& L, const int32_t* sizes, int policy) {
@@ -571,7 +688,7 @@ __device__ void clear_bids(const Layout& L) {
 // decided inside their tiles are decided again, to the same end.
 __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& gs,
                               const int32_t* sizes, int P, int policy,
-                              unsigned long long stamp, unsigned& nbar) {
+                              unsigned long long stamp, unsigned& nbar, DenseTables& tab) {
   WsHeader* h = L.hdr;
   State* st = L.state;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
@@ -586,7 +703,6 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
     L.stack[3] = 1, L.stack[4] = 0;
   }
   if (!grid_barrier_counted(h, ++nbar)) return;
-  __shared__ TileTables T;
   __shared__ int lev, cls;
   for (unsigned round = 0;; ++round) {
     if (threadIdx.x == 0) {
@@ -597,7 +713,8 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
     __syncthreads();
     if (lev < 0) break;   // the same decision in every block
     for (int t = blockIdx.x; t < gs.total_tiles; t += gridDim.x)
-      pair_tile<true>(lab, gs, L, sizes, P, policy, T, t, lev, (unsigned)cls, &h->status);
+      pair_tile<true, false>(lab, gs, L, sizes, P, policy, tab, t, lev, (unsigned)cls,
+                             &h->status);
     if (!grid_barrier_counted(h, ++nbar)) return;
     const bool split = *(volatile int*)&st->overflow != 0;
     if (!split) {
@@ -634,21 +751,37 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
 }
 
 // The decision, one cooperative launch (at most one block per SM, see
-// merge_run): bids and decisions over the global pair list (skipped when the
-// tiles decided everything), chains, cleanup, each phase behind a bounded grid
-// barrier.  The last step records the layout the guard cleared for.  When the
-// pair pass overflowed, the overflow path decides instead.
-__global__ void __launch_bounds__(kThreads)
+// merge_run): the dense tiles the pair pass left, bids and decisions over the
+// global pair list (each skipped when there is none), chains, cleanup, each
+// phase behind a bounded grid barrier.  The last step records the layout the
+// guard cleared for.  When the table overflowed, the overflow path decides
+// instead.
+__global__ void __launch_bounds__(kListThreads, 1)
 list_kernel(Layout L, const int32_t* lab, Geoms gs, const int32_t* sizes, int P, int policy,
             unsigned long long stamp) {
+  extern __shared__ __align__(16) unsigned char list_smem[];
+  DenseTables& tab = *reinterpret_cast<DenseTables*>(list_smem);
   WsHeader* h = L.hdr;
   // grid barriers passed (the guard zeroed the counter they count on)
   unsigned nbar = 0;
-  if (*(volatile int*)&L.state->overflow) {   // set before this launch: the same in every block
-    overflow_path(L, lab, gs, sizes, P, policy, stamp, nbar);
+  // written before this launch only: the same in every block
+  const unsigned dense = *(volatile unsigned*)&L.state->dense_count;
+  bool over = *(volatile int*)&L.state->overflow != 0;
+  if (dense && !over) {
+    for (unsigned k = blockIdx.x; k < dense; k += gridDim.x) {
+      const int tile = *(volatile int*)&L.dec[gs.total_px - 1 - k];
+      if (tile >= 0 && tile < gs.total_tiles)
+        pair_tile<false, false>(lab, gs, L, sizes, P, policy, tab, tile, 0, 0u, &h->status);
+    }
+    if (!grid_barrier_counted(h, ++nbar)) return;
+    over = *(volatile int*)&L.state->overflow != 0;   // every insert came before the barrier
+    // the overflow path resets the flag behind its next barrier
+  }
+  if (over) {
+    overflow_path(L, lab, gs, sizes, P, policy, stamp, nbar, tab);
     return;
   }
-  if (*(volatile unsigned*)&L.state->list_count) {   // likewise
+  if (*(volatile unsigned*)&L.state->list_count) {
     bid_phase(L, sizes, policy);
     if (!grid_barrier_counted(h, ++nbar)) return;
     decide_phase(L, policy);
@@ -704,6 +837,7 @@ __global__ void guard_kernel(WsHeader* h, unsigned long long stamp, Layout L, lo
     st->cap_log2 = L.cap_log2;
     st->overflow = 0;
     st->dec_count = 0;
+    st->dense_count = 0;
     h->barrier_count = 0;
   }
   if (*(volatile const unsigned long long*)&h->stamp == stamp) return;
@@ -715,6 +849,23 @@ __global__ void guard_kernel(WsHeader* h, unsigned long long stamp, Layout L, lo
   }
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
     L.best[i] = 0ull;
+}
+
+// The decision launch's shared memory is above the default limit: allowed once
+// per device (no stream work, so a graph capture may be under way).
+static int list_attributes() {
+  static std::mutex mu;
+  static bool done[64] = {false};
+  int dev = 0;
+  SG_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return SPLIT_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done[dev]) return SPLIT_OK;
+  SG_CUDA_TRY(cudaFuncSetAttribute((const void*)list_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(DenseTables)));
+  done[dev] = true;
+  return SPLIT_OK;
 }
 
 }  // namespace mrg
@@ -792,24 +943,15 @@ static int merge_run(int32_t* labels, const Geoms& gs, int P, int policy, const 
                ref ? chroma : nullptr, &l.hdr->status);
     SG_TRY(launch_status());
   }
-  launch_pdl(mrg::pair_kernel, dim3(gs.total_tiles), dim3(mrg::kThreads), 0, st, labels, gs, l,
+  launch_pdl(mrg::pair_kernel, dim3(gs.total_tiles), dim3(mrg::kPairThreads), 0, st, labels, gs, l,
              sizes, P, policy, &l.hdr->status);
   SG_TRY(launch_status());
   {
-    // At most one co-resident block per SM and one per 4096 pixels: the lists
-    // of most images are short and the decision is bound by its grid
-    // barriers, which slow with the block count.  Images and arenas of 2^24
-    // pixels and more can hold lists of millions of entries, walked with a
-    // dependent load or two per entry: there as many blocks as fit, up to 4
-    // per SM.
-    int per_sm = 0;
-    SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrg::list_kernel,
-                                                              mrg::kThreads, 0));
-    if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-    const int list_blocks =
-        n >= ((int64_t)1 << 24)
-            ? di.sm_count * std::min(per_sm, 4)
-            : (int)std::max<int64_t>(1, std::min<int64_t>(di.sm_count, n / 4096));
+    // At most one co-resident block per SM and one per 8192
+    // pixels: the lists of most images are short and the decision is bound by
+    // its grid barriers, which slow with the block count.
+    SG_TRY(mrg::list_attributes());
+    const int list_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(di.sm_count, n / 8192));
     unsigned long long stamp_arg = stamp;
     int P_arg = P, policy_arg = policy;
     const int32_t* sizes_arg = sizes;
@@ -817,7 +959,8 @@ static int merge_run(int32_t* labels, const Geoms& gs, int P, int policy, const 
     Geoms gs_arg = gs;
     void* args[] = {&l, &lab_arg, &gs_arg, &sizes_arg, &P_arg, &policy_arg, &stamp_arg};
     SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)mrg::list_kernel, dim3(list_blocks),
-                                            dim3(mrg::kThreads), args, 0, st));
+                                            dim3(mrg::kListThreads), args, sizeof(mrg::DenseTables),
+                                            st));
   }
   SG_TRY(launch_status());
   if (relabel_labels)

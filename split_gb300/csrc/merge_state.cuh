@@ -16,8 +16,9 @@ struct State {
   int cap_log2;
   int n;                 // pixels (segment ids lie in [0, n))
   int overflow;          // the pair pass found the table full (see split_round)
-  unsigned dec_count;    // decided segments of the rounds (overflow path)
-  int pad[6];
+  unsigned dec_count;    // decided segments
+  unsigned dense_count;  // tiles the pair pass left to the decision launch
+  int pad[5];
 };
 
 // Final label of a pixel whose pre-merge label is v.  Small segments take the

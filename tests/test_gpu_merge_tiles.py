@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
     ((32, 64), 1, 3, 50),       # one tile of speckle
     ((32, 64), 1, 1000, 2),     # more single-pixel segments than the tile's table holds
     ((33, 65), 2, 40, 6),       # the last tiles are one pixel wide or high
+    ((64, 128), 2, 1000, 6),    # more pairs than the decision launch's tables hold
     ((200, 330), 3, 5, 30),     # mixed sizes, many inside their tiles
     ((200, 330), 1, 60, 9),     # pair tables nearly full
     ((256, 320), 40, 9, 2000),  # every segment crosses tiles
