@@ -276,9 +276,10 @@ struct Smem {
   alignas(16) float cent[kMaxK * 8];
   float acc[kWarps][kMaxK * kMaxDim];
   int cnt[kWarps][kMaxK];
-  // the sums of the spans processed since the last flush, in fixed point
-  // (each span's converted on its own, then added as integers)
-  long long fix[kMaxK * kMaxDim];
+  // the sums of the spans processed since the last flush, in 64-bit fixed
+  // point (each span's converted on its own, then added as integers); two
+  // words, because shared memory adds 32 bits in one operation
+  unsigned fix_lo[kMaxK * kMaxDim], fix_hi[kMaxK * kMaxDim];
   int fixn[kMaxK];
   // n * c * 2^24 of every centroid value, n the pixels of a whole span
   long long nc[kMaxK * kMaxDim];
@@ -294,14 +295,12 @@ struct Smem {
   int stopped, more;
 };
 
-// Advance a (row, col) pair by s pixels along the row-major order.
-__device__ __forceinline__ void advance(int& row, int& col, int s, int w) {
-  col += s;
-  if (col >= w) {
-    int q = col / w;
-    row += q;
-    col -= q * w;
-  }
+// sum idx += v (64 bits, wrapping)
+__device__ __forceinline__ void fix_add(Smem& sm, int idx, long long v) {
+  const unsigned lo = (unsigned)v;
+  const unsigned old = atomicAdd(&sm.fix_lo[idx], lo);
+  const unsigned hi = (unsigned)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
+  if (hi) atomicAdd(&sm.fix_hi[idx], hi);
 }
 
 // acc[d] += x[d] - c[d] for every dimension, in IEEE single precision: the
@@ -421,19 +420,57 @@ __device__ __forceinline__ void nearest_px(const float (&f)[kPx][DIM],
   }
 }
 
+// Sums of N (4, 8 or 16) per-lane values over the warp, each in the butterfly
+// order of warp_sum (so the same bits): at each level a lane keeps half of its
+// values and sends the others, which takes N - 1 shuffles and a few instead of
+// 5 N.  Lane l returns the sum of value l / (32 / N).
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i >= h) continue;
+      const float send = upper ? v[i] : v[i + h];
+      const float keep = upper ? v[i + h] : v[i];
+      v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, o));
+    }
+  }
+#pragma unroll
+  for (int q = 32 / N / 2; q >= 1; q >>= 1)
+    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], q));
+  return v[0];
+}
+
 // Warp-collective: add the per-lane sums `acc` (label l, warp-uniform) to the
 // warp's shared slot.
 template <int DIM>
 __device__ __forceinline__ void flush_acc(Smem& sm, int warp, int l, const float (&acc)[DIM],
                                           int n) {
+  constexpr int N = DIM == 3 ? 4 : 8;
   const int lane = threadIdx.x & 31;
+  float v[N];
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    const float s = warp_sum(acc[d]);
-    if (lane == 0) sm.acc[warp][l * kMaxDim + d] = __fadd_rn(sm.acc[warp][l * kMaxDim + d], s);
+  for (int d = 0; d < N; ++d) v[d] = d < DIM ? acc[d < DIM ? d : 0] : 0.0f;
+  v[DIM] = (float)n;
+  const float s = warp_sums<N>(v);
+  const int d = lane / (32 / N);
+  __syncwarp();   // the slots may have been written by other lanes
+  if (lane % (32 / N) == 0) {
+    if (d < DIM)
+      sm.acc[warp][l * kMaxDim + d] = __fadd_rn(sm.acc[warp][l * kMaxDim + d], s);
+    else if (d == DIM)
+      sm.cnt[warp][l] += (int)s;
   }
-  const int c = __reduce_add_sync(0xffffffffu, n);
-  if (lane == 0) sm.cnt[warp][l] += c;
+}
+
+// A span's FP32 sum into the block's integer sums.
+__device__ __forceinline__ void sum_to_fix(Smem& sm, int idx, float v, int* status) {
+  if (!(fabsf(v) < kFixLimit)) set_status(status, SPLIT_ERR_OVERFLOW);
+  fix_add(sm, idx, __float2ll_rn(__fmul_rn(v, kFixScale)));
 }
 
 // The end of a span: the warp's FP32 sums (its slots, one per label it met)
@@ -442,7 +479,7 @@ __device__ __forceinline__ void flush_acc(Smem& sm, int warp, int l, const float
 // depend on which block or pass took the span, nor in what order.
 template <int DIM>
 __device__ __forceinline__ void warp_to_fix(Smem& sm, int warp, int K, int* status) {
-  __syncwarp();   // lane 0's slot updates are visible to the warp
+  __syncwarp();   // the lanes' slot updates are visible to the warp
   for (int k = threadIdx.x & 31; k < K; k += 32) {
     const int c = sm.cnt[warp][k];
     if (c == 0) continue;
@@ -453,61 +490,131 @@ __device__ __forceinline__ void warp_to_fix(Smem& sm, int warp, int K, int* stat
       const float v = sm.acc[warp][k * kMaxDim + d];
       if (v == 0.0f) continue;
       sm.acc[warp][k * kMaxDim + d] = 0.0f;
-      if (!(fabsf(v) < kFixLimit)) set_status(status, SPLIT_ERR_OVERFLOW);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&sm.fix[k * kMaxDim + d]),
-                (unsigned long long)__float2ll_rn(__fmul_rn(v, kFixScale)));
+      sum_to_fix(sm, k * kMaxDim + d, v, status);
     }
   }
   __syncwarp();
 }
 
-// Accumulate one batch whose kPx labels are all valid: the same sums, in the
-// same order, as the general path below.
+// The sums of a span whose pixels all carry one of two labels, straight into
+// the block's integer sums: what flush_acc into empty slots and warp_to_fix
+// would give.
 template <int DIM>
-__device__ __forceinline__ void accumulate_valid(Smem& sm, int warp, const float (&f)[kPx][DIM],
-                                                 const int (&lab)[kPx], int& acc_l, int& acc_n,
-                                                 float (&acc)[DIM]) {
+__device__ __forceinline__ void pair_to_fix(Smem& sm, int ka, int kb, const float (&acc)[DIM],
+                                            int n, const float (&acc2)[DIM], int n2,
+                                            int* status) {
+  constexpr int NV = DIM + 1;
+  constexpr int N = 2 * NV <= 8 ? 8 : 16;
+  const int lane = threadIdx.x & 31;
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    v[d] = acc[d];
+    v[NV + d] = acc2[d];
+  }
+  v[DIM] = (float)n;
+  v[NV + DIM] = (float)n2;
+  const float s = warp_sums<N>(v);
+  const int i = lane / (32 / N);
+  if (lane % (32 / N) != 0 || i >= 2 * NV || s == 0.0f) return;
+  const int k = i < NV ? ka : kb, d = i < NV ? i : i - NV;
+  if (d < DIM)
+    sum_to_fix(sm, k * kMaxDim + d, s, status);
+  else
+    atomicAdd(&sm.fixn[k], (int)s);
+}
+
+// Accumulate one batch of x - c_label; labels below 0 mark pixels outside the
+// image.  A batch of one label adds to the lanes' running sums; otherwise the
+// batch's labels, in groups, are summed over the warp into their slots.
+template <int DIM>
+__device__ __forceinline__ void accumulate(Smem& sm, int warp, int K, const float (&f)[kPx][DIM],
+                                           const int (&lab)[kPx], int& acc_l, int& acc_n,
+                                           float (&acc)[DIM]) {
   const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   constexpr int CS = cstride(DIM);
-  int mn = min(min(lab[0], lab[1]), min(lab[2], lab[3]));
-  int mx = max(max(lab[0], lab[1]), max(lab[2], lab[3]));
-  mn = __reduce_min_sync(full, mn);
-  mx = __reduce_max_sync(full, mx);
-  if (mn == mx) {
-    if (mn != acc_l) {
+  // the labels of the batch
+  unsigned m0 = 0, m1 = 0;
+#pragma unroll
+  for (int j = 0; j < kPx; ++j) {
+    const unsigned bit = 1u << (lab[j] & 31);
+    if (lab[j] >= 0 && lab[j] < 32) m0 |= bit;
+    if (lab[j] >= 32) m1 |= bit;
+  }
+  m0 = __reduce_or_sync(full, m0);
+  if (K > 32) m1 = __reduce_or_sync(full, m1);
+  const int nlab = __popc(m0) + __popc(m1);
+  if (nlab == 0) return;
+  if (nlab == 1) {
+    const int l = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+    if (l != acc_l) {
       if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
-      acc_l = mn;
+      acc_l = l;
       acc_n = 0;
 #pragma unroll
       for (int d = 0; d < DIM; ++d) acc[d] = 0.0f;
     }
     float c[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) c[d] = sm.cent[mn * CS + d];
+    for (int d = 0; d < DIM; ++d) c[d] = sm.cent[l * CS + d];
 #pragma unroll
-    for (int j = 0; j < kPx; ++j) add_centered<DIM>(f[j], c, acc);
-    acc_n += kPx;
+    for (int j = 0; j < kPx; ++j) {
+      if (lab[j] >= 0) {
+        add_centered<DIM>(f[j], c, acc);
+        ++acc_n;
+      }
+    }
     return;
   }
   if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
   acc_l = -1;
-  for (int l = mn; l != INT_MAX;) {
-    float sum[DIM];
-    int c = 0;
+  // each pixel's x - c_label
+  float t[kPx][DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) sum[d] = 0.0f;
-    int nxt = INT_MAX;
+  for (int j = 0; j < kPx; ++j) {
+    const float* c = sm.cent + max(lab[j], 0) * CS;
 #pragma unroll
-    for (int j = 0; j < kPx; ++j) {
-      if (lab[j] == l) {
-        add_centered<DIM>(f[j], sm.cent + l * CS, sum);
-        ++c;
-      } else if (lab[j] > l) {
-        nxt = min(nxt, lab[j]);
+    for (int d = 0; d < DIM; ++d) t[j][d] = __fsub_rn(f[j][d], c[d]);
+  }
+  constexpr int NV = DIM + 1;    // the sums and the count of a label
+  constexpr int G = 16 / NV;     // labels of a group
+  const int i = lane >> 1, g = i / NV, d = i - g * NV;   // what this lane receives
+  while (m0 | m1) {
+    float v[16];
+    int mine = -1;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      int l = -2;
+      if (m0) {
+        l = __ffs(m0) - 1;
+        m0 &= m0 - 1;
+      } else if (m1) {
+        l = 31 + __ffs(m1);
+        m1 &= m1 - 1;
+      }
+      if (g == q) mine = l;
+#pragma unroll
+      for (int j = 0; j < kPx; ++j) {
+        if (lab[j] == l) {
+#pragma unroll
+          for (int dd = 0; dd < DIM; ++dd) v[q * NV + dd] = __fadd_rn(v[q * NV + dd], t[j][dd]);
+          v[q * NV + DIM] += 1.0f;
+        }
       }
     }
-    flush_acc<DIM>(sm, warp, l, sum, c);
-    l = __reduce_min_sync(full, nxt);
+    const float s = warp_sums<16>(v);
+    __syncwarp();   // the slots may have been written by other lanes
+    if ((lane & 1) == 0 && g < G && mine >= 0) {
+      if (d < DIM)
+        sm.acc[warp][mine * kMaxDim + d] = __fadd_rn(sm.acc[warp][mine * kMaxDim + d], s);
+      else
+        sm.cnt[warp][mine] += (int)s;
+    }
   }
 }
 
@@ -523,47 +630,54 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// Staging of the float4 fast path: per warp two batches of kPx x 32 float4,
-// pixel j of lane l at [j][l] (conflict-free copies and reads).
-constexpr int kStageFloat4 = kWarps * 2 * 4 * 32;   // float4 elements per block
+// Staging of the float4 fast path: per warp kStages batches of kPx x 32
+// float4, pixel j of lane l at [j][l] (conflict-free copies and reads).  Four
+// hold a whole span of a 64-row unit: its loads are all under way at once.
+constexpr int kStages = 4;
+constexpr int kStageFloat4 = kWarps * kStages * 4 * 32;   // float4 elements per block
 constexpr size_t kStageBytes = (size_t)kStageFloat4 * 16;
 
-// Labels of the lane's pixels when the candidates are exactly ka < kb: the
+// The lane's pixels when the candidates are exactly ka < kb: labels by the
 // same distances, in the same order and with the same comparisons, as
-// nearest_px over a two-bit mask.
+// nearest_px over a two-bit mask, and each pixel's differences (those of its
+// distance) added to the sums of its label, in pixel order.
 template <int DIM>
-__device__ __forceinline__ void nearest_pair(const float (&f)[kPx][DIM],
-                                             const float* __restrict__ cs, int ka, int kb,
-                                             int (&lab)[kPx]) {
+__device__ __forceinline__ void pair_px(const float (&f)[kPx][DIM], const float* __restrict__ cs,
+                                        int ka, int kb, int (&lab)[kPx], float (&acc)[DIM],
+                                        int& acc_n, float (&acc2)[DIM], int& acc2_n) {
   constexpr int CS = cstride(DIM);
-  float best[kPx];
+  float ca[DIM], cb[DIM];
 #pragma unroll
-  for (int j = 0; j < kPx; ++j) {
-    best[j] = INFINITY;
-    lab[j] = 0;
+  for (int d = 0; d < DIM; ++d) {
+    ca[d] = cs[ka * CS + d];
+    cb[d] = cs[kb * CS + d];
   }
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int k = h ? kb : ka;
-    const float4 c0 = *reinterpret_cast<const float4*>(cs + k * CS);
-    const float cc[5] = {c0.x, c0.y, c0.z, c0.w, DIM == 5 ? cs[k * CS + 4] : 0.0f};
+  for (int q = 0; q < kPx / 2; ++q) {
+    float2 ta[DIM], tb[DIM], da, db;
 #pragma unroll
-    for (int q = 0; q < kPx / 2; ++q) {
-      const int a = 2 * q, b = 2 * q + 1;
-      float2 t = fsub2(make_float2(f[a][0], f[b][0]), make_float2(cc[0], cc[0]));
-      float2 d = fmul2(t, t);
+    for (int d = 0; d < DIM; ++d) {
+      const float2 x = make_float2(f[2 * q][d], f[2 * q + 1][d]);
+      ta[d] = fsub2(x, make_float2(ca[d], ca[d]));
+      tb[d] = fsub2(x, make_float2(cb[d], cb[d]));
+      da = d == 0 ? fmul2(ta[0], ta[0]) : ffma2(ta[d], ta[d], da);
+      db = d == 0 ? fmul2(tb[0], tb[0]) : ffma2(tb[d], tb[d], db);
+    }
 #pragma unroll
-      for (int dd = 1; dd < DIM; ++dd) {
-        t = fsub2(make_float2(f[a][dd], f[b][dd]), make_float2(cc[dd], cc[dd]));
-        d = ffma2(t, t, d);
-      }
-      if (d.x < best[a]) {
-        best[a] = d.x;
-        lab[a] = k;
-      }
-      if (d.y < best[b]) {
-        best[b] = d.y;
-        lab[b] = k;
+    for (int h = 0; h < 2; ++h) {
+      const float xa = h ? da.y : da.x, xb = h ? db.y : db.x;
+      const bool finite = xa < INFINITY;
+      const bool second = xb < (finite ? xa : INFINITY);
+      const int l = second ? kb : finite ? ka : 0;
+      lab[2 * q + h] = l;
+      if (l == ka) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) acc[d] = __fadd_rn(acc[d], h ? ta[d].y : ta[d].x);
+        ++acc_n;
+      } else {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) acc2[d] = __fadd_rn(acc2[d], h ? tb[d].y : tb[d].x);
+        ++acc2_n;
       }
     }
   }
@@ -594,8 +708,7 @@ template <int DIM>
 __device__ __forceinline__ void add_span_sums(Smem& sm, int k, long long s_lane, int n) {
   const int lane = threadIdx.x & 31;
   if (lane < DIM) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&sm.fix[k * kMaxDim + lane]),
-              (unsigned long long)(s_lane - sm.nc[k * kMaxDim + lane]));
+    fix_add(sm, k * kMaxDim + lane, s_lane - sm.nc[k * kMaxDim + lane]);
   } else if (lane == DIM) {
     atomicAdd(&sm.fixn[k], n);
   }
@@ -653,7 +766,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
                                              int col, int nbatches, unsigned long long mask,
                                              int ka, int kb, bool write_labels, bool vec_labels,
                                              int& acc_l, int& acc_n, float (&acc)[DIM],
-                                             long long* entry) {
+                                             long long* entry, int* status) {
   constexpr int CS = cstride(DIM);
   constexpr bool kFixSingle = KIND == kSpanSingle && MODE == kCluster;
   // the first iteration also keeps the words of spans with several candidates
@@ -676,7 +789,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
   // both are free of bank conflicts.
   extern __shared__ float4 km_stage[];
   const int ln = threadIdx.x & 31;
-  float4* stage = km_stage + warp * (2 * kPx * 32);
+  float4* stage = km_stage + warp * (kStages * kPx * 32);
   const int64_t gw = (int64_t)im.width;
   // batch pixel q = 64 r + c of the batch's first row (row_first - lrow)
   const float4* gb0 = static_cast<const float4*>(im.points) + (px0 - (int64_t)(ln / kLanesPerRow) * gw
@@ -685,34 +798,30 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
   // copies (q = ln + 32 j) and reads (q = 4 ln + j)
   const int cs0 = (ln & ~7) + ((ln + (ln >> 3)) & 7), cs1 = cs0 ^ 4;
   const int rs0 = 8 * (ln >> 1), rt = (4 * ln + (ln >> 1)) & 7;
-  const float4* grow1 = gb0 + gw;
-  if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
-    cp_async16(stage + cs0, gb0 + ln);
-    cp_async16(stage + 32 + cs1, gb0 + ln + 32);
-    cp_async16(stage + 64 + cs0, grow1 + ln);
-    cp_async16(stage + 96 + cs1, grow1 + ln + 32);
+  // batch b into buffer b % kStages (an empty group past the end, so that
+  // the groups in flight count batches)
+  auto fetch = [&](int b) {
+    if (b < nbatches) {
+      const float4* g = gb0 + (int64_t)b * step + ln;
+      float4* dst = stage + (b % kStages) * (kPx * 32);
+      cp_async16(dst + cs0, g);
+      cp_async16(dst + 32 + cs1, g + 32);
+      cp_async16(dst + 64 + cs0, g + gw);
+      cp_async16(dst + 96 + cs1, g + gw + 32);
+    }
     cp_async_commit();
+  };
+  if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
+#pragma unroll
+    for (int b = 0; b < kStages; ++b) fetch(b);
   }
   for (int b = 0; b < nbatches; ++b, px0 += step) {
     float f[kPx][DIM];
     if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
-      // every lane has read the buffer about to be refilled (batch b - 1)
-      __syncwarp();
-      if (b + 1 < nbatches) {
-        const float4* g = gb0 + (int64_t)(b + 1) * step + ln;
-        float4* dst = stage + ((b + 1) & 1) * (kPx * 32);
-        cp_async16(dst + cs0, g);
-        cp_async16(dst + 32 + cs1, g + 32);
-        cp_async16(dst + 64 + cs0, g + gw);
-        cp_async16(dst + 96 + cs1, g + gw + 32);
-        cp_async_commit();
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
+      cp_async_wait<kStages - 1>();
       // the copies of the other lanes must have landed too
       __syncwarp();
-      const float4* src = stage + (b & 1) * (kPx * 32);
+      const float4* src = stage + (b % kStages) * (kPx * 32);
 #pragma unroll
       for (int j = 0; j < kPx; ++j) {
         const float4 v = src[rs0 + ((rt + j) & 7)];
@@ -720,6 +829,8 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
         f[j][1] = v.y;
         f[j][2] = v.z;
       }
+      __syncwarp();   // every lane has read the buffer that is refilled now
+      fetch(b + kStages);
     } else {
       const uint32_t* p =
           reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(im.points) + 3 * px0);
@@ -752,7 +863,8 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
 #pragma unroll
       for (int j = 0; j < kPx; ++j) lab[j] = ka;
     } else if (KIND == kSpanPair) {
-      nearest_pair<DIM>(f, sm.cent, ka, kb, lab);
+      // the distances, and the sums from the same differences
+      pair_px<DIM>(f, sm.cent, ka, kb, lab, acc, acc_n, acc2, acc2_n);
     } else {
       nearest_px<DIM>(f, sm.cent, mask, lab);
     }
@@ -773,26 +885,13 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
           for (int j = 0; j < kPx; ++j) add_centered<DIM>(f[j], c, acc);
           acc_n += kPx;
         }
-      } else if (KIND == kSpanPair) {
-        const float* ca = sm.cent + ka * CS;
-        const float* cb = sm.cent + kb * CS;
-#pragma unroll
-        for (int j = 0; j < kPx; ++j) {
-          if (lab[j] == ka) {
-            add_centered<DIM>(f[j], ca, acc);
-            ++acc_n;
-          } else {
-            add_centered<DIM>(f[j], cb, acc2);
-            ++acc2_n;
-          }
-        }
-      } else {
-        accumulate_valid<DIM>(sm, warp, f, lab, acc_l, acc_n, acc);
+      } else if (KIND == kSpanAny) {
+        accumulate<DIM>(sm, warp, im.K, f, lab, acc_l, acc_n, acc);
       }
     }
   }
-  // the second candidate's sums (the first's stay running)
-  if (MODE != kAssignOnly && KIND == kSpanPair) flush_acc<DIM>(sm, warp, kb, acc2, acc2_n);
+  if (MODE != kAssignOnly && KIND == kSpanPair)
+    pair_to_fix<DIM>(sm, ka, kb, acc, acc_n, acc2, acc2_n, status);
   if (kFixSingle || keep) {
     const long long w = span_words<DIM>(qc, fx, im.xy_scale, row_first, nbatches);
     if (entry && (threadIdx.x & 31) < DIM) __stcg(entry + (threadIdx.x & 31), w);
@@ -817,7 +916,7 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
                                           int col, int nbatches, unsigned long long mask,
                                           bool write_labels, bool vec_labels, int& acc_l,
                                           int& acc_n, float (&acc)[DIM], long long* entry,
-                                          int it) {
+                                          int it, int* status) {
   constexpr int CS = cstride(DIM);
   // A mask with one cluster names every pixel's nearest centroid outright:
   // the span's box excludes all others for every pixel it holds (and the
@@ -844,27 +943,18 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
     if (write_labels) write_span_labels(im, row_first, col, nbatches, ka, vec_labels);
     return;
   }
-  // with one running label for the whole span the sums switch to it once
-  // (a clustering sums its single spans exactly instead)
-  if (MODE != kAssignOnly && ka >= 0 && ka != acc_l && !(MODE == kCluster && kind == kSpanSingle)) {
-    if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
-    acc_l = ka;
-    acc_n = 0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) acc[d] = 0.0f;
-  }
   if (kind == kSpanSingle)
     span_batches<LAYOUT, DIM, MODE, kSpanSingle>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                                  kb, write_labels, vec_labels, acc_l, acc_n, acc,
-                                                 entry);
+                                                 entry, status);
   else if (kind == kSpanPair)
     span_batches<LAYOUT, DIM, MODE, kSpanPair>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                                kb, write_labels, vec_labels, acc_l, acc_n, acc,
-                                               it == 0 ? entry : nullptr);
+                                               it == 0 ? entry : nullptr, status);
   else
     span_batches<LAYOUT, DIM, MODE, kSpanAny>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                               kb, write_labels, vec_labels, acc_l, acc_n, acc,
-                                              it == 0 ? entry : nullptr);
+                                              it == 0 ? entry : nullptr, status);
 }
 
 // Whether a warp span takes the fast path: xy features with colour known to
@@ -960,7 +1050,7 @@ __device__ bool process_span(const Image& im, int srow, int tx, Smem& sm, bool w
   if (fast)
     fast_span<LAYOUT, DIM, MODE>(im, sm, warp, row0 + lrow, col0 + lcol, wrows / kBatchRows,
                                  span_mask, write_labels, vec_labels, acc_l, acc_n, acc, entry,
-                                 it);
+                                 it, status);
   for (int b = 0; !fast && b < wrows / kBatchRows; ++b) {
     if (b * kBatchRows >= rows_in) break;
     const int row = row0 + b * kBatchRows + lrow;
@@ -1036,58 +1126,7 @@ __device__ bool process_span(const Image& im, int srow, int tx, Smem& sm, bool w
     }
     if (MODE == kAssignOnly) continue;
 
-    // ---- accumulate x - c_label
-    int mn = INT_MAX, mx = -1;
-#pragma unroll
-    for (int j = 0; j < kPx; ++j) {
-      if (lab[j] >= 0) {
-        mn = min(mn, lab[j]);
-        mx = max(mx, lab[j]);
-      }
-    }
-    mn = __reduce_min_sync(full, mn);
-    mx = __reduce_max_sync(full, mx);
-    if (mx < 0) continue;
-    if (mn == mx) {
-      if (mn != acc_l) {
-        if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
-        acc_l = mn;
-        acc_n = 0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) acc[d] = 0.0f;
-      }
-      float c[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) c[d] = sm.cent[mn * CS + d];
-#pragma unroll
-      for (int j = 0; j < kPx; ++j) {
-        if (lab[j] >= 0) {
-          add_centered<DIM>(f[j], c, acc);
-          ++acc_n;
-        }
-      }
-    } else {
-      if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
-      acc_l = -1;
-      for (int l = mn; l != INT_MAX;) {
-        float s[DIM];
-        int c = 0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) s[d] = 0.0f;
-        int nxt = INT_MAX;
-#pragma unroll
-        for (int j = 0; j < kPx; ++j) {
-          if (lab[j] == l) {
-            add_centered<DIM>(f[j], sm.cent + l * CS, s);
-            ++c;
-          } else if (lab[j] > l) {
-            nxt = min(nxt, lab[j]);
-          }
-        }
-        flush_acc<DIM>(sm, warp, l, s, c);
-        l = __reduce_min_sync(full, nxt);
-      }
-    }
+    accumulate<DIM>(sm, warp, im.K, f, lab, acc_l, acc_n, acc);
   }
   if (MODE != kAssignOnly) {
     if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
@@ -1108,9 +1147,11 @@ __device__ void block_to_accum(Smem& sm, const Params& p, int img, int K, int di
   unsigned long long* lo = p.acc_lo + acc_slot(p, slot, img) * (kMaxK * kMaxDim);
   unsigned long long* hi = p.acc_hi + acc_slot(p, slot, img) * (kMaxK * kMaxDim);
   for (int idx = threadIdx.x; idx < K * kMaxDim; idx += blockDim.x) {
-    const long long q = sm.fix[idx];
-    if (q == 0) continue;
-    sm.fix[idx] = 0;
+    const unsigned wlo = sm.fix_lo[idx], whi = sm.fix_hi[idx];
+    if ((wlo | whi) == 0u) continue;
+    const long long q = (long long)(((unsigned long long)whi << 32) | wlo);
+    sm.fix_lo[idx] = 0u;
+    sm.fix_hi[idx] = 0u;
     if ((idx % kMaxDim) < dim) {
       atomicAdd(lo + idx, (unsigned long long)q & 0xffffffffull);
       atomicAdd(hi + idx, (unsigned long long)(q >> 32));
@@ -1400,8 +1441,7 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
     const int k = __shfl_sync(full, k_lane, gs < kGroup ? gs : 0);
     if (gs < kGroup && e >= 0) {
       const long long w = __ldcg(im.span_sum + (size_t)e * kSpanSums + d);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&sm.fix[k * kMaxDim + d]),
-                (unsigned long long)(w - sm.nc[k * kMaxDim + d]));
+      fix_add(sm, k * kMaxDim + d, w - sm.nc[k * kMaxDim + d]);
     }
     if (lane < kGroup && e_lane >= 0) atomicAdd(&sm.fixn[k_lane], wrows * kTile);
   }
@@ -1426,7 +1466,7 @@ __device__ __forceinline__ void clear_sums(Smem& sm) {
   for (int i = threadIdx.x; i < kWarps * kMaxK * kMaxDim; i += blockDim.x)
     (&sm.acc[0][0])[i] = 0.0f;
   for (int i = threadIdx.x; i < kWarps * kMaxK; i += blockDim.x) (&sm.cnt[0][0])[i] = 0;
-  for (int i = threadIdx.x; i < kMaxK * kMaxDim; i += blockDim.x) sm.fix[i] = 0;
+  for (int i = threadIdx.x; i < kMaxK * kMaxDim; i += blockDim.x) sm.fix_lo[i] = sm.fix_hi[i] = 0u;
   for (int i = threadIdx.x; i < kMaxK; i += blockDim.x) sm.fixn[i] = 0;
   if (threadIdx.x == 0) {
     sm.nheavy = 0;
@@ -1752,13 +1792,8 @@ static int stage_attributes() {
   std::lock_guard<std::mutex> lock(mu);
   if (done[dev]) return SPLIT_OK;
   const void* kerns[] = {
-      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 3, kCluster>,
       (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kCluster>,
-      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 3, kUpdateOnly>,
-      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kUpdateOnly>,
-      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 3, kAssignOnly>,
       (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kAssignOnly>,
-      (const void*)kmeans_batch_kernel<SPLIT_LAYOUT_FLOAT4, 3>,
       (const void*)kmeans_batch_kernel<SPLIT_LAYOUT_FLOAT4, 5>};
   for (const void* k : kerns)
     SG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1774,7 +1809,9 @@ static int launch(Params& p, cudaStream_t st) {
   auto kern = kmeans_kernel<LAYOUT, DIM, MODE>;
   if constexpr (MODE == kCluster)
     if (p.images) kern = kmeans_batch_kernel<LAYOUT, DIM>;
-  const size_t dyn = LAYOUT == SPLIT_LAYOUT_FLOAT4 ? kStageBytes : 0;
+  // (3-D features never take the fast path)
+  const size_t dyn =
+      LAYOUT == SPLIT_LAYOUT_FLOAT4 && DIM == 5 && MODE != kUpdateOnly ? kStageBytes : 0;
   if (dyn) SG_TRY(stage_attributes());
   int per_sm = 0;
   SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, dyn));
