@@ -47,12 +47,10 @@
 namespace sg {
 namespace km {
 
-// Resident blocks per SM the register budget is set for.  Single images: 2
-// (up to 128 registers a thread) keeps the span passes free of spills; at 3
-// (80 registers) they spill, and small images, whose iterations are
-// latency-bound, lose more than the extra occupancy gives.  Batches (many
-// small images through the unit loop): 3, where the extra resident blocks
-// hide more latency than the spills cost.
+// Resident blocks per SM the register budget is set for: 2 (up to 128
+// registers a thread) keeps the span passes free of spills; at 3 (80
+// registers) they spill (512 x 512 alone: 0.323 against 0.287 ms in the unit
+// loop; the 48-image batch 3.67 against 3.58 ms in the span loop).
 #ifndef SG_KM_MINBLOCKS
 #define SG_KM_MINBLOCKS 2
 #endif
@@ -67,7 +65,7 @@ constexpr int kTile = 64;
 constexpr int kMaxK = 64;
 constexpr int kMaxDim = 5;
 constexpr int kSpanSums = 8;   // words of a span's entry in Image::span_sum (kMaxDim used)
-constexpr int kHeavyCap = 256; // deferred spans a block lists per iteration
+constexpr int kHeavyCap = 512; // deferred spans a block lists per iteration
 // Span sums are added into the image accumulators as multiples of 2^-24; a
 // span's FP32 sum must stay below 2^38 in magnitude (a span holds at most
 // 1024 pixels, so |x - c| below 2.6e8 everywhere).  Beyond it the call
@@ -281,6 +279,9 @@ struct Smem {
   // words, because shared memory adds 32 bits in one operation
   unsigned fix_lo[kMaxK * kMaxDim], fix_hi[kMaxK * kMaxDim];
   int fixn[kMaxK];
+  // classification of spans with xy features: the colour part of a centroid's
+  // bounds over the unit cube (lower, upper) and its xy
+  float4 bound[kMaxK];
   // n * c * 2^24 of every centroid value, n the pixels of a whole span
   long long nc[kMaxK * kMaxDim];
   // spans deferred to the second pass of an iteration (see span_pass)
@@ -1170,6 +1171,21 @@ __device__ __forceinline__ long long span_centre(const Image& im, float c) {
   return __float2ll_rn(__fmul_rn(c, (float)(im.unit_rows / kWarps * kTile) * kFixScale));
 }
 
+// Entry of Smem::bound for centroid k at c: the first three steps of the
+// fma chains of candidates() over lo = 0, hi = 1.
+template <int DIM>
+__device__ __forceinline__ float4 colour_bound(const float* c) {
+  float l = 0.0f, u = 0.0f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float g = fmaxf(fmaxf(0.0f - c[d], c[d] - 1.0f), 0.0f);
+    const float e = fmaxf(c[d] - 0.0f, 1.0f - c[d]);
+    l = __fmaf_rn(g, g, l);
+    u = __fmaf_rn(e, e, u);
+  }
+  return make_float4(l, u, c[DIM == 5 ? 3 : 0], c[DIM == 5 ? 4 : 0]);
+}
+
 // The centroids of slot `src` into shared memory (strides cstride(DIM) there,
 // 8 in the slot).
 template <int DIM>
@@ -1181,6 +1197,13 @@ __device__ __forceinline__ void load_centroids(const Image& im, const float* src
     sm.cent[idx] = c;
     if (d < DIM) sm.nc[k * kMaxDim + d] = span_centre(im, c);
   }
+  if (DIM == 5)
+    for (int k = threadIdx.x; k < im.K; k += blockDim.x) {
+      float c[5];
+#pragma unroll
+      for (int d = 0; d < 5; ++d) c[d] = __ldcg(src + k * 8 + d);
+      sm.bound[k] = colour_bound<5>(c);
+    }
 }
 
 // The squared "centroid shift" as the reference's cluster() measures it
@@ -1282,6 +1305,10 @@ __device__ bool form_centroids(const Params& p, int img, const Image& im, int i,
     __syncthreads();
     return false;
   }
+  if (DIM == 5 && threadIdx.x >= kThreads - kMaxK) {
+    const int k = (int)threadIdx.x - (kThreads - kMaxK);
+    if (k < im.K) sm.bound[k] = colour_bound<5>(sm.cent + k * CS);
+  }
   if (owner && threadIdx.x >= 32) {
     const size_t zb = acc_slot(p, (i + 1) % 3, img);
     const int t = (int)threadIdx.x - 32, nt = (int)blockDim.x - 32;
@@ -1327,31 +1354,20 @@ __device__ bool form_centroids(const Params& p, int img, const Image& im, int i,
 }
 
 // The spans a block takes of an image in an iteration: place j < count is
-// span (first + j * step) mod nspans (from the other end when `back`), read by
-// each warp in the order j = warp, warp + kWarps, ...
+// span first + j * step of the image (mod nspans when SCATTER; from the other
+// end when `back`).
+template <bool SCATTER>
 struct SpanShare {
   int first, step, count;
   bool back;
   int nspans, ntx;
-};
-struct SpanWalk {
-  int s, hop, nspans, ntx;
-  bool back;
-  __device__ __forceinline__ SpanWalk(const SpanShare& h, int warp)
-      : nspans(h.nspans), ntx(h.ntx), back(h.back) {
-    s = (int)(((long long)h.first + (long long)warp * h.step) % h.nspans);
-    hop = (int)((long long)kWarps * h.step % h.nspans);
-  }
-  // the next place's span
-  __device__ __forceinline__ void next(int& srow, int& tx) {
-    const int v = back ? nspans - 1 - s : s;
+  __device__ __forceinline__ void at(int j, int& srow, int& tx) const {
+    int v = SCATTER ? (int)(((long long)first + (long long)j * step) % nspans) : first + j * step;
+    if (back) v = nspans - 1 - v;
     srow = v / ntx;
     tx = v - srow * ntx;
-    s += hop;
-    if (s >= nspans) s -= nspans;
   }
 };
-
 // One iteration of the block's share of an image's spans.  There is no block
 // barrier and no global traffic per span: warps take places j = warp, warp +
 // kWarps, ..., each span's contribution is added to the block's integer sums,
@@ -1362,19 +1378,18 @@ struct SpanWalk {
 // need none of their pixels (one candidate: labels and sums known): the warps
 // finish those at once and list the others; the block's warps then take the
 // listed spans one at a time.
-template <int LAYOUT, int DIM, int MODE, bool COUNT>
+template <int LAYOUT, int DIM, int MODE, bool BATCH>
 __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image& im, int img,
-                                          const SpanShare& share, int it) {
+                                          const SpanShare<BATCH>& share, int it) {
   constexpr unsigned full = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wrows = im.unit_rows / kWarps;
   const bool wl = MODE == kAssignOnly ||
                   (MODE == kCluster && (im.threshold >= 0.0f || it == im.max_iter - 1));
   int* status = &p.hdr->status;
-  SpanWalk walk(share, warp);
   int counted = 0;
   auto count = [&]() {
-    if (!COUNT || it > 0) return;
+    if (!BATCH || it > 0) return;
     if (lane == 0 && counted) atomicAdd(&sm.counted, counted);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1382,81 +1397,99 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
       sm.counted = 0;
     }
   };
-  if (MODE != kCluster || it == 0 || !im.span_sum) {
+  // (with at most one span per warp nothing is gained by the second form)
+  if (MODE != kCluster || it == 0 || !im.span_sum || share.count <= kWarps) {
     for (int j = warp; j < share.count; j += kWarps) {
       int sr, tx;
-      walk.next(sr, tx);
+      share.at(j, sr, tx);
       counted += process_span<LAYOUT, DIM, MODE>(im, sr, tx, sm, wl, it, status);
     }
     count();
     if (MODE != kAssignOnly) block_to_accum(sm, p, img, im.K, DIM, it % 3);
     return;
   }
+  // Light spans, a lane each: classified from the geometry alone (the bounds
+  // and the test of candidates(), one centroid after the other, so that a
+  // warp bounds 32 spans at a time), their kept words added by their lanes.
+  // With a warp per span this pass took 4.5 us of a 4K iteration.
   const int rows = wrows / kBatchRows;
   const int lrow = lane / kLanesPerRow, lcol = (lane % kLanesPerRow) * kPx;
   const bool vec_labels = (reinterpret_cast<uintptr_t>(im.labels) & 15) == 0 && (im.width % kPx) == 0;
-  // Groups of up to kGroup of the warp's spans: classify each (candidates
-  // from the geometry alone), then one round of loads brings every light
-  // span's kept words (lane g * DIM + d: span g, dimension d).
-  constexpr int kGroup = 32 / DIM < 6 ? 32 / DIM : 6;
-  // with at most one span per warp (small images) nothing is gained by
-  // deferring: a warp does its span at once
-  const bool defer = share.count > kWarps;
-  for (int j0 = warp; j0 < share.count; j0 += kGroup * kWarps) {
-    int e_lane = -1, k_lane = -1;   // lane g: light span g's kept entry and its cluster
-    for (int g = 0; g < kGroup; ++g) {
-      const int j = j0 + g * kWarps;
-      if (j >= share.count) break;
-      int sr, tx;
-      walk.next(sr, tx);
-      int k = -1;
-      if (fast_geometry<LAYOUT, DIM, MODE>(im, sr * wrows, tx * kTile, wrows, vec_labels)) {
-        const unsigned long long m =
-            unit_box_mask<DIM>(im, sm, sr * wrows, tx * kTile, wrows, kTile);
-        if (m != 0ull && (m & (m - 1ull)) == 0ull) k = __ffsll((long long)m) - 1;
+  const int per = (share.count + kWarps - 1) / kWarps;
+  const int end = min((warp + 1) * per, share.count);
+  for (int j0 = warp * per; j0 < end; j0 += 32) {
+    const int j = j0 + lane;
+    const bool mine = j < end;
+    int sr = 0, tx = 0;
+    if (mine) share.at(j, sr, tx);
+    int k = -1;   // a light span's cluster
+    if (mine && fast_geometry<LAYOUT, DIM, MODE>(im, sr * wrows, tx * kTile, wrows, vec_labels)) {
+      const float lo3 = __fmul_rn(im.xy_scale, (float)(tx * kTile));
+      const float hi3 = __fmul_rn(im.xy_scale, (float)(tx * kTile + kTile - 1));
+      const float lo4 = __fmul_rn(im.xy_scale, (float)(sr * wrows));
+      const float hi4 = __fmul_rn(im.xy_scale, (float)(sr * wrows + wrows - 1));
+      float ub = INFINITY;
+      for (int q = 0; q < im.K; ++q) {
+        const float4 c = sm.bound[q];
+        const float e3 = fmaxf(c.z - lo3, hi3 - c.z), e4 = fmaxf(c.w - lo4, hi4 - c.w);
+        ub = fminf(ub, __fmaf_rn(e4, e4, __fmaf_rn(e3, e3, c.y)));
       }
-      if (k >= 0) {
-        if (lane == g) {
-          e_lane = sr * im.span_cols + tx;
-          k_lane = k;
-        }
-        if (wl) write_span_labels(im, sr * wrows + lrow, tx * kTile + lcol, rows, k, vec_labels);
-        continue;
-      }
-      ++counted;
-      if (defer) {
-        int slot = 0;
-        if (lane == 0) slot = atomicAdd(&sm.nheavy, 1);
-        slot = __shfl_sync(full, slot, 0);
-        if (slot < kHeavyCap) {
-          if (lane == 0) sm.heavy[slot] = sr * im.ntx + tx;
-          continue;
+      const float thr = ub * 1.0001f;
+      int n = 0;
+      for (int q = 0; q < im.K; ++q) {
+        const float4 c = sm.bound[q];
+        const float g3 = fmaxf(fmaxf(lo3 - c.z, c.z - hi3), 0.0f);
+        const float g4 = fmaxf(fmaxf(lo4 - c.w, c.w - hi4), 0.0f);
+        if (__fmaf_rn(g4, g4, __fmaf_rn(g3, g3, c.x)) <= thr) {
+          ++n;
+          k = q;
         }
       }
-      // not deferred, or the list is full: this one now
-      process_span<LAYOUT, DIM, MODE>(im, sr, tx, sm, wl, it, status);
+      if (n != 1) k = -1;
     }
-    const int gs = lane / DIM, d = lane - gs * DIM;
-    const int e = __shfl_sync(full, e_lane, gs < kGroup ? gs : 0);
-    const int k = __shfl_sync(full, k_lane, gs < kGroup ? gs : 0);
-    if (gs < kGroup && e >= 0) {
-      const long long w = __ldcg(im.span_sum + (size_t)e * kSpanSums + d);
-      fix_add(sm, k * kMaxDim + d, w - sm.nc[k * kMaxDim + d]);
+    if (k >= 0) {
+      const long long* e = im.span_sum + ((size_t)sr * im.span_cols + tx) * kSpanSums;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        fix_add(sm, k * kMaxDim + d, __ldcg(e + d) - sm.nc[k * kMaxDim + d]);
+      atomicAdd(&sm.fixn[k], wrows * kTile);
     }
-    if (lane < kGroup && e_lane >= 0) atomicAdd(&sm.fixn[k_lane], wrows * kTile);
+    if (wl) {
+      for (unsigned m = __ballot_sync(full, k >= 0); m; m &= m - 1) {
+        const int g = __ffs(m) - 1;
+        write_span_labels(im, __shfl_sync(full, sr, g) * wrows + lrow,
+                          __shfl_sync(full, tx, g) * kTile + lcol, rows, __shfl_sync(full, k, g),
+                          vec_labels);
+      }
+    }
+    unsigned heavy = __ballot_sync(full, mine && k < 0);
+    counted += __popc(heavy);
+    if (heavy) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&sm.nheavy, __popc(heavy));
+      base = __shfl_sync(full, base, 0);
+      const int slot = base + __popc(heavy & ((1u << lane) - 1u));
+      const bool listed = ((heavy >> lane) & 1u) && slot < kHeavyCap;
+      if (listed) sm.heavy[slot] = sr * im.ntx + tx;
+      heavy &= ~__ballot_sync(full, listed);
+    }
+    // the list is full: these now
+    for (; heavy; heavy &= heavy - 1) {
+      const int g = __ffs(heavy) - 1;
+      process_span<LAYOUT, DIM, MODE>(im, __shfl_sync(full, sr, g), __shfl_sync(full, tx, g), sm,
+                                      wl, it, status);
+    }
   }
-  if (defer) {
-    __syncthreads();
-    const int nh = min(sm.nheavy, kHeavyCap);
-    for (;;) {
-      int idx = 0;
-      if (lane == 0) idx = atomicAdd(&sm.next_heavy, 1);
-      idx = __shfl_sync(full, idx, 0);
-      if (idx >= nh) break;
-      const int s = sm.heavy[idx];
-      const int sr = s / im.ntx;
-      process_span<LAYOUT, DIM, MODE>(im, sr, s - sr * im.ntx, sm, wl, it, status);
-    }
+  __syncthreads();
+  const int nh = min(sm.nheavy, kHeavyCap);
+  for (;;) {
+    int idx = 0;
+    if (lane == 0) idx = atomicAdd(&sm.next_heavy, 1);
+    idx = __shfl_sync(full, idx, 0);
+    if (idx >= nh) break;
+    const int s = sm.heavy[idx];
+    const int sr = s / im.ntx;
+    process_span<LAYOUT, DIM, MODE>(im, sr, s - sr * im.ntx, sm, wl, it, status);
   }
   count();
   block_to_accum(sm, p, img, im.K, DIM, it % 3);
@@ -1487,7 +1520,7 @@ __global__ void __launch_bounds__(kThreads, SG_KM_MINBLOCKS) kmeans_kernel(Param
     for (int i = threadIdx.x; i < 256; i += blockDim.x) sm.lut[i] = (float)i / 255.0f;
   load_centroids<DIM>(im, p.cur, sm);
   __syncthreads();
-  SpanShare share;
+  SpanShare<false> share;
   share.first = (int)blockIdx.x;
   share.step = (int)gridDim.x;
   share.count = (im.nspans - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -1634,7 +1667,7 @@ __global__ void __launch_bounds__(kThreads, kBatchMinBlocks) kmeans_batch_kernel
           __syncthreads();
         }
         if (!more) continue;
-        SpanShare share;
+        SpanShare<true> share;
         share.first = (int)((long long)rl.begin[k] * im.scatter % im.nspans);
         share.step = im.scatter;
         share.count = rl.end[k] - rl.begin[k];
