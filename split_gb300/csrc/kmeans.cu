@@ -762,7 +762,7 @@ enum SpanKind { kSpanSingle = 0, kSpanPair = 1, kSpanAny = 2 };
 // words instead of running FP32 sums, and keeps them in `entry` (if any);
 // any other span given an `entry` (the first iteration's) also sums and keeps
 // its words, besides its FP32 sums.
-template <int LAYOUT, int DIM, int MODE, int KIND>
+template <int LAYOUT, int DIM, int MODE, int KIND, bool FIRST>
 __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp, int row_first,
                                              int col, int nbatches, unsigned long long mask,
                                              int ka, int kb, bool write_labels, bool vec_labels,
@@ -771,7 +771,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
   constexpr int CS = cstride(DIM);
   constexpr bool kFixSingle = KIND == kSpanSingle && MODE == kCluster;
   // the first iteration also keeps the words of spans with several candidates
-  const bool keep = MODE == kCluster && KIND != kSpanSingle && entry != nullptr;
+  const bool keep = MODE == kCluster && FIRST && KIND != kSpanSingle && entry != nullptr;
   long long qc[3] = {0, 0, 0};
   const int64_t step = (int64_t)kBatchRows * im.width;
   int64_t px0 = (int64_t)row_first * im.width + col;
@@ -895,7 +895,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
     pair_to_fix<DIM>(sm, ka, kb, acc, acc_n, acc2, acc2_n, status);
   if (kFixSingle || keep) {
     const long long w = span_words<DIM>(qc, fx, im.xy_scale, row_first, nbatches);
-    if (entry && (threadIdx.x & 31) < DIM) __stcg(entry + (threadIdx.x & 31), w);
+    if (FIRST && entry && (threadIdx.x & 31) < DIM) __stcg(entry + (threadIdx.x & 31), w);
     if (kFixSingle) add_span_sums<DIM>(sm, ka, w, 32 * kPx * nbatches);
   }
 }
@@ -912,12 +912,12 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
 // with one candidate reads it back instead of its pixels: its labels are
 // that candidate's (written when asked) and its sums are exact integers, so
 // nothing else needs the pixels.
-template <int LAYOUT, int DIM, int MODE>
+template <int LAYOUT, int DIM, int MODE, bool FIRST>
 __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, int row_first,
                                           int col, int nbatches, unsigned long long mask,
                                           bool write_labels, bool vec_labels, int& acc_l,
                                           int& acc_n, float (&acc)[DIM], long long* entry,
-                                          int it, int* status) {
+                                          int* status) {
   constexpr int CS = cstride(DIM);
   // A mask with one cluster names every pixel's nearest centroid outright:
   // the span's box excludes all others for every pixel it holds (and the
@@ -938,24 +938,24 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
       kb = b;
     }
   }
-  if (MODE == kCluster && kind == kSpanSingle && entry && it > 0) {
+  if (MODE == kCluster && !FIRST && kind == kSpanSingle && entry) {
     const int lane = threadIdx.x & 31;
     add_span_sums<DIM>(sm, ka, lane < DIM ? __ldcg(entry + lane) : 0ll, 32 * kPx * nbatches);
     if (write_labels) write_span_labels(im, row_first, col, nbatches, ka, vec_labels);
     return;
   }
   if (kind == kSpanSingle)
-    span_batches<LAYOUT, DIM, MODE, kSpanSingle>(im, sm, warp, row_first, col, nbatches, mask, ka,
+    span_batches<LAYOUT, DIM, MODE, kSpanSingle, FIRST>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                                  kb, write_labels, vec_labels, acc_l, acc_n, acc,
                                                  entry, status);
   else if (kind == kSpanPair)
-    span_batches<LAYOUT, DIM, MODE, kSpanPair>(im, sm, warp, row_first, col, nbatches, mask, ka,
+    span_batches<LAYOUT, DIM, MODE, kSpanPair, FIRST>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                                kb, write_labels, vec_labels, acc_l, acc_n, acc,
-                                               it == 0 ? entry : nullptr, status);
+                                               entry, status);
   else
-    span_batches<LAYOUT, DIM, MODE, kSpanAny>(im, sm, warp, row_first, col, nbatches, mask, ka,
+    span_batches<LAYOUT, DIM, MODE, kSpanAny, FIRST>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                               kb, write_labels, vec_labels, acc_l, acc_n, acc,
-                                              it == 0 ? entry : nullptr, status);
+                                              entry, status);
 }
 
 // Whether a warp span takes the fast path: xy features with colour known to
@@ -1012,9 +1012,9 @@ __device__ __forceinline__ unsigned long long unit_box_mask(const Image& im, con
 //
 // Returns whether the span needs its pixels in later iterations too (as long
 // as its candidates stay the same).
-template <int LAYOUT, int DIM, int MODE>
-__device__ bool process_span(const Image& im, int srow, int tx, Smem& sm, bool write_labels,
-                             int it, int* status) {
+template <int LAYOUT, int DIM, int MODE, bool FIRST>
+__device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, Smem& sm,
+                                             bool write_labels, int* status) {
   const unsigned full = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int CS = cstride(DIM);
@@ -1049,9 +1049,9 @@ __device__ bool process_span(const Image& im, int srow, int tx, Smem& sm, bool w
   for (int d = 0; d < DIM; ++d) acc[d] = 0.0f;
 
   if (fast)
-    fast_span<LAYOUT, DIM, MODE>(im, sm, warp, row0 + lrow, col0 + lcol, wrows / kBatchRows,
-                                 span_mask, write_labels, vec_labels, acc_l, acc_n, acc, entry,
-                                 it, status);
+    fast_span<LAYOUT, DIM, MODE, FIRST>(im, sm, warp, row0 + lrow, col0 + lcol, wrows / kBatchRows,
+                                 span_mask, write_labels, vec_labels, acc_l, acc_n, acc,
+                                        entry, status);
   for (int b = 0; !fast && b < wrows / kBatchRows; ++b) {
     if (b * kBatchRows >= rows_in) break;
     const int row = row0 + b * kBatchRows + lrow;
@@ -1368,56 +1368,25 @@ struct SpanShare {
     tx = v - srow * ntx;
   }
 };
-// One iteration of the block's share of an image's spans.  There is no block
-// barrier and no global traffic per span: warps take places j = warp, warp +
-// kWarps, ..., each span's contribution is added to the block's integer sums,
-// and those go to the image accumulators once, at the end.  A span's
-// contribution does not depend on who takes it, so neither does the result.
-//
-// After the first iteration, where the fast spans' sums are kept, most spans
-// need none of their pixels (one candidate: labels and sums known): the warps
-// finish those at once and list the others; the block's warps then take the
-// listed spans one at a time.
+// Places [w0, w1) of the block's share after the first iteration, a lane each:
+// classified from the geometry alone (the bounds and the test of candidates(),
+// one centroid after the other, so that a warp bounds 32 spans at a time).  A
+// span with one candidate is finished: its kept words are added and, when
+// asked, its labels written.  The others are listed.  With a warp per span
+// this took 4.5 us of a 4K iteration, now 2.1.
 template <int LAYOUT, int DIM, int MODE, bool BATCH>
-__device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image& im, int img,
-                                          const SpanShare<BATCH>& share, int it) {
+__device__ __forceinline__ void list_spans(Smem& sm, const Image& im,
+                                           const SpanShare<BATCH>& share, int w0, int w1,
+                                           bool wl) {
   constexpr unsigned full = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wrows = im.unit_rows / kWarps;
-  const bool wl = MODE == kAssignOnly ||
-                  (MODE == kCluster && (im.threshold >= 0.0f || it == im.max_iter - 1));
-  int* status = &p.hdr->status;
-  int counted = 0;
-  auto count = [&]() {
-    if (!BATCH || it > 0) return;
-    if (lane == 0 && counted) atomicAdd(&sm.counted, counted);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      atomicAdd(cost_at(p, img, it), kPixelCost * sm.counted + share.count);
-      sm.counted = 0;
-    }
-  };
-  // (with at most one span per warp nothing is gained by the second form)
-  if (MODE != kCluster || it == 0 || !im.span_sum || share.count <= kWarps) {
-    for (int j = warp; j < share.count; j += kWarps) {
-      int sr, tx;
-      share.at(j, sr, tx);
-      counted += process_span<LAYOUT, DIM, MODE>(im, sr, tx, sm, wl, it, status);
-    }
-    count();
-    if (MODE != kAssignOnly) block_to_accum(sm, p, img, im.K, DIM, it % 3);
-    return;
-  }
-  // Light spans, a lane each: classified from the geometry alone (the bounds
-  // and the test of candidates(), one centroid after the other, so that a
-  // warp bounds 32 spans at a time), their kept words added by their lanes.
-  // With a warp per span this pass took 4.5 us of a 4K iteration.
   const int rows = wrows / kBatchRows;
   const int lrow = lane / kLanesPerRow, lcol = (lane % kLanesPerRow) * kPx;
   const bool vec_labels = (reinterpret_cast<uintptr_t>(im.labels) & 15) == 0 && (im.width % kPx) == 0;
-  const int per = (share.count + kWarps - 1) / kWarps;
-  const int end = min((warp + 1) * per, share.count);
-  for (int j0 = warp * per; j0 < end; j0 += 32) {
+  const int per = (w1 - w0 + kWarps - 1) / kWarps;
+  const int end = min(w0 + (warp + 1) * per, w1);
+  for (int j0 = w0 + warp * per; j0 < end; j0 += 32) {
     const int j = j0 + lane;
     const bool mine = j < end;
     int sr = 0, tx = 0;
@@ -1462,37 +1431,86 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
                           vec_labels);
       }
     }
-    unsigned heavy = __ballot_sync(full, mine && k < 0);
-    counted += __popc(heavy);
+    const unsigned heavy = __ballot_sync(full, mine && k < 0);
     if (heavy) {
       int base = 0;
       if (lane == 0) base = atomicAdd(&sm.nheavy, __popc(heavy));
       base = __shfl_sync(full, base, 0);
-      const int slot = base + __popc(heavy & ((1u << lane) - 1u));
-      const bool listed = ((heavy >> lane) & 1u) && slot < kHeavyCap;
-      if (listed) sm.heavy[slot] = sr * im.ntx + tx;
-      heavy &= ~__ballot_sync(full, listed);
-    }
-    // the list is full: these now
-    for (; heavy; heavy &= heavy - 1) {
-      const int g = __ffs(heavy) - 1;
-      process_span<LAYOUT, DIM, MODE>(im, __shfl_sync(full, sr, g), __shfl_sync(full, tx, g), sm,
-                                      wl, it, status);
+      if ((heavy >> lane) & 1u) sm.heavy[base + __popc(heavy & ((1u << lane) - 1u))] = sr * im.ntx + tx;
     }
   }
-  __syncthreads();
-  const int nh = min(sm.nheavy, kHeavyCap);
-  for (;;) {
-    int idx = 0;
-    if (lane == 0) idx = atomicAdd(&sm.next_heavy, 1);
-    idx = __shfl_sync(full, idx, 0);
-    if (idx >= nh) break;
-    const int s = sm.heavy[idx];
-    const int sr = s / im.ntx;
-    process_span<LAYOUT, DIM, MODE>(im, sr, s - sr * im.ntx, sm, wl, it, status);
+}
+
+// One iteration of the block's share of an image's spans.  There is no block
+// barrier and no global traffic per span: warps take places j = warp, warp +
+// kWarps, ..., each span's contribution is added to the block's integer sums,
+// and those go to the image accumulators once, at the end.  A span's
+// contribution does not depend on who takes it, so neither does the result.
+//
+// After the first iteration, where the fast spans' sums are kept, most spans
+// need none of their pixels (one candidate: labels and sums known): the warps
+// finish those at once and list the others; the block's warps then take the
+// listed spans one at a time.
+template <int LAYOUT, int DIM, int MODE, bool BATCH>
+__device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image& im, int img,
+                                          const SpanShare<BATCH>& share, int it) {
+  constexpr unsigned full = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool wl = MODE == kAssignOnly ||
+                  (MODE == kCluster && (im.threshold >= 0.0f || it == im.max_iter - 1));
+  int* status = &p.hdr->status;
+  if (MODE != kCluster || it == 0) {
+    int counted = 0;
+    for (int j = warp; j < share.count; j += kWarps) {
+      int sr, tx;
+      share.at(j, sr, tx);
+      counted += process_span<LAYOUT, DIM, MODE, true>(im, sr, tx, sm, wl, status);
+    }
+    if (BATCH) {
+      // what the next iteration may cost: spans, and those that need pixels
+      if (lane == 0 && counted) atomicAdd(&sm.counted, counted);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        atomicAdd(cost_at(p, img, it), kPixelCost * sm.counted + share.count);
+        sm.counted = 0;
+      }
+    }
+  } else {
+    // (with at most one span per warp nothing is gained by listing)
+    const bool light = im.span_sum && share.count > kWarps;
+    for (int w0 = 0; w0 < share.count;) {
+      const int w1 = light ? min(share.count, w0 + kHeavyCap) : share.count;
+      if (light) {
+        list_spans<LAYOUT, DIM, MODE, BATCH>(sm, im, share, w0, w1, wl);
+        __syncthreads();
+      }
+      const int n = light ? sm.nheavy : w1;
+      for (int own = warp;; own += kWarps) {
+        int idx = own;
+        if (light) {
+          if (lane == 0) idx = atomicAdd(&sm.next_heavy, 1);
+          idx = __shfl_sync(full, idx, 0);
+        }
+        if (idx >= n) break;
+        int sr, tx;
+        if (light) {
+          const int s = sm.heavy[idx];
+          sr = s / im.ntx;
+          tx = s - sr * im.ntx;
+        } else {
+          share.at(idx, sr, tx);
+        }
+        process_span<LAYOUT, DIM, MODE, false>(im, sr, tx, sm, wl, status);
+      }
+      w0 = w1;
+      if (w0 < share.count) {   // another window
+        __syncthreads();
+        if (threadIdx.x == 0) sm.nheavy = sm.next_heavy = 0;
+        __syncthreads();
+      }
+    }
   }
-  count();
-  block_to_accum(sm, p, img, im.K, DIM, it % 3);
+  if (MODE != kAssignOnly) block_to_accum(sm, p, img, im.K, DIM, it % 3);
 }
 
 __device__ __forceinline__ void clear_sums(Smem& sm) {
