@@ -388,8 +388,9 @@ typedef struct split_pipeline_params {
   float xy_scale;
   int kmeans_iters;
   float kmeans_threshold; /* < 0: exactly kmeans_iters iterations            */
-  int features;           /* SPLIT_LAYOUT_FLOAT4: pack float4 features first;
-                             SPLIT_LAYOUT_RGB8: read the bytes directly;
+  int features;           /* SPLIT_LAYOUT_FLOAT4: byte / 255 with the results
+                             of packed float4 features (read from the bytes);
+                             SPLIT_LAYOUT_RGB8: the RGB8 layout's results;
                              SPLIT_PIPELINE_FEATURES_LAB_BETA: the sample's
                              (beta, a*, b*) features (split_pack_lab_beta;
                              in a batch with per-image maxima)             */
@@ -424,9 +425,8 @@ size_t split_pipeline_workspace_size(int width, int height,
  * 3 x w*h float out (may be null when compute_normals == 0).
  * stage_events: null, or 2 * SPLIT_PIPELINE_STAGES cudaEvent_t recorded
  * before/after each stage (a skipped stage records both back to back).  With
- * SPLIT_LAYOUT_FLOAT4 features and compute_normals set, one pass over the
- * bytes writes both the features and the normals: the first stage times it
- * and the normals stage is empty. */
+ * SPLIT_LAYOUT_FLOAT4 features and compute_normals set, the first stage is the
+ * normals pass and the normals stage is empty. */
 int split_pipeline_run(const uint8_t* rgb, int width, int height,
                        const split_pipeline_params* params, float* centroids,
                        int32_t* cluster_labels, int32_t* segment_labels,

@@ -30,7 +30,7 @@ int lab_beta_geoms(const uint8_t* rgb, const Geoms& gs, float mu, float* feature
 constexpr int kFeaturesLabBeta = SPLIT_PIPELINE_FEATURES_LAB_BETA;
 // the batch packs float4 features (RGB / 255, or Lab + beta) before k-means
 inline bool packs_float4(const split_pipeline_params& p) {
-  return p.features == SPLIT_LAYOUT_FLOAT4 || p.features == kFeaturesLabBeta;
+  return p.features == kFeaturesLabBeta;   // byte / 255 features are read from the bytes
 }
 }  // namespace sg
 
@@ -212,13 +212,11 @@ extern "C" int split_batch_bind(split_batch* b, const uint8_t* rgb, float* centr
   b->normals = normals;
   b->ws = workspace;
   std::vector<KmBatchImage> kmi = km_images(*b, l);
-  // byte / 255 features lie in the unit cube; Lab + beta ones do not
-  const int layout = b->params.features == SPLIT_LAYOUT_FLOAT4
-                         ? (SPLIT_LAYOUT_FLOAT4 | SPLIT_FEATURES_UNIT_RANGE)
-                         : b->params.features == kFeaturesLabBeta ? SPLIT_LAYOUT_FLOAT4
-                                                                  : SPLIT_LAYOUT_RGB8;
-  SG_TRY(kmeans_batch_prepare(kmi.data(), (int)kmi.size(), layout, b->params.dim,
-                              b->params.xy_scale, l.km_ws, b->km_bytes, st, &b->km));
+  SG_TRY(kmeans_batch_prepare(kmi.data(), (int)kmi.size(),
+                              packs_float4(b->params) ? SPLIT_LAYOUT_FLOAT4 : SPLIT_LAYOUT_RGB8,
+                              b->params.dim, b->params.xy_scale,
+                              b->params.features == SPLIT_LAYOUT_FLOAT4, l.km_ws, b->km_bytes, st,
+                              &b->km));
   const size_t ni = b->images.size();
   std::vector<ImgGeom> geoms(ni);
   std::vector<CUtensorMap> lab_maps(ni), rgb_maps(ni);
@@ -272,15 +270,13 @@ extern "C" int split_batch_run_events(split_batch* b, void* const* stage_events,
   ss.p[ss.n++] = &static_cast<WsHeader*>(l.km_ws)->status;
   ss.p[ss.n++] = &static_cast<WsHeader*>(l.ccl_ws)->status;
   if (l.mrg_ws) ss.p[ss.n++] = &static_cast<WsHeader*>(l.mrg_ws)->status;
-  // 0: byte / 255 features with the normals, from one read of the bytes
+  // 0: features (with SPLIT_LAYOUT_FLOAT4 the normals instead: the k-means reads
+  // the bytes)
   SG_TRY(mark(0));
-  const bool fused = p.features == SPLIT_LAYOUT_FLOAT4 && p.compute_normals;
-  if (fused)
-    SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals,
-                              l.features4, st));
-  else if (p.features == SPLIT_LAYOUT_FLOAT4)
-    SG_TRY(split_pack_rgb8(b->rgb, b->arena_px, l.features4, nullptr, stream));
-  else if (p.features == kFeaturesLabBeta)
+  const bool first = p.features == SPLIT_LAYOUT_FLOAT4 && p.compute_normals;
+  if (first)
+    SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals, st));
+  else if (packs_float4(p))
     SG_TRY(lab_beta_geoms(b->rgb, device_geoms(*b, l, nullptr), p.beta_mu, l.features4, l.maxima,
                           st));
   SG_TRY(mark(1));
@@ -311,11 +307,10 @@ extern "C" int split_batch_run_events(split_batch* b, void* const* stage_events,
   SG_TRY(erode_geoms(l.seg, b->segment_labels, device_geoms(*b, l, l.lab_maps), p.erode_radius,
                      mstate, mfin, 1, st));
   SG_TRY(mark(9));
-  // 5: normals (empty when the features pass wrote them)
+  // 5: normals (empty when stage 0 wrote them)
   SG_TRY(mark(10));
-  if (p.compute_normals && !fused)
-    SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals,
-                              nullptr, st));
+  if (p.compute_normals && !first)
+    SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals, st));
   // errors the stages recorded in their own workspace headers, into the
   // batch's status word
   SG_TRY(fold_status(&l.hdr->status, ss, st));

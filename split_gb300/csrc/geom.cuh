@@ -87,9 +87,14 @@ __device__ __forceinline__ TileRef tile_ref(const Geoms& gs, int tile) {
   return r;
 }
 
-// Sobel normals of the L* plane straight from RGB8 over a geometry table;
-// with features4 set, the same pass writes the float4 byte / 255 features.
+// Sobel normals of the L* plane straight from RGB8 over a geometry table.
 int normals_rgb8_geoms(const uint8_t* rgb, const Geoms& gs, float depth, float* normals,
-                       float* features4, cudaStream_t st);
+                       cudaStream_t st);
+
+// k-means over byte / 255 features read from the bytes, with the results of the
+// packed float4 ones (kmeans.cu).
+int kmeans_cluster_bytes(const uint8_t* rgb, int dim, int64_t n, int width, float xy_scale,
+                         float* centroids, int K, int32_t* labels, void* ws, size_t ws_bytes,
+                         int max_iter, float threshold, cudaStream_t st);
 
 }  // namespace sg

@@ -78,6 +78,7 @@ enum Mode { kCluster = 0, kUpdateOnly = 1, kAssignOnly = 2 };
 struct Image {
   const void* points;
   int unit_range;           // colour features known to lie in [0, 1]
+  int any_width;            // RGB8: fast spans at any width and alignment
   int64_t npoints;
   int width;
   float xy_scale;
@@ -152,7 +153,6 @@ struct Loader {
   const void* pts;
   int64_t n;
   float xy;
-  const float* lut;
   __device__ __forceinline__ void load(int64_t i, int row, int col,
                                        float (&f)[DIM]) const {
     if (LAYOUT == SPLIT_LAYOUT_PLANAR) {
@@ -167,9 +167,8 @@ struct Loader {
       f[2] = v.z;
     } else {
       const uint8_t* p = static_cast<const uint8_t*>(pts) + 3 * i;
-      f[0] = lut[__ldg(p + 0)];
-      f[1] = lut[__ldg(p + 1)];
-      f[2] = lut[__ldg(p + 2)];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) f[c] = __fdiv_rn((float)__ldg(p + c), 255.0f);
     }
     if (DIM == 5) {
       f[3] = __fmul_rn(xy, (float)col);
@@ -230,40 +229,6 @@ __device__ __forceinline__ unsigned long long candidates(const float (&lo)[DIM],
   return ((unsigned long long)m1 << 32) | m0;
 }
 
-// Nearest centroid among `mask`: d = fma chain of (x - c)^2 in dimension
-// order, strict < in ascending k, so ties go to the lowest k (label.cu:23-32,
-// :98-105).
-template <int DIM>
-__device__ __forceinline__ int nearest(const float (&f)[DIM], const float* __restrict__ cs,
-                                       unsigned long long mask) {
-  constexpr int CS = cstride(DIM);
-  float best = INFINITY;
-  int bk = 0;
-  while (mask) {
-    const int k = __ffsll((long long)mask) - 1;
-    mask &= mask - 1;
-    const float4 c0 = *reinterpret_cast<const float4*>(cs + k * CS);
-    float t = __fsub_rn(f[0], c0.x);
-    float d = __fmul_rn(t, t);
-    t = __fsub_rn(f[1], c0.y);
-    d = __fmaf_rn(t, t, d);
-    t = __fsub_rn(f[2], c0.z);
-    d = __fmaf_rn(t, t, d);
-    if (DIM == 5) {
-      // dims 0..3 sit in c0 (x = column feature in c0.w), dim 4 right after
-      t = __fsub_rn(f[3], c0.w);
-      d = __fmaf_rn(t, t, d);
-      t = __fsub_rn(f[4], cs[k * CS + 4]);
-      d = __fmaf_rn(t, t, d);
-    }
-    if (d < best) {
-      best = d;
-      bk = k;
-    }
-  }
-  return bk;
-}
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -286,10 +251,11 @@ struct Smem {
   long long nc[kMaxK * kMaxDim];
   // spans deferred to the second pass of an iteration (see span_pass)
   int heavy[kHeavyCap];
+  unsigned long long heavy_mask[kHeavyCap];   // their candidates
+  unsigned finite[2];   // bit k: centroid k has no infinity and no NaN
   int nheavy;
   int next_heavy;
   int counted;   // spans of the pass that needed their pixels (batches)
-  float lut[256];
   // centroid forming: squared shifts, the last shift, the decisions
   float sdiff[kMaxK * kMaxDim];
   float delta;
@@ -329,46 +295,86 @@ constexpr int kLanesPerRow = kTile / kPx;  // 16 lanes cover a tile row
 constexpr int kBatchRows = 32 / kLanesPerRow;
 static_assert((kTile / kWarps) % kBatchRows == 0, "whole batches per warp span");
 
-// The lane's kPx consecutive pixels of image row `row` starting at column
-// `col`; ok[j] marks pixels inside the image.
-template <int LAYOUT, int DIM>
-__device__ __forceinline__ void load_px(const Image& im, const float* lut, int row, int col,
-                                        float (&f)[kPx][DIM], bool (&ok)[kPx]) {
-  const int64_t n = im.npoints;
-  const int64_t px0 = (int64_t)row * im.width + col;
-#pragma unroll
-  for (int j = 0; j < kPx; ++j) ok[j] = row < im.height && col + j < im.width && px0 + j < n;
-  if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
-    const float4* p = static_cast<const float4*>(im.points) + px0;
-#pragma unroll
-    for (int j = 0; j < kPx; ++j) {
-      const float4 v = ok[j] ? __ldg(p + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-      f[j][0] = v.x;
-      f[j][1] = v.y;
-      f[j][2] = v.z;
-    }
-  } else if (LAYOUT == SPLIT_LAYOUT_RGB8) {
-    const uint8_t* p = static_cast<const uint8_t*>(im.points) + 3 * px0;
-#pragma unroll
-    for (int j = 0; j < kPx; ++j)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) f[j][c] = ok[j] ? lut[__ldg(p + 3 * j + c)] : 0.0f;
-  } else {
-    const float* p = static_cast<const float*>(im.points);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d)
-#pragma unroll
-      for (int j = 0; j < kPx; ++j) f[j][d] = ok[j] ? __ldg(p + (int64_t)d * n + px0 + j) : 0.0f;
-  }
-  if (DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR) {
-    const float fy = __fmul_rn(im.xy_scale, (float)row);
-#pragma unroll
-    for (int j = 0; j < kPx; ++j) {
-      f[j][3] = __fmul_rn(im.xy_scale, (float)(col + j));
-      f[j][4] = fy;
-    }
-  }
+// byte / 255 of a pair of values, correctly rounded like the division: with r
+// = 1 / 255 rounded and e the rest, fma(b, r, b * e) gives it for every byte
+// (no table look-ups and no bank conflicts).
+__device__ __forceinline__ float2 unit_pair(float2 b) {
+  constexpr float r = 1.0f / 255.0f;
+  constexpr float e = (float)(1.0 / 255.0 - (double)r);
+  return ffma2(b, make_float2(r, r), fmul2(b, make_float2(e, e)));
 }
+
+// The lane's kPx consecutive pixels of a row as loaded (RGB8: the words that
+// hold their bytes), so that a batch's loads are under way before the one
+// before it is examined.
+template <int LAYOUT, int DIM>
+struct RawPx {
+  float v[LAYOUT == SPLIT_LAYOUT_RGB8 ? 1 : kPx][LAYOUT == SPLIT_LAYOUT_PLANAR ? DIM : 3];
+  uint32_t w[LAYOUT == SPLIT_LAYOUT_RGB8 ? 4 : 1];
+  int shift;   // RGB8: bits before the first byte
+
+  // pixels px0 .. px0 + valid - 1 (valid <= kPx; 0: nothing is read).  Every
+  // word that is read holds a byte of them.
+  __device__ __forceinline__ void load(const Image& im, int64_t px0, int valid) {
+    if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
+      const float4* p = static_cast<const float4*>(im.points) + px0;
+#pragma unroll
+      for (int j = 0; j < kPx; ++j) {
+        const float4 x = j < valid ? __ldg(p + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[j][0] = x.x;
+        v[j][1] = x.y;
+        v[j][2] = x.z;
+      }
+    } else if (LAYOUT == SPLIT_LAYOUT_RGB8) {
+      const uintptr_t at = reinterpret_cast<uintptr_t>(im.points) + 3 * px0;
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
+      const int skip = (int)(at & 3);
+      shift = 8 * skip;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = valid > 0 && 4 * i < 3 * valid + skip ? __ldg(p + i) : 0u;
+    } else {
+      const float* p = static_cast<const float*>(im.points) + px0;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+#pragma unroll
+        for (int j = 0; j < kPx; ++j) v[j][d] = j < valid ? __ldg(p + (int64_t)d * im.npoints + j) : 0.0f;
+    }
+  }
+  __device__ __forceinline__ void features(const Image& im, int row, int col,
+                                           float (&f)[kPx][DIM]) const {
+    if (LAYOUT == SPLIT_LAYOUT_RGB8) {
+      uint32_t x[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) x[i] = __funnelshift_r(w[i], w[i + 1], shift);
+#pragma unroll
+      for (int q = 0; q < kPx / 2; ++q)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int a = 6 * q + c, b = a + 3;
+          // 2^23 + byte, minus 2^23
+          const float2 m = make_float2(
+              __uint_as_float(__byte_perm(x[a >> 2], 0x4b000000u, 0x7540u | (a & 3))),
+              __uint_as_float(__byte_perm(x[b >> 2], 0x4b000000u, 0x7540u | (b & 3))));
+          const float2 u = unit_pair(fadd2(m, make_float2(-8388608.0f, -8388608.0f)));
+          f[2 * q][c] = u.x;
+          f[2 * q + 1][c] = u.y;
+        }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kPx; ++j)
+#pragma unroll
+        for (int d = 0; d < (LAYOUT == SPLIT_LAYOUT_PLANAR ? DIM : 3); ++d) f[j][d] = v[j][d];
+    }
+    if (DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR) {
+      const float fy = __fmul_rn(im.xy_scale, (float)row);
+#pragma unroll
+      for (int j = 0; j < kPx; ++j) {
+        f[j][3] = __fmul_rn(im.xy_scale, (float)(col + j));
+        f[j][4] = fy;
+      }
+    }
+  }
+};
 
 // Nearest centroid among `mask` for the lane's pixels; the distance is the
 // fma chain of (x - c)^2 in dimension order, strict < in ascending k (ties to
@@ -812,9 +818,14 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
     }
     cp_async_commit();
   };
+  // RGB8: the next batches' words in registers, moved up as they are used
+  RawPx<SPLIT_LAYOUT_RGB8, DIM> raw[kStages];
   if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
 #pragma unroll
     for (int b = 0; b < kStages; ++b) fetch(b);
+  } else {
+#pragma unroll
+    for (int b = 0; b < kStages; ++b) raw[b].load(im, px0 + b * step, b < nbatches ? kPx : 0);
   }
   for (int b = 0; b < nbatches; ++b, px0 += step) {
     float f[kPx][DIM];
@@ -833,16 +844,10 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
       __syncwarp();   // every lane has read the buffer that is refilled now
       fetch(b + kStages);
     } else {
-      const uint32_t* p =
-          reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(im.points) + 3 * px0);
-      const uint32_t w[3] = {__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+      raw[0].features(im, 0, 0, f);
 #pragma unroll
-      for (int j = 0; j < kPx; ++j)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int byte = 3 * j + c;
-          f[j][c] = sm.lut[(w[byte >> 2] >> (8 * (byte & 3))) & 0xffu];
-        }
+      for (int i = 0; i + 1 < kStages; ++i) raw[i] = raw[i + 1];
+      raw[kStages - 1].load(im, px0 + kStages * step, b + kStages < nbatches ? kPx : 0);
     }
     if (DIM == 5) {
       const float fy = __fmul_rn(im.xy_scale, (float)(row_first + b * kBatchRows));
@@ -905,7 +910,8 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
 // or RGB8 read as three 32-bit words per 4 pixels) and a candidate mask known
 // for the whole span: no per-pixel bounds checks, one pointer step per batch,
 // the column feature hoisted.  Results equal the general path's labels; the
-// sums are the same pixels' in a fixed, data-dependent order.
+// sums are the same pixels' in a fixed, data-dependent order.  Returns whether
+// those sums have gone into the block's (kSpanAny leaves its in the slots).
 //
 // In a clustering, `entry` is the span's slot of kept feature words (or
 // null).  Iteration 0 writes it for every span; in later iterations a span
@@ -913,7 +919,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
 // that candidate's (written when asked) and its sums are exact integers, so
 // nothing else needs the pixels.
 template <int LAYOUT, int DIM, int MODE, bool FIRST>
-__device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, int row_first,
+__device__ __forceinline__ bool fast_span(const Image& im, Smem& sm, int warp, int row_first,
                                           int col, int nbatches, unsigned long long mask,
                                           bool write_labels, bool vec_labels, int& acc_l,
                                           int& acc_n, float (&acc)[DIM], long long* entry,
@@ -928,10 +934,7 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
     ka = __ffsll((long long)mask) - 1;
   } else if (MODE != kAssignOnly && __popcll((long long)mask) == 2) {
     const int a = __ffsll((long long)mask) - 1, b = 63 - __clzll((long long)mask);
-    bool fin = true;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d)
-      fin = fin && isfinite(sm.cent[a * CS + d]) && isfinite(sm.cent[b * CS + d]);
+    const bool fin = ((sm.finite[a >> 5] >> (a & 31)) & (sm.finite[b >> 5] >> (b & 31)) & 1u) != 0u;
     if (fin) {
       kind = kSpanPair;
       ka = a;
@@ -942,7 +945,7 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
     const int lane = threadIdx.x & 31;
     add_span_sums<DIM>(sm, ka, lane < DIM ? __ldcg(entry + lane) : 0ll, 32 * kPx * nbatches);
     if (write_labels) write_span_labels(im, row_first, col, nbatches, ka, vec_labels);
-    return;
+    return true;
   }
   if (kind == kSpanSingle)
     span_batches<LAYOUT, DIM, MODE, kSpanSingle, FIRST>(im, sm, warp, row_first, col, nbatches, mask, ka,
@@ -956,6 +959,7 @@ __device__ __forceinline__ void fast_span(const Image& im, Smem& sm, int warp, i
     span_batches<LAYOUT, DIM, MODE, kSpanAny, FIRST>(im, sm, warp, row_first, col, nbatches, mask, ka,
                                               kb, write_labels, vec_labels, acc_l, acc_n, acc,
                                               entry, status);
+  return MODE == kCluster && kind != kSpanAny;
 }
 
 // Whether a warp span takes the fast path: xy features with colour known to
@@ -970,8 +974,9 @@ __device__ __forceinline__ bool fast_geometry(const Image& im, int row0, int col
   return MODE != kUpdateOnly && unit_box && row0 + wrows <= im.height &&
          col0 + kTile <= im.width &&
          (LAYOUT == SPLIT_LAYOUT_FLOAT4 ||
-          (LAYOUT == SPLIT_LAYOUT_RGB8 && vec_labels &&
-           (reinterpret_cast<uintptr_t>(im.points) & 3) == 0));
+          (LAYOUT == SPLIT_LAYOUT_RGB8 &&
+           (im.any_width ||
+            (vec_labels && (reinterpret_cast<uintptr_t>(im.points) & 3) == 0))));
 }
 
 // The candidate mask of a span with xy features and colour in [0, 1]: the
@@ -1012,9 +1017,11 @@ __device__ __forceinline__ unsigned long long unit_box_mask(const Image& im, con
 //
 // Returns whether the span needs its pixels in later iterations too (as long
 // as its candidates stay the same).
+// listed: span_mask is the span's candidate mask already (list_spans).
 template <int LAYOUT, int DIM, int MODE, bool FIRST>
 __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, Smem& sm,
-                                             bool write_labels, int* status) {
+                                             bool write_labels, int* status,
+                                             unsigned long long span_mask, bool listed) {
   const unsigned full = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int CS = cstride(DIM);
@@ -1039,8 +1046,7 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
                          ? im.span_sum + ((size_t)srow * im.span_cols + tx) * kSpanSums
                          : nullptr;
 
-  unsigned long long span_mask = 0;
-  if (MODE != kUpdateOnly && unit_box)
+  if (MODE != kUpdateOnly && unit_box && !listed)
     span_mask = unit_box_mask<DIM>(im, sm, row0, col0, rows_in, cols_in);
 
   int acc_l = -1, acc_n = 0;
@@ -1048,19 +1054,39 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
 #pragma unroll
   for (int d = 0; d < DIM; ++d) acc[d] = 0.0f;
 
+  bool direct = false;   // the sums are in the block's already
   if (fast)
-    fast_span<LAYOUT, DIM, MODE, FIRST>(im, sm, warp, row0 + lrow, col0 + lcol, wrows / kBatchRows,
+    direct = fast_span<LAYOUT, DIM, MODE, FIRST>(im, sm, warp, row0 + lrow, col0 + lcol, wrows / kBatchRows,
                                  span_mask, write_labels, vec_labels, acc_l, acc_n, acc,
                                         entry, status);
-  for (int b = 0; !fast && b < wrows / kBatchRows; ++b) {
-    if (b * kBatchRows >= rows_in) break;
+  // the lane's pixels inside the image in the span's rows
+  auto valid_px = [&](int row) {
+    const int64_t left = im.npoints - ((int64_t)row * im.width + col0 + lcol);
+    return row < im.height ? (int)max((int64_t)0, min((int64_t)min(kPx, im.width - col0 - lcol), left))
+                           : 0;
+  };
+  const int nb = fast ? 0 : (rows_in + kBatchRows - 1) / kBatchRows;
+  RawPx<LAYOUT, DIM> raw;
+  int valid_next = 0;
+  if (!fast) {
+    valid_next = valid_px(row0 + lrow);
+    raw.load(im, (int64_t)(row0 + lrow) * im.width + col0 + lcol, valid_next);
+  }
+  for (int b = 0; b < nb; ++b) {
     const int row = row0 + b * kBatchRows + lrow;
     const int col = col0 + lcol;
+    const int valid = valid_next;
     float f[kPx][DIM];
     bool ok[kPx];
-    load_px<LAYOUT, DIM>(im, sm.lut, row, col, f, ok);
-    const bool all_ok = ok[kPx - 1];
+    raw.features(im, row, col, f);
+#pragma unroll
+    for (int j = 0; j < kPx; ++j) ok[j] = j < valid;
+    const bool all_ok = valid == kPx;
     const int64_t px0 = (int64_t)row * im.width + col;
+    if (b + 1 < nb) {   // the next batch's loads go out now
+      valid_next = valid_px(row + kBatchRows);
+      raw.load(im, px0 + (int64_t)kBatchRows * im.width, valid_next);
+    }
     int lab[kPx];
     if (MODE == kUpdateOnly) {
       if (all_ok && vec_labels) {
@@ -1129,7 +1155,7 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
 
     accumulate<DIM>(sm, warp, im.K, f, lab, acc_l, acc_n, acc);
   }
-  if (MODE != kAssignOnly) {
+  if (MODE != kAssignOnly && !direct) {
     if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
     warp_to_fix<DIM>(sm, warp, im.K, status);
   }
@@ -1171,19 +1197,30 @@ __device__ __forceinline__ long long span_centre(const Image& im, float c) {
   return __float2ll_rn(__fmul_rn(c, (float)(im.unit_rows / kWarps * kTile) * kFixScale));
 }
 
-// Entry of Smem::bound for centroid k at c: the first three steps of the
-// fma chains of candidates() over lo = 0, hi = 1.
-template <int DIM>
-__device__ __forceinline__ float4 colour_bound(const float* c) {
-  float l = 0.0f, u = 0.0f;
+// Smem::bound and Smem::finite of centroid k < kMaxK (two whole warps call
+// this): the first three steps of the fma chains of candidates() over lo = 0,
+// hi = 1, and the centroid's xy.
+__device__ __forceinline__ void set_bounds(Smem& sm, int k, int K, const float* src, int stride) {
+  bool fin = false;
+  if (k < K) {
+    float c[5], l = 0.0f, u = 0.0f;
+    fin = true;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float g = fmaxf(fmaxf(0.0f - c[d], c[d] - 1.0f), 0.0f);
-    const float e = fmaxf(c[d] - 0.0f, 1.0f - c[d]);
-    l = __fmaf_rn(g, g, l);
-    u = __fmaf_rn(e, e, u);
+    for (int d = 0; d < 5; ++d) {
+      c[d] = src[k * stride + d];
+      fin = fin && isfinite(c[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float g = fmaxf(fmaxf(0.0f - c[d], c[d] - 1.0f), 0.0f);
+      const float e = fmaxf(c[d] - 0.0f, 1.0f - c[d]);
+      l = __fmaf_rn(g, g, l);
+      u = __fmaf_rn(e, e, u);
+    }
+    sm.bound[k] = make_float4(l, u, c[3], c[4]);
   }
-  return make_float4(l, u, c[DIM == 5 ? 3 : 0], c[DIM == 5 ? 4 : 0]);
+  const unsigned m = __ballot_sync(0xffffffffu, fin);
+  if ((k & 31) == 0) sm.finite[k >> 5] = m;
 }
 
 // The centroids of slot `src` into shared memory (strides cstride(DIM) there,
@@ -1197,13 +1234,7 @@ __device__ __forceinline__ void load_centroids(const Image& im, const float* src
     sm.cent[idx] = c;
     if (d < DIM) sm.nc[k * kMaxDim + d] = span_centre(im, c);
   }
-  if (DIM == 5)
-    for (int k = threadIdx.x; k < im.K; k += blockDim.x) {
-      float c[5];
-#pragma unroll
-      for (int d = 0; d < 5; ++d) c[d] = __ldcg(src + k * 8 + d);
-      sm.bound[k] = colour_bound<5>(c);
-    }
+  if (DIM == 5 && threadIdx.x < kMaxK) set_bounds(sm, threadIdx.x, im.K, src, 8);
 }
 
 // The squared "centroid shift" as the reference's cluster() measures it
@@ -1222,9 +1253,9 @@ __device__ __forceinline__ void load_centroids(const Image& im, const float* src
 // read words no call of the iteration wrote).
 template <int LAYOUT, int DIM>
 __device__ float reference_shift(const Image& im, const float* cent, const float* c_old,
-                                 const unsigned* cnt, const float* lut) {
+                                 const unsigned* cnt) {
   constexpr int CS = cstride(DIM);
-  Loader<LAYOUT, DIM> ld{im.points, im.npoints, im.xy_scale, lut};
+  Loader<LAYOUT, DIM> ld{im.points, im.npoints, im.xy_scale};
   const int64_t base = 2 * im.npoints;
   float acc = 0.0f;
   for (int j = 0; j < im.K * 3; ++j) {
@@ -1305,10 +1336,8 @@ __device__ bool form_centroids(const Params& p, int img, const Image& im, int i,
     __syncthreads();
     return false;
   }
-  if (DIM == 5 && threadIdx.x >= kThreads - kMaxK) {
-    const int k = (int)threadIdx.x - (kThreads - kMaxK);
-    if (k < im.K) sm.bound[k] = colour_bound<5>(sm.cent + k * CS);
-  }
+  if (DIM == 5 && threadIdx.x >= kThreads - kMaxK)
+    set_bounds(sm, (int)threadIdx.x - (kThreads - kMaxK), im.K, sm.cent, CS);
   if (owner && threadIdx.x >= 32) {
     const size_t zb = acc_slot(p, (i + 1) % 3, img);
     const int t = (int)threadIdx.x - 32, nt = (int)blockDim.x - 32;
@@ -1327,7 +1356,7 @@ __device__ bool form_centroids(const Params& p, int img, const Image& im, int i,
     for (int idx = threadIdx.x; idx < im.K * DIM; idx += 32) acc = __fadd_rn(acc, sm.sdiff[idx]);
     acc = warp_sum(acc);
     if (DIM == 3 && im.ref_shift && threadIdx.x == 0)
-      acc = reference_shift<LAYOUT, DIM>(im, sm.cent, c_old, cnt, sm.lut);
+      acc = reference_shift<LAYOUT, DIM>(im, sm.cent, c_old, cnt);
     if (threadIdx.x == 0) {
       const float delta = sqrtf(acc);
       bool more = i < im.max_iter && fabsf(delta - sm.delta) > im.threshold;
@@ -1392,11 +1421,14 @@ __device__ __forceinline__ void list_spans(Smem& sm, const Image& im,
     int sr = 0, tx = 0;
     if (mine) share.at(j, sr, tx);
     int k = -1;   // a light span's cluster
-    if (mine && fast_geometry<LAYOUT, DIM, MODE>(im, sr * wrows, tx * kTile, wrows, vec_labels)) {
-      const float lo3 = __fmul_rn(im.xy_scale, (float)(tx * kTile));
-      const float hi3 = __fmul_rn(im.xy_scale, (float)(tx * kTile + kTile - 1));
-      const float lo4 = __fmul_rn(im.xy_scale, (float)(sr * wrows));
-      const float hi4 = __fmul_rn(im.xy_scale, (float)(sr * wrows + wrows - 1));
+    unsigned long long mask = 0;
+    if (mine) {
+      const int row0 = sr * wrows, col0 = tx * kTile;
+      const int rows_in = min(wrows, im.height - row0), cols_in = min(kTile, im.width - col0);
+      const float lo3 = __fmul_rn(im.xy_scale, (float)col0);
+      const float hi3 = __fmul_rn(im.xy_scale, (float)(col0 + cols_in - 1));
+      const float lo4 = __fmul_rn(im.xy_scale, (float)row0);
+      const float hi4 = __fmul_rn(im.xy_scale, (float)(row0 + rows_in - 1));
       float ub = INFINITY;
       for (int q = 0; q < im.K; ++q) {
         const float4 c = sm.bound[q];
@@ -1404,17 +1436,15 @@ __device__ __forceinline__ void list_spans(Smem& sm, const Image& im,
         ub = fminf(ub, __fmaf_rn(e4, e4, __fmaf_rn(e3, e3, c.y)));
       }
       const float thr = ub * 1.0001f;
-      int n = 0;
       for (int q = 0; q < im.K; ++q) {
         const float4 c = sm.bound[q];
         const float g3 = fmaxf(fmaxf(lo3 - c.z, c.z - hi3), 0.0f);
         const float g4 = fmaxf(fmaxf(lo4 - c.w, c.w - hi4), 0.0f);
-        if (__fmaf_rn(g4, g4, __fmaf_rn(g3, g3, c.x)) <= thr) {
-          ++n;
-          k = q;
-        }
+        if (__fmaf_rn(g4, g4, __fmaf_rn(g3, g3, c.x)) <= thr) mask |= 1ull << q;
       }
-      if (n != 1) k = -1;
+      if (mask != 0ull && (mask & (mask - 1ull)) == 0ull &&
+          fast_geometry<LAYOUT, DIM, MODE>(im, row0, col0, wrows, vec_labels))
+        k = __ffsll((long long)mask) - 1;
     }
     if (k >= 0) {
       const long long* e = im.span_sum + ((size_t)sr * im.span_cols + tx) * kSpanSums;
@@ -1436,7 +1466,11 @@ __device__ __forceinline__ void list_spans(Smem& sm, const Image& im,
       int base = 0;
       if (lane == 0) base = atomicAdd(&sm.nheavy, __popc(heavy));
       base = __shfl_sync(full, base, 0);
-      if ((heavy >> lane) & 1u) sm.heavy[base + __popc(heavy & ((1u << lane) - 1u))] = sr * im.ntx + tx;
+      if ((heavy >> lane) & 1u) {
+        const int slot = base + __popc(heavy & ((1u << lane) - 1u));
+        sm.heavy[slot] = sr * im.ntx + tx;
+        sm.heavy_mask[slot] = mask;
+      }
     }
   }
 }
@@ -1464,7 +1498,7 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
     for (int j = warp; j < share.count; j += kWarps) {
       int sr, tx;
       share.at(j, sr, tx);
-      counted += process_span<LAYOUT, DIM, MODE, true>(im, sr, tx, sm, wl, status);
+      counted += process_span<LAYOUT, DIM, MODE, true>(im, sr, tx, sm, wl, status, 0ull, false);
     }
     if (BATCH) {
       // what the next iteration may cost: spans, and those that need pixels
@@ -1477,7 +1511,9 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
     }
   } else {
     // (with at most one span per warp nothing is gained by listing)
-    const bool light = im.span_sum && share.count > kWarps;
+    constexpr bool kXY = DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR;
+    const bool light = kXY && (LAYOUT == SPLIT_LAYOUT_RGB8 || im.unit_range) && im.span_sum &&
+                       share.count > kWarps;
     for (int w0 = 0; w0 < share.count;) {
       const int w1 = light ? min(share.count, w0 + kHeavyCap) : share.count;
       if (light) {
@@ -1500,7 +1536,8 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
         } else {
           share.at(idx, sr, tx);
         }
-        process_span<LAYOUT, DIM, MODE, false>(im, sr, tx, sm, wl, status);
+        process_span<LAYOUT, DIM, MODE, false>(im, sr, tx, sm, wl, status,
+                                               light ? sm.heavy_mask[idx] : 0ull, light);
       }
       w0 = w1;
       if (w0 < share.count) {   // another window
@@ -1534,8 +1571,6 @@ __global__ void __launch_bounds__(kThreads, SG_KM_MINBLOCKS) kmeans_kernel(Param
   __shared__ Smem sm;
   const Image& im = p.img0;
   clear_sums(sm);
-  if (LAYOUT == SPLIT_LAYOUT_RGB8)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) sm.lut[i] = (float)i / 255.0f;
   load_centroids<DIM>(im, p.cur, sm);
   __syncthreads();
   SpanShare<false> share;
@@ -1588,8 +1623,6 @@ __global__ void __launch_bounds__(kThreads, kBatchMinBlocks) kmeans_batch_kernel
   __shared__ RangeList rl;
   __shared__ Image im;
   clear_sums(sm);
-  if (LAYOUT == SPLIT_LAYOUT_RGB8)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) sm.lut[i] = (float)i / 255.0f;
   __syncthreads();
   auto take_image = [&](int img) {
     const int* src = reinterpret_cast<const int*>(p.images + img);
@@ -1920,7 +1953,7 @@ static int run(int mode, const void* points, int layout, int dim, int64_t n,
                int width, float xy_scale, float* centroids,
                const float* centroids_in, int K, int32_t* labels,
                const int32_t* labels_in, void* ws, size_t ws_bytes, int max_iter,
-               float threshold, int32_t* d_iter, cudaStream_t st) {
+               float threshold, int32_t* d_iter, cudaStream_t st, bool any_width = false) {
   if (!valid_features(points, layout, dim, n, width, K)) return SPLIT_ERR_INVALID;
   const int unit_range = (layout & SPLIT_FEATURES_UNIT_RANGE) ? 1 : 0;
   const int ref_shift = (layout & SPLIT_KMEANS_REFERENCE_SHIFT) ? 1 : 0;
@@ -1944,6 +1977,7 @@ static int run(int mode, const void* points, int layout, int dim, int64_t n,
   Image& im = p.img0;
   im.points = points;
   im.unit_range = unit_range;
+  im.any_width = any_width;
   im.npoints = n;
   im.width = width;
   im.xy_scale = xy_scale;
@@ -2042,6 +2076,22 @@ extern "C" int split_kmeans_cluster(const void* points, int layout, int dim, int
                  centroids, nclusters, labels, nullptr, workspace, workspace_bytes, max_iter,
                  threshold, d_iterations, as_stream(stream));
 }
+
+// byte / 255 features straight from the bytes, with the results of
+// split_kmeans_cluster on the packed float4 ones (unit range): the same values
+// and, at any image width, the same fast spans.
+namespace sg {
+int kmeans_cluster_bytes(const uint8_t* rgb, int dim, int64_t n, int width, float xy_scale,
+                         float* centroids, int K, int32_t* labels, void* ws, size_t ws_bytes,
+                         int max_iter, float threshold, cudaStream_t st) {
+  if (K > km::kMaxK)
+    return kmw::run(true, rgb, SPLIT_LAYOUT_RGB8, dim, n, width, xy_scale, centroids, centroids,
+                    K, labels, ws, ws_bytes, max_iter, threshold, nullptr, st);
+  return km::run(km::kCluster, rgb, SPLIT_LAYOUT_RGB8, dim, n, width, xy_scale, centroids,
+                 centroids, K, labels, nullptr, ws, ws_bytes, max_iter, threshold, nullptr, st,
+                 true);
+}
+}  // namespace sg
 
 extern "C" size_t split_kmeans_assign_workspace_size(int64_t npoints, int nclusters) {
   // one assignment keeps no span sums
@@ -2237,8 +2287,8 @@ size_t kmeans_batch_workspace(const KmBatchImage* imgs, int nimages) {
 }
 
 int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int dim,
-                         float xy_scale, void* ws, size_t ws_bytes, cudaStream_t st,
-                         KmBatchPlan* plan) {
+                         float xy_scale, bool any_width, void* ws, size_t ws_bytes,
+                         cudaStream_t st, KmBatchPlan* plan) {
   using namespace km;
   if (!imgs || nimages < 1 || (dim != 3 && dim != 5)) return SPLIT_ERR_INVALID;
   // kernel attributes now: the batch's launches may be captured into a graph
@@ -2267,6 +2317,7 @@ int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int 
     memset(&im, 0, sizeof(im));
     im.points = b.points;
     im.unit_range = unit_range;
+    im.any_width = any_width;
     im.npoints = b.npoints;
     im.width = b.width;
     im.xy_scale = xy_scale;

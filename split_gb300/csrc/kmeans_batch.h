@@ -28,9 +28,11 @@ struct KmBatchPlan {
 
 size_t kmeans_batch_workspace(const KmBatchImage* imgs, int nimages);
 // Uploads the image descriptors (synchronises `st`; call outside capture).
+// any_width: RGB8 spans take the fast path at any width and alignment, as
+// float4 ones do (bytes in the place of packed features).
 int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int dim,
-                         float xy_scale, void* ws, size_t ws_bytes, cudaStream_t st,
-                         KmBatchPlan* plan);
+                         float xy_scale, bool any_width, void* ws, size_t ws_bytes,
+                         cudaStream_t st, KmBatchPlan* plan);
 // Launches only (capturable into a CUDA graph).
 int kmeans_batch_run(const KmBatchPlan& plan, void* ws, cudaStream_t st);
 

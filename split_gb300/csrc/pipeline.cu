@@ -11,9 +11,10 @@ namespace pipe {
 // The sample's Lab + beta features (float4 per pixel) instead of RGB / 255.
 constexpr int kFeaturesLabBeta = SPLIT_PIPELINE_FEATURES_LAB_BETA;
 
-inline bool packs(const split_pipeline_params& p) {
-  return p.features == SPLIT_LAYOUT_FLOAT4 || p.features == kFeaturesLabBeta;
-}
+// Only the Lab + beta features are packed.  The byte / 255 features of
+// SPLIT_LAYOUT_FLOAT4 have the values the k-means forms from the bytes: packing
+// them wrote and read 16 bytes per pixel for the 3 it reads now.
+inline bool packs(const split_pipeline_params& p) { return p.features == kFeaturesLabBeta; }
 
 struct Layout {
   WsHeader* hdr;
@@ -114,29 +115,28 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
       ((unsigned long long)l.bytes << 7) ^ ((unsigned long long)p.features << 3) ^
       (unsigned long long)(p.merge_P > 0) ^ ((unsigned long long)p.merge_policy << 1);
   if (!layout_unchanged(workspace, layout_key)) SG_TRY(clear_status(ss, st));
-  // byte / 255 features with the normals, from one read of the bytes (the
-  // normals stage below is then empty)
-  const bool fused = p.features == SPLIT_LAYOUT_FLOAT4 && p.compute_normals;
-  if (fused)
-    SG_TRY(normals_rgb8_geoms(rgb, single_geom(width, height), p.depth, normals, l.features4,
-                              st));
-  else if (p.features == SPLIT_LAYOUT_FLOAT4)
-    SG_TRY(split_pack_rgb8(rgb, n, l.features4, nullptr, stream));
-  else if (p.features == pipe::kFeaturesLabBeta)
+  // with SPLIT_LAYOUT_FLOAT4 the normals come first (the normals stage below is
+  // then empty)
+  const bool first = p.features == SPLIT_LAYOUT_FLOAT4 && p.compute_normals;
+  if (first)
+    SG_TRY(normals_rgb8_geoms(rgb, single_geom(width, height), p.depth, normals, st));
+  else if (pipe::packs(p))
     SG_TRY(split_pack_lab_beta(rgb, n, p.beta_mu, SPLIT_LAYOUT_FLOAT4, l.features4, nullptr,
                                l.pack_ws, 512, stream));
   SG_TRY(mark(1));
   // 1: k-means
   SG_TRY(mark(2));
-  const void* pts = pipe::packs(p) ? static_cast<const void*>(l.features4)
-                             : static_cast<const void*>(rgb);
-  // byte / 255 features lie in the unit cube; Lab + beta ones do not
-  const int layout = p.features == SPLIT_LAYOUT_FLOAT4
-                         ? (SPLIT_LAYOUT_FLOAT4 | SPLIT_FEATURES_UNIT_RANGE)
-                         : pipe::packs(p) ? SPLIT_LAYOUT_FLOAT4 : p.features;
-  SG_TRY(split_kmeans_cluster(pts, layout, p.dim, n, width, p.xy_scale, centroids,
-                              p.nclusters, cluster_labels, l.km_ws, l.km_bytes, p.kmeans_iters,
-                              p.kmeans_threshold, nullptr, stream));
+  if (p.features == SPLIT_LAYOUT_FLOAT4)
+    SG_TRY(kmeans_cluster_bytes(rgb, p.dim, n, width, p.xy_scale, centroids, p.nclusters,
+                                cluster_labels, l.km_ws, l.km_bytes, p.kmeans_iters,
+                                p.kmeans_threshold, st));
+  else
+    SG_TRY(split_kmeans_cluster(pipe::packs(p) ? static_cast<const void*>(l.features4)
+                                               : static_cast<const void*>(rgb),
+                                pipe::packs(p) ? SPLIT_LAYOUT_FLOAT4 : SPLIT_LAYOUT_RGB8, p.dim,
+                                n, width, p.xy_scale, centroids, p.nclusters, cluster_labels,
+                                l.km_ws, l.km_bytes, p.kmeans_iters, p.kmeans_threshold, nullptr,
+                                stream));
   SG_TRY(mark(3));
   // 2: connected components (+ component sizes for the merge)
   SG_TRY(mark(4));
@@ -171,7 +171,7 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
   SG_TRY(mark(9));
   // 5: normals of the luminance plane, straight from the bytes
   SG_TRY(mark(10));
-  if (p.compute_normals && !fused)
+  if (p.compute_normals && !first)
     SG_TRY(split_sobel_normals_rgb8(rgb, width, height, p.depth, normals, stream));
   // errors the stages recorded in their own workspace headers, into the
   // pipeline's status word
