@@ -55,7 +55,10 @@ namespace km {
 #define SG_KM_MINBLOCKS 2
 #endif
 constexpr int kBatchMinBlocks = 2;
-constexpr int kPixelCost = 10;   // of a span that needs its pixels, against one that does not
+// Costs of a batch's partition: a span that needs its pixels against one that
+// does not, and taking up an image (in spans, and in clocks).
+constexpr int kPixelCost = 20;
+constexpr int kImageSpans = 32, kImageClocks = 20000;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 // A unit is a tile of unit_rows x kTile pixels (unit_rows = 16 to 128, per
@@ -1643,13 +1646,16 @@ __global__ void __launch_bounds__(kThreads, kBatchMinBlocks) kmeans_batch_kernel
     // the running images' cost up to each thread's images
     const int per = (p.nimages + kThreads - 1) / kThreads;
     const int i0 = min(p.nimages, (int)threadIdx.x * per), i1 = min(p.nimages, i0 + per);
+    // (what a block pays to take up an image comes first: a range that holds the
+    // end of one image and the start of another gets less of both)
+    const long long fixed = it < 2 ? kImageSpans : kImageClocks >> 8;
     auto cost_of = [&](int img) -> long long {
       if (p.images[img].max_iter <= it) return 0;
       // stopped at the start of an iteration before this one (one that stops
       // in this iteration still has its spans in the ranges)
       const int done = __ldcg(&p.state[img].done);
       if (done != 0 && done < it) return 0;
-      return it == 0 ? p.images[img].nspans : max(1, __ldcg(cost_at(p, img, it - 1)));
+      return fixed + (it == 0 ? p.images[img].nspans : max(1, __ldcg(cost_at(p, img, it - 1))));
     };
     long long mine = 0;
     for (int i = i0; i < i1; ++i) mine += cost_of(i);
@@ -1693,8 +1699,12 @@ __global__ void __launch_bounds__(kThreads, kBatchMinBlocks) kmeans_batch_kernel
         const long long c = cost_of(i);
         if (c > 0 && x + c > w0) {
           const long long n = p.images[i].nspans;
-          const int a = w0 <= x ? 0 : (int)((w0 - x) * n / c);
-          const int b = w1 >= x + c ? (int)n : (int)((w1 - x) * n / c);
+          // where the range cuts the image's spans
+          auto cut = [&](long long w) {
+            const long long in = min(max(w - x - fixed, 0ll), c - fixed);
+            return (int)(in * n / (c - fixed));
+          };
+          const int a = cut(w0), b = cut(w1);
           if (a < b) {
             const int k = atomicAdd(&rl.n, 1);
             rl.img[k] = i;
