@@ -36,6 +36,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -94,6 +95,7 @@ struct Image {
   int32_t* d_iterations;
   int nspans;               // warp spans: ceil(height / (unit_rows / kWarps)) * ntx
   int scatter;              // batches: a step coprime to nspans, about 0.618 of it
+  int first_cost;           // batches: cost of the first iteration, in spans
   int height;               // rows (ceil(npoints / width))
   int ntx;                  // tiles per row of tiles
   int unit_rows;            // rows of a unit (kTile or 2 * kTile, from the tuning table)
@@ -1655,7 +1657,7 @@ __global__ void __launch_bounds__(kThreads, kBatchMinBlocks) kmeans_batch_kernel
       // in this iteration still has its spans in the ranges)
       const int done = __ldcg(&p.state[img].done);
       if (done != 0 && done < it) return 0;
-      return fixed + (it == 0 ? p.images[img].nspans : max(1, __ldcg(cost_at(p, img, it - 1))));
+      return fixed + (it == 0 ? p.images[img].first_cost : max(1, __ldcg(cost_at(p, img, it - 1))));
     };
     long long mine = 0;
     for (int i = i0; i < i1; ++i) mine += cost_of(i);
@@ -2340,6 +2342,13 @@ int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int 
     im.nspans = spans_of(b.npoints, b.width, im.unit_rows);
     im.scatter = std::max(1, (int)(0.6180339887 * im.nspans));
     while (std::gcd(im.scatter, im.nspans) != 1) ++im.scatter;
+    // Every span reads its pixels in the first iteration; one with several
+    // candidates costs about five times as much.  Their share, from the size
+    // of a cluster's cell against a span's 64 + 8: sqrt(K) 72 / sqrt(W H)
+    // (0.13 for K = 4 at 1000 x 1200, 0.40 for K = 32 at 1300 x 800).
+    const double several =
+        dim == 5 ? std::min(1.0, 72.0 * std::sqrt((double)b.nclusters / (double)b.npoints)) : 1.0;
+    im.first_cost = (int)(im.nspans * (1.0 + 4.0 * several));
     spans += im.nspans;
     im.height = height_of(b.npoints, b.width);
     im.ntx = tiles_x(b.width);
