@@ -14,10 +14,16 @@
 //
 // No N x 16 edge array and no comparison sort: the edges are written by an
 // order-preserving compaction (per-block counts, one scan, a write pass that
-// recomputes each item's outputs), and the pairs are sorted as 64-bit keys
-// by a stable LSD radix sort (8-bit digits; a digit equal in every key is
-// skipped), after which the same compaction keeps the first pair of every
-// run of equal pairs.  Counts come back through device words.
+// recomputes each item's outputs).  The pairs need no order before the sort,
+// and a boundary repeats its pair at every pixel: each tile keeps its distinct
+// pairs in a shared-memory set and appends those (a 1080p labelling of 400
+// segments and 4000 single pixels: about 20 thousand keys to sort for 0.9
+// million edges).  The keys, 64 bits, are sorted by a stable LSD radix sort
+// (8-bit digits; a digit equal in every key is skipped), after which the
+// compaction keeps the first pair of every run of equal pairs.  Counts come
+// back through device words.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sg {
@@ -31,12 +37,12 @@ constexpr int kScanThreads = 1024;
 // 16 n edge words must stay addressable with int32 (as in the reference)
 constexpr int64_t kMaxPixels = (1ll << 27) - 1;
 
-enum Mode { kEdges = 0, kPairs = 1, kUnique = 2 };
+enum Mode { kEdges = 0, kUnique = 1 };
 
 struct Layout {
   WsHeader* hdr;
   int* block_sum;                   // [blocks + 1]: per-block counts, then their prefix
-  int* total;                       // [2]: edges (or pairs), distinct pairs
+  int* total;                       // [2]: keys to sort
   unsigned long long* bits;         // [2]: OR and AND of every pair key
   unsigned long long* keys[2];      // [8 n] each: pair keys, sort ping-pong
   unsigned* hist;                   // [256 * sort blocks]: digit counts, then offsets
@@ -45,6 +51,17 @@ struct Layout {
 
 __host__ __device__ inline int blocks_of(int64_t items) {
   return (int)((items + kTile - 1) / kTile);
+}
+
+// The sort's tiles: up to kFewKeys keys (most labellings) 512, so that the
+// passes spread over many blocks with two rounds each; more keys 4096, so that
+// the one-block scan of the digit counts stays short.  20 thousand keys: a
+// pass 28 us in tiles of 4096, 17 us in tiles of 512.
+constexpr int64_t kFewKeys = 1 << 18;
+__host__ __device__ inline int sort_rounds(int64_t keys) { return keys <= kFewKeys ? 2 : kItems; }
+__host__ __device__ inline int sort_tiles(int64_t keys) {
+  const int64_t tile = (int64_t)sort_rounds(keys) * kThreads;
+  return (int)((keys + tile - 1) / tile);
 }
 
 static Layout carve(void* ws, int64_t n, bool pairs) {
@@ -58,7 +75,8 @@ static Layout carve(void* ws, int64_t n, bool pairs) {
   if (pairs) {
     l.keys[0] = c.take<unsigned long long>((size_t)(8 * n));
     l.keys[1] = c.take<unsigned long long>((size_t)(8 * n));
-    l.hist = c.take<unsigned>((size_t)256 * blocks_of(8 * n));
+    l.hist = c.take<unsigned>((size_t)256 * std::max(sort_tiles(8 * n),
+                                                     sort_tiles(std::min(8 * n, kFewKeys))));
   }
   l.bytes = c.size();
   return l;
@@ -92,7 +110,7 @@ __device__ __forceinline__ int pass_parity(const unsigned long long* bits, int p
 }
 
 struct Items {
-  const int32_t* labels;   // kEdges / kPairs
+  const int32_t* labels;   // kEdges
   int w, h;
   // kUnique: the sort buffers and the key bits that name the sorted one
   const unsigned long long* keys0;
@@ -104,7 +122,7 @@ struct Items {
 };
 
 // Outputs of item i: the bitmask of neighbours that border another segment
-// (kEdges / kPairs), or whether a sorted pair starts a run (kUnique).
+// (kEdges), or whether a sorted pair starts a run (kUnique).
 template <int MODE>
 __device__ __forceinline__ unsigned item_mask(const Items& it, int i) {
   if (MODE == kUnique) {
@@ -123,27 +141,29 @@ __device__ __forceinline__ unsigned item_mask(const Items& it, int i) {
 
 __device__ __forceinline__ int n_items(const int* d_n, int n) { return d_n ? *d_n : n; }
 
-// Block totals of the items' outputs (contiguous kItems per thread).
+// Totals of the items' outputs per tile of items (contiguous kItems per
+// thread), a block taking every gridDim.x-th tile.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) count_kernel(Items it, int n, const int* d_n,
                                                           int* block_sum) {
   pdl_wait();
   const int nn = n_items(d_n, n);
-  const int base = blockIdx.x * kTile;
-  if (base >= nn) return;
-  int c = 0;
-  for (int k = 0; k < kItems; ++k) {
-    const int i = base + threadIdx.x * kItems + k;
-    if (i < nn) c += __popc(item_mask<MODE>(it, i));
-  }
   __shared__ int ws[kWarps];
-  c = __reduce_add_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < kWarps; ++w) s += ws[w];
-    block_sum[blockIdx.x] = s;
+  for (int b = blockIdx.x; b < blocks_of(nn); b += gridDim.x) {
+    int c = 0;
+    for (int k = 0; k < kItems; ++k) {
+      const int i = b * kTile + threadIdx.x * kItems + k;
+      if (i < nn) c += __popc(item_mask<MODE>(it, i));
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int s = 0;
+      for (int w = 0; w < kWarps; ++w) s += ws[w];
+      block_sum[b] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -187,93 +207,160 @@ __device__ void block_scan(T* a, int count, int* total) {
   if (threadIdx.x == 0 && total) *total = (int)carry;
 }
 
-// Prefix of the block totals (their total to *total); with `bits`, also
-// resets the key OR / AND words that the write pass then fills.
+// Prefix of the block totals (their total to *total).
 __global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(int n, const int* d_n,
-                                                                   int* block_sum, int* total,
-                                                                   unsigned long long* bits) {
+                                                                   int* block_sum, int* total) {
   pdl_wait();
-  const int nb = blocks_of(n_items(d_n, n));
-  if (bits && threadIdx.x == 0) {
-    bits[0] = 0ull;
-    bits[1] = ~0ull;
-  }
-  block_scan<int>(block_sum, nb, total);
+  block_scan<int>(block_sum, blocks_of(n_items(d_n, n)), total);
 }
 
 // Writes every item's outputs at its place in the order of the items (a
-// block-wide exclusive scan of the threads' counts, plus the block prefix).
+// block-wide exclusive scan of the threads' counts, plus the tile's prefix).
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) write_kernel(Items it, int n, const int* d_n,
                                                           const int* block_sum, const int* total,
-                                                          int32_t* out0, int32_t* out1,
-                                                          unsigned long long* keys,
-                                                          unsigned long long* bits) {
+                                                          int32_t* out0, int32_t* out1) {
   pdl_wait();
   const int nn = n_items(d_n, n);
-  const int base = blockIdx.x * kTile;
-  if (base >= nn) return;
-  const int first = base + threadIdx.x * kItems;
-  int c = 0;
-  for (int k = 0; k < kItems; ++k)
-    if (first + k < nn) c += __popc(item_mask<MODE>(it, first + k));
-  // exclusive scan of c over the block
   __shared__ int ws[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int s = c;
+  for (int b = blockIdx.x; b < blocks_of(nn); b += gridDim.x) {
+    const int first = b * kTile + threadIdx.x * kItems;
+    int c = 0;
+    for (int k = 0; k < kItems; ++k)
+      if (first + k < nn) c += __popc(item_mask<MODE>(it, first + k));
+    // exclusive scan of c over the block
+    int s = c;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, s, o);
-    if (lane >= o) s += u;
-  }
-  if (lane == 31) ws[warp] = s;
-  __syncthreads();
-  int before = block_sum[blockIdx.x] + s - c;
-  for (int w = 0; w < warp; ++w) before += ws[w];
-  const int m = *total;
-  unsigned long long o_or = 0ull, o_and = ~0ull;
-  for (int k = 0; k < kItems; ++k) {
-    const int i = first + k;
-    if (i >= nn) break;
-    unsigned mask = item_mask<MODE>(it, i);
-    if (MODE == kUnique) {
-      if (mask) {
-        const unsigned long long key = it.sorted()[i];
-        out0[before] = (int)((unsigned)(key >> 32) ^ 0x80000000u);
-        out1[before] = (int)((unsigned)key ^ 0x80000000u);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += u;
+    }
+    if (lane == 31) ws[warp] = s;
+    __syncthreads();
+    int before = block_sum[b] + s - c;
+    for (int w = 0; w < warp; ++w) before += ws[w];
+    const int m = *total;
+    for (int k = 0; k < kItems; ++k) {
+      const int i = first + k;
+      if (i >= nn) break;
+      unsigned mask = item_mask<MODE>(it, i);
+      if (MODE == kUnique) {
+        if (mask) {
+          const unsigned long long key = it.sorted()[i];
+          out0[before] = (int)((unsigned)(key >> 32) ^ 0x80000000u);
+          out1[before] = (int)((unsigned)key ^ 0x80000000u);
+          ++before;
+        }
+        continue;
+      }
+      const int x = i % it.w, y = i / it.w;
+      while (mask) {
+        const int d = __ffs(mask) - 1;
+        mask &= mask - 1;
+        out0[before] = i;
+        out0[m + before] = neighbour(x, y, it.w, it.h, d);
         ++before;
       }
-      continue;
     }
-    const int x = i % it.w, y = i / it.w;
-    const int v = MODE == kPairs ? __ldg(it.labels + i) : 0;
-    while (mask) {
-      const int d = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int j = neighbour(x, y, it.w, it.h, d);
-      if (MODE == kEdges) {
-        out0[before] = i;
-        out0[m + before] = j;
-      } else {
-        const unsigned long long key = pair_key(v, __ldg(it.labels + j));
-        keys[before] = key;
-        o_or |= key;
-        o_and &= key;
+    __syncthreads();
+  }
+}
+
+// ---- the keys to sort ----------------------------------------------------------
+// no keys yet, and the OR / AND of none
+__global__ void reset_kernel(const Layout l) {
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    l.total[0] = 0;
+    l.bits[0] = 0ull;
+    l.bits[1] = ~0ull;
+  }
+}
+
+// The distinct pair keys of one tile of pixels, appended to keys[0] in any
+// order; a pair that the set has no room for within a short probe is appended
+// as it is (the sort brings the copies together).  A key is never 0: its two
+// labels differ.  Every append has an edge of its own, so 8 n keys hold all.
+constexpr int kPixH = 32, kPixW = 64, kHaloW = kPixW + 2, kHaloH = kPixH + 2;
+constexpr int kSetBits = 11, kSetProbes = 16;
+__global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restrict__ lab, int w,
+                                                         int h, const Layout l) {
+  __shared__ int tile[kHaloH * kHaloW];
+  __shared__ unsigned long long set[1 << kSetBits];
+  __shared__ int found, base;
+  pdl_wait();
+  const int tiles_x = (w + kPixW - 1) / kPixW;
+  const int x0 = (int)(blockIdx.x % tiles_x) * kPixW, y0 = (int)(blockIdx.x / tiles_x) * kPixH;
+  // pixels outside the image take the nearest inside: a neighbour of its own
+  // tile's pixel, so no pair is added
+  bool mixed = false;
+  const int first = __ldg(lab + (size_t)y0 * w + x0);
+  for (int q = threadIdx.x; q < kHaloH * kHaloW; q += kThreads) {
+    const int y = min(max(y0 - 1 + q / kHaloW, 0), h - 1);
+    const int x = min(max(x0 - 1 + q % kHaloW, 0), w - 1);
+    tile[q] = __ldg(lab + (size_t)y * w + x);
+    mixed |= tile[q] != first;
+  }
+  if (!__syncthreads_or(mixed)) return;
+  for (int i = threadIdx.x; i < (1 << kSetBits); i += kThreads) set[i] = 0ull;
+  if (threadIdx.x == 0) found = 0;
+  __syncthreads();
+  unsigned long long o_or = 0ull, o_and = ~0ull;
+  auto append = [&](unsigned long long key, int at) {
+    l.keys[0][at] = key;
+    o_or |= key;
+    o_and &= key;
+  };
+  for (int q = threadIdx.x; q < kPixH * kPixW; q += kThreads) {
+    const int lx = q % kPixW, ly = q / kPixW;
+    if (x0 + lx >= w || y0 + ly >= h) continue;
+    const int* c = tile + (ly + 1) * kHaloW + lx + 1;
+    const int v = *c;
+    const int t[8] = {c[-kHaloW - 1], c[-kHaloW], c[-kHaloW + 1], c[-1],
+                      c[1],           c[kHaloW - 1], c[kHaloW],   c[kHaloW + 1]};
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      bool add = t[a] != v;
+#pragma unroll
+      for (int b = 0; b < a; ++b) add = add && t[b] != t[a];
+      if (!add) continue;
+      const unsigned long long key = pair_key(v, t[a]);
+      unsigned s = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kSetBits));
+      bool in = false;
+      for (int probe = 0; probe < kSetProbes && !in; ++probe, s = (s + 1) & ((1 << kSetBits) - 1)) {
+        unsigned long long k = *(volatile unsigned long long*)&set[s];
+        if (k == 0ull) k = atomicCAS(&set[s], 0ull, key);
+        in = k == 0ull || k == key;
       }
-      ++before;
+      if (!in) append(key, atomicAdd(l.total, 1));
     }
   }
-  if (MODE == kPairs) {
-    // digits that differ between keys (a digit equal in all is not sorted on)
+  __syncthreads();
+  // the set's keys, with one place in the list per block
+  constexpr int kPer = (1 << kSetBits) / kThreads;
+  int mine = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      o_or |= __shfl_xor_sync(0xffffffffu, o_or, o);
-      o_and &= __shfl_xor_sync(0xffffffffu, o_and, o);
-    }
-    if (lane == 0) {
-      atomicOr(bits, o_or);
-      atomicAnd(bits + 1, o_and);
-    }
+  for (int k = 0; k < kPer; ++k) mine += set[threadIdx.x + k * kThreads] != 0ull;
+  int at = mine ? atomicAdd(&found, mine) : 0;
+  __syncthreads();
+  if (threadIdx.x == 0) base = found ? atomicAdd(l.total, found) : 0;
+  __syncthreads();
+  at += base;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const unsigned long long key = set[threadIdx.x + k * kThreads];
+    if (key != 0ull) append(key, at++);
+  }
+  // digits that differ between keys (a digit equal in all is not sorted on)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    o_or |= __shfl_xor_sync(0xffffffffu, o_or, o);
+    o_and &= __shfl_xor_sync(0xffffffffu, o_and, o);
+  }
+  if ((threadIdx.x & 31) == 0 && (o_or != 0ull || o_and != ~0ull)) {
+    atomicOr(l.bits, o_or);
+    atomicAnd(l.bits + 1, o_and);
   }
 }
 
@@ -282,24 +369,27 @@ __global__ void __launch_bounds__(kThreads) write_kernel(Items it, int n, const 
 __global__ void __launch_bounds__(kThreads) hist_kernel(const Layout l, int p) {
   pdl_wait();
   const int n = *l.total;
-  const int nb = blocks_of(n), b = blockIdx.x;
-  if (b >= nb || !pass_runs(l.bits, p)) return;
+  const int nb = sort_tiles(n), rounds = sort_rounds(n);
+  if ((int)blockIdx.x >= nb || !pass_runs(l.bits, p)) return;
   const unsigned long long* in = l.keys[pass_parity(l.bits, p)];
   __shared__ unsigned h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  for (int k = 0; k < kItems; ++k) {
-    const int i = b * kTile + k * kThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(in[i] >> (8 * p)) & 0xff], 1u);
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    for (int k = 0; k < rounds; ++k) {
+      const int i = (b * rounds + k) * kThreads + threadIdx.x;
+      if (i < n) atomicAdd(&h[(in[i] >> (8 * p)) & 0xff], 1u);
+    }
+    __syncthreads();
+    l.hist[threadIdx.x * nb + b] = h[threadIdx.x];
+    __syncthreads();
   }
-  __syncthreads();
-  l.hist[threadIdx.x * nb + b] = h[threadIdx.x];
 }
 
 __global__ void __launch_bounds__(kScanThreads) hist_scan_kernel(const Layout l, int p) {
   pdl_wait();
   if (!pass_runs(l.bits, p)) return;
-  block_scan<unsigned>(l.hist, 256 * blocks_of(*l.total), nullptr);
+  block_scan<unsigned>(l.hist, 256 * sort_tiles(*l.total), nullptr);
 }
 
 // Stable scatter: a block moves its items in index order, kThreads at a
@@ -309,57 +399,58 @@ __global__ void __launch_bounds__(kScanThreads) hist_scan_kernel(const Layout l,
 __global__ void __launch_bounds__(kThreads) scatter_kernel(const Layout l, int p) {
   pdl_wait();
   const int n = *l.total;
-  const int nb = blocks_of(n), b = blockIdx.x;
-  if (b >= nb || !pass_runs(l.bits, p)) return;
+  const int nb = sort_tiles(n), rounds = sort_rounds(n);
+  if ((int)blockIdx.x >= nb || !pass_runs(l.bits, p)) return;
   const int q = pass_parity(l.bits, p);
   const unsigned long long* in = l.keys[q];
   unsigned long long* out = l.keys[q ^ 1];
   __shared__ unsigned off[256];
   __shared__ unsigned wc[kWarps][256];
   const int warp = threadIdx.x >> 5;
-  off[threadIdx.x] = l.hist[threadIdx.x * nb + b];
-  for (int w = 0; w < kWarps; ++w) wc[w][threadIdx.x] = 0;
-  __syncthreads();
   unsigned lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-  for (int k = 0; k < kItems; ++k) {
-    const int i = b * kTile + k * kThreads + threadIdx.x;
-    const bool ok = i < n;
-    const unsigned long long key = ok ? in[i] : 0ull;
-    const int digit = ok ? (int)((key >> (8 * p)) & 0xff) : 256;
-    const unsigned peers = __match_any_sync(0xffffffffu, digit);
-    const int rank = __popc(peers & lt);
-    if (ok && rank == 0) wc[warp][digit] = __popc(peers);
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    off[threadIdx.x] = l.hist[threadIdx.x * nb + b];
+    for (int w = 0; w < kWarps; ++w) wc[w][threadIdx.x] = 0;
     __syncthreads();
-    if (ok) {
-      unsigned pos = off[digit] + rank;
-      for (int w = 0; w < warp; ++w) pos += wc[w][digit];
-      out[pos] = key;
+    for (int k = 0; k < rounds; ++k) {
+      const int i = (b * rounds + k) * kThreads + threadIdx.x;
+      if (i - (int)threadIdx.x >= n) break;   // the same in every thread
+      const bool ok = i < n;
+      const unsigned long long key = ok ? in[i] : 0ull;
+      const int digit = ok ? (int)((key >> (8 * p)) & 0xff) : 256;
+      const unsigned peers = __match_any_sync(0xffffffffu, digit);
+      const int rank = __popc(peers & lt);
+      if (ok && rank == 0) wc[warp][digit] = __popc(peers);
+      __syncthreads();
+      if (ok) {
+        unsigned pos = off[digit] + rank;
+        for (int w = 0; w < warp; ++w) pos += wc[w][digit];
+        out[pos] = key;
+      }
+      __syncthreads();
+      // the round's counts move into the digit offsets
+      unsigned t = 0;
+      for (int w = 0; w < kWarps; ++w) {
+        t += wc[w][threadIdx.x];
+        wc[w][threadIdx.x] = 0;
+      }
+      off[threadIdx.x] += t;
+      __syncthreads();
     }
-    __syncthreads();
-    // the round's counts move into the digit offsets
-    unsigned t = 0;
-    for (int w = 0; w < kWarps; ++w) {
-      t += wc[w][threadIdx.x];
-      wc[w][threadIdx.x] = 0;
-    }
-    off[threadIdx.x] += t;
-    __syncthreads();
   }
 }
 
+// `tiles`: tiles of items at most (blocks stride over those there are)
 template <int MODE>
-static int compaction(const Items& it, int n, const int* d_n, int max_blocks, const Layout& l,
-                      int* total, int32_t* out0, int32_t* out1, unsigned long long* keys,
-                      unsigned long long* bits, cudaStream_t st) {
-  launch_pdl(count_kernel<MODE>, dim3(max_blocks), dim3(kThreads), 0, st, it, n, d_n,
-             l.block_sum);
+static int compaction(const Items& it, int n, const int* d_n, int tiles, const Layout& l,
+                      int* total, int32_t* out0, int32_t* out1, cudaStream_t st) {
+  launch_pdl(count_kernel<MODE>, dim3(tiles), dim3(kThreads), 0, st, it, n, d_n, l.block_sum);
   SG_TRY(launch_status());
-  launch_pdl(scan_blocks_kernel, dim3(1), dim3(kScanThreads), 0, st, n, d_n, l.block_sum, total,
-             bits);
+  launch_pdl(scan_blocks_kernel, dim3(1), dim3(kScanThreads), 0, st, n, d_n, l.block_sum, total);
   SG_TRY(launch_status());
-  launch_pdl(write_kernel<MODE>, dim3(max_blocks), dim3(kThreads), 0, st, it, n, d_n,
-             (const int*)l.block_sum, (const int*)total, out0, out1, keys, bits);
+  launch_pdl(write_kernel<MODE>, dim3(tiles), dim3(kThreads), 0, st, it, n, d_n,
+             (const int*)l.block_sum, (const int*)total, out0, out1);
   return launch_status();
 }
 
@@ -386,7 +477,7 @@ extern "C" int split_segment_adjacency_edges(const int32_t* labels, int width, i
   cudaStream_t st = as_stream(stream);
   adj::Items it{labels, width, height, nullptr, nullptr, nullptr};
   return adj::compaction<adj::kEdges>(it, (int)n, nullptr, adj::blocks_of(n), l, d_count, edges,
-                                      nullptr, nullptr, nullptr, st);
+                                      nullptr, st);
 }
 
 extern "C" size_t split_segment_adjacency_workspace_size(int width, int height) {
@@ -406,12 +497,19 @@ extern "C" int split_segment_adjacency(const int32_t* labels, int width, int hei
     return SPLIT_ERR_WORKSPACE;
   l = adj::carve(workspace, n, true);
   cudaStream_t st = as_stream(stream);
-  // 1: the pair key of every edge, in edge order, and the digits that vary
-  adj::Items it{labels, width, height, nullptr, nullptr, nullptr};
-  SG_TRY(adj::compaction<adj::kPairs>(it, (int)n, nullptr, adj::blocks_of(n), l, l.total, nullptr,
-                                      nullptr, l.keys[0], l.bits, st));
-  // 2: stable radix passes
-  const int sort_blocks = adj::blocks_of(8 * n);
+  // 1: the distinct pair keys of every tile, and the digits that vary
+  launch_pdl(adj::reset_kernel, dim3(1), dim3(32), 0, st, l);
+  SG_TRY(launch_status());
+  const int tiles = ((width + adj::kPixW - 1) / adj::kPixW) * ((height + adj::kPixH - 1) / adj::kPixH);
+  launch_pdl(adj::pair_kernel, dim3(tiles), dim3(adj::kThreads), 0, st, labels, width, height, l);
+  SG_TRY(launch_status());
+  // 2: stable radix passes.  The key count is known on the device only and is
+  // usually a small part of 8 n: the blocks stride over the tiles there are (a
+  // block for every possible tile took 4 us a launch to find nothing to do).
+  DeviceInfo di;
+  SG_TRY(device_info(&di));
+  const int sort_blocks =
+      std::min(std::max(adj::blocks_of(8 * n), adj::sort_tiles(8 * n)), 4 * di.sm_count);
   for (int p = 0; p < 8; ++p) {
     launch_pdl(adj::hist_kernel, dim3(sort_blocks), dim3(adj::kThreads), 0, st, l, p);
     SG_TRY(launch_status());
@@ -424,5 +522,5 @@ extern "C" int split_segment_adjacency(const int32_t* labels, int width, int hei
   // sorted keys depends on the passes that ran: named on the device)
   adj::Items u{nullptr, width, height, l.keys[0], l.keys[1], l.bits};
   return adj::compaction<adj::kUnique>(u, 0, l.total, sort_blocks, l, d_count, keys, adjacency,
-                                       nullptr, nullptr, st);
+                                       st);
 }
