@@ -44,6 +44,7 @@
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "fixsum.cuh"
+#include "pixels.cuh"
 
 namespace sg {
 namespace km {
@@ -295,91 +296,9 @@ __device__ __forceinline__ void add_centered(const float (&x)[DIM], const float*
   }
 }
 
-constexpr int kPx = 4;                 // consecutive pixels per lane
 constexpr int kLanesPerRow = kTile / kPx;  // 16 lanes cover a tile row
 constexpr int kBatchRows = 32 / kLanesPerRow;
 static_assert((kTile / kWarps) % kBatchRows == 0, "whole batches per warp span");
-
-// byte / 255 of a pair of values, correctly rounded like the division: with r
-// = 1 / 255 rounded and e the rest, fma(b, r, b * e) gives it for every byte
-// (no table look-ups and no bank conflicts).
-__device__ __forceinline__ float2 unit_pair(float2 b) {
-  constexpr float r = 1.0f / 255.0f;
-  constexpr float e = (float)(1.0 / 255.0 - (double)r);
-  return ffma2(b, make_float2(r, r), fmul2(b, make_float2(e, e)));
-}
-
-// The lane's kPx consecutive pixels of a row as loaded (RGB8: the words that
-// hold their bytes), so that a batch's loads are under way before the one
-// before it is examined.
-template <int LAYOUT, int DIM>
-struct RawPx {
-  float v[LAYOUT == SPLIT_LAYOUT_RGB8 ? 1 : kPx][LAYOUT == SPLIT_LAYOUT_PLANAR ? DIM : 3];
-  uint32_t w[LAYOUT == SPLIT_LAYOUT_RGB8 ? 4 : 1];
-  int shift;   // RGB8: bits before the first byte
-
-  // pixels px0 .. px0 + valid - 1 (valid <= kPx; 0: nothing is read).  Every
-  // word that is read holds a byte of them.
-  __device__ __forceinline__ void load(const Image& im, int64_t px0, int valid) {
-    if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
-      const float4* p = static_cast<const float4*>(im.points) + px0;
-#pragma unroll
-      for (int j = 0; j < kPx; ++j) {
-        const float4 x = j < valid ? __ldg(p + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[j][0] = x.x;
-        v[j][1] = x.y;
-        v[j][2] = x.z;
-      }
-    } else if (LAYOUT == SPLIT_LAYOUT_RGB8) {
-      const uintptr_t at = reinterpret_cast<uintptr_t>(im.points) + 3 * px0;
-      const uint32_t* p = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
-      const int skip = (int)(at & 3);
-      shift = 8 * skip;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) w[i] = valid > 0 && 4 * i < 3 * valid + skip ? __ldg(p + i) : 0u;
-    } else {
-      const float* p = static_cast<const float*>(im.points) + px0;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d)
-#pragma unroll
-        for (int j = 0; j < kPx; ++j) v[j][d] = j < valid ? __ldg(p + (int64_t)d * im.npoints + j) : 0.0f;
-    }
-  }
-  __device__ __forceinline__ void features(const Image& im, int row, int col,
-                                           float (&f)[kPx][DIM]) const {
-    if (LAYOUT == SPLIT_LAYOUT_RGB8) {
-      uint32_t x[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) x[i] = __funnelshift_r(w[i], w[i + 1], shift);
-#pragma unroll
-      for (int q = 0; q < kPx / 2; ++q)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int a = 6 * q + c, b = a + 3;
-          // 2^23 + byte, minus 2^23
-          const float2 m = make_float2(
-              __uint_as_float(__byte_perm(x[a >> 2], 0x4b000000u, 0x7540u | (a & 3))),
-              __uint_as_float(__byte_perm(x[b >> 2], 0x4b000000u, 0x7540u | (b & 3))));
-          const float2 u = unit_pair(fadd2(m, make_float2(-8388608.0f, -8388608.0f)));
-          f[2 * q][c] = u.x;
-          f[2 * q + 1][c] = u.y;
-        }
-    } else {
-#pragma unroll
-      for (int j = 0; j < kPx; ++j)
-#pragma unroll
-        for (int d = 0; d < (LAYOUT == SPLIT_LAYOUT_PLANAR ? DIM : 3); ++d) f[j][d] = v[j][d];
-    }
-    if (DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR) {
-      const float fy = __fmul_rn(im.xy_scale, (float)row);
-#pragma unroll
-      for (int j = 0; j < kPx; ++j) {
-        f[j][3] = __fmul_rn(im.xy_scale, (float)(col + j));
-        f[j][4] = fy;
-      }
-    }
-  }
-};
 
 // Nearest centroid among `mask` for the lane's pixels; the distance is the
 // fma chain of (x - c)^2 in dimension order, strict < in ascending k (ties to
@@ -830,7 +749,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
     for (int b = 0; b < kStages; ++b) fetch(b);
   } else {
 #pragma unroll
-    for (int b = 0; b < kStages; ++b) raw[b].load(im, px0 + b * step, b < nbatches ? kPx : 0);
+    for (int b = 0; b < kStages; ++b) raw[b].load(im.points, im.npoints, px0 + b * step, b < nbatches ? kPx : 0);
   }
   for (int b = 0; b < nbatches; ++b, px0 += step) {
     float f[kPx][DIM];
@@ -849,10 +768,10 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
       __syncwarp();   // every lane has read the buffer that is refilled now
       fetch(b + kStages);
     } else {
-      raw[0].features(im, 0, 0, f);
+      raw[0].features(0.0f, 0, 0, f);
 #pragma unroll
       for (int i = 0; i + 1 < kStages; ++i) raw[i] = raw[i + 1];
-      raw[kStages - 1].load(im, px0 + kStages * step, b + kStages < nbatches ? kPx : 0);
+      raw[kStages - 1].load(im.points, im.npoints, px0 + kStages * step, b + kStages < nbatches ? kPx : 0);
     }
     if (DIM == 5) {
       const float fy = __fmul_rn(im.xy_scale, (float)(row_first + b * kBatchRows));
@@ -1075,7 +994,7 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
   int valid_next = 0;
   if (!fast) {
     valid_next = valid_px(row0 + lrow);
-    raw.load(im, (int64_t)(row0 + lrow) * im.width + col0 + lcol, valid_next);
+    raw.load(im.points, im.npoints, (int64_t)(row0 + lrow) * im.width + col0 + lcol, valid_next);
   }
   for (int b = 0; b < nb; ++b) {
     const int row = row0 + b * kBatchRows + lrow;
@@ -1083,14 +1002,14 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
     const int valid = valid_next;
     float f[kPx][DIM];
     bool ok[kPx];
-    raw.features(im, row, col, f);
+    raw.features(im.xy_scale, row, col, f);
 #pragma unroll
     for (int j = 0; j < kPx; ++j) ok[j] = j < valid;
     const bool all_ok = valid == kPx;
     const int64_t px0 = (int64_t)row * im.width + col;
     if (b + 1 < nb) {   // the next batch's loads go out now
       valid_next = valid_px(row + kBatchRows);
-      raw.load(im, px0 + (int64_t)kBatchRows * im.width, valid_next);
+      raw.load(im.points, im.npoints, px0 + (int64_t)kBatchRows * im.width, valid_next);
     }
     int lab[kPx];
     if (MODE == kUpdateOnly) {

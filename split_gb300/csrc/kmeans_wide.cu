@@ -2,21 +2,21 @@
 // memory (64 < K <= 2^20): label_points (split/src/split/device/kmeans/
 // label.cu:74-106) and cluster (cluster.cu:27-93), which set no limit on K.
 //
-// Assignment (assign_kernel): a warp takes 128 consecutive pixels per round
-// (4 per lane, measured as two packed FP32x2 pairs), the block walks the
-// centroids in shared-memory chunks of 32 KB (1024 centroids of 5
-// dimensions, 2048 of 3), and each warp prunes them exactly with bounds over
-// its pixels' feature box before measuring the survivors.  The squared distance is the reference's sum of
-// (x - c)^2 in dimension order (label.cu:23-32) with one rounding per
-// operation, and ties go to the lowest cluster index (strict < in ascending
-// k, as the reference's argmin over the distance row, label.cu:98-105).  In
-// a clustering the same pass adds every pixel's features to its cluster's
-// fixed-point sums (fixsum.cuh), so the update reads no pixel again: for
-// features below 2^32 as one 64-bit word per dimension, summed first over a
-// lane's four pixels where the warp's 128 pixels share one label.
+// Assignment (assign_kernel): a block takes 64 x 16 pixels at a time, a warp
+// 32 x 4 of them (4 consecutive ones per lane, measured as two packed FP32x2
+// pairs).  The centroids come in shared-memory chunks of 32 KB (1024
+// centroids of 5 dimensions, 2048 of 3).  The block prunes a chunk exactly
+// with bounds over its tile's feature box to a list, each warp the list over
+// its own pixels' box, and measures the survivors.  The squared distance is
+// the reference's sum of (x - c)^2 in dimension order (label.cu:23-32) with
+// one rounding per operation, and ties go to the lowest cluster index (strict
+// < in ascending k, as the reference's argmin over the distance row,
+// label.cu:98-105).  In a clustering the same pass adds every pixel's
+// features to its cluster's fixed-point sums (fixsum.cuh), so the update reads
+// no pixel again; a tile's sums are added up in shared memory first.
 //
 // Clustering: per iteration one assignment launch and one forming launch
-// (form_kernel, one block), all max_iter pairs queued at once, each launch a
+// (form_kernel), all max_iter pairs queued at once, each launch a
 // programmatic dependent of the one before.  The forming launch turns the
 // sums into means (FP64 division of the exact sum, rounded once to FP32; a
 // cluster without members keeps its centroid), measures the centroid shift,
@@ -30,6 +30,7 @@
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "fixsum.cuh"
+#include "pixels.cuh"
 
 namespace sg {
 namespace kmw {
@@ -37,15 +38,22 @@ namespace kmw {
 constexpr int kMinK = 65;                 // smaller K runs in the persistent kernel
 constexpr int kMaxClusters = 1 << 20;
 constexpr int kThreads = 256;
-constexpr int kPix = 4;                   // pixels per thread and round (two pairs)
+constexpr int kPix = kPx;                 // pixels per thread (two pairs)
+constexpr int kTileW = 64, kTileH = 16;   // a block's pixels
+constexpr int kSubW = 32, kSubH = 4;      // a warp's
+constexpr int kWarps = kThreads / 32;
+static_assert(kTileW * kTileH == kThreads * kPix && kSubW * kSubH == 32 * kPix, "one lane each");
+constexpr int kSlots = 128;               // clusters of a tile summed in shared memory
 constexpr int kChunkF4 = 2048;            // float4 slots of one centroid chunk (32 KB)
-constexpr int kFormThreads = 1024;
+constexpr int kFormSlots = 1024;          // strided partials of the shift
+constexpr int kFormThreads = 256;
+constexpr int kFormBlocks = 16;
 
 struct State {
   float delta;   // shift of the last formed iteration (0 before the first)
   int iters;     // iterations formed
   int done;      // no further iteration runs
-  int pad;
+  unsigned arrived;   // forming blocks that have finished their share
 };
 
 struct Layout {
@@ -56,6 +64,7 @@ struct Layout {
   unsigned long long* hi;    // [K][DIM] high words (signed)
   unsigned* cnt;             // [K] member counts
   float* word;               // [3K] squared terms of the reference's shift
+  float* part;               // [kFormSlots] partials of the L2 shift
   size_t bytes;
 };
 
@@ -69,6 +78,7 @@ inline Layout carve(void* ws, int K, int dim) {
   l.hi = c.take<unsigned long long>((size_t)K * dim);
   l.cnt = c.take<unsigned>((size_t)K);
   l.word = c.take<float>((size_t)3 * K);
+  l.part = c.take<float>(kFormSlots);
   l.bytes = c.size();
   return l;
 }
@@ -160,26 +170,113 @@ __device__ __forceinline__ void closer(const float (&fp)[DIM], const float (&fq)
   }
 }
 
-// A warp takes 128 consecutive pixels per round: lane l holds pixels
-// base + 32 j + l, j < 4, so each of its four loads is coalesced and labels
-// come in runs across the lanes for the fixed-point sums.
-//
-// Exact pruning per warp and round, over the box [lo, hi] of its 128
-// pixels' features: for a centroid, LB = squared distance to the box (below
-// every pixel's distance) and UB = squared distance to the farthest corner
-// (above it).  thr = the smallest UB seen so far (over this chunk and the
-// ones before) bounds every pixel's best distance, so a centroid whose LB
-// exceeds thr by more than the 1e-4 relative margin is strictly farther than
-// another centroid from every pixel, even after FP32 rounding (a few ulp),
-// and is skipped: every argmin, ties included, is unchanged.  Lanes bound 32
-// centroids at a time; the survivors of a ballot are then measured against
-// the warp's pixels in ascending k, as pairs on the packed FP32x2 pipe.
+// Exact pruning over a box [lo, hi] of pixels' features: for a centroid, LB =
+// squared distance to the box (below every pixel's distance) and UB = squared
+// distance to the farthest corner (above it).  thr = the smallest UB seen so
+// far (over this chunk and the ones before) bounds every pixel's best
+// distance, so a centroid whose LB exceeds thr by more than the 1e-4 relative
+// margin is strictly farther than another centroid from every pixel, even
+// after FP32 rounding (a few ulp), and is skipped: every argmin, ties
+// included, is unchanged.
+template <int DIM>
+__device__ __forceinline__ float upper_bound(const float* c, const float (&lo)[DIM],
+                                             const float (&hi)[DIM]) {
+  float u = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const float e = fmaxf(c[d] - lo[d], hi[d] - c[d]);
+    u = __fmaf_rn(e, e, u);
+  }
+  return u;
+}
+template <int DIM>
+__device__ __forceinline__ float lower_bound(const float* c, const float (&lo)[DIM],
+                                             const float (&hi)[DIM]) {
+  float l = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const float g = fmaxf(fmaxf(lo[d] - c[d], c[d] - hi[d]), 0.0f);
+    l = __fmaf_rn(g, g, l);
+  }
+  return l;
+}
+
+// The tile's sums per list entry (64-bit fixed point in two words).
+template <int DIM>
+struct TileSums {
+  unsigned lo[kSlots * DIM], hi[kSlots * DIM];
+  unsigned cnt[kSlots];
+};
+
+template <int DIM>
+__device__ __forceinline__ void tile_add(TileSums<DIM>& ts, int idx, unsigned long long v) {
+  const unsigned lo = (unsigned)v;
+  const unsigned old = atomicAdd(&ts.lo[idx], lo);
+  const unsigned hi = (unsigned)(v >> 32) + (old + lo < old ? 1u : 0u);
+  if (hi) atomicAdd(&ts.hi[idx], hi);
+}
+
+// Adds the warp's pixels (features in [0, 2^14)) to the sums of their list
+// entries `at` (below 0: none), entry by entry: the lanes' words split at bit
+// 24, so that each half's warp sum fits the 32-bit warp reduction.
+template <int LAYOUT, int DIM>
+__device__ __forceinline__ void warp_to_tile(TileSums<DIM>& ts, const float (&f)[kPix][DIM],
+                                             const int (&at)[kPix]) {
+  constexpr unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  unsigned long long q[kPix][DIM];
+#pragma unroll
+  for (int j = 0; j < kPix; ++j)
+#pragma unroll
+    for (int d = 0; d < DIM; ++d)
+      q[j][d] = (unsigned long long)__float2ll_rn(__fmul_rn(f[j][d], fix::kScale));
+  int left = -1;   // entries up to this one are done
+  for (;;) {
+    unsigned next = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < kPix; ++j)
+      if (at[j] > left) next = min(next, (unsigned)at[j]);
+    const unsigned p = __reduce_min_sync(full, next);
+    if (p == 0xffffffffu) break;
+    left = (int)p;
+    unsigned n = 0;
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int j = 0; j < kPix; ++j) n += at[j] == left ? 1u : 0u;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      unsigned long long s = 0;
+#pragma unroll
+      for (int j = 0; j < kPix; ++j) s += at[j] == left ? q[j][d] : 0ull;
+      unsigned long long total;
+      if (LAYOUT == SPLIT_LAYOUT_RGB8 && d < 3)   // values up to 1: at most 2^31 in all
+        total = __reduce_add_sync(full, (unsigned)s);
+      else
+        total = ((unsigned long long)__reduce_add_sync(full, (unsigned)(s >> 24)) << 24) +
+                __reduce_add_sync(full, (unsigned)s & 0xffffffu);
+      if (lane == d) mine = total;
+    }
+    n = __reduce_add_sync(full, n);
+    if (lane < DIM) tile_add(ts, left * DIM + lane, mine);
+    if (lane == DIM) atomicAdd(&ts.cnt[left], n);
+  }
+}
+
+// What bounds it: instruction issue (a pixel's labels and sums are a few
+// bytes).  Bounding every centroid against every 128 pixels and sending each
+// warp's sums to global memory took 120 us an iteration at 2560 x 1440, K =
+// 256, 5-D (75 without the sums); with the tile's list and sums in shared
+// memory 56 (54 for the labels alone).
 template <int LAYOUT, int DIM, bool ACC>
 __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
   constexpr int CS = DIM == 5 ? 2 : 1;          // float4 slots per centroid
   constexpr int kChunk = kChunkF4 / CS;         // centroids per chunk
   constexpr unsigned full = 0xffffffffu;
   __shared__ float4 cs[kChunkF4];
+  __shared__ unsigned short list[kChunk];       // the tile's candidates, ascending
+  __shared__ TileSums<DIM> sums;   // (clusterings only)
+  __shared__ float boxes[kWarps][2 * DIM], box[2 * DIM], least[kWarps];
+  __shared__ int counts[kWarps];
   __shared__ int stop;
   pdl_wait();
   if (ACC) {
@@ -188,12 +285,13 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
     if (stop) return;
   }
   const int K = a.K;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nchunks = (K + kChunk - 1) / kChunk;
-  const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-  const int64_t gw = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  const int64_t rounds = (a.P.n + warps * 128 - 1) / (warps * 128);
   float* csf = reinterpret_cast<float*>(cs);
+  const int W = a.P.width;
+  const int H = (int)((a.P.n + W - 1) / W);
+  const int tiles_x = (W + kTileW - 1) / kTileW;
+  const int tiles = tiles_x * ((H + kTileH - 1) / kTileH);
 
   auto load_chunk = [&](int ch) {
     const int k0 = ch * kChunk;
@@ -206,19 +304,22 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
     __syncthreads();
   };
   if (nchunks == 1) load_chunk(0);
+  if constexpr (ACC) {
+    for (int i = threadIdx.x; i < kSlots * DIM; i += kThreads) sums.lo[i] = sums.hi[i] = 0u;
+    for (int i = threadIdx.x; i < kSlots; i += kThreads) sums.cnt[i] = 0u;
+  }
 
-  for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t base = (r * warps + gw) * 128 + lane;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
+    const int row = ty * kTileH + (warp >> 1) * kSubH + lane / (kSubW / kPix);
+    const int col = tx * kTileW + (warp & 1) * kSubW + (lane % (kSubW / kPix)) * kPix;
+    const int64_t px0 = (int64_t)row * W + col;
+    const int valid =
+        row < H ? (int)max((int64_t)0, min((int64_t)min(kPix, W - col), a.P.n - px0)) : 0;
+    RawPx<LAYOUT, DIM> raw;
+    raw.load(a.P.pts, a.P.n, px0, valid);
     float f[kPix][DIM];
-    bool ok[kPix];
-#pragma unroll
-    for (int j = 0; j < kPix; ++j) {
-      const int64_t i = base + 32 * j;
-      ok[j] = i < a.P.n;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) f[j][d] = 0.0f;
-      if (ok[j]) load_px<LAYOUT, DIM>(a.P, i, f[j]);
-    }
+    raw.features(a.P.xy, row, col, f);
     // box of the warp's pixels; fminf / fmaxf skip NaN (a NaN pixel's
     // distances all compare false, so it keeps label 0 whatever is skipped)
     float lo[DIM], hi[DIM];
@@ -227,111 +328,161 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
       float x = INFINITY, z = -INFINITY;
 #pragma unroll
       for (int j = 0; j < kPix; ++j) {
-        if (ok[j]) {
+        if (j < valid) {
           x = fminf(x, f[j][d]);
           z = fmaxf(z, f[j][d]);
         }
       }
       lo[d] = fkey_inv(__reduce_min_sync(full, fkey(x)));
       hi[d] = fkey_inv(__reduce_max_sync(full, fkey(z)));
+      if (lane == 0) {
+        boxes[warp][d] = lo[d];
+        boxes[warp][DIM + d] = hi[d];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * DIM) {
+      float v = boxes[0][threadIdx.x];
+      for (int w = 1; w < kWarps; ++w)
+        v = threadIdx.x < DIM ? fminf(v, boxes[w][threadIdx.x]) : fmaxf(v, boxes[w][threadIdx.x]);
+      box[threadIdx.x] = v;
+    }
+    __syncthreads();
+    float blo[DIM], bhi[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      blo[d] = box[d];
+      bhi[d] = box[DIM + d];
     }
     float best[kPix];
-    int bk[kPix];
+    int bk[kPix];   // with one chunk the list entry, otherwise the cluster
 #pragma unroll
     for (int j = 0; j < kPix; ++j) {
       best[j] = INFINITY;
-      bk[j] = 0;
+      bk[j] = -1;   // (no distance compares: label 0)
     }
-    float ub_min = INFINITY;
+    float tile_ub = INFINITY, ub_min = INFINITY;
+    int nlist = 0;
     for (int ch = 0; ch < nchunks; ++ch) {
       if (nchunks > 1) load_chunk(ch);
       const int k0 = ch * kChunk;
       const int kc = min(kChunk, K - k0);
-      // smallest UB over this chunk (and the chunks before)
-      float um = ub_min;
-      for (int k = lane; k < kc; k += 32) {
-        float u = 0.0f;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          const float c = csf[k * (4 * CS) + d];
-          const float e = fmaxf(c - lo[d], hi[d] - c);
-          u = __fmaf_rn(e, e, u);
-        }
-        um = fminf(um, u);
-      }
+      // the tile's candidates of the chunk
+      float um = tile_ub;
+      for (int k = threadIdx.x; k < kc; k += kThreads)
+        um = fminf(um, upper_bound<DIM>(csf + k * (4 * CS), blo, bhi));
       // UB >= 0: its bit pattern orders like the value
+      um = __int_as_float(__reduce_min_sync(full, __float_as_int(um)));
+      if (lane == 0) least[warp] = um;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) tile_ub = fminf(tile_ub, least[w]);
+      const float tile_thr = tile_ub * 1.0001f;
+      nlist = 0;
+      for (int g = 0; g < kc; g += kThreads) {
+        const int k = g + (int)threadIdx.x;
+        const bool in = k < kc && lower_bound<DIM>(csf + k * (4 * CS), blo, bhi) <= tile_thr;
+        const unsigned m = __ballot_sync(full, in);
+        if (lane == 0) counts[warp] = __popc(m);
+        __syncthreads();
+        int before = nlist;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+          if (w < warp) before += counts[w];
+          nlist += counts[w];
+        }
+        if (in) list[before + __popc(m & ((1u << lane) - 1u))] = (unsigned short)k;
+        __syncthreads();
+      }
+      // the warp's, 32 list entries at a time
+      um = ub_min;
+      for (int i = lane; i < nlist; i += 32)
+        um = fminf(um, upper_bound<DIM>(csf + list[i] * (4 * CS), lo, hi));
       ub_min = __int_as_float(__reduce_min_sync(full, __float_as_int(um)));
       const float thr = ub_min * 1.0001f;
-      for (int g = 0; g < kc; g += 32) {
-        const int k = g + lane;
-        float l = __int_as_float(0x7fffffff);   // past the chunk: never a candidate
-        if (k < kc) {
-          l = 0.0f;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            const float c = csf[k * (4 * CS) + d];
-            const float gg = fmaxf(fmaxf(lo[d] - c, c - hi[d]), 0.0f);
-            l = __fmaf_rn(gg, gg, l);
-          }
-        }
-        unsigned m = __ballot_sync(full, l <= thr);
+      for (int g = 0; g < nlist; g += 32) {
+        const int i = g + lane;
+        const bool in = i < nlist && lower_bound<DIM>(csf + list[i] * (4 * CS), lo, hi) <= thr;
+        unsigned m = __ballot_sync(full, in);
         while (m) {
-          const int kk = g + __ffs(m) - 1;
+          const int p = g + __ffs(m) - 1;
           m &= m - 1;
+          const int kk = list[p];
+          const int name = nchunks == 1 ? p : k0 + kk;
           const float4 c = cs[kk * CS];
           const float c4 = DIM == 5 ? cs[kk * CS + (CS - 1)].x : 0.0f;
-          closer<DIM>(f[0], f[1], c, c4, k0 + kk, best[0], best[1], bk[0], bk[1]);
-          closer<DIM>(f[2], f[3], c, c4, k0 + kk, best[2], best[3], bk[2], bk[3]);
+          closer<DIM>(f[0], f[1], c, c4, name, best[0], best[1], bk[0], bk[1]);
+          closer<DIM>(f[2], f[3], c, c4, name, best[2], best[3], bk[2], bk[3]);
         }
       }
     }
+    int lab[kPix];
 #pragma unroll
     for (int j = 0; j < kPix; ++j)
-      if (ok[j]) a.labels[base + 32 * j] = bk[j];
-    if (ACC) {
-      // Features below 2^32 (the common case by far): the narrow fixed-point
-      // form, and where all 128 pixels share one label each lane first adds
-      // its four pixels' words.  Otherwise the general form, pixel by pixel.
-      bool small = true;
+      lab[j] = bk[j] < 0 ? 0 : nchunks == 1 ? (int)list[bk[j]] : bk[j];
+    if (valid == kPix && (W & 3) == 0 && (reinterpret_cast<uintptr_t>(a.labels) & 15) == 0) {
+      *reinterpret_cast<int4*>(a.labels + px0) = make_int4(lab[0], lab[1], lab[2], lab[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kPix; ++j)
+        if (j < valid) a.labels[px0 + j] = lab[j];
+    }
+    if constexpr (ACC) {
+      // Features in [0, 2^14) whose clusters fit the tile's sums (the common
+      // case by far); below 2^32, the narrow fixed-point form straight into
+      // the global sums; otherwise the general form.
+      bool tiled = nchunks == 1 && nlist <= kSlots, small = true;
 #pragma unroll
       for (int j = 0; j < kPix; ++j)
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) small = small && (!ok[j] || fabsf(f[j][d]) < 4294967296.0f);
-      const int b0 = __shfl_sync(full, bk[0], 0);   // every lane, before any branch
-      bool one = ok[kPix - 1];                        // (ok[3] implies ok[0..2])
+        for (int d = 0; d < DIM; ++d) {
+          tiled = tiled && (j >= valid || (f[j][d] >= 0.0f && f[j][d] < 16384.0f));
+          small = small && (j >= valid || fabsf(f[j][d]) < 4294967296.0f);
+        }
+      if (__all_sync(full, tiled)) {
+        int at[kPix];
 #pragma unroll
-      for (int j = 1; j < kPix; ++j) one = one && bk[j] == bk[0];
-      if (__all_sync(full, small)) {
-        if (__all_sync(full, one && bk[0] == b0)) {
+        for (int j = 0; j < kPix; ++j) at[j] = j < valid ? bk[j] : -1;
+        warp_to_tile<LAYOUT, DIM>(sums, f, at);
+      } else if (__all_sync(full, small)) {
+#pragma unroll
+        for (int j = 0; j < kPix; ++j) {
+          const int l = j < valid ? lab[j] : -1;
           long long q[DIM];
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            q[d] = 0;
-#pragma unroll
-            for (int j = 0; j < kPix; ++j) q[d] += __float2ll_rn(__fmul_rn(f[j][d], fix::kScale));
-          }
-          fix::warp_add_narrow<DIM>(b0, q, kPix, a.lo, a.hi, a.cnt);
-        } else {
-#pragma unroll
-          for (int j = 0; j < kPix; ++j) {
-            const int l = ok[j] ? bk[j] : -1;
-            long long q[DIM];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-              q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
-            fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
-          }
+          for (int d = 0; d < DIM; ++d)
+            q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
+          fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < kPix; ++j) {
           unsigned long long qlo[DIM], qhi[DIM];
-          const int l = ok[j] ? bk[j] : -1;
+          const int l = j < valid ? lab[j] : -1;
           fix::quantize<DIM>(f[j], l, a.status, qlo, qhi);
           fix::warp_add<DIM>(l, qlo, qhi, a.lo, a.hi, a.cnt);
         }
       }
+      // the tile's sums into the global ones (a block has few tiles: the list
+      // changes with the tile)
+      __syncthreads();
+      const int used = nchunks == 1 ? min(nlist, kSlots) : 0;
+      for (int i = threadIdx.x; i < used * DIM; i += kThreads) {
+        const unsigned wl = sums.lo[i], wh = sums.hi[i];
+        if ((wl | wh) == 0u) continue;
+        sums.lo[i] = sums.hi[i] = 0u;
+        const size_t s = (size_t)list[i / DIM] * DIM + i % DIM;
+        atomicAdd(a.lo + s, (unsigned long long)wl);
+        if (wh) atomicAdd(a.hi + s, (unsigned long long)wh);
+      }
+      for (int i = threadIdx.x; i < used; i += kThreads) {
+        const unsigned n = sums.cnt[i];
+        if (n == 0u) continue;
+        sums.cnt[i] = 0u;
+        atomicAdd(a.cnt + list[i], n);
+      }
     }
+    __syncthreads();   // the list and the boxes are the next tile's
   }
 }
 
@@ -346,7 +497,7 @@ __global__ void setup_kernel(Layout L, int K, int dim, const float* __restrict__
     s.delta = 0.0f;
     s.iters = 0;
     s.done = max_iter <= 0;
-    s.pad = 0;
+    s.arrived = 0u;
     *L.state = s;
     if (d_iter && max_iter <= 0) *d_iter = 0;
   }
@@ -372,9 +523,12 @@ struct FormArgs {
 };
 
 // Centroids of iteration i from the sums of its assignment, the shift, the
-// decision.  One block: every sum is read once and cleared for the next
-// iteration.  The L2 shift is summed in a fixed order (per-thread strided
-// partials, then a fixed tree), so it does not vary between runs.
+// decision.  Every sum is read once and cleared for the next iteration.  The
+// L2 shift is summed in a fixed order (kFormSlots strided partials, then a
+// fixed tree), so it does not vary between runs.  FP64 runs at two lanes per
+// clock and SM, and the means divide in FP64: one block took 10.4 us for K =
+// 256, so the slots are spread over kFormBlocks blocks and the last to finish
+// measures the shift and decides.
 //
 // With ref_shift the shift is the reference's own measure (cluster.cu:40-50,
 // :73-87): it compares the new planar centroids, entry j = d * K + k, with
@@ -386,8 +540,8 @@ struct FormArgs {
 // and sums (c_new[j] - word[j])^2 in FP32 in j order.
 template <int LAYOUT, int DIM>
 __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
-  __shared__ float part[kFormThreads];
-  __shared__ int stop, more;
+  __shared__ float part[kFormSlots];
+  __shared__ int stop, last, more;
   pdl_wait();
   if (threadIdx.x == 0) stop = __ldcg(&a.L.state->done);
   __syncthreads();
@@ -396,21 +550,31 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
   const int64_t kd = (int64_t)K * DIM;
   const float* c_old = a.L.cur + (size_t)((a.i - 1) & 1) * kd;
   float* c_new = a.L.cur + (size_t)(a.i & 1) * kd;
-  float acc = 0.0f;
-  for (int64_t idx = threadIdx.x; idx < kd; idx += kFormThreads) {
-    const int d = (int)(idx / K), k = (int)(idx - (int64_t)d * K);
-    const float c = c_old[idx];
-    const unsigned n = __ldcg(a.L.cnt + k);
-    const size_t s = (size_t)k * DIM + d;
-    const float cn = n ? fix::mean(__ldcg(a.L.lo + s), __ldcg(a.L.hi + s), n) : c;
-    a.L.lo[s] = 0ull;
-    a.L.hi[s] = 0ull;
-    c_new[idx] = cn;
-    const float df = __fsub_rn(cn, c);
-    acc = __fadd_rn(acc, __fmul_rn(df, df));
+  for (int slot = (int)blockIdx.x + (int)threadIdx.x * kFormBlocks; slot < kFormSlots;
+       slot += kFormBlocks * kFormThreads) {
+    float acc = 0.0f;
+    for (int64_t idx = slot; idx < kd; idx += kFormSlots) {
+      const int d = (int)(idx / K), k = (int)(idx - (int64_t)d * K);
+      const float c = __ldcg(c_old + idx);
+      const unsigned n = __ldcg(a.L.cnt + k);
+      const size_t s = (size_t)k * DIM + d;
+      const float cn = n ? fix::mean(__ldcg(a.L.lo + s), __ldcg(a.L.hi + s), n) : c;
+      a.L.lo[s] = 0ull;
+      a.L.hi[s] = 0ull;
+      __stcg(c_new + idx, cn);
+      const float df = __fsub_rn(cn, c);
+      acc = __fadd_rn(acc, __fmul_rn(df, df));
+    }
+    __stcg(a.L.part + slot, acc);
   }
-  part[threadIdx.x] = acc;
-  __syncthreads();   // every c_new entry written
+  // the block that finishes last has every block's words
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&a.L.state->arrived, 1u) + 1u == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < kFormSlots; i += kFormThreads) part[i] = __ldcg(a.L.part + i);
   if (DIM == 3 && a.ref_shift) {
     const int64_t base = 2 * a.P.n;
     for (int64_t j = threadIdx.x; j < 3 * (int64_t)K; j += kFormThreads) {
@@ -426,18 +590,18 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
         float w = 0.0f;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
-          const float t = __fsub_rn(f[d], c_old[(int64_t)d * K + c]);
+          const float t = __fsub_rn(f[d], __ldcg(c_old + (int64_t)d * K + c));
           w = d == 0 ? __fmul_rn(t, t) : __fadd_rn(w, __fmul_rn(t, t));
         }
         word = w;
       }
-      const float t = __fsub_rn(c_new[j], word);
+      const float t = __fsub_rn(__ldcg(c_new + j), word);
       a.L.word[j] = __fmul_rn(t, t);
     }
   }
   __syncthreads();
-  for (int s = kFormThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) part[threadIdx.x] = __fadd_rn(part[threadIdx.x], part[threadIdx.x + s]);
+  for (int s = kFormSlots / 2; s > 0; s >>= 1) {
+    for (int i = threadIdx.x; i < s; i += kFormThreads) part[i] = __fadd_rn(part[i], part[i + s]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -451,6 +615,7 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
     const bool m = a.i < a.max_iter && fabsf(delta - old_delta) > a.threshold;
     a.L.state->delta = delta;
     a.L.state->iters = a.i;
+    a.L.state->arrived = 0u;
     if (!m) {
       a.L.state->done = 1;
       if (a.d_iter) *a.d_iter = a.i;
@@ -459,7 +624,8 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
   }
   __syncthreads();
   if (!more)
-    for (int64_t idx = threadIdx.x; idx < kd; idx += kFormThreads) a.centroids[idx] = c_new[idx];
+    for (int64_t idx = threadIdx.x; idx < kd; idx += kFormThreads)
+      a.centroids[idx] = __ldcg(c_new + idx);
   for (int k = threadIdx.x; k < K; k += kFormThreads) a.L.cnt[k] = 0u;
 }
 
@@ -475,7 +641,8 @@ static int queue(bool cluster, const Points& P, int K, const float* cent, float*
   auto ak = cluster ? assign_kernel<LAYOUT, DIM, true> : assign_kernel<LAYOUT, DIM, false>;
   SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ak, kThreads, 0));
   if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-  int64_t blocks = (P.n + (int64_t)kThreads * kPix - 1) / ((int64_t)kThreads * kPix);
+  const int64_t rows = (P.n + P.width - 1) / P.width;
+  int64_t blocks = ((P.width + kTileW - 1) / kTileW) * ((rows + kTileH - 1) / kTileH);
   const int64_t cap = (int64_t)di.sm_count * per_sm;
   if (blocks > cap) blocks = cap;
   AssignArgs aa{};
@@ -512,7 +679,7 @@ static int queue(bool cluster, const Points& P, int K, const float* cent, float*
     SG_CUDA_TRY(launch_pdl(ak, dim3((unsigned)blocks), dim3(kThreads), 0, st, aa));
     SG_TRY(launch_status());
     fa.i = i;
-    SG_CUDA_TRY(launch_pdl(form_kernel<LAYOUT, DIM>, dim3(1), dim3(kFormThreads), 0, st, fa));
+    SG_CUDA_TRY(launch_pdl(form_kernel<LAYOUT, DIM>, dim3(kFormBlocks), dim3(kFormThreads), 0, st, fa));
     SG_TRY(launch_status());
   }
   return SPLIT_OK;
