@@ -303,18 +303,20 @@ static_assert((kTile / kWarps) % kBatchRows == 0, "whole batches per warp span")
 // Nearest centroid among `mask` for the lane's pixels; the distance is the
 // fma chain of (x - c)^2 in dimension order, strict < in ascending k (ties to
 // the lowest k; label.cu:23-32, :98-105), evaluated on pixel pairs with the
-// packed f32x2 pipe.
-template <int DIM>
-__device__ __forceinline__ void nearest_px(const float (&f)[kPx][DIM],
+// packed f32x2 pipe.  NB batches share the walk over the mask.
+template <int DIM, int NB>
+__device__ __forceinline__ void nearest_px(const float (&f)[NB][kPx][DIM],
                                            const float* __restrict__ cs,
-                                           unsigned long long mask, int (&lab)[kPx]) {
+                                           unsigned long long mask, int (&lab)[NB][kPx]) {
   constexpr int CS = cstride(DIM);
-  float best[kPx];
+  float best[NB][kPx];
 #pragma unroll
-  for (int j = 0; j < kPx; ++j) {
-    best[j] = INFINITY;
-    lab[j] = 0;
-  }
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < kPx; ++j) {
+      best[i][j] = INFINITY;
+      lab[i][j] = 0;
+    }
   // ascending k over the two 32-bit halves of the mask
   unsigned m = (unsigned)mask, hi = (unsigned)(mask >> 32);
   int base = 0;
@@ -330,24 +332,26 @@ __device__ __forceinline__ void nearest_px(const float (&f)[kPx][DIM],
     const float4 c0 = *reinterpret_cast<const float4*>(cs + k * CS);
     const float cc[5] = {c0.x, c0.y, c0.z, c0.w, DIM == 5 ? cs[k * CS + 4] : 0.0f};
 #pragma unroll
-    for (int q = 0; q < kPx / 2; ++q) {
-      const int a = 2 * q, b = 2 * q + 1;
-      float2 t = fsub2(make_float2(f[a][0], f[b][0]), make_float2(cc[0], cc[0]));
-      float2 d = fmul2(t, t);
+    for (int i = 0; i < NB; ++i)
 #pragma unroll
-      for (int dd = 1; dd < DIM; ++dd) {
-        t = fsub2(make_float2(f[a][dd], f[b][dd]), make_float2(cc[dd], cc[dd]));
-        d = ffma2(t, t, d);
+      for (int q = 0; q < kPx / 2; ++q) {
+        const int a = 2 * q, b = 2 * q + 1;
+        float2 t = fsub2(make_float2(f[i][a][0], f[i][b][0]), make_float2(cc[0], cc[0]));
+        float2 d = fmul2(t, t);
+#pragma unroll
+        for (int dd = 1; dd < DIM; ++dd) {
+          t = fsub2(make_float2(f[i][a][dd], f[i][b][dd]), make_float2(cc[dd], cc[dd]));
+          d = ffma2(t, t, d);
+        }
+        if (d.x < best[i][a]) {
+          best[i][a] = d.x;
+          lab[i][a] = k;
+        }
+        if (d.y < best[i][b]) {
+          best[i][b] = d.y;
+          lab[i][b] = k;
+        }
       }
-      if (d.x < best[a]) {
-        best[a] = d.x;
-        lab[a] = k;
-      }
-      if (d.y < best[b]) {
-        best[b] = d.y;
-        lab[b] = k;
-      }
-    }
   }
 }
 
@@ -796,7 +800,8 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
       // the distances, and the sums from the same differences
       pair_px<DIM>(f, sm.cent, ka, kb, lab, acc, acc_n, acc2, acc2_n);
     } else {
-      nearest_px<DIM>(f, sm.cent, mask, lab);
+      nearest_px<DIM, 1>(reinterpret_cast<const float(&)[1][kPx][DIM]>(f), sm.cent, mask,
+                         reinterpret_cast<int(&)[1][kPx]>(lab));
     }
     if (write_labels) {
       if (vec_labels) {
@@ -989,58 +994,68 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
     return row < im.height ? (int)max((int64_t)0, min((int64_t)min(kPx, im.width - col0 - lcol), left))
                            : 0;
   };
+  // Three-dimensional features: two batches per step share the box, the
+  // candidates and the walk over them, whose latencies (box 0.2 us, candidates
+  // 0.2 us, 0.1 us a candidate) are most of a step; more dimensions do not fit
+  // the registers.  The next step's loads go out before this one is examined.
+  constexpr int NB = DIM == 3 ? 2 : 1;
   const int nb = fast ? 0 : (rows_in + kBatchRows - 1) / kBatchRows;
-  RawPx<LAYOUT, DIM> raw;
-  int valid_next = 0;
-  if (!fast) {
-    valid_next = valid_px(row0 + lrow);
-    raw.load(im.points, im.npoints, (int64_t)(row0 + lrow) * im.width + col0 + lcol, valid_next);
-  }
-  for (int b = 0; b < nb; ++b) {
-    const int row = row0 + b * kBatchRows + lrow;
-    const int col = col0 + lcol;
-    const int valid = valid_next;
-    float f[kPx][DIM];
-    bool ok[kPx];
-    raw.features(im.xy_scale, row, col, f);
+  const int col = col0 + lcol;
+  RawPx<LAYOUT, DIM> raw[NB];
+  int valid_next[NB];
+  auto load = [&](int b) {
 #pragma unroll
-    for (int j = 0; j < kPx; ++j) ok[j] = j < valid;
-    const bool all_ok = valid == kPx;
-    const int64_t px0 = (int64_t)row * im.width + col;
-    if (b + 1 < nb) {   // the next batch's loads go out now
-      valid_next = valid_px(row + kBatchRows);
-      raw.load(im.points, im.npoints, px0 + (int64_t)kBatchRows * im.width, valid_next);
+    for (int i = 0; i < NB; ++i) {
+      const int row = row0 + (b + i) * kBatchRows + lrow;
+      valid_next[i] = b + i < nb ? valid_px(row) : 0;
+      raw[i].load(im.points, im.npoints, (int64_t)row * im.width + col, valid_next[i]);
     }
-    int lab[kPx];
+  };
+  if (!fast) load(0);
+  for (int b = 0; b < nb; b += NB) {
+    float f[NB][kPx][DIM];
+    int valid[NB], lab[NB][kPx];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      valid[i] = valid_next[i];
+      raw[i].features(im.xy_scale, row0 + (b + i) * kBatchRows + lrow, col, f[i]);
+    }
+    if (b + NB < nb) load(b + NB);
     if (MODE == kUpdateOnly) {
-      if (all_ok && vec_labels) {
-        const int4 v = __ldg(reinterpret_cast<const int4*>(im.labels_in + px0));
-        lab[0] = v.x; lab[1] = v.y; lab[2] = v.z; lab[3] = v.w;
-      } else {
 #pragma unroll
-        for (int j = 0; j < kPx; ++j) lab[j] = ok[j] ? __ldg(im.labels_in + px0 + j) : -1;
+      for (int i = 0; i < NB; ++i) {
+        const int64_t px0 = (int64_t)(row0 + (b + i) * kBatchRows + lrow) * im.width + col;
+        if (valid[i] == kPx && vec_labels) {
+          const int4 v = __ldg(reinterpret_cast<const int4*>(im.labels_in + px0));
+          lab[i][0] = v.x; lab[i][1] = v.y; lab[i][2] = v.z; lab[i][3] = v.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < kPx; ++j) lab[i][j] = j < valid[i] ? __ldg(im.labels_in + px0 + j) : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < kPx; ++j)
+          if (j >= valid[i] || lab[i][j] < 0 || lab[i][j] >= im.K) lab[i][j] = -1;
       }
-#pragma unroll
-      for (int j = 0; j < kPx; ++j)
-        if (!ok[j] || lab[j] < 0 || lab[j] >= im.K) lab[j] = -1;
     } else {
       unsigned long long mask = span_mask;
       if (!unit_box) {
-        // Box of the batch.  fminf / fmaxf skip NaN: a NaN pixel gets label
-        // 0 whatever the mask (every distance compares false), and the box
-        // still bounds all other pixels.
+        // Box of the step's pixels.  fminf / fmaxf skip NaN: a NaN pixel gets
+        // label 0 whatever the mask (every distance compares false), and the
+        // box still bounds all other pixels.
         float lo[DIM], hi[DIM];
         constexpr int kBoxDims = kXY ? 3 : DIM;
 #pragma unroll
         for (int d = 0; d < kBoxDims; ++d) {
           float a = INFINITY, z = -INFINITY;
 #pragma unroll
-          for (int j = 0; j < kPx; ++j) {
-            if (ok[j]) {
-              a = fminf(a, f[j][d]);
-              z = fmaxf(z, f[j][d]);
+          for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int j = 0; j < kPx; ++j) {
+              if (j < valid[i]) {
+                a = fminf(a, f[i][j][d]);
+                z = fmaxf(z, f[i][j][d]);
+              }
             }
-          }
           lo[d] = fkey_inv(__reduce_min_sync(full, fkey(a)));
           hi[d] = fkey_inv(__reduce_max_sync(full, fkey(z)));
         }
@@ -1049,7 +1064,7 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
           lo[3] = __fmul_rn(im.xy_scale, (float)col0);
           hi[3] = __fmul_rn(im.xy_scale, (float)(col0 + cols_in - 1));
           lo[4] = __fmul_rn(im.xy_scale, (float)r0);
-          hi[4] = __fmul_rn(im.xy_scale, (float)min(r0 + kBatchRows - 1, im.height - 1));
+          hi[4] = __fmul_rn(im.xy_scale, (float)min(r0 + NB * kBatchRows - 1, im.height - 1));
         }
         mask = candidates<DIM>(lo, hi, sm.cent, im.K);
       }
@@ -1058,26 +1073,34 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
         // the unit cube: none is NaN), as on the fast path
         const int k1 = __ffsll((long long)mask) - 1;
 #pragma unroll
-        for (int j = 0; j < kPx; ++j) lab[j] = k1;
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+          for (int j = 0; j < kPx; ++j) lab[i][j] = k1;
       } else {
-        nearest_px<DIM>(f, sm.cent, mask, lab);
+        nearest_px<DIM, NB>(f, sm.cent, mask, lab);
       }
-      if (write_labels) {
-        if (all_ok && vec_labels) {
-          *reinterpret_cast<int4*>(im.labels + px0) = make_int4(lab[0], lab[1], lab[2], lab[3]);
-        } else {
 #pragma unroll
-          for (int j = 0; j < kPx; ++j)
-            if (ok[j]) im.labels[px0 + j] = lab[j];
+      for (int i = 0; i < NB; ++i) {
+        const int64_t px0 = (int64_t)(row0 + (b + i) * kBatchRows + lrow) * im.width + col;
+        if (write_labels) {
+          if (valid[i] == kPx && vec_labels) {
+            *reinterpret_cast<int4*>(im.labels + px0) =
+                make_int4(lab[i][0], lab[i][1], lab[i][2], lab[i][3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < kPx; ++j)
+              if (j < valid[i]) im.labels[px0 + j] = lab[i][j];
+          }
         }
-      }
 #pragma unroll
-      for (int j = 0; j < kPx; ++j)
-        if (!ok[j]) lab[j] = -1;
+        for (int j = 0; j < kPx; ++j)
+          if (j >= valid[i]) lab[i][j] = -1;
+      }
     }
     if (MODE == kAssignOnly) continue;
-
-    accumulate<DIM>(sm, warp, im.K, f, lab, acc_l, acc_n, acc);
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      accumulate<DIM>(sm, warp, im.K, f[i], lab[i], acc_l, acc_n, acc);
   }
   if (MODE != kAssignOnly && !direct) {
     if (acc_l >= 0) flush_acc<DIM>(sm, warp, acc_l, acc, acc_n);
