@@ -19,10 +19,13 @@
 // thrust::less, a predicate, as the reduction), so the stated intent above
 // is what this restates.
 //
-// Pair statistics live in an open-addressing table (key (s, t), edge count,
-// 96-bit fixed-point sum of the edge norms at scale 2^32), so the means do
-// not depend on the order edges are added in.  Bids are one 64-bit atomicMax
-// per pair on ~((bits(mean) << 32) | t).
+// An edge and its reverse have the same norm, so a pair's statistics are those
+// of its reverse: the table holds unordered pairs (s < t), filled from four of
+// the eight neighbours, and every entry bids for both segments.  The table is
+// open-addressing (key, edge count, 96-bit fixed-point sum of the edge norms
+// at scale 2^32), so the means do not depend on the order edges are added in.
+// Bids are one 64-bit atomicMax per segment and pair on
+// ~((bits(mean) << 32) | t).
 #include "geom.cuh"
 
 namespace sg {
@@ -32,25 +35,30 @@ constexpr int kThreads = 256;
 constexpr int kProbeCap = 1 << 16;
 constexpr unsigned kChainCap = 1u << 24;
 
+// One pair of segments.
+struct Slot {
+  unsigned long long key;       // 0: free
+  unsigned long long lo, hi;    // sums of the norms' low and high 32-bit words
+  unsigned count;
+  unsigned pad;
+};
+
 struct Layout {
   WsHeader* hdr;
   unsigned* maxsq;              // bits of the largest |x|^2 (non-negative float)
   unsigned* list_count;
+  unsigned* call;               // the call's number: marks this call's entries of fin
   unsigned long long* best;     // [n] winning bid per segment, 0 = none
-  int32_t* map;                 // [n]
-  int32_t* fin;                 // [n]
-  unsigned long long* keys;     // [cap]
-  unsigned* counts;             // [cap]
-  unsigned long long* dlo;      // [cap] low 32-bit words of the norm sums
-  unsigned long long* dhi;      // [cap] high words
+  unsigned long long* fin;      // [n] (call number, final label)
+  Slot* slots;                  // [cap]
   int32_t* list;                // [cap] claimed slots
   int cap_log2;
   size_t bytes;
 };
 
 inline int cap_log2_for(int64_t n) {
-  int l = 12;
-  while ((1ll << l) < 2 * n && l < 31) ++l;
+  int l = 11;
+  while ((1ll << l) < n && l < 30) ++l;
   return l;
 }
 
@@ -58,51 +66,48 @@ inline Layout carve(void* ws, int64_t n) {
   Carver c(ws);
   Layout l;
   l.hdr = c.take<WsHeader>(1);
-  l.maxsq = c.take<unsigned>(1);
-  l.list_count = c.take<unsigned>(1);
+  l.maxsq = l.hdr ? l.hdr->work_counter : nullptr;
+  l.list_count = l.hdr ? l.hdr->work_counter + 1 : nullptr;
+  l.call = l.hdr ? reinterpret_cast<unsigned*>(l.hdr->pad) : nullptr;
   l.best = c.take<unsigned long long>((size_t)n);
-  l.map = c.take<int32_t>((size_t)n);
-  l.fin = c.take<int32_t>((size_t)n);
+  l.fin = c.take<unsigned long long>((size_t)n);
   l.cap_log2 = cap_log2_for(n);
   const size_t cap = (size_t)1 << l.cap_log2;
-  l.keys = c.take<unsigned long long>(cap);
-  l.counts = c.take<unsigned>(cap);
-  l.dlo = c.take<unsigned long long>(cap);
-  l.dhi = c.take<unsigned long long>(cap);
+  l.slots = c.take<Slot>(cap);
   l.list = c.take<int32_t>(cap);
   l.bytes = c.size();
   return l;
 }
 
 __device__ __forceinline__ unsigned long long pair_key(int s, int t) {
-  return (((unsigned long long)(unsigned)s << 32) | (unsigned)t) + 1ull;
+  return ((unsigned long long)(unsigned)min(s, t) << 32) | (unsigned)max(s, t);
 }
-__device__ __forceinline__ int key_s(unsigned long long k) { return (int)((k - 1ull) >> 32); }
-__device__ __forceinline__ int key_t(unsigned long long k) {
-  return (int)(unsigned)((k - 1ull) & 0xffffffffull);
+__device__ __forceinline__ int key_s(unsigned long long k) { return (int)(k >> 32); }
+__device__ __forceinline__ int key_t(unsigned long long k) { return (int)(unsigned)k; }
+__device__ __forceinline__ unsigned key_hash(unsigned long long key, int bits) {
+  return (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - bits));
 }
 
-// |x_p - x_q| over feature rows 0..2, the sum of squares in row order
-__device__ __forceinline__ float edge_norm(const float* pts, long long n, long long p,
-                                           long long q) {
+// |p - q| over feature rows 0..2, the sum of squares in row order
+__device__ __forceinline__ float edge_norm(const float (&p)[3], const float (&q)[3]) {
   float s = 0.0f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float v = __fsub_rn(__ldg(pts + d * n + p), __ldg(pts + d * n + q));
+    const float v = __fsub_rn(p[d], q[d]);
     s = __fadd_rn(s, __fmul_rn(v, v));
   }
   return __fsqrt_rn(s);
 }
 
-__device__ void insert(const Layout& L, int s, int t, unsigned m, unsigned long long lo,
+__device__ void insert(const Layout& L, unsigned long long key, unsigned m, unsigned long long lo,
                        unsigned long long hi, int* status) {
-  const unsigned long long key = pair_key(s, t);
   const unsigned mask = (1u << L.cap_log2) - 1u;
-  unsigned h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - L.cap_log2));
+  unsigned h = key_hash(key, L.cap_log2);
   for (int probe = 0; probe < kProbeCap; ++probe, h = (h + 1) & mask) {
-    unsigned long long k = *(volatile unsigned long long*)(L.keys + h);
+    Slot* const e = L.slots + h;
+    unsigned long long k = *(volatile unsigned long long*)&e->key;
     if (k == 0ull) {
-      k = atomicCAS(L.keys + h, 0ull, key);
+      k = atomicCAS(&e->key, 0ull, key);
       if (k == 0ull) {
         const unsigned idx = atomicAdd(L.list_count, 1u);
         L.list[idx] = (int)h;
@@ -110,204 +115,272 @@ __device__ void insert(const Layout& L, int s, int t, unsigned m, unsigned long 
       }
     }
     if (k == key) {
-      atomicAdd(L.counts + h, m);
-      atomicAdd(L.dlo + h, lo);
-      atomicAdd(L.dhi + h, hi);
+      atomicAdd(&e->count, m);
+      atomicAdd(&e->lo, lo);
+      if (hi) atomicAdd(&e->hi, hi);
       return;
     }
   }
   set_status(status, SPLIT_ERR_OVERFLOW);
 }
 
-__global__ void __launch_bounds__(kThreads)
-maxnorm_kernel(const float* __restrict__ pts, long long n, Layout L) {
-  unsigned best = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float v = __ldg(pts + d * n + i);
-      s = __fadd_rn(s, __fmul_rn(v, v));
-    }
-    // non-negative floats order like their bit patterns (NaN is skipped)
-    if (s >= 0.0f) best = max(best, __float_as_uint(s));
-  }
-  best = __reduce_max_sync(0xffffffffu, best);
-  if ((threadIdx.x & 31) == 0) atomicMax(L.maxsq, best);
-}
+// One block per 32 x 64 tile: the largest feature norm, and the statistics of
+// the tile's boundary edges (to the east, south-west, south and south-east).
+//
+// Bound by the reads of the features when few pixels lie on a boundary and by
+// the latency of the edges otherwise.  The features are read once for the
+// norm; the pixels that have an edge go to a list, which the block then walks
+// densely, so that a boundary's loads overlap instead of following each other
+// down the columns of one warp; the edges of a pair meet in a shared-memory
+// table and reach the global one as one entry per tile and pair.  The norms'
+// 62-bit values are added as four 16-bit pieces: a tile has at most 2^13
+// edges, so a piece's sum stays below 2^29.  A pair that the tile's table has
+// no room for within a short probe goes to the global one directly.
+constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 1;
+constexpr int kPairBits = 9, kPairs = 1 << kPairBits, kPairProbes = 16;
+constexpr int kTilePx = kTileH * kTileW;
+static_assert(kTilePx <= 1 << 11 && kThreads % kTileW == 0, "list entries; pixels per thread");
 
-// one block per 32 x 64 tile: every pixel adds its out-going boundary edges,
-// aggregated per distinct neighbour label
 __global__ void __launch_bounds__(kThreads)
 edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geoms gs, Layout L,
             int* status) {
+  __shared__ int tile[kHaloH * kHaloW];
+  __shared__ unsigned long long key[kPairs];
+  __shared__ unsigned count[kPairs], piece[4][kPairs];
+  __shared__ unsigned short todo[kTilePx];   // local pixel, then its edges in 4 bits
+  __shared__ unsigned ntodo, maxsq;
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, blockIdx.x);
   const int W = tr.W, H = tr.H;
-  for (int q = threadIdx.x; q < kTileH * kTileW; q += blockDim.x) {
-    const int x = tr.tx0 + q % kTileW, y = tr.ty0 + q / kTileW;
-    if (x >= W || y >= H) continue;
-    const long long i = tr.off + (long long)y * W + x;
-    const int s = __ldg(lab + i);
-    if (s < 0 || s >= n) {
-      set_status(status, SPLIT_ERR_INVALID);
-      continue;
-    }
-    int t[8];
-    long long j[8];
-    int nt = 0;
-#pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const int dx = (d == 0 || d == 3 || d == 5) ? -1 : (d == 2 || d == 4 || d == 7) ? 1 : 0;
-      const int dy = d < 3 ? -1 : d > 4 ? 1 : 0;
-      const int nx = x + dx, ny = y + dy;
-      if (nx < 0 || ny < 0 || nx >= W || ny >= H) continue;
-      const long long k = tr.off + (long long)ny * W + nx;
-      const int v = __ldg(lab + k);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *L.call += 1u;
+  if (threadIdx.x == 0) ntodo = maxsq = 0u;
+  // -1: outside the image, or no label
+  bool bad = false;
+  for (int q = threadIdx.x; q < kHaloH * kHaloW; q += kThreads) {
+    const int x = tr.tx0 - 1 + q % kHaloW, y = tr.ty0 + q / kHaloW;
+    int v = -1;
+    if (x >= 0 && x < W && y < H) {
+      v = __ldg(lab + tr.off + (long long)y * W + x);
       if (v < 0 || v >= n) {
-        set_status(status, SPLIT_ERR_INVALID);
-        continue;
-      }
-      if (v != s) {
-        t[nt] = v;
-        j[nt] = k;
-        ++nt;
+        bad = true;
+        v = -1;
       }
     }
-    for (int a = 0; a < nt; ++a) {
-      bool first = true;
-      for (int b = 0; b < a; ++b) first &= (t[b] != t[a]);
-      if (!first) continue;
-      unsigned m = 0;
-      unsigned long long slo = 0, shi = 0;
-      for (int b = a; b < nt; ++b) {
-        if (t[b] != t[a]) continue;
-        ++m;
-        const float e = edge_norm(pts, n, i, j[b]);
-        if (!(e < 1073741824.0f)) set_status(status, SPLIT_ERR_OVERFLOW);   // 2^30, or NaN
-        const long long q = __float2ll_rn(__fmul_rn(e, 4294967296.0f));
-        slo += (unsigned long long)q & 0xffffffffull;
-        shi += (unsigned long long)(q >> 32);
+    tile[q] = v;
+  }
+  if (bad) set_status(status, SPLIT_ERR_INVALID);
+  for (int i = threadIdx.x; i < kPairs; i += kThreads) {
+    key[i] = 0ull;
+    count[i] = piece[0][i] = piece[1][i] = piece[2][i] = piece[3][i] = 0u;
+  }
+  __syncthreads();
+  const int lx = threadIdx.x % kTileW, ly0 = threadIdx.x / kTileW;
+  unsigned largest = 0u;
+#pragma unroll
+  for (int r = 0; r < kTileH; r += kThreads / kTileW) {
+    const int ly = ly0 + r;
+    const int* c = tile + ly * kHaloW + lx + 1;
+    const int v = c[0];
+    if (tr.tx0 + lx < W && tr.ty0 + ly < H) {
+      const long long i = tr.off + (long long)(tr.ty0 + ly) * W + tr.tx0 + lx;
+      float s = 0.0f;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float f = __ldg(pts + d * n + i);
+        s = __fadd_rn(s, __fmul_rn(f, f));
       }
-      insert(L, s, t[a], m, slo, shi, status);
+      // non-negative floats order like their bit patterns (NaN is skipped)
+      if (s >= 0.0f) largest = max(largest, __float_as_uint(s));
+    }
+    const int e = c[1], sw = c[kHaloW - 1], so = c[kHaloW], se = c[kHaloW + 1];
+    unsigned m = 0u;
+    if (v >= 0)
+      m = (e >= 0 && e != v ? 1u : 0u) | (sw >= 0 && sw != v ? 2u : 0u) |
+          (so >= 0 && so != v ? 4u : 0u) | (se >= 0 && se != v ? 8u : 0u);
+    const unsigned any = __ballot_sync(0xffffffffu, m != 0u);
+    if (any) {
+      const int lane = threadIdx.x & 31;
+      unsigned at = lane == 0 ? atomicAdd(&ntodo, (unsigned)__popc(any)) : 0u;
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(any & ((1u << lane) - 1u));
+      if (m) todo[at] = (unsigned short)((ly * kTileW + lx) << 4 | m);
     }
   }
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  if ((threadIdx.x & 31) == 0) atomicMax(&maxsq, largest);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(L.maxsq, maxsq);
+  const unsigned nt = ntodo;
+  if (nt == 0u) return;
+  for (unsigned q = threadIdx.x; q < nt; q += kThreads) {
+    const unsigned item = todo[q], m = item & 15u, px = item >> 4;
+    const int* c = tile + (px / kTileW) * kHaloW + px % kTileW + 1;
+    const int v = c[0];
+    const long long i =
+        tr.off + (long long)(tr.ty0 + (int)(px / kTileW)) * W + tr.tx0 + (int)(px % kTileW);
+    const int t[4] = {c[1], c[kHaloW - 1], c[kHaloW], c[kHaloW + 1]};
+    const long long j[4] = {i + 1, i + W - 1, i + W, i + W + 1};
+    float f[3], g[4][3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      f[d] = __ldg(pts + d * n + i);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) g[k][d] = m >> k & 1u ? __ldg(pts + d * n + j[k]) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!(m >> k & 1u)) continue;
+      const float e = edge_norm(f, g[k]);
+      const bool large = !(e < 1073741824.0f);   // 2^30, or NaN
+      if (large) set_status(status, SPLIT_ERR_OVERFLOW);
+      const long long w = __float2ll_rn(__fmul_rn(e, 4294967296.0f));
+      const unsigned long long kk = pair_key(v, t[k]);
+      unsigned h = key_hash(kk, kPairBits);
+      bool in = false;
+      for (int probe = large ? kPairProbes : 0; probe < kPairProbes;
+           ++probe, h = (h + 1) & (kPairs - 1)) {
+        unsigned long long o = *(volatile unsigned long long*)&key[h];
+        if (o == 0ull) o = atomicCAS(&key[h], 0ull, kk);
+        in = o == 0ull || o == kk;
+        if (in) break;
+      }
+      if (!in) {
+        insert(L, kk, 1u, (unsigned long long)w & 0xffffffffull, (unsigned long long)(w >> 32),
+               status);
+        continue;
+      }
+      atomicAdd(&count[h], 1u);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const unsigned p = (unsigned)(w >> (16 * a)) & 0xffffu;
+        if (p) atomicAdd(&piece[a][h], p);
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kPairs; i += kThreads)
+    if (key[i])
+      insert(L, key[i], count[i], piece[0][i] + ((unsigned long long)piece[1][i] << 16),
+             piece[2][i] + ((unsigned long long)piece[3][i] << 16), status);
 }
 
 // mean edge norm of a slot, rounded to FP32 (the reference keeps it as real);
 // edge norms are below 2^30, so the high words sum to below 2^62
-__device__ __forceinline__ float slot_mean(const Layout& L, int h) {
-  const double hi = (double)(long long)L.dhi[h];
-  const double lo = (double)L.dlo[h];
+__device__ __forceinline__ float slot_mean(const Slot& e) {
+  const double hi = (double)(long long)e.hi;
+  const double lo = (double)e.lo;
   const double S = __dadd_rn(__dmul_rn(hi, 4294967296.0), lo);
-  return __double2float_rn(__ddiv_rn(__dmul_rn(S, 1.0 / 4294967296.0), (double)L.counts[h]));
+  return __double2float_rn(__ddiv_rn(__dmul_rn(S, 1.0 / 4294967296.0), (double)e.count));
 }
 
 __device__ void bid_phase(const Layout& L, float threshold) {
   const unsigned cnt = *(volatile unsigned*)L.list_count;
   const float D = __fmul_rn(threshold, __fsqrt_rn(__uint_as_float(*(volatile unsigned*)L.maxsq)));
   for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const int h = L.list[j];
-    const unsigned long long k = L.keys[h];
-    const int s = key_s(k), t = key_t(k);
-    const float d = slot_mean(L, h);
-    if (!(d < D) || L.counts[h] <= 15u) continue;
-    atomicMax(L.best + s, ~(((unsigned long long)__float_as_uint(d) << 32) | (unsigned)t));
+    const Slot e = L.slots[L.list[j]];
+    const int s = key_s(e.key), t = key_t(e.key);
+    if (e.count <= 15u) continue;
+    const float d = slot_mean(e);
+    if (!(d < D)) continue;
+    const unsigned long long mean = (unsigned long long)__float_as_uint(d) << 32;
+    atomicMax(L.best + s, ~(mean | (unsigned)t));
+    atomicMax(L.best + t, ~(mean | (unsigned)s));
   }
 }
 
+// the winning bid of segment r after the bids are in
+__device__ __forceinline__ unsigned long long bid_of(const Layout& L, int r) {
+  return *(volatile unsigned long long*)(L.best + r);
+}
 __device__ __forceinline__ int bid_target(unsigned long long b) {
   return (int)(unsigned)((~b) & 0xffffffffull);
 }
 
-__device__ void decide_phase(const Layout& L) {
-  const unsigned cnt = *(volatile unsigned*)L.list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    const unsigned long long b = L.best[s];
-    if (b && bid_target(b) == t) L.map[s] = t;
+// The segment that r maps to: its bid's target; r itself without a bid, and
+// the larger id of a pair that bid for each other.
+__device__ __forceinline__ int next_of(const Layout& L, int r) {
+  const unsigned long long b = bid_of(L, r);
+  if (b == 0ull) return r;
+  const int t = bid_target(b);
+  if (r > t) {
+    const unsigned long long back = bid_of(L, t);
+    if (back != 0ull && bid_target(back) == r) return r;
   }
+  return t;
 }
 
-__device__ __forceinline__ int next_of(const Layout& L, int n, int r) {
-  if (*(volatile unsigned long long*)(L.best + r) == 0ull) return r;
-  const int nx = *(volatile int*)(L.map + r);
-  if (nx < 0 || nx >= n) {
-    set_status(&L.hdr->status, SPLIT_ERR_INVALID);
-    return r;
-  }
-  return nx;
-}
-
-// mutual pairs: the larger id keeps itself
-__device__ void cycle_phase(const Layout& L, int n) {
-  const unsigned cnt = *(volatile unsigned*)L.list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    const unsigned long long b = L.best[s];
-    if (!b || bid_target(b) != t) continue;
-    if (next_of(L, n, t) == s && s > t) *(volatile int*)(L.map + s) = s;
-  }
-}
-
-__device__ void resolve_phase(const Layout& L, int n) {
-  const unsigned cnt = *(volatile unsigned*)L.list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const unsigned long long k = L.keys[L.list[j]];
-    const int s = key_s(k), t = key_t(k);
-    const unsigned long long b = L.best[s];
-    if (!b || bid_target(b) != t) continue;
-    int r = s;
-    for (unsigned steps = 0;; ++steps) {
-      const int nx = next_of(L, n, r);
-      if (nx == r) break;
-      r = nx;
-      if (steps > kChainCap) {
-        set_status(&L.hdr->status, SPLIT_ERR_NOT_CONVERGED);
-        break;
-      }
+// The end of s's chain, for a segment that has a bid; one of its pairs, the
+// one it bid for, does it.
+__device__ __forceinline__ void resolve(const Layout& L, int s, int t, unsigned long long call) {
+  const unsigned long long b = bid_of(L, s);
+  if (!b || bid_target(b) != t) return;
+  int r = s;
+  for (unsigned steps = 0;; ++steps) {
+    const int nx = next_of(L, r);
+    if (nx == r) break;
+    r = nx;
+    if (steps > kChainCap) {
+      set_status(&L.hdr->status, SPLIT_ERR_NOT_CONVERGED);
+      break;
     }
-    L.fin[s] = r;
   }
+  L.fin[s] = call << 32 | (unsigned)r;
 }
 
-// The decision over the (segment, neighbour) list, one cooperative launch (one
-// block per SM): bids, decisions, mutual-pair fix, chains, each phase behind a
-// bounded grid barrier.
-__global__ void __launch_bounds__(kThreads) list_kernel(Layout L, float threshold, int n) {
+// The decision over the pairs, one cooperative launch (one block per SM): the
+// bids, a bounded grid barrier, then every segment's chain.  The fix of mutual
+// pairs needs both bids and nothing else, so the chain reads it off the bids
+// as it goes: no phase writes maps first, and two barriers of 1.5 us each are
+// not needed.
+__global__ void __launch_bounds__(kThreads) list_kernel(Layout L, float threshold) {
   bid_phase(L, threshold);
   if (!grid_barrier(L.hdr)) return;
-  decide_phase(L);
-  if (!grid_barrier(L.hdr)) return;
-  cycle_phase(L, n);
-  if (!grid_barrier(L.hdr)) return;
-  resolve_phase(L, n);
-}
-
-__global__ void __launch_bounds__(kThreads)
-relabel_kernel(int32_t* __restrict__ lab, long long n, Layout L) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int v = lab[i];
-    if (v < 0 || v >= n) continue;
-    if (L.best[v]) lab[i] = L.fin[v];
+  const unsigned cnt = *(volatile unsigned*)L.list_count;
+  const unsigned long long call = *L.call;
+  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
+    const unsigned long long k = L.slots[L.list[j]].key;
+    resolve(L, key_s(k), key_t(k), call);
+    resolve(L, key_t(k), key_s(k), call);
   }
 }
 
-// table slots and bids back to zero for the next call
-__global__ void cleanup_kernel(Layout L) {
-  const unsigned cnt = *(volatile unsigned*)L.list_count;
-  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
-    const int h = L.list[j];
-    const int s = key_s(L.keys[h]);
-    L.best[s] = 0ull;
-    L.keys[h] = 0ull;
-    L.counts[h] = 0u;
-    L.dlo[h] = 0ull;
-    L.dhi[h] = 0ull;
+__device__ __forceinline__ int final_of(const Layout& L, unsigned n, unsigned call, int v) {
+  if ((unsigned)v >= n) return v;
+  const unsigned long long f = __ldg(L.fin + v);
+  return (unsigned)(f >> 32) == call ? (int)(unsigned)f : v;
+}
+
+// Final labels, four pixels per thread where the address allows it (equal
+// neighbours share one look-up), and the slots and bids of the call back to
+// zero for the next.  The look-up needs one word: an entry of fin counts when
+// it carries the call's number, so fin is never cleared.
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads)
+relabel_kernel(int32_t* __restrict__ lab, long long n, Layout L) {
+  pdl_wait();
+  const unsigned call = *L.call, cnt = *L.list_count;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned un = (unsigned)n;
+  long long i = first;
+  if (VEC) {
+    for (; i < n / 4; i += step) {
+      const int4 v = reinterpret_cast<const int4*>(lab)[i];
+      int4 r;
+      r.x = final_of(L, un, call, v.x);
+      r.y = v.y == v.x ? r.x : final_of(L, un, call, v.y);
+      r.z = v.z == v.y ? r.y : final_of(L, un, call, v.z);
+      r.w = v.w == v.z ? r.z : final_of(L, un, call, v.w);
+      if (r.x != v.x || r.y != v.y || r.z != v.z || r.w != v.w)
+        reinterpret_cast<int4*>(lab)[i] = r;
+    }
+    i = n / 4 * 4 + first;
+  }
+  for (; i < n; i += step) lab[i] = final_of(L, un, call, lab[i]);
+  for (long long j = first; j < cnt; j += step) {
+    Slot* const e = L.slots + L.list[j];
+    L.best[key_s(e->key)] = 0ull;
+    L.best[key_t(e->key)] = 0ull;
+    *e = Slot{};
   }
 }
 
@@ -333,37 +406,32 @@ extern "C" int split_merge_smooth(int32_t* labels, int width, int height, const 
     return SPLIT_ERR_WORKSPACE;
   l = carve(workspace, n);
   cudaStream_t st = as_stream(stream);
-  // header words after the status, the norm maximum and the slot counter
-  // start at zero; the table and the bids are kept clean by cleanup_kernel
-  // (a fresh workspace is zero-filled by its owner)
-  SG_CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(l.hdr) + sizeof(int), 0,
-                              reinterpret_cast<char*>(l.best) -
-                                  reinterpret_cast<char*>(l.hdr) - sizeof(int), st));
+  // the barrier words, the norm maximum and the slot counter start at zero;
+  // the table and the bids are kept clean by relabel_kernel (a fresh workspace
+  // is zero-filled by its owner)
+  SG_CUDA_TRY(cudaMemsetAsync(&l.hdr->barrier_count, 0, 4 * sizeof(unsigned), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
   const Geoms gs = single_geom(width, height);
-  int64_t blocks = (n + kThreads - 1) / kThreads;
-  const int64_t cap = (int64_t)di.sm_count * 8;
-  if (blocks > cap) blocks = cap;
-  maxnorm_kernel<<<(int)blocks, kThreads, 0, st>>>(points, n, l);
-  SG_TRY(launch_status());
   edge_kernel<<<gs.total_tiles, kThreads, 0, st>>>(labels, points, gs, l, &l.hdr->status);
   SG_TRY(launch_status());
-  const int grid = di.sm_count * 4;
   {
     // one co-resident block per SM; the header clear above zeroed the barrier
     int per_sm = 0;
     SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, list_kernel, kThreads, 0));
     if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
     float thr = threshold;
-    int n32 = (int)n;
-    void* args[] = {&l, &thr, &n32};
+    void* args[] = {&l, &thr};
     SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)list_kernel, dim3(di.sm_count),
                                             dim3(kThreads), args, 0, st));
   }
   SG_TRY(launch_status());
-  relabel_kernel<<<(int)blocks, kThreads, 0, st>>>(labels, n, l);
-  SG_TRY(launch_status());
-  cleanup_kernel<<<grid, kThreads, 0, st>>>(l);
+  const bool vec = (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
+  const int64_t items = vec ? (n + 3) / 4 : n;
+  int64_t blocks = (items + kThreads - 1) / kThreads;
+  const int64_t cap = (int64_t)di.sm_count * 8;
+  if (blocks > cap) blocks = cap;
+  launch_pdl(vec ? relabel_kernel<true> : relabel_kernel<false>, dim3((unsigned)blocks),
+             dim3(kThreads), 0, st, labels, (long long)n, l);
   return launch_status();
 }
