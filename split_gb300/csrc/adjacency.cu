@@ -12,16 +12,16 @@
 //     those edges, sorted by key then value (:279-284), without repeats
 //     (:286).
 //
-// No N x 16 edge array and no comparison sort: the edges are written by an
-// order-preserving compaction (per-block counts, one scan, a write pass that
-// recomputes each item's outputs).  The pairs need no order before the sort,
-// and a boundary repeats its pair at every pixel: each tile keeps its distinct
-// pairs in a shared-memory set and appends those (a 1080p labelling of 400
-// segments and 4000 single pixels: about 20 thousand keys to sort for 0.9
-// million edges).  The keys, 64 bits, are sorted by a stable LSD radix sort
-// (8-bit digits; a digit equal in every key is skipped), after which the
-// compaction keeps the first pair of every run of equal pairs.  Counts come
-// back through device words.
+// No N x 16 edge array and no comparison sort of the edges: the edges are
+// written by an order-preserving compaction (per-block counts, one scan, a
+// write pass that recomputes each item's outputs).  The pairs need no order
+// before the sort, and a boundary repeats its pair at every pixel: each tile
+// keeps its distinct pairs in a shared-memory set and appends those (a 1080p
+// labelling of 400 segments and 4000 single pixels: about 20 thousand keys to
+// sort for 0.9 million edges).  One cooperative launch sorts the keys, 64 bits,
+// and keeps one of each: a few by their ranks in sorted tiles, more by a stable
+// LSD radix sort (8-bit digits; a digit equal in every key is skipped).
+// Counts come back through device words.
 #include <algorithm>
 
 #include "common.cuh"
@@ -37,15 +37,14 @@ constexpr int kScanThreads = 1024;
 // 16 n edge words must stay addressable with int32 (as in the reference)
 constexpr int64_t kMaxPixels = (1ll << 27) - 1;
 
-enum Mode { kEdges = 0, kUnique = 1 };
-
 struct Layout {
   WsHeader* hdr;
   int* block_sum;                   // [blocks + 1]: per-block counts, then their prefix
   int* total;                       // [2]: keys to sort
   unsigned long long* bits;         // [2]: OR and AND of every pair key
-  unsigned long long* keys[2];      // [8 n] each: pair keys, sort ping-pong
-  unsigned* hist;                   // [256 * sort blocks]: digit counts, then offsets
+  unsigned long long* keys[2];      // [8 n] each, whole rank tiles: pair keys, sort ping-pong
+  unsigned* hist;                   // [256 * sort blocks + 256]: digit counts, then offsets;
+                                    // the digits' totals
   size_t bytes;
 };
 
@@ -53,16 +52,11 @@ __host__ __device__ inline int blocks_of(int64_t items) {
   return (int)((items + kTile - 1) / kTile);
 }
 
-// The sort's tiles: up to kFewKeys keys (most labellings) 512, so that the
-// passes spread over many blocks with two rounds each; more keys 4096, so that
-// the one-block scan of the digit counts stays short.  20 thousand keys: a
-// pass 28 us in tiles of 4096, 17 us in tiles of 512.
-constexpr int64_t kFewKeys = 1 << 18;
-__host__ __device__ inline int sort_rounds(int64_t keys) { return keys <= kFewKeys ? 2 : kItems; }
-__host__ __device__ inline int sort_tiles(int64_t keys) {
-  const int64_t tile = (int64_t)sort_rounds(keys) * kThreads;
-  return (int)((keys + tile - 1) / tile);
-}
+// Up to kFewKeys keys are ranked, more are sorted by digits.  Ranking costs
+// every key a search in every tile of kRankTile keys and three barriers; a
+// digit pass three barriers and two passes over the keys, six to eight times.
+constexpr int64_t kFewKeys = 1 << 17;
+constexpr int kRankBits = 10, kRankTile = 1 << kRankBits;
 
 static Layout carve(void* ws, int64_t n, bool pairs) {
   Carver c(ws);
@@ -73,10 +67,10 @@ static Layout carve(void* ws, int64_t n, bool pairs) {
   l.total = c.take<int>(2);
   l.bits = c.take<unsigned long long>(2);
   if (pairs) {
-    l.keys[0] = c.take<unsigned long long>((size_t)(8 * n));
-    l.keys[1] = c.take<unsigned long long>((size_t)(8 * n));
-    l.hist = c.take<unsigned>((size_t)256 * std::max(sort_tiles(8 * n),
-                                                     sort_tiles(std::min(8 * n, kFewKeys))));
+    const size_t cap = (size_t)((8 * n + kRankTile - 1) / kRankTile * kRankTile);
+    l.keys[0] = c.take<unsigned long long>(cap);
+    l.keys[1] = c.take<unsigned long long>(cap);
+    l.hist = c.take<unsigned>((size_t)256 * blocks_of(8 * n) + 256);
   }
   l.bytes = c.size();
   return l;
@@ -109,169 +103,120 @@ __device__ __forceinline__ int pass_parity(const unsigned long long* bits, int p
   return q & 1;
 }
 
-struct Items {
-  const int32_t* labels;   // kEdges
-  int w, h;
-  // kUnique: the sort buffers and the key bits that name the sorted one
-  const unsigned long long* keys0;
-  const unsigned long long* keys1;
-  const unsigned long long* bits;
-  __device__ __forceinline__ const unsigned long long* sorted() const {
-    return pass_parity(bits, 8) ? keys1 : keys0;
-  }
-};
-
-// Outputs of item i: the bitmask of neighbours that border another segment
-// (kEdges), or whether a sorted pair starts a run (kUnique).
-template <int MODE>
-__device__ __forceinline__ unsigned item_mask(const Items& it, int i) {
-  if (MODE == kUnique) {
-    const unsigned long long* s = it.sorted();
-    return (i == 0 || s[i] != s[i - 1]) ? 1u : 0u;
-  }
-  const int x = i % it.w, y = i / it.w, v = __ldg(it.labels + i);
+// the neighbours of pixel i that border another segment, a bit each
+__device__ __forceinline__ unsigned edge_mask(const int32_t* lab, int w, int h, int i) {
+  const int x = i % w, y = i / w, v = __ldg(lab + i);
   unsigned m = 0;
 #pragma unroll
   for (int d = 0; d < 8; ++d) {
-    const int j = neighbour(x, y, it.w, it.h, d);
-    if (j >= 0 && __ldg(it.labels + j) != v) m |= 1u << d;
+    const int j = neighbour(x, y, w, h, d);
+    if (j >= 0 && __ldg(lab + j) != v) m |= 1u << d;
   }
   return m;
 }
 
-__device__ __forceinline__ int n_items(const int* d_n, int n) { return d_n ? *d_n : n; }
-
-// Totals of the items' outputs per tile of items (contiguous kItems per
-// thread), a block taking every gridDim.x-th tile.
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) count_kernel(Items it, int n, const int* d_n,
-                                                          int* block_sum) {
+// Edges per tile of pixels (contiguous kItems per thread).
+__global__ void __launch_bounds__(kThreads) count_kernel(const int32_t* __restrict__ lab, int w,
+                                                          int h, int* block_sum) {
   pdl_wait();
-  const int nn = n_items(d_n, n);
+  const int n = w * h;
   __shared__ int ws[kWarps];
-  for (int b = blockIdx.x; b < blocks_of(nn); b += gridDim.x) {
-    int c = 0;
-    for (int k = 0; k < kItems; ++k) {
-      const int i = b * kTile + threadIdx.x * kItems + k;
-      if (i < nn) c += __popc(item_mask<MODE>(it, i));
-    }
-    c = __reduce_add_sync(0xffffffffu, c);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int s = 0;
-      for (int w = 0; w < kWarps; ++w) s += ws[w];
-      block_sum[b] = s;
-    }
-    __syncthreads();
+  int c = 0;
+  for (int k = 0; k < kItems; ++k) {
+    const int i = blockIdx.x * kTile + threadIdx.x * kItems + k;
+    if (i < n) c += __popc(edge_mask(lab, w, h, i));
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int s = 0;
+    for (int k = 0; k < kWarps; ++k) s += ws[k];
+    block_sum[blockIdx.x] = s;
   }
 }
 
-// Exclusive scan of `count` words in place by one block, in tiles of
-// kScanThreads with a carried prefix; the grand total goes to *total (when
-// given).
-template <typename T>
-__device__ void block_scan(T* a, int count, int* total) {
-  __shared__ T part[kScanThreads / 32];
-  __shared__ T carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
+// Exclusive scan of one value per thread over the block; the total to every
+// thread.
+template <int THREADS, typename T>
+__device__ T scan_threads(T v, T& total) {
+  __shared__ T part[THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int t0 = 0; t0 < count; t0 += kScanThreads) {
-    const int i = t0 + threadIdx.x;
-    const T v = i < count ? a[i] : 0;
-    T s = v;
+  T s = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T u = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += u;
-    }
-    if (lane == 31) part[warp] = s;
-    __syncthreads();
-    if (warp == 0) {
-      T p = lane < kScanThreads / 32 ? part[lane] : 0;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const T u = __shfl_up_sync(0xffffffffu, p, o);
-        if (lane >= o) p += u;
-      }
-      if (lane < kScanThreads / 32) part[lane] = p;
-    }
-    __syncthreads();
-    const T before = carry + (warp ? part[warp - 1] : 0) + s - v;
-    if (i < count) a[i] = before;
-    __syncthreads();
-    if (threadIdx.x == kScanThreads - 1) carry = before + v;
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const T u = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += u;
   }
-  if (threadIdx.x == 0 && total) *total = (int)carry;
+  __syncthreads();
+  if (lane == 31) part[warp] = s;
+  __syncthreads();
+  T before = 0, all = 0;
+#pragma unroll
+  for (int k = 0; k < THREADS / 32; ++k) {
+    if (k == warp) before = all;
+    all += part[k];
+  }
+  total = all;
+  return before + s - v;
+}
+
+// Exclusive scan of `count` words in place by one block, in tiles of THREADS
+// with a carried prefix; returns the grand total.
+template <int THREADS, typename T>
+__device__ T block_scan(T* a, int count) {
+  T carry = 0;
+  for (int t0 = 0; t0 < count; t0 += THREADS) {
+    const int i = t0 + threadIdx.x;
+    T total;
+    const T before = scan_threads<THREADS, T>(i < count ? a[i] : 0, total);
+    if (i < count) a[i] = carry + before;
+    carry += total;
+  }
+  return carry;
 }
 
 // Prefix of the block totals (their total to *total).
-__global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(int n, const int* d_n,
-                                                                   int* block_sum, int* total) {
+__global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(int count, int* block_sum,
+                                                                   int* total) {
   pdl_wait();
-  block_scan<int>(block_sum, blocks_of(n_items(d_n, n)), total);
+  const int all = block_scan<kScanThreads>(block_sum, count);
+  if (threadIdx.x == 0) *total = all;
 }
 
-// Writes every item's outputs at its place in the order of the items (a
+// Writes every pixel's edges at their place in the order of the pixels (a
 // block-wide exclusive scan of the threads' counts, plus the tile's prefix).
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) write_kernel(Items it, int n, const int* d_n,
-                                                          const int* block_sum, const int* total,
-                                                          int32_t* out0, int32_t* out1) {
+__global__ void __launch_bounds__(kThreads) write_kernel(const int32_t* __restrict__ lab, int w,
+                                                          int h, const int* block_sum,
+                                                          const int* total, int32_t* edges) {
   pdl_wait();
-  const int nn = n_items(d_n, n);
-  __shared__ int ws[kWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int b = blockIdx.x; b < blocks_of(nn); b += gridDim.x) {
-    const int first = b * kTile + threadIdx.x * kItems;
-    int c = 0;
-    for (int k = 0; k < kItems; ++k)
-      if (first + k < nn) c += __popc(item_mask<MODE>(it, first + k));
-    // exclusive scan of c over the block
-    int s = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += u;
+  const int n = w * h;
+  const int first = blockIdx.x * kTile + threadIdx.x * kItems;
+  int c = 0;
+  for (int k = 0; k < kItems; ++k)
+    if (first + k < n) c += __popc(edge_mask(lab, w, h, first + k));
+  int all;
+  int at = block_sum[blockIdx.x] + scan_threads<kThreads>(c, all);
+  const int m = *total;
+  for (int k = 0; k < kItems; ++k) {
+    const int i = first + k;
+    if (i >= n) break;
+    const int x = i % w, y = i / w;
+    for (unsigned mask = edge_mask(lab, w, h, i); mask; mask &= mask - 1) {
+      edges[at] = i;
+      edges[m + at] = neighbour(x, y, w, h, __ffs(mask) - 1);
+      ++at;
     }
-    if (lane == 31) ws[warp] = s;
-    __syncthreads();
-    int before = block_sum[b] + s - c;
-    for (int w = 0; w < warp; ++w) before += ws[w];
-    const int m = *total;
-    for (int k = 0; k < kItems; ++k) {
-      const int i = first + k;
-      if (i >= nn) break;
-      unsigned mask = item_mask<MODE>(it, i);
-      if (MODE == kUnique) {
-        if (mask) {
-          const unsigned long long key = it.sorted()[i];
-          out0[before] = (int)((unsigned)(key >> 32) ^ 0x80000000u);
-          out1[before] = (int)((unsigned)key ^ 0x80000000u);
-          ++before;
-        }
-        continue;
-      }
-      const int x = i % it.w, y = i / it.w;
-      while (mask) {
-        const int d = __ffs(mask) - 1;
-        mask &= mask - 1;
-        out0[before] = i;
-        out0[m + before] = neighbour(x, y, it.w, it.h, d);
-        ++before;
-      }
-    }
-    __syncthreads();
   }
 }
 
 // ---- the keys to sort ----------------------------------------------------------
-// no keys yet, and the OR / AND of none
-__global__ void reset_kernel(const Layout l) {
+// no keys and no pairs yet, the OR / AND of none, and the sort's barrier
+__global__ void reset_kernel(const Layout l, int* d_count) {
   pdl_wait();
   if (threadIdx.x == 0) {
+    *d_count = 0;
+    l.hdr->barrier_count = 0u;
     l.total[0] = 0;
     l.bits[0] = 0ull;
     l.bits[1] = ~0ull;
@@ -364,94 +309,237 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
   }
 }
 
-// ---- stable LSD radix sort of the pair keys ----------------------------------
-// Digit counts per block, digit-major (hist[d * nb + b]).
-__global__ void __launch_bounds__(kThreads) hist_kernel(const Layout l, int p) {
-  pdl_wait();
-  const int n = *l.total;
-  const int nb = sort_tiles(n), rounds = sort_rounds(n);
-  if ((int)blockIdx.x >= nb || !pass_runs(l.bits, p)) return;
-  const unsigned long long* in = l.keys[pass_parity(l.bits, p)];
-  __shared__ unsigned h[256];
-  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    h[threadIdx.x] = 0;
+// ---- distinct keys in order, by their ranks -----------------------------------
+// Tiles of kRankTile keys are sorted in shared memory; a key that no earlier
+// tile holds (and that is the first of its run in its own) goes out, at the
+// number of such keys below it in all tiles: one binary search per tile, whose
+// loads meet in the caches, the keys of a warp being neighbours in order.
+// Bound by the barriers and the searches' latency, four tiles in flight.
+// 20 thousand keys (20 tiles): 50 us; the 27 launches of a digit sort and
+// compaction took 158 us.
+
+// places of `key` in tiles t0 .. t0 + 3 (tiles past the last repeat it)
+__device__ __forceinline__ void lower_bounds(const unsigned long long* a, int t0, int tiles,
+                                             unsigned long long key, int (&at)[4]) {
+  const unsigned long long* s[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    s[g] = a + (size_t)min(t0 + g, tiles - 1) * kRankTile;
+    at[g] = 0;
+  }
+#pragma unroll
+  for (int step = kRankTile / 2; step > 0; step >>= 1)
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      if (s[g][at[g] + step - 1] < key) at[g] += step;
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    if (s[g][at[g]] < key) ++at[g];
+}
+
+__device__ void rank_keys(const Layout& l, int n, int32_t* out0, int32_t* out1, int* d_count,
+                          unsigned long long* sm) {
+  const int tiles = (n + kRankTile - 1) / kRankTile;
+  const int step = gridDim.x * kThreads, first = blockIdx.x * kThreads + threadIdx.x;
+  // a tile's keys in order, filled up with the largest value (no key: the two
+  // labels of a pair differ)
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (int i = threadIdx.x; i < kRankTile; i += kThreads)
+      sm[i] = t * kRankTile + i < n ? l.keys[0][t * kRankTile + i] : ~0ull;
+    for (int size = 2; size <= kRankTile; size <<= 1)
+      for (int d = size >> 1; d > 0; d >>= 1) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < kRankTile / 2; q += kThreads) {
+          const int i = ((q & ~(d - 1)) << 1) | (q & (d - 1)), j = i | d;
+          const unsigned long long a = sm[i], b = sm[j];
+          if ((a > b) == ((i & size) == 0)) {
+            sm[i] = b;
+            sm[j] = a;
+          }
+        }
+      }
     __syncthreads();
-    for (int k = 0; k < rounds; ++k) {
-      const int i = (b * rounds + k) * kThreads + threadIdx.x;
-      if (i < n) atomicAdd(&h[(in[i] >> (8 * p)) & 0xff], 1u);
+    for (int i = threadIdx.x; i < kRankTile; i += kThreads)
+      l.keys[1][t * kRankTile + i] = sm[i];
+    __syncthreads();
+  }
+  if (!grid_barrier(l.hdr)) return;
+  // per tile, the keys that go out (1), then the number of those before each
+  // and, past the last, of all
+  int* const out = reinterpret_cast<int*>(l.keys[0]);   // [tiles][kRankTile + 1]
+  const unsigned long long* const a = l.keys[1];
+  for (int i = first; i < n; i += step) {
+    const unsigned long long key = a[i];
+    const int t = i / kRankTile;
+    bool seen = i % kRankTile != 0 && a[i - 1] == key;
+    for (int e = 0; e < t && !seen; e += 4) {
+      int at[4];
+      lower_bounds(a, e, t, key, at);
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        seen |= at[g] < kRankTile && a[min(e + g, t - 1) * kRankTile + at[g]] == key;
     }
-    __syncthreads();
-    l.hist[threadIdx.x * nb + b] = h[threadIdx.x];
-    __syncthreads();
+    out[i + t] = !seen;
+  }
+  if (!grid_barrier(l.hdr)) return;
+  constexpr int kPer = kRankTile / kThreads;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    int* const o = out + t * (kRankTile + 1);
+    int v[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x * kPer + k;
+      v[k] = t * kRankTile + i < n ? o[i] : 0;
+      sum += v[k];
+    }
+    int all;
+    int at = scan_threads<kThreads>(sum, all);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      o[threadIdx.x * kPer + k] = at;
+      at += v[k];
+    }
+    if (threadIdx.x == 0) o[kRankTile] = all;
+  }
+  if (!grid_barrier(l.hdr)) return;
+  for (int i = first; i < n; i += step) {
+    const int* const o = out + i + i / kRankTile;
+    if (o[0] == o[1]) continue;
+    const unsigned long long key = a[i];
+    int pos = 0;
+    for (int e = 0; e < tiles; e += 4) {
+      int at[4];
+      lower_bounds(a, e, tiles, key, at);
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (e + g < tiles) pos += out[(e + g) * (kRankTile + 1) + at[g]];
+    }
+    out0[pos] = (int)((unsigned)(key >> 32) ^ 0x80000000u);
+    out1[pos] = (int)((unsigned)key ^ 0x80000000u);
+  }
+  if (blockIdx.x == 0) {
+    int mine = 0, all;
+    for (int t = threadIdx.x; t < tiles; t += kThreads) mine += out[t * (kRankTile + 1) + kRankTile];
+    scan_threads<kThreads>(mine, all);
+    if (threadIdx.x == 0) *d_count = all;
   }
 }
 
-__global__ void __launch_bounds__(kScanThreads) hist_scan_kernel(const Layout l, int p) {
-  pdl_wait();
-  if (!pass_runs(l.bits, p)) return;
-  block_scan<unsigned>(l.hist, 256 * sort_tiles(*l.total), nullptr);
-}
+// ---- distinct keys in order, by a stable LSD radix sort -----------------------
+// Per digit: counts per tile, digit-major (hist[d * nb + b]); each digit's
+// counts scanned by one block, its total behind them; then the stable scatter.
+// A block moves a tile's items in index order, kThreads at a time; an item's
+// place is its digit's offset for the tile, plus the items of that digit in
+// earlier rounds, in earlier warps of this round, and in earlier lanes of its
+// warp.  Last, the first key of every run goes out.
+struct RadixSmem {
+  unsigned off[256], wc[kWarps][256];
+};
 
-// Stable scatter: a block moves its items in index order, kThreads at a
-// time; an item's place is its digit's offset for the block, plus the items
-// of that digit in earlier rounds, in earlier warps of this round, and in
-// earlier lanes of its warp.
-__global__ void __launch_bounds__(kThreads) scatter_kernel(const Layout l, int p) {
-  pdl_wait();
-  const int n = *l.total;
-  const int nb = sort_tiles(n), rounds = sort_rounds(n);
-  if ((int)blockIdx.x >= nb || !pass_runs(l.bits, p)) return;
-  const int q = pass_parity(l.bits, p);
-  const unsigned long long* in = l.keys[q];
-  unsigned long long* out = l.keys[q ^ 1];
-  __shared__ unsigned off[256];
-  __shared__ unsigned wc[kWarps][256];
-  const int warp = threadIdx.x >> 5;
+__device__ void radix_keys(const Layout& l, int n, int32_t* out0, int32_t* out1, int* d_count,
+                           RadixSmem& sm) {
+  const int nb = blocks_of(n), warp = threadIdx.x >> 5;
+  unsigned* const totals = l.hist + (size_t)256 * nb;
   unsigned lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+  for (int p = 0; p < 8; ++p) {
+    if (!pass_runs(l.bits, p)) continue;
+    const int q = pass_parity(l.bits, p);
+    const unsigned long long* in = l.keys[q];
+    unsigned long long* out = l.keys[q ^ 1];
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+      sm.off[threadIdx.x] = 0;
+      __syncthreads();
+#pragma unroll 4
+      for (int k = 0; k < kItems; ++k) {
+        const int i = (b * kItems + k) * kThreads + threadIdx.x;
+        if (i < n) atomicAdd(&sm.off[(in[i] >> (8 * p)) & 0xff], 1u);
+      }
+      __syncthreads();
+      l.hist[(size_t)threadIdx.x * nb + b] = sm.off[threadIdx.x];
+      __syncthreads();
+    }
+    if (!grid_barrier(l.hdr)) return;
+    for (int d = blockIdx.x; d < 256; d += gridDim.x) {
+      const unsigned all = block_scan<kThreads>(l.hist + (size_t)d * nb, nb);
+      if (threadIdx.x == 0) totals[d] = all;
+    }
+    if (!grid_barrier(l.hdr)) return;
+    unsigned all;
+    const unsigned below = scan_threads<kThreads>(totals[threadIdx.x], all);
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+      sm.off[threadIdx.x] = below + l.hist[(size_t)threadIdx.x * nb + b];
+      for (int w = 0; w < kWarps; ++w) sm.wc[w][threadIdx.x] = 0;
+      __syncthreads();
+      for (int k = 0; k < kItems; ++k) {
+        const int i = (b * kItems + k) * kThreads + threadIdx.x;
+        if (i - (int)threadIdx.x >= n) break;   // the same in every thread
+        const bool ok = i < n;
+        const unsigned long long key = ok ? in[i] : 0ull;
+        const int digit = ok ? (int)((key >> (8 * p)) & 0xff) : 256;
+        const unsigned peers = __match_any_sync(0xffffffffu, digit);
+        const int rank = __popc(peers & lt);
+        if (ok && rank == 0) sm.wc[warp][digit] = __popc(peers);
+        __syncthreads();
+        if (ok) {
+          unsigned pos = sm.off[digit] + rank;
+          for (int w = 0; w < warp; ++w) pos += sm.wc[w][digit];
+          out[pos] = key;
+        }
+        __syncthreads();
+        // the round's counts move into the digit offsets
+        unsigned t = 0;
+        for (int w = 0; w < kWarps; ++w) {
+          t += sm.wc[w][threadIdx.x];
+          sm.wc[w][threadIdx.x] = 0;
+        }
+        sm.off[threadIdx.x] += t;
+        __syncthreads();
+      }
+    }
+    if (!grid_barrier(l.hdr)) return;
+  }
+  const unsigned long long* const a = l.keys[pass_parity(l.bits, 8)];
+  auto starts = [&](int i) { return i < n && (i == 0 || a[i] != a[i - 1]); };
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    off[threadIdx.x] = l.hist[threadIdx.x * nb + b];
-    for (int w = 0; w < kWarps; ++w) wc[w][threadIdx.x] = 0;
-    __syncthreads();
-    for (int k = 0; k < rounds; ++k) {
-      const int i = (b * rounds + k) * kThreads + threadIdx.x;
-      if (i - (int)threadIdx.x >= n) break;   // the same in every thread
-      const bool ok = i < n;
-      const unsigned long long key = ok ? in[i] : 0ull;
-      const int digit = ok ? (int)((key >> (8 * p)) & 0xff) : 256;
-      const unsigned peers = __match_any_sync(0xffffffffu, digit);
-      const int rank = __popc(peers & lt);
-      if (ok && rank == 0) wc[warp][digit] = __popc(peers);
-      __syncthreads();
-      if (ok) {
-        unsigned pos = off[digit] + rank;
-        for (int w = 0; w < warp; ++w) pos += wc[w][digit];
-        out[pos] = key;
+    int c = 0, all;
+#pragma unroll 4
+    for (int k = 0; k < kItems; ++k) c += starts((b * kItems + k) * kThreads + threadIdx.x);
+    scan_threads<kThreads>(c, all);
+    if (threadIdx.x == 0) l.block_sum[b] = all;
+  }
+  if (!grid_barrier(l.hdr)) return;
+  if (blockIdx.x == 0) {
+    const int all = block_scan<kThreads>(l.block_sum, nb);
+    if (threadIdx.x == 0) *d_count = all;
+  }
+  if (!grid_barrier(l.hdr)) return;
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    int base = l.block_sum[b];
+    for (int k = 0; k < kItems; ++k) {
+      const int i = (b * kItems + k) * kThreads + threadIdx.x;
+      int all;
+      const int at = base + scan_threads<kThreads>((int)starts(i), all);
+      if (starts(i)) {
+        out0[at] = (int)((unsigned)(a[i] >> 32) ^ 0x80000000u);
+        out1[at] = (int)((unsigned)a[i] ^ 0x80000000u);
       }
-      __syncthreads();
-      // the round's counts move into the digit offsets
-      unsigned t = 0;
-      for (int w = 0; w < kWarps; ++w) {
-        t += wc[w][threadIdx.x];
-        wc[w][threadIdx.x] = 0;
-      }
-      off[threadIdx.x] += t;
-      __syncthreads();
+      base += all;
     }
   }
 }
 
-// `tiles`: tiles of items at most (blocks stride over those there are)
-template <int MODE>
-static int compaction(const Items& it, int n, const int* d_n, int tiles, const Layout& l,
-                      int* total, int32_t* out0, int32_t* out1, cudaStream_t st) {
-  launch_pdl(count_kernel<MODE>, dim3(tiles), dim3(kThreads), 0, st, it, n, d_n, l.block_sum);
-  SG_TRY(launch_status());
-  launch_pdl(scan_blocks_kernel, dim3(1), dim3(kScanThreads), 0, st, n, d_n, l.block_sum, total);
-  SG_TRY(launch_status());
-  launch_pdl(write_kernel<MODE>, dim3(tiles), dim3(kThreads), 0, st, it, n, d_n,
-             (const int*)l.block_sum, (const int*)total, out0, out1);
-  return launch_status();
+// One cooperative launch: the number of keys is known on the device only, and
+// launches for the path not taken would cost more than ranking does.
+__global__ void __launch_bounds__(kThreads) sort_kernel(const Layout l, int32_t* out0,
+                                                         int32_t* out1, int* d_count) {
+  __shared__ union {
+    unsigned long long tile[kRankTile];
+    RadixSmem radix;
+  } sm;
+  const int n = *l.total;
+  if (n <= kFewKeys) rank_keys(l, n, out0, out1, d_count, sm.tile);
+  else radix_keys(l, n, out0, out1, d_count, sm.radix);
 }
 
 }  // namespace adj
@@ -475,9 +563,16 @@ extern "C" int split_segment_adjacency_edges(const int32_t* labels, int width, i
     return SPLIT_ERR_WORKSPACE;
   l = adj::carve(workspace, n, false);
   cudaStream_t st = as_stream(stream);
-  adj::Items it{labels, width, height, nullptr, nullptr, nullptr};
-  return adj::compaction<adj::kEdges>(it, (int)n, nullptr, adj::blocks_of(n), l, d_count, edges,
-                                      nullptr, st);
+  const int tiles = adj::blocks_of(n);
+  launch_pdl(adj::count_kernel, dim3(tiles), dim3(adj::kThreads), 0, st, labels, width, height,
+             l.block_sum);
+  SG_TRY(launch_status());
+  launch_pdl(adj::scan_blocks_kernel, dim3(1), dim3(adj::kScanThreads), 0, st, tiles, l.block_sum,
+             d_count);
+  SG_TRY(launch_status());
+  launch_pdl(adj::write_kernel, dim3(tiles), dim3(adj::kThreads), 0, st, labels, width, height,
+             (const int*)l.block_sum, (const int*)d_count, edges);
+  return launch_status();
 }
 
 extern "C" size_t split_segment_adjacency_workspace_size(int width, int height) {
@@ -498,29 +593,22 @@ extern "C" int split_segment_adjacency(const int32_t* labels, int width, int hei
   l = adj::carve(workspace, n, true);
   cudaStream_t st = as_stream(stream);
   // 1: the distinct pair keys of every tile, and the digits that vary
-  launch_pdl(adj::reset_kernel, dim3(1), dim3(32), 0, st, l);
+  launch_pdl(adj::reset_kernel, dim3(1), dim3(32), 0, st, l, (int*)d_count);
   SG_TRY(launch_status());
   const int tiles = ((width + adj::kPixW - 1) / adj::kPixW) * ((height + adj::kPixH - 1) / adj::kPixH);
   launch_pdl(adj::pair_kernel, dim3(tiles), dim3(adj::kThreads), 0, st, labels, width, height, l);
   SG_TRY(launch_status());
-  // 2: stable radix passes.  The key count is known on the device only and is
-  // usually a small part of 8 n: the blocks stride over the tiles there are (a
-  // block for every possible tile took 4 us a launch to find nothing to do).
+  // 2: sorted, one of each
   DeviceInfo di;
   SG_TRY(device_info(&di));
-  const int sort_blocks =
-      std::min(std::max(adj::blocks_of(8 * n), adj::sort_tiles(8 * n)), 4 * di.sm_count);
-  for (int p = 0; p < 8; ++p) {
-    launch_pdl(adj::hist_kernel, dim3(sort_blocks), dim3(adj::kThreads), 0, st, l, p);
-    SG_TRY(launch_status());
-    launch_pdl(adj::hist_scan_kernel, dim3(1), dim3(adj::kScanThreads), 0, st, l, p);
-    SG_TRY(launch_status());
-    launch_pdl(adj::scatter_kernel, dim3(sort_blocks), dim3(adj::kThreads), 0, st, l, p);
-    SG_TRY(launch_status());
-  }
-  // 3: the first pair of every run of equal pairs (which buffer holds the
-  // sorted keys depends on the passes that ran: named on the device)
-  adj::Items u{nullptr, width, height, l.keys[0], l.keys[1], l.bits};
-  return adj::compaction<adj::kUnique>(u, 0, l.total, sort_blocks, l, d_count, keys, adjacency,
-                                       st);
+  int per_sm = 0;
+  SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adj::sort_kernel,
+                                                            adj::kThreads, 0));
+  if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
+  int* count = d_count;
+  void* args[] = {&l, &keys, &adjacency, &count};
+  SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)adj::sort_kernel,
+                                          dim3(di.sm_count * std::min(per_sm, 2)),
+                                          dim3(adj::kThreads), args, 0, st));
+  return launch_status();
 }
