@@ -2101,14 +2101,38 @@ extern "C" int split_kmeans_update(const int32_t* labels, const void* points, in
 }
 
 namespace {
-__global__ void propagate_kernel(const int32_t* __restrict__ labels, int64_t n,
-                                 const float* __restrict__ cent, int K, int dim,
-                                 float* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+// Bound by the stores.  Four pixels per thread where rows of n floats keep the
+// alignment (equal neighbours share one look-up): 2 Mpx to three rows, 33 MB,
+// 12.6 us a pixel at a time, 8.4 us four at a time.
+__device__ __forceinline__ float centroid_of(const float* row, int K, int l) {
+  return l >= 0 && l < K ? __ldg(row + l) : 0.0f;
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+propagate_kernel(const int32_t* __restrict__ labels, int64_t n, const float* __restrict__ cent,
+                 int K, int dim, float* __restrict__ out) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (VEC) {
+    for (; i < n / 4; i += step) {
+      const int4 l = __ldg(reinterpret_cast<const int4*>(labels) + i);
+#pragma unroll 3
+      for (int d = 0; d < dim; ++d) {
+        const float* const row = cent + (int64_t)d * K;
+        float4 v;
+        v.x = centroid_of(row, K, l.x);
+        v.y = l.y == l.x ? v.x : centroid_of(row, K, l.y);
+        v.z = l.z == l.y ? v.y : centroid_of(row, K, l.z);
+        v.w = l.w == l.z ? v.z : centroid_of(row, K, l.w);
+        reinterpret_cast<float4*>(out + d * n)[i] = v;
+      }
+    }
+    return;
+  }
+  for (; i < n; i += step) {
     const int l = __ldg(labels + i);
-    const bool ok = l >= 0 && l < K;
-    for (int d = 0; d < dim; ++d) out[d * n + i] = ok ? __ldg(cent + d * K + l) : 0.0f;
+    for (int d = 0; d < dim; ++d) out[d * n + i] = centroid_of(cent + (int64_t)d * K, K, l);
   }
 }
 }  // namespace
@@ -2120,11 +2144,14 @@ extern "C" int split_kmeans_propagate(const int32_t* labels, int64_t npoints,
     return SPLIT_ERR_INVALID;
   DeviceInfo di;
   SG_TRY(device_info(&di));
-  int64_t blocks = (npoints + 255) / 256;
+  const bool vec = npoints % 4 == 0 && ((reinterpret_cast<uintptr_t>(labels) |
+                                         reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  int64_t blocks = ((vec ? npoints / 4 : npoints) + 255) / 256;
   const int64_t cap = (int64_t)di.sm_count * 8;
   if (blocks > cap) blocks = cap;
-  propagate_kernel<<<(int)blocks, 256, 0, as_stream(stream)>>>(labels, npoints, centroids,
-                                                                nclusters, dim, out);
+  (vec ? propagate_kernel<true> : propagate_kernel<false>)
+      <<<(int)blocks, 256, 0, as_stream(stream)>>>(labels, npoints, centroids, nclusters, dim,
+                                                   out);
   return launch_status();
 }
 
@@ -2383,9 +2410,8 @@ extern "C" int split_tune_get(split_tune_entry* out, int capacity) {
 // of segments).  Per-cluster sums of the member features in the same 96-bit
 // fixed point as the k-means update (each feature rounded to a multiple of
 // 2^-24, low and high words added with 64-bit atomics), so the result is the
-// same whatever order pixels are added in.  A warp whose 32 pixels share one
-// label adds one warp sum; mixed warps add per pixel.  Means in FP64,
-// rounded to FP32; a cluster without members keeps its input centroid.
+// same whatever order pixels are added in.  Means in FP64, rounded to FP32; a
+// cluster without members keeps its input centroid.
 // ---------------------------------------------------------------------------
 namespace sg {
 namespace segm {
@@ -2411,48 +2437,137 @@ inline Layout carve(void* ws, int K, int dim) {
   return l;
 }
 
+// the features of pixel i
+template <int LAYOUT, int DIM>
+__device__ __forceinline__ void pixel_features(const void* points, int64_t n, int64_t i, int width,
+                                               float xy_scale, float (&f)[DIM]) {
+  if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
+    const float4 v = __ldg(static_cast<const float4*>(points) + i);
+    f[0] = v.x;
+    f[1] = v.y;
+    f[2] = v.z;
+  } else if (LAYOUT == SPLIT_LAYOUT_RGB8) {
+    const uint8_t* p = static_cast<const uint8_t*>(points) + 3 * i;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = __fdiv_rn((float)__ldg(p + c), 255.0f);
+  } else {
+    const float* p = static_cast<const float*>(points);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) f[d] = __ldg(p + (int64_t)d * n + i);
+  }
+  if (DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR) {
+    const int64_t row = i / width;
+    f[3] = __fmul_rn(xy_scale, (float)(i - row * width));
+    f[4] = __fmul_rn(xy_scale, (float)row);
+  }
+}
+
+// Adds a run of pixels of one label, its words as 32-bit sums.
+template <int DIM>
+__device__ __forceinline__ void add_run(const Layout& L, int l, const unsigned (&q)[DIM],
+                                        unsigned count) {
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+    atomicAdd(L.lo + (size_t)l * DIM + d, (unsigned long long)q[d]);
+  atomicAdd(L.cnt + l, count);
+}
+
+// Bound by the reductions of runs and the atomics that they end in.  Four
+// consecutive pixels per thread.  A warp whose features all lie in [0, 1]
+// (colours do) has words of at most 2^24, so the sums of its 128 pixels fit 32
+// bits and their high words are zero: a thread adds the runs that end inside
+// its four pixels as they are, and its last run takes part in a segmented
+// reduction over the lanes, whose run heads add.  Other warps add the 96-bit
+// words, a pixel of every lane at a time.  2 Mpx in 24 thousand segments,
+// planar colours: 27.4 us with the 96-bit words throughout, 15.4 us.
+constexpr int kPer = 4;
+
 template <int LAYOUT, int DIM>
 __global__ void __launch_bounds__(kThreads)
 accumulate_kernel(const int32_t* __restrict__ labels, const void* __restrict__ points,
-                  int64_t n, int width, float xy_scale, int K, Layout L) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  // every lane runs the same number of rounds (warp-wide shuffles below)
-  const int64_t rounds = (n + stride - 1) / stride;
-  for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t i = r * stride + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int l = -1;
-    float f[DIM];
+                  int64_t n, int width, float xy_scale, int K, Layout L, bool vec) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i0 = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * kPer;
+  int l[kPer];
+  float f[kPer][DIM];
+  if (vec && i0 + kPer <= n) {   // n is a multiple of kPer
+    const int4 v = __ldg(reinterpret_cast<const int4*>(labels + i0));
+    l[0] = v.x; l[1] = v.y; l[2] = v.z; l[3] = v.w;
+  } else {
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) f[d] = 0.0f;
-    if (i < n) {
-      l = __ldg(labels + i);
-      if (l < 0 || l >= K) l = -1;
-    }
-    if (l >= 0) {
-      if (LAYOUT == SPLIT_LAYOUT_FLOAT4) {
-        const float4 v = __ldg(static_cast<const float4*>(points) + i);
-        f[0] = v.x;
-        f[1] = v.y;
-        f[2] = v.z;
-      } else if (LAYOUT == SPLIT_LAYOUT_RGB8) {
-        const uint8_t* p = static_cast<const uint8_t*>(points) + 3 * i;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] = __fdiv_rn((float)__ldg(p + c), 255.0f);
-      } else {
-        const float* p = static_cast<const float*>(points);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) f[d] = __ldg(p + (int64_t)d * n + i);
-      }
-      if (DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR) {
-        const int64_t row = i / width;
-        f[3] = __fmul_rn(xy_scale, (float)(i - row * width));
-        f[4] = __fmul_rn(xy_scale, (float)row);
-      }
-    }
-    unsigned long long qlo[DIM], qhi[DIM];
-    fix::quantize<DIM>(f, l, &L.hdr->status, qlo, qhi);
-    fix::warp_add<DIM>(l, qlo, qhi, L.lo, L.hi, L.cnt);
+    for (int j = 0; j < kPer; ++j) l[j] = i0 + j < n ? __ldg(labels + i0 + j) : -1;
   }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j)
+    if (l[j] >= K) l[j] = -1;
+  if (LAYOUT == SPLIT_LAYOUT_PLANAR && vec) {
+    const float* p = static_cast<const float*>(points);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const float4 v = i0 < n ? __ldg(reinterpret_cast<const float4*>(p + (int64_t)d * n + i0))
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      f[0][d] = v.x; f[1][d] = v.y; f[2][d] = v.z; f[3][d] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) f[j][d] = 0.0f;
+      if (l[j] >= 0) pixel_features<LAYOUT, DIM>(points, n, i0 + j, width, xy_scale, f[j]);
+    }
+  }
+  bool unit = true;   // false for NaN
+#pragma unroll
+  for (int j = 0; j < kPer; ++j)
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) unit &= l[j] < 0 || (f[j][d] >= 0.0f && f[j][d] <= 1.0f);
+  if (!__all_sync(0xffffffffu, unit)) {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int lj = l[j] < 0 ? -1 : l[j];
+      unsigned long long qlo[DIM], qhi[DIM];
+      fix::quantize<DIM>(f[j], lj, &L.hdr->status, qlo, qhi);
+      fix::warp_add<DIM>(lj, qlo, qhi, L.lo, L.hi, L.cnt);
+    }
+    return;
+  }
+  unsigned q[DIM], c = 0u;
+  int cur = l[0];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) q[d] = 0u;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (j > 0 && l[j] != cur) {
+      if (cur >= 0) add_run<DIM>(L, cur, q, c);
+      cur = l[j];
+      c = 0u;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) q[d] = 0u;
+    }
+    ++c;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) q[d] += __float2uint_rn(__fmul_rn(f[j][d], fix::kScale));
+  }
+  // the lanes' last runs: a lane adds from lane + o while that lane is in its
+  // run; a lane that began its run with fewer than four pixels is a head, its
+  // label not the lane's before (or cut off by the runs already added)
+  const int before = __shfl_up_sync(0xffffffffu, cur, 1);
+  const unsigned heads =
+      __ballot_sync(0xffffffffu, lane == 0 || cur != before || c != (unsigned)kPer);
+  const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
+  const int run_end = after ? __ffs(after) - 1 : 32;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const bool in_run = lane + o < run_end;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const unsigned a = __shfl_down_sync(0xffffffffu, q[d], o);
+      if (in_run) q[d] += a;
+    }
+    const unsigned a = __shfl_down_sync(0xffffffffu, c, o);
+    if (in_run) c += a;
+  }
+  if (cur >= 0 && (heads >> lane & 1u)) add_run<DIM>(L, cur, q, c);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -2485,13 +2600,15 @@ int run(const int32_t* labels, const void* points, int layout, int dim, int64_t 
                               l.bytes - sizeof(int), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
-  int64_t blocks = (n + kThreads - 1) / kThreads;
-  const int64_t cap = (int64_t)di.sm_count * 8;
-  if (blocks > cap) blocks = cap;
+  // whole vectors of labels and, planar, of every feature row
+  const bool vec = n % kPer == 0 && ((reinterpret_cast<uintptr_t>(labels) |
+                                      (layout == SPLIT_LAYOUT_PLANAR
+                                           ? reinterpret_cast<uintptr_t>(points) : 0)) & 15) == 0;
 #define SG_SEG_CASE(LY, D)                                                                 \
   if (layout == LY && dim == D) {                                                          \
-    accumulate_kernel<LY, D><<<(int)blocks, kThreads, 0, st>>>(labels, points, n, width,  \
-                                                               xy_scale, K, l);            \
+    accumulate_kernel<LY, D><<<(int)((n + kThreads * kPer - 1) / (kThreads * kPer)),       \
+                               kThreads, 0, st>>>(labels, points, n, width, xy_scale, K,  \
+                                                  l, vec);                                 \
   }
   SG_SEG_CASE(SPLIT_LAYOUT_PLANAR, 3)
   SG_SEG_CASE(SPLIT_LAYOUT_PLANAR, 5)
@@ -2501,6 +2618,7 @@ int run(const int32_t* labels, const void* points, int layout, int dim, int64_t 
   SG_SEG_CASE(SPLIT_LAYOUT_RGB8, 5)
 #undef SG_SEG_CASE
   SG_TRY(launch_status());
+  const int64_t cap = (int64_t)di.sm_count * 8;
   int64_t fb = ((int64_t)K * dim + kThreads - 1) / kThreads;
   if (fb > cap) fb = cap;
   finish_kernel<<<(int)fb, kThreads, 0, st>>>(l, K, dim, centroids);
