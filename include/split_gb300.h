@@ -91,6 +91,13 @@ const char* split_status_string(int status);
  * work queued on `stream` completes.  Synchronises `stream`. */
 int split_workspace_status(void* workspace, void* stream, int* out_status);
 
+/* A device word inside the workspace that a call may be given for its count
+ * (the d_count of split_compress_labels, split_segment_adjacency and
+ * split_segment_adjacency_edges), and the read of that word together with the
+ * status (which it clears): one round trip instead of two.  Synchronises
+ * `stream`. */
+int32_t* split_workspace_result(void* workspace);
+int split_workspace_finish(void* workspace, void* stream, int* out_status, int32_t* out_result);
 
 /* ======================================================================== */
 /* k-means                                                                  */

@@ -26,6 +26,8 @@ _SIGS = {
     "split_version": (C.c_char_p, []),
     "split_status_string": (C.c_char_p, [_i32]),
     "split_workspace_status": (_i32, [_vp, _vp, C.POINTER(C.c_int)]),
+    "split_workspace_result": (_vp, [_vp]),
+    "split_workspace_finish": (_i32, [_vp, _vp, C.POINTER(C.c_int), C.POINTER(_i32)]),
     "split_kmeans_set_wait_test": (None, [C.c_uint, _i32]),
     "split_kmeans_cluster_workspace_size": (_sz, [_i64, _i32, _i32]),
     "split_kmeans_cluster_workspace_size_2d": (_sz, [_i64, _i32, _i32, _i32]),

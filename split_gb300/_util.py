@@ -75,6 +75,20 @@ class Workspace:
         if st != N.OK:
             raise N.SplitError(st, where + " (device)")
 
+    @property
+    def result(self):
+        """Device address of the word a call may leave its count in."""
+        return C.c_void_p(N.load().split_workspace_result(self.ptr))
+
+    def finish(self, where: str, stream=None) -> int:
+        """The count in `result`, after the check of the status: one round trip."""
+        st, count = C.c_int(0), C.c_int(0)
+        N.check(N.load().split_workspace_finish(self.ptr, stream_handle(stream), C.byref(st),
+                                                C.byref(count)), "split_workspace_finish")
+        if st.value != N.OK:
+            raise N.SplitError(st.value, where + " (device)")
+        return count.value
+
 
 def ensure_workspace(ws: Workspace | None, nbytes: int, device) -> Workspace:
     if ws is None or ws.nbytes < nbytes:

@@ -54,12 +54,10 @@ def compress_labels(labels: torch.Tensor, temp: Workspace | None = None, *,
     require_cuda(labels, "labels", torch.int32)
     n = labels.numel()
     ws = ensure_workspace(temp, compress_labels_workspace(n), labels.device)
-    count = torch.zeros(1, dtype=torch.int32, device=labels.device)
-    st = N.load().split_compress_labels(ptr(labels), n, ptr(count), ws.ptr, ws.nbytes,
+    st = N.load().split_compress_labels(ptr(labels), n, ws.result, ws.ptr, ws.nbytes,
                                         stream_handle(stream))
     N.check(st, "ccl.compress_labels")
-    ws.check("ccl.compress_labels", stream)
-    return int(count.item())
+    return ws.finish("ccl.compress_labels", stream)
 
 
 def segment_adjacency_edges_workspace(width: int, height: int) -> int:
@@ -82,12 +80,10 @@ def segment_adjacency_edges(labels: torch.Tensor, edges: torch.Tensor,
     if edges.numel() < 16 * h * w:
         raise ValueError("edges must hold 16 entries per pixel")
     ws = ensure_workspace(temp, segment_adjacency_edges_workspace(w, h), labels.device)
-    count = torch.zeros(1, dtype=torch.int32, device=labels.device)
-    st = N.load().split_segment_adjacency_edges(ptr(labels), w, h, ptr(edges), ptr(count),
+    st = N.load().split_segment_adjacency_edges(ptr(labels), w, h, ptr(edges), ws.result,
                                                 ws.ptr, ws.nbytes, stream_handle(stream))
     N.check(st, "ccl.segment_adjacency_edges")
-    ws.check("ccl.segment_adjacency_edges", stream)
-    return int(count.item())
+    return ws.finish("ccl.segment_adjacency_edges", stream)
 
 
 def segment_adjacency_workspace(width: int, height: int) -> int:
@@ -110,12 +106,10 @@ def segment_adjacency(labels: torch.Tensor, keys: torch.Tensor, adjacency: torch
     if keys.numel() < 8 * h * w or adjacency.numel() < 8 * h * w:
         raise ValueError("keys and adjacency must hold 8 entries per pixel")
     ws = ensure_workspace(temp, segment_adjacency_workspace(w, h), labels.device)
-    count = torch.zeros(1, dtype=torch.int32, device=labels.device)
     st = N.load().split_segment_adjacency(ptr(labels), w, h, ptr(keys), ptr(adjacency),
-                                          ptr(count), ws.ptr, ws.nbytes, stream_handle(stream))
+                                          ws.result, ws.ptr, ws.nbytes, stream_handle(stream))
     N.check(st, "ccl.segment_adjacency")
-    ws.check("ccl.segment_adjacency", stream)
-    return int(count.item())
+    return ws.finish("ccl.segment_adjacency", stream)
 
 
 def merge_small_segments_workspace(width: int, height: int) -> int:

@@ -103,13 +103,32 @@ int clear_status(const StatusSources& s, cudaStream_t st) {
 }
 }  // namespace sg
 
+// The header's first words in one copy; the status word goes back to zero, which
+// it nearly always is already (a clear is a launch).
+static int read_header(void* workspace, void* stream, int* out_status, int* out_result) {
+  cudaStream_t st = as_stream(stream);
+  struct {
+    int words[offsetof(WsHeader, result) / sizeof(int) + 1];
+  } h;
+  SG_CUDA_TRY(cudaMemcpyAsync(&h, workspace, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h.words[0] != 0) SG_CUDA_TRY(cudaMemsetAsync(workspace, 0, sizeof(int), st));
+  *out_status = h.words[0];
+  if (out_result) *out_result = h.words[sizeof(h) / sizeof(int) - 1];
+  return SPLIT_OK;
+}
+
 extern "C" int split_workspace_status(void* workspace, void* stream, int* out_status) {
   if (!workspace || !out_status) return SPLIT_ERR_INVALID;
-  cudaStream_t st = as_stream(stream);
-  int h = 0;
-  SG_CUDA_TRY(cudaMemcpyAsync(&h, workspace, sizeof(int), cudaMemcpyDeviceToHost, st));
-  SG_CUDA_TRY(cudaStreamSynchronize(st));
-  SG_CUDA_TRY(cudaMemsetAsync(workspace, 0, sizeof(int), st));
-  *out_status = h;
-  return SPLIT_OK;
+  return read_header(workspace, stream, out_status, nullptr);
+}
+
+extern "C" int32_t* split_workspace_result(void* workspace) {
+  return workspace ? &static_cast<WsHeader*>(workspace)->result : nullptr;
+}
+
+extern "C" int split_workspace_finish(void* workspace, void* stream, int* out_status,
+                                      int32_t* out_result) {
+  if (!workspace || !out_status || !out_result) return SPLIT_ERR_INVALID;
+  return read_header(workspace, stream, out_status, out_result);
 }

@@ -83,8 +83,8 @@ struct WsHeader {
   int status;
   unsigned barrier_count;
   unsigned barrier_gen;
-  unsigned work_counter[2];
-  int pad0;
+  unsigned counter[2];   // per call, cleared by its first launch
+  int result;            // a call's count, for callers that read it with the status
   // layout the workspace's persistent state was last cleared for (0: never)
   unsigned long long stamp;
   int pad[56];

@@ -66,8 +66,8 @@ inline Layout carve(void* ws, int64_t n) {
   Carver c(ws);
   Layout l;
   l.hdr = c.take<WsHeader>(1);
-  l.maxsq = l.hdr ? l.hdr->work_counter : nullptr;
-  l.list_count = l.hdr ? l.hdr->work_counter + 1 : nullptr;
+  l.maxsq = l.hdr ? l.hdr->counter : nullptr;
+  l.list_count = l.hdr ? l.hdr->counter + 1 : nullptr;
   l.call = l.hdr ? reinterpret_cast<unsigned*>(l.hdr->pad) : nullptr;
   l.best = c.take<unsigned long long>((size_t)n);
   l.fin = c.take<unsigned long long>((size_t)n);
