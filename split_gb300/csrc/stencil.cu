@@ -123,6 +123,9 @@ struct ErodeArgs {
   int* status;
 };
 
+// every entry point refuses a larger one
+constexpr int kMaxRadius = 16;
+
 // TMA bits of ImgGeom::tma_ok
 constexpr int kTmaLabels = 1, kTmaRgb = 2;
 
@@ -147,25 +150,19 @@ erode_kernel(const __grid_constant__ CUtensorMap tmap, bool use_tma, ErodeArgs a
   if (!stage<int32_t>(lab, map, a.in + t.off, W, H, tx0 - XP, ty0 - R, SW, SH, &bar, a.status))
     return;
   if (a.mstate) {
+    // four consecutive entries per step (the staged tile is 16-byte aligned,
+    // its rows are whole int4s); an entry equal to the one before it takes
+    // that one's result instead of gathering again
     const mrg::State ms = *a.mstate;
-    if (R1) {
-      // 72 x 34 entries, four consecutive ones per step (the staged tile is
-      // 16-byte aligned); an entry equal to the one before it takes that
-      // one's result instead of gathering again
-      static_assert((TW + 8) * (TH + 2) % 4 == 0, "whole int4 steps");
-      int4* l4 = reinterpret_cast<int4*>(lab);
-      for (int i = threadIdx.x; i < SW * SH / 4; i += blockDim.x) {
-        const int4 v = l4[i];
-        int4 o;
-        o.x = mrg::relabel(ms, a.mfin, v.x);
-        o.y = v.y == v.x ? o.x : mrg::relabel(ms, a.mfin, v.y);
-        o.z = v.z == v.y ? o.y : mrg::relabel(ms, a.mfin, v.z);
-        o.w = v.w == v.z ? o.z : mrg::relabel(ms, a.mfin, v.w);
-        l4[i] = o;
-      }
-    } else {
-      for (int i = threadIdx.x; i < SW * SH; i += blockDim.x)
-        lab[i] = mrg::relabel(ms, a.mfin, lab[i]);
+    int4* l4 = reinterpret_cast<int4*>(lab);
+    for (int i = threadIdx.x; i < SW * SH / 4; i += blockDim.x) {
+      const int4 v = l4[i];
+      int4 o;
+      o.x = mrg::relabel(ms, a.mfin, v.x);
+      o.y = v.y == v.x ? o.x : mrg::relabel(ms, a.mfin, v.y);
+      o.z = v.z == v.y ? o.y : mrg::relabel(ms, a.mfin, v.z);
+      o.w = v.w == v.z ? o.z : mrg::relabel(ms, a.mfin, v.w);
+      l4[i] = o;
     }
     __syncthreads();
   }
@@ -201,28 +198,56 @@ erode_kernel(const __grid_constant__ CUtensorMap tmap, bool use_tma, ErodeArgs a
     }
     return;
   }
-  // separable square window: vertical run test per staged column, then the
-  // horizontal test over the vertical flags
+  // Separable square window, the same work for any radius.  Down each staged
+  // column the length of the run of equal labels that ends at a row says
+  // whether the window that ends there is constant; kStrips threads share a
+  // column.  Along each row two masks of a bit per staged column, that flag and
+  // "flagged, and equal to the left", say whether the flags of a window are all
+  // set and its labels all equal.  1283 x 957, radius 10: 39.8 us with a test
+  // per window entry, 26.8.
+  constexpr int kStrips = 2, kRows = TH / kStrips, kWords = (TW + 2 * kMaxRadius + 31) / 32;
+  __shared__ unsigned flags[TH][kWords], links[TH][kWords];
   unsigned char* vert = smem + (size_t)SW * SH * sizeof(int32_t);
-  for (int i = threadIdx.x; i < TH * SW; i += blockDim.x) {
-    const int r = i / SW, c = i % SW;
-    const int* p = lab + (r + R) * SW + c;
-    const int v = p[0];
-    bool ok = true;
-    for (int dy = -R; dy <= R && ok; ++dy) ok = p[dy * SW] == v;
-    vert[i] = ok;
+  for (int i = threadIdx.x; i < kStrips * SW; i += blockDim.x) {
+    const int c = i % SW, a0 = i / SW * kRows;
+    const int* p = lab + a0 * SW + c;
+    int run = 0, last = 0;
+    for (int s = 0; s < kRows + 2 * R; ++s, p += SW) {
+      const int v = *p;
+      run = run > 0 && v == last ? run + 1 : 1;
+      last = v;
+      if (s >= 2 * R) vert[(a0 + s - 2 * R) * SW + c] = run > 2 * R;
+    }
   }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < TH; r += kThreads / 32)
+    for (int w = 0; w < (SW + 31) / 32; ++w) {
+      const int c = 32 * w + lane;
+      const int* p = lab + (r + R) * SW + c;
+      const bool v = c < SW && vert[r * SW + c];
+      const unsigned f = __ballot_sync(0xffffffffu, v);
+      const unsigned l = __ballot_sync(0xffffffffu, v && c > 0 && p[0] == p[-1]);
+      if (lane == 0) {
+        flags[r][w] = f;
+        links[r][w] = l;
+      }
+    }
   __syncthreads();
   for (int i = threadIdx.x; i < TH * TW; i += blockDim.x) {
     const int r = i / TW, c = i % TW;
     const int x = tx0 + c, y = ty0 + r;
     if (x >= W || y >= H) continue;
-    const int* p = lab + (r + R) * SW + (c + XP);
-    const unsigned char* f = vert + r * SW + (c + XP);
-    const int v = p[0];
-    bool keep = x >= R && y >= R && x + R < W && y + R < H;
-    for (int dx = -R; dx <= R && keep; ++dx) keep = p[dx] == v && f[dx];
-    out[(size_t)y * W + x] = keep ? v - base : -1;
+    // staged columns lo .. hi: the first flagged, the others linked
+    const int lo = c + XP - R, hi = c + XP + R;
+    bool keep = x >= R && y >= R && x + R < W && y + R < H && (flags[r][lo >> 5] >> (lo & 31) & 1u);
+    for (int w = (lo + 1) >> 5; keep && w <= hi >> 5; ++w) {
+      unsigned m = 0xffffffffu;
+      if (w == (lo + 1) >> 5) m &= 0xffffffffu << ((lo + 1) & 31);
+      if (w == hi >> 5) m &= 0xffffffffu >> (31 - (hi & 31));
+      if (lo < hi) keep = (links[r][w] & m) == m;
+    }
+    out[(size_t)y * W + x] = keep ? lab[(r + R) * SW + (c + XP)] - base : -1;
   }
 }
 
@@ -273,12 +298,18 @@ __device__ __forceinline__ float lin100(int byte) {
 }
 
 // L* / 100 from linear channels (conversion.inl:22-24 Y row, :46-64 L*).
-__device__ __forceinline__ float lum_from_lin(float r, float g, float b) {
-  const float Y = __fadd_rn(__fadd_rn(__fmul_rn(r, 0.2126729f), __fmul_rn(g, 0.7151522f)),
-                            __fmul_rn(b, 0.0721750f));
+__device__ __forceinline__ float lum_r(float r) { return __fmul_rn(r, 0.2126729f); }
+__device__ __forceinline__ float lum_g(float g) { return __fmul_rn(g, 0.7151522f); }
+__device__ __forceinline__ float lum_b(float b) { return __fmul_rn(b, 0.0721750f); }
+__device__ __forceinline__ float lum_from_parts(float r, float g, float b) {
+  const float Y = __fadd_rn(__fadd_rn(r, g), b);
   const float y = __fmul_rn(Y, 0.01f);
   const float fy = y > 0.008856f ? cbrtf(y) : __fadd_rn(__fmul_rn(7.787f, y), 16.0f / 116.0f);
   return __fmul_rn(__fsub_rn(__fmul_rn(116.0f, fy), 16.0f), 0.01f);
+}
+
+__device__ __forceinline__ float lum_from_lin(float r, float g, float b) {
+  return lum_from_parts(lum_r(r), lum_g(g), lum_b(b));
 }
 
 // ---- Sobel normals --------------------------------------------------------------
@@ -376,28 +407,57 @@ normals_kernel(const __grid_constant__ CUtensorMap tmap, bool use_tma, NormArgs 
 
 // RGB8 -> luminance tile -> normals; staged bytes (3 TW + 32) x (TH + 2)
 // from byte column 3 tx0 - 16.
+//
+// Bound by instruction issue, most of it the luminance.  A thread takes four
+// pixels, twelve bytes in three words and one 16-byte store, and the products
+// of a channel's 256 values with its weight come from a table of their own
+// (the same products; the cube roots of four pixels overlap).  3840 x 2160:
+// 35.5 us with a pixel at a time, 32.7; the bytes read and floats
+// written take 18.4 us.
 __global__ void __launch_bounds__(kThreads)
 normals_rgb8_kernel(const __grid_constant__ CUtensorMap tmap, bool use_tma, NormArgs a,
                     Geoms gs) {
   pdl_wait();
-  constexpr int SWB = 3 * TW + 32, SH = TH + 2, HP = TW + 2;
+  // a row of luminances: the pixels at column kLumX, so that they start on 16
+  // bytes, the halo on either side
+  constexpr int SWB = 3 * TW + 32, SH = TH + 2, kLumX = 4, HP = TW + 8, kQuads = TW / 4;
   __shared__ __align__(128) unsigned char bytes[SWB * SH];
-  __shared__ float lum[SH * HP];
-  __shared__ float lin[256];
+  __shared__ __align__(16) float lum[SH * HP];
+  __shared__ float weighted[3][256];
   __shared__ __align__(8) uint64_t bar;
   const TileRef t = tile_ref(gs, blockIdx.x);
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) lin[i] = lin100(i);
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    const float v = lin100(i);
+    weighted[0][i] = lum_r(v);
+    weighted[1][i] = lum_g(v);
+    weighted[2][i] = lum_b(v);
+  }
   const CUtensorMap* map = pick_map(gs, t, use_tma ? &tmap : nullptr, kTmaRgb);
   if (!stage<unsigned char>(bytes, map, a.rgb + 3 * t.off, 3 * t.W, t.H, 3 * t.tx0 - 16,
                             t.ty0 - 1, SWB, SH, &bar, a.status))
     return;
-  for (int i = threadIdx.x; i < SH * HP; i += blockDim.x) {
-    const int r = i / HP, c = i % HP;  // pixel x = tx0 - 1 + c
+  auto luminance = [&](unsigned r, unsigned g, unsigned b) {
+    return lum_from_parts(weighted[0][r], weighted[1][g], weighted[2][b]);
+  };
+  for (int i = threadIdx.x; i < SH * kQuads; i += blockDim.x) {
+    const int r = i / kQuads, q = i % kQuads;
+    const unsigned* w = reinterpret_cast<const unsigned*>(bytes + r * SWB + 16 + 12 * q);
+    const unsigned w0 = w[0], w1 = w[1], w2 = w[2];
+    float4 v;
+    v.x = luminance(w0 & 255u, w0 >> 8 & 255u, w0 >> 16 & 255u);
+    v.y = luminance(w0 >> 24, w1 & 255u, w1 >> 8 & 255u);
+    v.z = luminance(w1 >> 16 & 255u, w1 >> 24, w2 & 255u);
+    v.w = luminance(w2 >> 8 & 255u, w2 >> 16 & 255u, w2 >> 24);
+    *reinterpret_cast<float4*>(lum + r * HP + kLumX + 4 * q) = v;
+  }
+  // the halo columns, from the threads that had one quad fewer
+  for (int i = (int)blockDim.x - 1 - (int)threadIdx.x; i < 2 * SH; i += blockDim.x) {
+    const int r = i >> 1, c = (i & 1) * (TW + 1);   // pixel x = tx0 - 1 + c
     const unsigned char* p = bytes + r * SWB + 3 * c + 13;
-    lum[i] = lum_from_lin(lin[p[0]], lin[p[1]], lin[p[2]]);
+    lum[r * HP + kLumX - 1 + c] = luminance(p[0], p[1], p[2]);
   }
   __syncthreads();
-  sobel_tile(lum, HP, t.tx0, t.ty0, t.W, t.H, a.zinv, a.out + 3 * t.off);
+  sobel_tile(lum + kLumX - 1, HP, t.tx0, t.ty0, t.W, t.H, a.zinv, a.out + 3 * t.off);
 }
 
 // ---- feature packing ------------------------------------------------------------
@@ -487,12 +547,19 @@ __global__ void lab_max_kernel(const uint8_t* __restrict__ rgb, int64_t n, unsig
     kl = max(kl, okey(c.L));
     ka = max(ka, okey(fabsf(c.a)));
   }
+  // one atomic per block and word: a warp's each, 19 thousand on two addresses,
+  // were half of the 18 us at 1.2 Mpx (now 9.0)
+  __shared__ unsigned top[2];
+  if (threadIdx.x < 2) top[threadIdx.x] = 0u;
+  __syncthreads();
   kl = __reduce_max_sync(0xffffffffu, kl);
   ka = __reduce_max_sync(0xffffffffu, ka);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(maxima, kl);
-    atomicMax(maxima + 1, ka);
+    atomicMax(top, kl);
+    atomicMax(top + 1, ka);
   }
+  __syncthreads();
+  if (threadIdx.x < 2) atomicMax(maxima + threadIdx.x, top[threadIdx.x]);
 }
 
 // pass 2: (beta, a*, b*) features and L* (beta_feature.cu:26-45: beta = -mu
@@ -596,7 +663,8 @@ using namespace sg;
 
 extern "C" int split_erode(const int32_t* labels_in, int32_t* labels_out, int width, int height,
                            int radius, void* stream) {
-  if (!labels_in || !labels_out || width < 1 || height < 1 || radius < 1 || radius > 16)
+  if (!labels_in || !labels_out || width < 1 || height < 1 || radius < 1 ||
+      radius > stn::kMaxRadius)
     return SPLIT_ERR_INVALID;
   if ((int64_t)width * height > 0x7fffffffLL) return SPLIT_ERR_INVALID;
   const size_t n = (size_t)width * height;
@@ -611,7 +679,7 @@ extern "C" int split_erode_mapped(const int32_t* labels_in, int32_t* labels_out,
                                   int height, int radius, const void* merge_workspace,
                                   void* stream) {
   if (!labels_in || !labels_out || !merge_workspace || width < 1 || height < 1 || radius < 1 ||
-      radius > 16)
+      radius > stn::kMaxRadius)
     return SPLIT_ERR_INVALID;
   if ((int64_t)width * height > 0x7fffffffLL) return SPLIT_ERR_INVALID;
   const size_t n = (size_t)width * height;
