@@ -17,7 +17,7 @@
 // write pass that recomputes each item's outputs).  The pairs need no order
 // before the sort, and a boundary repeats its pair at every pixel: each tile
 // keeps its distinct pairs in a shared-memory set and appends those (a 1080p
-// labelling of 400 segments and 4000 single pixels: about 20 thousand keys to
+// labelling of 400 segments and 4000 single pixels: 12 to 20 thousand keys to
 // sort for 0.9 million edges).  One cooperative launch sorts the keys, 64 bits,
 // and keeps one of each: a few by their ranks in sorted tiles, more by a stable
 // LSD radix sort (8-bit digits; a digit equal in every key is skipped).
@@ -314,54 +314,87 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
 // tile holds (and that is the first of its run in its own) goes out, at the
 // number of such keys below it in all tiles: one binary search per tile, whose
 // loads meet in the caches, the keys of a warp being neighbours in order.
-// Bound by the barriers and the searches' latency, four tiles in flight.
-// 20 thousand keys (20 tiles): 50 us; the 27 launches of a digit sort and
-// compaction took 158 us.
+// Bound by the barriers and the searches' latency, kWide tiles in flight.
+// 12 thousand keys (12 tiles): 28 us, of which the three barriers are 7; with
+// four searches in flight and the tiles sorted in shared memory 50; the 27
+// launches of a digit sort and compaction took 158 us.
 
-// places of `key` in tiles t0 .. t0 + 3 (tiles past the last repeat it)
+// places of `key` in the kWide tiles from t0 on (tiles past the last repeat it)
+constexpr int kWide = 16;
 __device__ __forceinline__ void lower_bounds(const unsigned long long* a, int t0, int tiles,
-                                             unsigned long long key, int (&at)[4]) {
-  const unsigned long long* s[4];
+                                             unsigned long long key, int (&at)[kWide]) {
+  int base[kWide];
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    s[g] = a + (size_t)min(t0 + g, tiles - 1) * kRankTile;
+  for (int g = 0; g < kWide; ++g) {
+    base[g] = min(t0 + g, tiles - 1) * kRankTile;
     at[g] = 0;
   }
 #pragma unroll
   for (int step = kRankTile / 2; step > 0; step >>= 1)
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      if (s[g][at[g] + step - 1] < key) at[g] += step;
+    for (int g = 0; g < kWide; ++g)
+      if (a[base[g] + at[g] + step - 1] < key) at[g] += step;
 #pragma unroll
-  for (int g = 0; g < 4; ++g)
-    if (s[g][at[g]] < key) ++at[g];
+  for (int g = 0; g < kWide; ++g)
+    if (a[base[g] + at[g]] < key) ++at[g];
+}
+
+// Bitonic sort of a block's kRankTile keys, kPer per thread: key j of a thread
+// is element warp * kRun + 32 j + lane.  Partners up to 16 apart are in another
+// lane, 32 and 64 apart in the same thread, further in another warp and reached
+// through shared memory (6 of the 55 stages; all of them through it took 13 us
+// a tile).
+constexpr int kPer = kRankTile / kThreads, kRun = 32 * kPer;
+static_assert(kPer == 4, "partners within a thread");
+
+__device__ __forceinline__ void sort_tile(unsigned long long (&k)[kPer], unsigned long long* sm) {
+  const int e0 = (threadIdx.x >> 5) * kRun + (threadIdx.x & 31);
+  for (int size = 2; size <= kRankTile; size <<= 1)
+    for (int d = size >> 1; d > 0; d >>= 1) {
+      unsigned long long o[kPer];
+      if (d >= kRun) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) sm[e0 + 32 * j] = k[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) o[j] = sm[(e0 + 32 * j) ^ d];
+      } else if (d >= 32) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) o[j] = d == 32 ? k[j ^ 1] : k[j ^ 2];
+      } else {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) o[j] = __shfl_xor_sync(0xffffffffu, k[j], d);
+      }
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const int e = e0 + 32 * j;
+        // the lower partner keeps the smaller key where the run ascends
+        const bool smaller = ((e & d) == 0) == ((e & size) == 0);
+        if ((o[j] < k[j]) == smaller) k[j] = o[j];
+      }
+    }
 }
 
 __device__ void rank_keys(const Layout& l, int n, int32_t* out0, int32_t* out1, int* d_count,
                           unsigned long long* sm) {
   const int tiles = (n + kRankTile - 1) / kRankTile;
-  const int step = gridDim.x * kThreads, first = blockIdx.x * kThreads + threadIdx.x;
+  // warps of consecutive keys, dealt out over the blocks
+  const int step = gridDim.x * kThreads;
+  const int first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
   // a tile's keys in order, filled up with the largest value (no key: the two
   // labels of a pair differ)
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-    for (int i = threadIdx.x; i < kRankTile; i += kThreads)
-      sm[i] = t * kRankTile + i < n ? l.keys[0][t * kRankTile + i] : ~0ull;
-    for (int size = 2; size <= kRankTile; size <<= 1)
-      for (int d = size >> 1; d > 0; d >>= 1) {
-        __syncthreads();
-        for (int q = threadIdx.x; q < kRankTile / 2; q += kThreads) {
-          const int i = ((q & ~(d - 1)) << 1) | (q & (d - 1)), j = i | d;
-          const unsigned long long a = sm[i], b = sm[j];
-          if ((a > b) == ((i & size) == 0)) {
-            sm[i] = b;
-            sm[j] = a;
-          }
-        }
-      }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kRankTile; i += kThreads)
-      l.keys[1][t * kRankTile + i] = sm[i];
-    __syncthreads();
+    unsigned long long k[kPer];
+    const int e0 = (threadIdx.x >> 5) * kRun + (threadIdx.x & 31);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = t * kRankTile + e0 + 32 * j;
+      k[j] = i < n ? l.keys[0][i] : ~0ull;
+    }
+    sort_tile(k, sm);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) l.keys[1][t * kRankTile + e0 + 32 * j] = k[j];
   }
   if (!grid_barrier(l.hdr)) return;
   // per tile, the keys that go out (1), then the number of those before each
@@ -372,17 +405,16 @@ __device__ void rank_keys(const Layout& l, int n, int32_t* out0, int32_t* out1, 
     const unsigned long long key = a[i];
     const int t = i / kRankTile;
     bool seen = i % kRankTile != 0 && a[i - 1] == key;
-    for (int e = 0; e < t && !seen; e += 4) {
-      int at[4];
+    for (int e = 0; e < t && !seen; e += kWide) {
+      int at[kWide];
       lower_bounds(a, e, t, key, at);
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
+      for (int g = 0; g < kWide; ++g)
         seen |= at[g] < kRankTile && a[min(e + g, t - 1) * kRankTile + at[g]] == key;
     }
     out[i + t] = !seen;
   }
   if (!grid_barrier(l.hdr)) return;
-  constexpr int kPer = kRankTile / kThreads;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     int* const o = out + t * (kRankTile + 1);
     int v[kPer], sum = 0;
@@ -407,11 +439,11 @@ __device__ void rank_keys(const Layout& l, int n, int32_t* out0, int32_t* out1, 
     if (o[0] == o[1]) continue;
     const unsigned long long key = a[i];
     int pos = 0;
-    for (int e = 0; e < tiles; e += 4) {
-      int at[4];
+    for (int e = 0; e < tiles; e += kWide) {
+      int at[kWide];
       lower_bounds(a, e, tiles, key, at);
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
+      for (int g = 0; g < kWide; ++g)
         if (e + g < tiles) pos += out[(e + g) * (kRankTile + 1) + at[g]];
     }
     out0[pos] = (int)((unsigned)(key >> 32) ^ 0x80000000u);
@@ -531,7 +563,8 @@ __device__ void radix_keys(const Layout& l, int n, int32_t* out0, int32_t* out1,
 
 // One cooperative launch: the number of keys is known on the device only, and
 // launches for the path not taken would cost more than ranking does.
-__global__ void __launch_bounds__(kThreads) sort_kernel(const Layout l, int32_t* out0,
+// Two blocks per SM: the searches' registers, and half the arrivals of four.
+__global__ void __launch_bounds__(kThreads, 2) sort_kernel(const Layout l, int32_t* out0,
                                                          int32_t* out1, int* d_count) {
   __shared__ union {
     unsigned long long tile[kRankTile];

@@ -135,13 +135,16 @@ __device__ void insert(const Layout& L, unsigned long long key, unsigned m, unsi
 // table and reach the global one as one entry per tile and pair.  The norms'
 // 62-bit values are added as four 16-bit pieces: a tile has at most 2^13
 // edges, so a piece's sum stays below 2^29.  A pair that the tile's table has
-// no room for within a short probe goes to the global one directly.
+// no room for within a short probe goes to the global one directly.  1080p, 400
+// segments and 4000 single pixels: 81 us for a norm kernel and a kernel that
+// pushed every directed edge into the global table, 24 us; seven blocks per SM
+// hold the 1020 tiles at once (six: 33 us).
 constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 1;
 constexpr int kPairBits = 9, kPairs = 1 << kPairBits, kPairProbes = 16;
 constexpr int kTilePx = kTileH * kTileW;
 static_assert(kTilePx <= 1 << 11 && kThreads % kTileW == 0, "list entries; pixels per thread");
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 7)
 edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geoms gs, Layout L,
             int* status) {
   __shared__ int tile[kHaloH * kHaloW];
