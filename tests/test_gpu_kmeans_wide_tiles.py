@@ -1,0 +1,37 @@
+"""More than 64 clusters at the edges of the 64 x 16 tiles: ragged tiles, rows of
+odd widths, tiles whose candidate list is longer than their 128 sums, negative
+and large features (which leave the tile's 32-bit sums); labels equal the
+FP32-exact oracle's and the centroids the FP64 means, within 1e-5 relative:
+features are summed exactly after rounding to multiples of 2^-24."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,k,scale,shift", [
+    (64, 16, 70, 1.0, 0.0), (65, 17, 70, 1.0, 0.0), (63, 33, 200, 1.0, 0.0),
+    (130, 31, 300, 1.0, 0.0),              # noise: every cluster is a candidate
+    (7, 50, 65, 1.0, -0.5), (96, 40, 100, 30000.0, 0.0), (1, 70, 65, 1.0, 0.0)])
+@pytest.mark.parametrize("dim", [3, 5])
+def test_tiles(cuda, w, h, k, scale, shift, dim):
+    import torch
+    from split_gb300 import kmeans
+    rng = np.random.default_rng(w * h + dim)
+    n = w * h
+    feats = ((rng.random((dim, n)) + shift) * scale).astype(np.float32)
+    c0 = feats[:, rng.choice(n, size=k, replace=n < k)].copy()
+    cent = torch.from_numpy(c0).to(cuda)
+    labels = torch.full((n,), -7, dtype=torch.int32, device=cuda)
+    ws = kmeans.cluster(torch.from_numpy(feats).to(cuda), cent, labels, None, 1, -1.0, dim=dim,
+                        width=w)
+    torch.cuda.synchronize()
+    ws.check("cluster")
+    lab = labels.cpu().numpy()
+    assert np.array_equal(lab, oracle.kmeans_assign_f32(feats, c0))
+    want = oracle.kmeans_update_f64(lab, feats, c0)
+    want = want[0] if isinstance(want, tuple) else want
+    got = cent.cpu().numpy().astype(np.float64)
+    assert (np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1e-3)).all()
