@@ -224,53 +224,76 @@ __global__ void reset_kernel(const Layout l, int* d_count) {
 }
 
 // The distinct pair keys of one tile of pixels, appended to keys[0] in any
-// order; a pair that the set has no room for within a short probe is appended
-// as it is (the sort brings the copies together).  A key is never 0: its two
-// labels differ.  Every append has an edge of its own, so 8 n keys hold all.
-constexpr int kPixH = 32, kPixW = 64, kHaloW = kPixW + 2, kHaloH = kPixH + 2;
-constexpr int kSetBits = 11, kSetProbes = 16;
+// order.  A pair borders both ways, so four of the eight neighbours (east,
+// south-west, south, south-east) find it and both its keys are appended; a
+// pair that the set has no room for within a short probe is appended as it is
+// (the sort brings the copies together).  A key is never 0: its two labels
+// differ.  Every pair appended has an edge of its own, at most 4 n there are,
+// so 8 n keys hold all.  The pixels that have an edge go to a list first, which
+// the block walks densely.  1080p, 400 segments and 4000 single pixels: 23 us
+// with all eight neighbours at every pixel, 14 us.
+constexpr int kPixH = 32, kPixW = 64, kHaloW = kPixW + 2, kHaloH = kPixH + 1;
+constexpr int kSetBits = 10, kSetProbes = 16;
+static_assert(kPixH * kPixW <= 1 << 11 && kThreads % kPixW == 0, "list entries; whole rows");
 __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restrict__ lab, int w,
                                                          int h, const Layout l) {
   __shared__ int tile[kHaloH * kHaloW];
   __shared__ unsigned long long set[1 << kSetBits];
-  __shared__ int found, base;
+  __shared__ unsigned short todo[kPixH * kPixW];   // local pixel, then its edges in 4 bits
+  __shared__ int ntodo, found, base;
   pdl_wait();
   const int tiles_x = (w + kPixW - 1) / kPixW;
   const int x0 = (int)(blockIdx.x % tiles_x) * kPixW, y0 = (int)(blockIdx.x / tiles_x) * kPixH;
-  // pixels outside the image take the nearest inside: a neighbour of its own
-  // tile's pixel, so no pair is added
-  bool mixed = false;
-  const int first = __ldg(lab + (size_t)y0 * w + x0);
+  if (threadIdx.x == 0) ntodo = found = 0;
+  // pixels outside the image take the nearest inside: the pixel itself or
+  // another of its neighbours, so no pair is added
   for (int q = threadIdx.x; q < kHaloH * kHaloW; q += kThreads) {
-    const int y = min(max(y0 - 1 + q / kHaloW, 0), h - 1);
+    const int y = min(y0 + q / kHaloW, h - 1);
     const int x = min(max(x0 - 1 + q % kHaloW, 0), w - 1);
     tile[q] = __ldg(lab + (size_t)y * w + x);
-    mixed |= tile[q] != first;
   }
-  if (!__syncthreads_or(mixed)) return;
   for (int i = threadIdx.x; i < (1 << kSetBits); i += kThreads) set[i] = 0ull;
-  if (threadIdx.x == 0) found = 0;
   __syncthreads();
+  const int lane = threadIdx.x & 31, lx = threadIdx.x % kPixW;
+#pragma unroll
+  for (int r = 0; r < kPixH; r += kThreads / kPixW) {
+    const int ly = threadIdx.x / kPixW + r;
+    const int* c = tile + ly * kHaloW + lx + 1;
+    const int v = c[0];
+    unsigned m = 0u;
+    if (x0 + lx < w && y0 + ly < h)
+      m = (c[1] != v ? 1u : 0u) | (c[kHaloW - 1] != v ? 2u : 0u) | (c[kHaloW] != v ? 4u : 0u) |
+          (c[kHaloW + 1] != v ? 8u : 0u);
+    const unsigned any = __ballot_sync(0xffffffffu, m != 0u);
+    if (any) {
+      int at = lane == 0 ? atomicAdd(&ntodo, __popc(any)) : 0;
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(any & ((1u << lane) - 1u));
+      if (m) todo[at] = (unsigned short)((ly * kPixW + lx) << 4 | m);
+    }
+  }
+  __syncthreads();
+  const int nt = ntodo;
+  if (nt == 0) return;
   unsigned long long o_or = 0ull, o_and = ~0ull;
   auto append = [&](unsigned long long key, int at) {
+    const unsigned long long back = key << 32 | key >> 32;
     l.keys[0][at] = key;
-    o_or |= key;
-    o_and &= key;
+    l.keys[0][at + 1] = back;
+    o_or |= key | back;
+    o_and &= key & back;
   };
-  for (int q = threadIdx.x; q < kPixH * kPixW; q += kThreads) {
-    const int lx = q % kPixW, ly = q / kPixW;
-    if (x0 + lx >= w || y0 + ly >= h) continue;
-    const int* c = tile + (ly + 1) * kHaloW + lx + 1;
+  for (int q = threadIdx.x; q < nt; q += kThreads) {
+    const unsigned item = todo[q], m = item & 15u, px = item >> 4;
+    const int* c = tile + (px / kPixW) * kHaloW + px % kPixW + 1;
     const int v = *c;
-    const int t[8] = {c[-kHaloW - 1], c[-kHaloW], c[-kHaloW + 1], c[-1],
-                      c[1],           c[kHaloW - 1], c[kHaloW],   c[kHaloW + 1]};
+    const int t[4] = {c[1], c[kHaloW - 1], c[kHaloW], c[kHaloW + 1]};
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      bool add = t[a] != v;
+    for (int a = 0; a < 4; ++a) {
+      bool add = m >> a & 1u;
 #pragma unroll
       for (int b = 0; b < a; ++b) add = add && t[b] != t[a];
       if (!add) continue;
-      const unsigned long long key = pair_key(v, t[a]);
+      const unsigned long long key = pair_key(min(v, t[a]), max(v, t[a]));
       unsigned s = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kSetBits));
       bool in = false;
       for (int probe = 0; probe < kSetProbes && !in; ++probe, s = (s + 1) & ((1 << kSetBits) - 1)) {
@@ -278,24 +301,26 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
         if (k == 0ull) k = atomicCAS(&set[s], 0ull, key);
         in = k == 0ull || k == key;
       }
-      if (!in) append(key, atomicAdd(l.total, 1));
+      if (!in) append(key, atomicAdd(l.total, 2));
     }
   }
   __syncthreads();
   // the set's keys, with one place in the list per block
-  constexpr int kPer = (1 << kSetBits) / kThreads;
+  constexpr int kMine = (1 << kSetBits) / kThreads;
   int mine = 0;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) mine += set[threadIdx.x + k * kThreads] != 0ull;
-  int at = mine ? atomicAdd(&found, mine) : 0;
+  for (int k = 0; k < kMine; ++k) mine += set[threadIdx.x + k * kThreads] != 0ull;
+  int at = mine ? atomicAdd(&found, 2 * mine) : 0;
   __syncthreads();
   if (threadIdx.x == 0) base = found ? atomicAdd(l.total, found) : 0;
   __syncthreads();
   at += base;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
+  for (int k = 0; k < kMine; ++k) {
     const unsigned long long key = set[threadIdx.x + k * kThreads];
-    if (key != 0ull) append(key, at++);
+    if (key == 0ull) continue;
+    append(key, at);
+    at += 2;
   }
   // digits that differ between keys (a digit equal in all is not sorted on)
 #pragma unroll
@@ -303,7 +328,7 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
     o_or |= __shfl_xor_sync(0xffffffffu, o_or, o);
     o_and &= __shfl_xor_sync(0xffffffffu, o_and, o);
   }
-  if ((threadIdx.x & 31) == 0 && (o_or != 0ull || o_and != ~0ull)) {
+  if (lane == 0 && (o_or != 0ull || o_and != ~0ull)) {
     atomicOr(l.bits, o_or);
     atomicAnd(l.bits + 1, o_and);
   }
