@@ -88,6 +88,23 @@ __device__ __forceinline__ unsigned key_hash(unsigned long long key, int bits) {
   return (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - bits));
 }
 
+// The call's words of the header to zero; and, when the workspace was last used
+// for another layout (another image size moves the pieces over each other),
+// the pieces that every call leaves clean.  A fresh workspace (stamp 0) is
+// zero-filled by its owner; relabel_kernel records the layout.
+__global__ void __launch_bounds__(kThreads)
+guard_kernel(Layout L, unsigned long long stamp, long long n) {
+  pdl_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    L.hdr->barrier_count = *L.maxsq = *L.list_count = 0u;
+  const unsigned long long last = L.hdr->stamp;
+  if (last == stamp || last == 0ull) return;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = first; i < n; i += step) L.best[i] = L.fin[i] = 0ull;
+  for (long long i = first; i < 1ll << L.cap_log2; i += step) L.slots[i] = Slot{};
+}
+
 // |p - q| over feature rows 0..2, the sum of squares in row order
 __device__ __forceinline__ float edge_norm(const float (&p)[3], const float (&q)[3]) {
   float s = 0.0f;
@@ -152,6 +169,7 @@ edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geom
   __shared__ unsigned count[kPairs], piece[4][kPairs];
   __shared__ unsigned short todo[kTilePx];   // local pixel, then its edges in 4 bits
   __shared__ unsigned ntodo, maxsq;
+  pdl_wait();
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, blockIdx.x);
   const int W = tr.W, H = tr.H;
@@ -358,8 +376,9 @@ __device__ __forceinline__ int final_of(const Layout& L, unsigned n, unsigned ca
 // it carries the call's number, so fin is never cleared.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
-relabel_kernel(int32_t* __restrict__ lab, long long n, Layout L) {
+relabel_kernel(int32_t* __restrict__ lab, long long n, Layout L, unsigned long long stamp) {
   pdl_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0) L.hdr->stamp = stamp;
   const unsigned call = *L.call, cnt = *L.list_count;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -409,14 +428,16 @@ extern "C" int split_merge_smooth(int32_t* labels, int width, int height, const 
     return SPLIT_ERR_WORKSPACE;
   l = carve(workspace, n);
   cudaStream_t st = as_stream(stream);
-  // the barrier words, the norm maximum and the slot counter start at zero;
-  // the table and the bids are kept clean by relabel_kernel (a fresh workspace
-  // is zero-filled by its owner)
-  SG_CUDA_TRY(cudaMemsetAsync(&l.hdr->barrier_count, 0, 4 * sizeof(unsigned), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
   const Geoms gs = single_geom(width, height);
-  edge_kernel<<<gs.total_tiles, kThreads, 0, st>>>(labels, points, gs, l, &l.hdr->status);
+  // the high bit: another workspace layout than the small-segment merge's
+  const unsigned long long stamp =
+      1ull << 63 | (unsigned long long)l.cap_log2 << 40 | (unsigned long long)n;
+  launch_pdl(guard_kernel, dim3(di.sm_count), dim3(kThreads), 0, st, l, stamp, (long long)n);
+  SG_TRY(launch_status());
+  launch_pdl(edge_kernel, dim3(gs.total_tiles), dim3(kThreads), 0, st, (const int32_t*)labels,
+             points, gs, l, &l.hdr->status);
   SG_TRY(launch_status());
   {
     // one co-resident block per SM; the header clear above zeroed the barrier
@@ -435,6 +456,6 @@ extern "C" int split_merge_smooth(int32_t* labels, int width, int height, const 
   const int64_t cap = (int64_t)di.sm_count * 8;
   if (blocks > cap) blocks = cap;
   launch_pdl(vec ? relabel_kernel<true> : relabel_kernel<false>, dim3((unsigned)blocks),
-             dim3(kThreads), 0, st, labels, (long long)n, l);
+             dim3(kThreads), 0, st, labels, (long long)n, l, stamp);
   return launch_status();
 }

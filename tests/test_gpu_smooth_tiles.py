@@ -37,3 +37,20 @@ def test_merge_over_tiles(cuda, shape, block, salt, offset):
         ws = ccl.merge_smooth_boundaries(dev, 0, got, ws, threshold)
         ws.check("merge_smooth")
         assert np.array_equal(got.cpu().numpy(), ref)
+
+
+def test_workspace_across_sizes(cuda):
+    """One workspace for images of different sizes, back and forth."""
+    import torch
+    from split_gb300 import ccl
+    ws = ccl.Workspace(ccl.merge_smooth_boundaries_workspace(300, 200), cuda)
+    for w, h in ((300, 200), (70, 50), (290, 190), (300, 200), (128, 64), (300, 200)):
+        rng = np.random.default_rng(w)
+        y, x = np.mgrid[0:h, 0:w]
+        seg = (y // 9 * 9 * w + x // 9 * 9).astype(np.int32)
+        pts = (rng.integers(0, 3, size=h * w)[seg.ravel()] * 0.4
+               + rng.random((3, h * w)) * 0.02).astype(np.float32)
+        got = torch.from_numpy(seg).to(cuda)
+        ccl.merge_smooth_boundaries(torch.from_numpy(pts).to(cuda), 0, got, ws, 0.05)
+        ws.check("merge_smooth")
+        assert np.array_equal(got.cpu().numpy(), oracle.merge_smooth(seg, pts, 0.05)), (w, h)
