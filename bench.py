@@ -327,7 +327,7 @@ def run_batched(dev, nimages, steps, seed=SEED + 1000):
                 for i, name in enumerate(N.PIPELINE_STAGES)}
     peak, peak_kind = peaks()
     km_bytes = sum(w * h * (16 * it + 4) for w, h, _, it in shapes)
-    bpp = {"pack": 31 * total_px, "kmeans": km_bytes, "ccl": 8 * total_px,
+    bpp = {"pack": 15 * total_px, "kmeans": km_bytes, "ccl": 8 * total_px,
            "merge": 4 * total_px, "erode": 8 * total_px}
     stages = {}
     for name, ms in stage_ms.items():
@@ -406,7 +406,7 @@ def run_batched(dev, nimages, steps, seed=SEED + 1000):
             "stages": stages,
             "stages_note": "CUDA-event time of each stage of the batch launched call by call "
                            "(median of runs, L2 flushed before each); frac = algorithmic bytes "
-                           "(features + normals 31 B/px, k-means 16 B/px per iteration + 4, "
+                           "(normals 15 B/px, k-means 16 B/px per iteration + 4, "
                            f"labelling 8, merge pair pass 4, erosion 8) / time / {peak_kind} "
                            "HBM peak",
             "launches_per_run": {"batched": int(batch_launches), "plain": int(plain_launches)}}
