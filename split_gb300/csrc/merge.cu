@@ -764,19 +764,24 @@ list_kernel(Layout L, const int32_t* lab, Geoms gs, const int32_t* sizes, int P,
   WsHeader* h = L.hdr;
   // grid barriers passed (the guard zeroed the counter they count on)
   unsigned nbar = 0;
-  // written before this launch only: the same in every block
+  // written before this launch only: the same in every block, so all of them
+  // pass the barrier or none
   const unsigned dense = *(volatile unsigned*)&L.state->dense_count;
-  bool over = *(volatile int*)&L.state->overflow != 0;
-  if (dense && !over) {
+  if (dense) {
+    // (a tile that starts after an overflow was flagged returns at once)
     for (unsigned k = blockIdx.x; k < dense; k += gridDim.x) {
       const int tile = *(volatile int*)&L.dec[gs.total_px - 1 - k];
       if (tile >= 0 && tile < gs.total_tiles)
         pair_tile<false, false>(lab, gs, L, sizes, P, policy, tab, tile, 0, 0u, &h->status);
     }
     if (!grid_barrier_counted(h, ++nbar)) return;
-    over = *(volatile int*)&L.state->overflow != 0;   // every insert came before the barrier
-    // the overflow path resets the flag behind its next barrier
   }
+  // The dense tiles set the flag too, so it is read behind that barrier only:
+  // every insert has come before, and the overflow path resets the flag behind
+  // its next barrier.  A block that read it earlier could miss a faster
+  // block's overflow, or see one and leave out a barrier that the others wait
+  // at.
+  const bool over = *(volatile int*)&L.state->overflow != 0;
   if (over) {
     overflow_path(L, lab, gs, sizes, P, policy, stamp, nbar, tab);
     return;

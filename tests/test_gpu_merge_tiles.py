@@ -38,3 +38,26 @@ def test_merge_tile_tables(cuda, policy, shape, block, values, P):
         torch.cuda.synchronize()
         ws.check("merge")
         assert np.array_equal(g.cpu().numpy(), want), k
+
+
+@pytest.mark.parametrize("policy", [0, 1])
+def test_merge_overflow_from_dense_tiles(cuda, policy):
+    """The pair pass leaves every tile to the decision launch, whose sixteen
+    blocks then overflow the global table: all of them have to go on to the
+    class-by-class decision together."""
+    import torch
+    from split_gb300 import ccl
+    h, w, block, P = 256, 512, 2, 6
+    rng = np.random.default_rng(11 + policy)
+    lab = rng.integers(0, 1000, size=(h // block, w // block))
+    seg = oracle.ccl(np.ascontiguousarray(lab.repeat(block, 0).repeat(block, 1)).astype(np.int32),
+                     8, 0)
+    chroma = (rng.integers(0, 256, size=(2, h * w)) / 256.0).astype(np.float32)
+    want = oracle.merge_small(seg, P, policy, chroma)
+    ws = None
+    for k in range(3):
+        g = torch.from_numpy(seg).to(cuda)
+        ws = ccl.merge_small_segments(torch.from_numpy(chroma).to(cuda), g, ws, P, policy=policy)
+        torch.cuda.synchronize()
+        ws.check("merge")
+        assert np.array_equal(g.cpu().numpy(), want), k
