@@ -46,6 +46,7 @@ constexpr int kThreads = 256;
 constexpr int kPairThreads = 256, kPairBlocks = 6;
 constexpr int kListThreads = 512;   // the decision launch (1024: the 4K frame 4 us more)
 constexpr int kProbeCap = 1 << 16;
+constexpr int kNearProbes = 9;   // from one of eight starts: sixteen slots of a segment
 constexpr unsigned kChainCap = 1u << 24;
 // overflow path: pending classes (level, class) on a stack, and a bound on rounds
 constexpr int kStackCap = 64;
@@ -107,12 +108,18 @@ __device__ __forceinline__ int key_t(unsigned long long k) { return (int)(unsign
 __device__ __forceinline__ int claim(const Layout& L, int s, int t, unsigned m) {
   const unsigned long long key = pair_key(s, t);
   const unsigned mask = (1u << L.cap_log2) - 1u;
-  // a segment's pairs start within eight slots of each other: its claims,
-  // counts and bids share a cache line or two
+  // A segment's first pairs share sixteen slots, so that its claims, counts and
+  // bids meet in a cache line or two; a pair that finds no room there goes on at
+  // a hash of both ids.  Without that a segment of d neighbours probes a run of
+  // its own pairs d long.
   unsigned h = (((unsigned)s * 0x9E3779B9u) >> (32 - L.cap_log2)) +
                (((unsigned)t * 0x9E3779B9u) >> 29);
   h &= mask;
-  for (int probe = 0; probe < kProbeCap; ++probe, h = (h + 1) & mask) {
+  for (int probe = 0; probe < kProbeCap; ++probe) {
+    if (probe == kNearProbes)
+      h = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - L.cap_log2));
+    else if (probe > 0)
+      h = (h + 1) & mask;
     unsigned long long k = *(volatile unsigned long long*)(L.keys + h);
     if (k == 0ull) {
       k = atomicCAS(L.keys + h, 0ull, key);

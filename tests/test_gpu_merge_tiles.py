@@ -61,3 +61,24 @@ def test_merge_overflow_from_dense_tiles(cuda, policy):
         torch.cuda.synchronize()
         ws.check("merge")
         assert np.array_equal(g.cpu().numpy(), want), k
+
+
+@pytest.mark.parametrize("policy", [0, 1])
+@pytest.mark.parametrize("step,P", [(2, 1 << 20), (3, 1 << 20), (2, 2)])
+def test_merge_many_neighbours(cuda, policy, step, P):
+    """Backgrounds that are themselves below P and border tens of thousands of
+    single pixels: thousands of pairs of one segment in the global table."""
+    import torch
+    from split_gb300 import ccl
+    h, w = 900, 777
+    y, x = np.mgrid[0:h, 0:w]
+    base = np.where(x < w // 2, 0, w // 2)   # two backgrounds side by side
+    lab = np.where((y % step == 1) & (x % step == 1), y * w + x, base).astype(np.int32)
+    rng = np.random.default_rng(step)
+    chroma = (rng.integers(0, 256, size=(2, h * w)) / 256.0).astype(np.float32)
+    want = oracle.merge_small(lab, P, policy, chroma)
+    g = torch.from_numpy(lab).to(cuda)
+    ws = ccl.merge_small_segments(torch.from_numpy(chroma).to(cuda), g, None, P, policy=policy)
+    torch.cuda.synchronize()
+    ws.check("merge")
+    assert np.array_equal(g.cpu().numpy(), want)
