@@ -85,11 +85,14 @@ struct WsHeader {
   unsigned barrier_gen;
   unsigned counter[2];   // per call, cleared by its first launch
   int result;            // a call's count, for callers that read it with the status
-  // layout the workspace's persistent state was last cleared for (0: never)
+  // layout the workspace's persistent state is clean for (no layout's: 0, never
+  // used, and kStampDirty)
   unsigned long long stamp;
   int pad[56];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
+// a call that keeps state between calls is under way, or has failed
+constexpr unsigned long long kStampDirty = ~0ull;
 
 // Bump allocator over a caller workspace; with base == nullptr it only
 // measures, so size queries and carving share one code path.

@@ -604,6 +604,9 @@ pair_kernel(const int32_t* __restrict__ lab, Geoms gs, Layout L, const int32_t* 
             int policy, int* status) {
   __shared__ PassTables tab;
   pdl_wait();
+  // from here the table and the bids hold this call's words: the stamp comes
+  // back only when the call has cleared them
+  if (blockIdx.x == 0 && threadIdx.x == 0) L.hdr->stamp = kStampDirty;
   pair_tile<false, true>(lab, gs, L, sizes, P, policy, tab, blockIdx.x, 0, 0u, status);
 }
 
@@ -688,6 +691,13 @@ __device__ void clear_bids(const Layout& L) {
     L.best[L.dec[j]] = 0ull;
 }
 
+// Records that the table and the bids are clean for the layout `stamp`, at the
+// end of a call and behind its last barrier.  A call that gave up has bids of
+// segments that no list names: its next call clears everything.
+__device__ __forceinline__ void set_stamp(WsHeader* h, unsigned long long stamp) {
+  if (*(volatile int*)&h->status == SPLIT_OK) h->stamp = stamp;
+}
+
 // ---- overflow path -----------------------------------------------------
 // The pair pass overflowed: decide class by class (see the top of the file).
 // Runs inside the cooperative decision launch; every phase sits behind a
@@ -754,7 +764,7 @@ __device__ void overflow_path(const Layout& L, const int32_t* lab, const Geoms& 
   resolve_phase(L, sizes, P, &h->status);
   if (!grid_barrier_counted(h, ++nbar)) return;
   clear_bids(L);
-  if (lead) h->stamp = stamp;
+  if (lead) set_stamp(h, stamp);
 }
 
 // The decision, one cooperative launch (at most one block per SM, see
@@ -803,7 +813,7 @@ list_kernel(Layout L, const int32_t* lab, Geoms gs, const int32_t* sizes, int P,
   if (!grid_barrier_counted(h, ++nbar)) return;
   clear_table(L);
   clear_bids(L);
-  if (blockIdx.x == 0 && threadIdx.x == 0) h->stamp = stamp;
+  if (blockIdx.x == 0 && threadIdx.x == 0) set_stamp(h, stamp);
 }
 
 // out = the final label of every pixel (out may be in), four pixels per
@@ -834,7 +844,8 @@ __global__ void relabel_kernel(const int32_t* in, int32_t* out, int64_t n, const
 // Sets the run's parameters (block 0) and clears the state that every call
 // leaves at zero (hash table, bids) when the workspace was last used with
 // another layout (or never): reusing one workspace for images of different
-// sizes moves these regions.  list_kernel records the new layout at its end.
+// sizes moves these regions.  list_kernel records the new layout at its end,
+// unless the call failed.
 __global__ void guard_kernel(WsHeader* h, unsigned long long stamp, Layout L, long long n,
                              const int32_t* sizes, int P, int policy) {
   pdl_wait();

@@ -82,3 +82,29 @@ def test_merge_many_neighbours(cuda, policy, step, P):
     torch.cuda.synchronize()
     ws.check("merge")
     assert np.array_equal(g.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("policy", [0, 1])
+def test_merge_after_refused_call(cuda, policy):
+    """A call that gives up leaves nothing behind for the next one."""
+    import torch
+    from split_gb300 import ccl
+    from split_gb300._native import SplitError
+    h, w = 64, 128
+    y, x = np.mgrid[0:h, 0:w]
+    rng = np.random.default_rng(5)
+    chroma = (rng.integers(0, 256, size=(2, h * w)) / 256.0).astype(np.float32)
+    ch = torch.from_numpy(chroma).to(cuda)
+    # one segment on half of the pixels, every other pixel its own: more pairs of
+    # one segment than half the table
+    many = np.where((x + y) % 2 == 1, y * w + x, 0).astype(np.int32)
+    g = torch.from_numpy(many).to(cuda)
+    ws = ccl.merge_small_segments(ch, g, None, h * w + 1, policy=policy)
+    with pytest.raises(SplitError):
+        ws.check("merge")
+    seg = oracle.ccl(rng.integers(0, 3, size=(h, w)).astype(np.int32), 4, 0)
+    want = oracle.merge_small(seg, 9, policy, chroma)
+    g = torch.from_numpy(seg).to(cuda)
+    ccl.merge_small_segments(ch, g, ws, 9, policy=policy)
+    ws.check("merge")
+    assert np.array_equal(g.cpu().numpy(), want)
