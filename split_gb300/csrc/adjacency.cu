@@ -178,8 +178,9 @@ __device__ T block_scan(T* a, int count) {
 
 // Prefix of the block totals (their total to *total).
 __global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(int count, int* block_sum,
-                                                                   int* total) {
+                                                                   int* total, WsHeader* hdr) {
   pdl_wait();
+  if (threadIdx.x == 0) hdr->stamp = kStampDirty;
   const int all = block_scan<kScanThreads>(block_sum, count);
   if (threadIdx.x == 0) *total = all;
 }
@@ -217,6 +218,7 @@ __global__ void reset_kernel(const Layout l, int* d_count) {
   if (threadIdx.x == 0) {
     *d_count = 0;
     l.hdr->barrier_count = 0u;
+    l.hdr->stamp = kStampDirty;
     l.total[0] = 0;
     l.bits[0] = 0ull;
     l.bits[1] = ~0ull;
@@ -626,7 +628,7 @@ extern "C" int split_segment_adjacency_edges(const int32_t* labels, int width, i
              l.block_sum);
   SG_TRY(launch_status());
   launch_pdl(adj::scan_blocks_kernel, dim3(1), dim3(adj::kScanThreads), 0, st, tiles, l.block_sum,
-             d_count);
+             d_count, l.hdr);
   SG_TRY(launch_status());
   launch_pdl(adj::write_kernel, dim3(tiles), dim3(adj::kThreads), 0, st, labels, width, height,
              (const int*)l.block_sum, (const int*)d_count, edges);

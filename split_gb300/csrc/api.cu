@@ -60,21 +60,22 @@ extern "C" const char* split_status_string(int status) {
 
 namespace sg {
 // first error in source order wins, as with set_status
-__global__ void fold_status_kernel(int* dst, StatusSources s) {
+__global__ void fold_status_kernel(WsHeader* hdr, StatusSources s) {
   pdl_wait();
   if (threadIdx.x != 0) return;
+  hdr->stamp = kStampDirty;
   for (int i = 0; i < s.n; ++i) {
     volatile int* q = s.p[i];
     const int v = *q;
     if (v) {
-      set_status(dst, v);
+      set_status(&hdr->status, v);
       *q = 0;
     }
   }
 }
 
-int fold_status(int* dst, const StatusSources& s, cudaStream_t st) {
-  launch_pdl(fold_status_kernel, dim3(1), dim3(32), 0, st, dst, s);
+int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st) {
+  launch_pdl(fold_status_kernel, dim3(1), dim3(32), 0, st, hdr, s);
   return launch_status();
 }
 

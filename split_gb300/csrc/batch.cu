@@ -313,6 +313,6 @@ extern "C" int split_batch_run_events(split_batch* b, void* const* stage_events,
     SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals, st));
   // errors the stages recorded in their own workspace headers, into the
   // batch's status word
-  SG_TRY(fold_status(&l.hdr->status, ss, st));
+  SG_TRY(fold_status(l.hdr, ss, st));
   return mark(11);
 }

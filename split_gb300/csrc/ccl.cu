@@ -503,8 +503,10 @@ border_kernel(const int32_t* __restrict__ in, Geoms gs, int* P, const int* __res
 // root's size (nobody adds to a hooked root, so its count is final).
 __global__ void __launch_bounds__(kThreads)
 flatten_kernel(int* P, Geoms gs, int32_t* __restrict__ sizes, const int* __restrict__ tword,
-               int* status) {
+               WsHeader* hdr) {
   pdl_wait();
+  int* const status = &hdr->status;
+  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->stamp = kStampDirty;
   const TileRef t = tile_ref(gs, blockIdx.x);
   const int W = t.W, tx0 = t.tx0, ty0 = t.ty0;
   const int tw = min(TW, W - tx0), th = min(TH, t.H - ty0);
@@ -624,7 +626,7 @@ static int run(const int32_t* in, const Geoms& gs, int32_t* out, int32_t* sizes,
              &hdr->status);
   SG_TRY(launch_status());
   launch_pdl(flatten_kernel, dim3(gs.total_tiles), dim3(kThreads), 0, st, out, gs, sizes,
-             (const int*)tword, &hdr->status);
+             (const int*)tword, hdr);
   return launch_status();
 }
 
@@ -697,7 +699,8 @@ __device__ __forceinline__ void load4(const int32_t* labels, int64_t n, int64_t 
 // per thread, 7.5 us with four.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads) mark_kernel(const int32_t* __restrict__ labels,
-                                                        int64_t n, uint32_t* bits, int* status) {
+                                                        int64_t n, uint32_t* bits, WsHeader* hdr) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->stamp = kStampDirty;
   const int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
   int v[4];
   load4<VEC>(labels, n, i, v);
@@ -708,7 +711,7 @@ __global__ void __launch_bounds__(kThreads) mark_kernel(const int32_t* __restric
       bad = true;
       v[j] = -2;
     }
-  if (bad) set_status(status, SPLIT_ERR_INVALID);
+  if (bad) set_status(&hdr->status, SPLIT_ERR_INVALID);
   int prev = __shfl_up_sync(0xffffffffu, v[3], 1);
   if ((threadIdx.x & 31) == 0) prev = -2;
   bool head[4];
@@ -872,7 +875,7 @@ extern "C" int split_compress_labels(int32_t* labels, int64_t n, int32_t* d_coun
   const int64_t quads = (cmp::words_of(n) + 3) / 4;
   SG_CUDA_TRY(cudaMemsetAsync(l.bits, 0, sizeof(uint4) * (size_t)quads, st));
   (vec ? cmp::mark_kernel<true> : cmp::mark_kernel<false>)
-      <<<grid, cmp::kThreads, 0, st>>>(labels, n, l.bits, &l.hdr->status);
+      <<<grid, cmp::kThreads, 0, st>>>(labels, n, l.bits, l.hdr);
   SG_TRY(launch_status());
   launch_pdl(cmp::tile_sum_kernel, dim3(tiles), dim3(cmp::kScanThreads), 0, st,
              (const uint32_t*)l.bits, quads, l.tile_sums);

@@ -91,7 +91,9 @@ struct WsHeader {
   int pad[56];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
-// a call that keeps state between calls is under way, or has failed
+// The body holds something else: a call that keeps state between calls is under
+// way or has failed, or an entry point that keeps none has used the workspace
+// (each writes this, or a zero, before it returns).
 constexpr unsigned long long kStampDirty = ~0ull;
 
 // Bump allocator over a caller workspace; with base == nullptr it only
@@ -126,8 +128,8 @@ struct StatusSources {
   int* p[8];
   int n;
 };
-__global__ void fold_status_kernel(int* dst, StatusSources s);
-int fold_status(int* dst, const StatusSources& s, cudaStream_t st);
+__global__ void fold_status_kernel(WsHeader* hdr, StatusSources s);
+int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st);
 // Clears the sources' status words before the stages run: a reused
 // workspace may hold anything where this call's sub-workspace headers lie.
 int clear_status(const StatusSources& s, cudaStream_t st);

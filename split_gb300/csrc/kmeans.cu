@@ -1775,6 +1775,7 @@ __global__ void setup_kernel(Params p, unsigned* zero, int zero_words) {
   if (threadIdx.x == 0) {
     p.hdr->barrier_count = 0u;
     p.hdr->barrier_gen = 0u;
+    p.hdr->stamp = kStampDirty;
     if (im.d_iterations && im.max_iter <= 0) *im.d_iterations = 0;
   }
   for (int i = threadIdx.x; i < zero_words; i += blockDim.x) zero[i] = 0u;

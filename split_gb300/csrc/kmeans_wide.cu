@@ -499,6 +499,7 @@ __global__ void setup_kernel(Layout L, int K, int dim, const float* __restrict__
     s.done = max_iter <= 0;
     s.arrived = 0u;
     *L.state = s;
+    L.hdr->stamp = kStampDirty;
     if (d_iter && max_iter <= 0) *d_iter = 0;
   }
   const int64_t kd = (int64_t)K * dim;

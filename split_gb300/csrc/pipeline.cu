@@ -175,7 +175,7 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
     SG_TRY(split_sobel_normals_rgb8(rgb, width, height, p.depth, normals, stream));
   // errors the stages recorded in their own workspace headers, into the
   // pipeline's status word
-  SG_TRY(fold_status(&l.hdr->status, ss, st));
+  SG_TRY(fold_status(l.hdr, ss, st));
   SG_TRY(mark(11));
   return SPLIT_OK;
 }

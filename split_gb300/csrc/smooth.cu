@@ -88,17 +88,17 @@ __device__ __forceinline__ unsigned key_hash(unsigned long long key, int bits) {
   return (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - bits));
 }
 
-// The call's words of the header to zero; and, when the workspace was last used
-// for another layout (another image size moves the pieces over each other),
-// the pieces that every call leaves clean.  A fresh workspace (stamp 0) is
-// zero-filled by its owner; relabel_kernel records the layout.
+// The call's words of the header to zero; and, unless the workspace was last
+// used for this layout and left clean (another image size moves the pieces over
+// each other, another entry point writes over them), the pieces that every call
+// leaves clean.  relabel_kernel records the layout.  The call numbers start
+// again when they run out: the entries of fin go with them.
 __global__ void __launch_bounds__(kThreads)
 guard_kernel(Layout L, unsigned long long stamp, long long n) {
   pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0)
     L.hdr->barrier_count = *L.maxsq = *L.list_count = 0u;
-  const unsigned long long last = L.hdr->stamp;
-  if (last == stamp || last == 0ull) return;
+  if (L.hdr->stamp == stamp && *L.call != ~0u) return;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = first; i < n; i += step) L.best[i] = L.fin[i] = 0ull;
@@ -173,7 +173,11 @@ edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geom
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, blockIdx.x);
   const int W = tr.W, H = tr.H;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *L.call += 1u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const unsigned last = *L.call;
+    *L.call = last == ~0u ? 1u : last + 1u;   // never 0, the mark of a cleared entry
+    L.hdr->stamp = kStampDirty;               // until the call has cleared its words
+  }
   if (threadIdx.x == 0) ntodo = maxsq = 0u;
   // -1: outside the image, or no label
   bool bad = false;
@@ -317,11 +321,16 @@ __device__ __forceinline__ int bid_target(unsigned long long b) {
 }
 
 // The segment that r maps to: its bid's target; r itself without a bid, and
-// the larger id of a pair that bid for each other.
-__device__ __forceinline__ int next_of(const Layout& L, int r) {
+// the larger id of a pair that bid for each other.  A bid's target is a segment
+// id; anything else is a corrupted workspace: the chain stops here.
+__device__ __forceinline__ int next_of(const Layout& L, int n, int r) {
   const unsigned long long b = bid_of(L, r);
   if (b == 0ull) return r;
   const int t = bid_target(b);
+  if (t < 0 || t >= n) {
+    set_status(&L.hdr->status, SPLIT_ERR_INVALID);
+    return r;
+  }
   if (r > t) {
     const unsigned long long back = bid_of(L, t);
     if (back != 0ull && bid_target(back) == r) return r;
@@ -331,12 +340,13 @@ __device__ __forceinline__ int next_of(const Layout& L, int r) {
 
 // The end of s's chain, for a segment that has a bid; one of its pairs, the
 // one it bid for, does it.
-__device__ __forceinline__ void resolve(const Layout& L, int s, int t, unsigned long long call) {
+__device__ __forceinline__ void resolve(const Layout& L, int n, int s, int t,
+                                        unsigned long long call) {
   const unsigned long long b = bid_of(L, s);
   if (!b || bid_target(b) != t) return;
   int r = s;
   for (unsigned steps = 0;; ++steps) {
-    const int nx = next_of(L, r);
+    const int nx = next_of(L, n, r);
     if (nx == r) break;
     r = nx;
     if (steps > kChainCap) {
@@ -352,15 +362,15 @@ __device__ __forceinline__ void resolve(const Layout& L, int s, int t, unsigned 
 // pairs needs both bids and nothing else, so the chain reads it off the bids
 // as it goes: no phase writes maps first, and two barriers of 1.5 us each are
 // not needed.
-__global__ void __launch_bounds__(kThreads) list_kernel(Layout L, float threshold) {
+__global__ void __launch_bounds__(kThreads) list_kernel(Layout L, float threshold, int n) {
   bid_phase(L, threshold);
   if (!grid_barrier(L.hdr)) return;
   const unsigned cnt = *(volatile unsigned*)L.list_count;
   const unsigned long long call = *L.call;
   for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
     const unsigned long long k = L.slots[L.list[j]].key;
-    resolve(L, key_s(k), key_t(k), call);
-    resolve(L, key_t(k), key_s(k), call);
+    resolve(L, n, key_s(k), key_t(k), call);
+    resolve(L, n, key_t(k), key_s(k), call);
   }
 }
 
@@ -378,7 +388,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 relabel_kernel(int32_t* __restrict__ lab, long long n, Layout L, unsigned long long stamp) {
   pdl_wait();
-  if (blockIdx.x == 0 && threadIdx.x == 0) L.hdr->stamp = stamp;
+  // (a call that failed may have left anything: the next one clears)
+  if (blockIdx.x == 0 && threadIdx.x == 0 && L.hdr->status == SPLIT_OK) L.hdr->stamp = stamp;
   const unsigned call = *L.call, cnt = *L.list_count;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -445,7 +456,8 @@ extern "C" int split_merge_smooth(int32_t* labels, int width, int height, const 
     SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, list_kernel, kThreads, 0));
     if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
     float thr = threshold;
-    void* args[] = {&l, &thr};
+    int n32 = (int)n;
+    void* args[] = {&l, &thr, &n32};
     SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)list_kernel, dim3(di.sm_count),
                                             dim3(kThreads), args, 0, st));
   }

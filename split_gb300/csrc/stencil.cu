@@ -536,8 +536,10 @@ __device__ __forceinline__ float okey_inv(unsigned k) {
 }
 
 // pass 1: the largest L* and the largest |a*| of the image (beta_feature.cu:52-64)
-__global__ void lab_max_kernel(const uint8_t* __restrict__ rgb, int64_t n, unsigned* maxima) {
+__global__ void lab_max_kernel(const uint8_t* __restrict__ rgb, int64_t n, unsigned* maxima,
+                               WsHeader* hdr) {
   __shared__ float lin[256];
+  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->stamp = kStampDirty;
   for (int i = threadIdx.x; i < 256; i += blockDim.x) lin[i] = lin100(i);
   __syncthreads();
   unsigned kl = 0, ka = 0;
@@ -804,7 +806,8 @@ extern "C" int split_pack_lab_beta(const uint8_t* rgb, int64_t npixels, float mu
   SG_TRY(device_info(&di));
   int64_t blocks = (npixels + 255) / 256;
   if (blocks > (int64_t)di.sm_count * 8) blocks = (int64_t)di.sm_count * 8;
-  stn::lab_max_kernel<<<(int)blocks, 256, 0, st>>>(rgb, npixels, maxima);
+  stn::lab_max_kernel<<<(int)blocks, 256, 0, st>>>(rgb, npixels, maxima,
+                                                    static_cast<WsHeader*>(workspace));
   SG_TRY(launch_status());
   stn::lab_beta_kernel<<<(int)blocks, 256, 0, st>>>(rgb, npixels, maxima, mu, features,
                                                      layout == SPLIT_LAYOUT_FLOAT4, luminance);
