@@ -60,10 +60,10 @@ extern "C" const char* split_status_string(int status) {
 
 namespace sg {
 // first error in source order wins, as with set_status
-__global__ void fold_status_kernel(WsHeader* hdr, StatusSources s) {
+__global__ void fold_status_kernel(WsHeader* hdr, StatusSources s, unsigned long long stamp) {
   pdl_wait();
   if (threadIdx.x != 0) return;
-  hdr->stamp = kStampDirty;
+  hdr->stamp = stamp;
   for (int i = 0; i < s.n; ++i) {
     volatile int* q = s.p[i];
     const int v = *q;
@@ -74,32 +74,21 @@ __global__ void fold_status_kernel(WsHeader* hdr, StatusSources s) {
   }
 }
 
-int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st) {
-  launch_pdl(fold_status_kernel, dim3(1), dim3(32), 0, st, hdr, s);
+int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st,
+                unsigned long long stamp) {
+  launch_pdl(fold_status_kernel, dim3(1), dim3(32), 0, st, hdr, s, stamp);
   return launch_status();
 }
 
-bool layout_unchanged(const void* workspace, unsigned long long key) {
-  struct Entry {
-    const void* ws;
-    unsigned long long key;
-  };
-  static std::mutex mu;
-  static Entry memo[256] = {};
-  const size_t i = (reinterpret_cast<uintptr_t>(workspace) >> 8) & 255;
-  std::lock_guard<std::mutex> lock(mu);
-  const bool same = memo[i].ws == workspace && memo[i].key == key;
-  memo[i] = Entry{workspace, key};
-  return same;
-}
-
-__global__ void clear_status_kernel(StatusSources s) {
+__global__ void clear_stages_kernel(StageHeaders s) {
   pdl_wait();
-  if ((int)threadIdx.x < s.n) *s.p[threadIdx.x] = 0;
+  if (threadIdx.x != 0) return;
+  enter_stages(s);
+  s.hdr->stamp = kStampDirty;
 }
 
-int clear_status(const StatusSources& s, cudaStream_t st) {
-  launch_pdl(clear_status_kernel, dim3(1), dim3(32), 0, st, s);
+int clear_stages(const StageHeaders& s, cudaStream_t st) {
+  launch_pdl(clear_stages_kernel, dim3(1), dim3(32), 0, st, s);
   return launch_status();
 }
 }  // namespace sg

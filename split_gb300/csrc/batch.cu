@@ -239,11 +239,15 @@ extern "C" int split_batch_bind(split_batch* b, const uint8_t* rgb, float* centr
                               cudaMemcpyHostToDevice, st));
   // a rebound arena may hold anything where this layout's stage headers lie
   {
-    StatusSources ss{};
+    StageHeaders sh{};
+    sh.hdr = l.hdr;
+    sh.stamp = kStampNone;
+    StatusSources& ss = sh.status;
     ss.p[ss.n++] = &static_cast<WsHeader*>(l.km_ws)->status;
     ss.p[ss.n++] = &static_cast<WsHeader*>(l.ccl_ws)->status;
     if (l.mrg_ws) ss.p[ss.n++] = &static_cast<WsHeader*>(l.mrg_ws)->status;
-    SG_TRY(clear_status(ss, st));
+    sh.keeps = static_cast<WsHeader*>(l.mrg_ws);
+    SG_TRY(clear_stages(sh, st));
   }
   SG_CUDA_TRY(cudaStreamSynchronize(st));
   b->bound = true;

@@ -95,6 +95,7 @@ static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 // way or has failed, or an entry point that keeps none has used the workspace
 // (each writes this, or a zero, before it returns).
 constexpr unsigned long long kStampDirty = ~0ull;
+constexpr unsigned long long kStampNone = ~0ull - 1;   // recorded by nobody
 
 // Bump allocator over a caller workspace; with base == nullptr it only
 // measures, so size queries and carving share one code path.
@@ -123,21 +124,32 @@ __device__ __forceinline__ void set_status(int* st, int code) {
 // carves from its own: fold_status moves the first error among them into the
 // composite workspace's own status word (read by split_workspace_status) and
 // clears them, so that a sub-stage error is never lost and never reported
-// twice.
+// twice.  It records `stamp`: the stages' headers are as this layout leaves
+// them.
 struct StatusSources {
   int* p[8];
   int n;
 };
-__global__ void fold_status_kernel(WsHeader* hdr, StatusSources s);
-int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st);
-// Clears the sources' status words before the stages run: a reused
-// workspace may hold anything where this call's sub-workspace headers lie.
-int clear_status(const StatusSources& s, cudaStream_t st);
-// Whether `workspace` was last used with layout `key` (a small direct-mapped
-// memo; records the key).  After the first run of a layout the fold leaves
-// the stage status words at zero, so the clear is needed only on a change
-// (a miss only costs a clear).
-bool layout_unchanged(const void* workspace, unsigned long long key);
+int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st,
+                unsigned long long stamp = kStampDirty);
+// What a composite call finds where its stages' headers lie: the stages' as its
+// last run left them, or, when another call or another layout has used the
+// workspace since, anything.  Then the status words go to zero and the stage
+// that keeps state (the merge) is told so.
+struct StageHeaders {
+  WsHeader* hdr;              // the composite's own (null: not a composite call)
+  unsigned long long stamp;   // its layout
+  StatusSources status;
+  WsHeader* keeps;            // may be null
+};
+// By one thread of the first launch that writes to a stage's workspace.
+__device__ __forceinline__ void enter_stages(const StageHeaders& s) {
+  if (!s.hdr || s.hdr->stamp == s.stamp) return;
+  for (int i = 0; i < s.status.n; ++i) *s.status.p[i] = 0;
+  if (s.keeps) s.keeps->stamp = kStampDirty;
+}
+// The same in a launch of its own.
+int clear_stages(const StageHeaders& s, cudaStream_t st);
 
 // Iteration limit of every spin wait (about a second with the back-off below).
 constexpr unsigned kSpinLimit = 1u << 24;

@@ -91,10 +91,11 @@ __device__ __forceinline__ TileRef tile_ref(const Geoms& gs, int tile) {
 int normals_rgb8_geoms(const uint8_t* rgb, const Geoms& gs, float depth, float* normals,
                        cudaStream_t st);
 
-// k-means over byte / 255 features read from the bytes, with the results of the
-// packed float4 ones (kmeans.cu).
-int kmeans_cluster_bytes(const uint8_t* rgb, int dim, int64_t n, int width, float xy_scale,
-                         float* centroids, int K, int32_t* labels, void* ws, size_t ws_bytes,
-                         int max_iter, float threshold, cudaStream_t st);
+// split_kmeans_cluster as a composite call's stage; `bytes` (RGB8): with the
+// results of the packed float4 features (kmeans.cu).
+int kmeans_cluster_stage(const void* points, int layout, bool bytes, int dim, int64_t n, int width,
+                         float xy_scale, float* centroids, int K, int32_t* labels, void* ws,
+                         size_t ws_bytes, int max_iter, float threshold, const StageHeaders& own,
+                         cudaStream_t st);
 
 }  // namespace sg

@@ -1767,12 +1767,14 @@ __global__ void init_kernel(Params p) {
 // Per-call setup of a single-image clustering in one launch: the header's
 // barrier and work counters and all three accumulator slots to zero
 // (`zero` .. `zero` + zero_words: the slots and the counts), the iteration
-// state (cluster.cu:65-68), and the caller's planar centroids into slot 0.
+// state (cluster.cu:65-68), and the caller's planar centroids into slot 0.  It is
+// a composite call's first launch that writes to a stage's workspace.
 template <int DIM>
-__global__ void setup_kernel(Params p, unsigned* zero, int zero_words) {
+__global__ void setup_kernel(Params p, unsigned* zero, int zero_words, StageHeaders own) {
   pdl_wait();
   const Image& im = p.img0;
   if (threadIdx.x == 0) {
+    enter_stages(own);
     p.hdr->barrier_count = 0u;
     p.hdr->barrier_gen = 0u;
     p.hdr->stamp = kStampDirty;
@@ -1908,7 +1910,8 @@ static int run(int mode, const void* points, int layout, int dim, int64_t n,
                int width, float xy_scale, float* centroids,
                const float* centroids_in, int K, int32_t* labels,
                const int32_t* labels_in, void* ws, size_t ws_bytes, int max_iter,
-               float threshold, int32_t* d_iter, cudaStream_t st, bool any_width = false) {
+               float threshold, int32_t* d_iter, cudaStream_t st, bool any_width = false,
+               const StageHeaders& own = StageHeaders{}) {
   if (!valid_features(points, layout, dim, n, width, K)) return SPLIT_ERR_INVALID;
   const int unit_range = (layout & SPLIT_FEATURES_UNIT_RANGE) ? 1 : 0;
   const int ref_shift = (layout & SPLIT_KMEANS_REFERENCE_SHIFT) ? 1 : 0;
@@ -1968,8 +1971,8 @@ static int run(int mode, const void* points, int layout, int dim, int64_t n,
   unsigned* zero = reinterpret_cast<unsigned*>(l.acc_lo);
   const int zero_words = (int)((reinterpret_cast<char*>(l.cur) -
                                 reinterpret_cast<char*>(l.acc_lo)) / sizeof(unsigned));
-  if (dim == 3) launch_pdl(setup_kernel<3>, dim3(1), dim3(256), 0, st, p, zero, zero_words);
-  else launch_pdl(setup_kernel<5>, dim3(1), dim3(256), 0, st, p, zero, zero_words);
+  if (dim == 3) launch_pdl(setup_kernel<3>, dim3(1), dim3(256), 0, st, p, zero, zero_words, own);
+  else launch_pdl(setup_kernel<5>, dim3(1), dim3(256), 0, st, p, zero, zero_words, own);
   SG_TRY(launch_status());
   if (max_iter <= 0) return SPLIT_OK;
   if (mode == kCluster) return dispatch<kCluster>(layout, dim, p, st);
@@ -1988,7 +1991,7 @@ namespace kmw {
 int run(bool cluster, const void* points, int layout, int dim, int64_t n, int width,
         float xy_scale, float* centroids, const float* cent_in, int K, int32_t* labels,
         void* ws, size_t ws_bytes, int max_iter, float threshold, int32_t* d_iter,
-        cudaStream_t st);
+        cudaStream_t st, const StageHeaders& own = StageHeaders{});
 size_t workspace_bytes(int K, int dim);
 }  // namespace kmw
 }  // namespace sg
@@ -2032,19 +2035,20 @@ extern "C" int split_kmeans_cluster(const void* points, int layout, int dim, int
                  threshold, d_iterations, as_stream(stream));
 }
 
-// byte / 255 features straight from the bytes, with the results of
+// A composite call's clustering (`own`: its stage headers).  With `bytes`
+// byte / 255 features straight from RGB8, with the results of
 // split_kmeans_cluster on the packed float4 ones (unit range): the same values
 // and, at any image width, the same fast spans.
 namespace sg {
-int kmeans_cluster_bytes(const uint8_t* rgb, int dim, int64_t n, int width, float xy_scale,
-                         float* centroids, int K, int32_t* labels, void* ws, size_t ws_bytes,
-                         int max_iter, float threshold, cudaStream_t st) {
+int kmeans_cluster_stage(const void* points, int layout, bool bytes, int dim, int64_t n, int width,
+                         float xy_scale, float* centroids, int K, int32_t* labels, void* ws,
+                         size_t ws_bytes, int max_iter, float threshold, const StageHeaders& own,
+                         cudaStream_t st) {
   if (K > km::kMaxK)
-    return kmw::run(true, rgb, SPLIT_LAYOUT_RGB8, dim, n, width, xy_scale, centroids, centroids,
-                    K, labels, ws, ws_bytes, max_iter, threshold, nullptr, st);
-  return km::run(km::kCluster, rgb, SPLIT_LAYOUT_RGB8, dim, n, width, xy_scale, centroids,
-                 centroids, K, labels, nullptr, ws, ws_bytes, max_iter, threshold, nullptr, st,
-                 true);
+    return kmw::run(true, points, layout, dim, n, width, xy_scale, centroids, centroids, K, labels,
+                    ws, ws_bytes, max_iter, threshold, nullptr, st, own);
+  return km::run(km::kCluster, points, layout, dim, n, width, xy_scale, centroids, centroids, K,
+                 labels, nullptr, ws, ws_bytes, max_iter, threshold, nullptr, st, bytes, own);
 }
 }  // namespace sg
 

@@ -488,11 +488,12 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
 
 // Initial state, the caller's centroids into cur[0], zero sums.
 __global__ void setup_kernel(Layout L, int K, int dim, const float* __restrict__ cent,
-                             int32_t* d_iter, int max_iter) {
+                             int32_t* d_iter, int max_iter, StageHeaders own) {
   pdl_wait();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nt = (int64_t)gridDim.x * blockDim.x;
   if (t == 0) {
+    enter_stages(own);
     State s;
     s.delta = 0.0f;
     s.iters = 0;
@@ -635,7 +636,7 @@ size_t workspace_bytes(int K, int dim) { return carve(nullptr, K, dim).bytes; }
 template <int LAYOUT, int DIM>
 static int queue(bool cluster, const Points& P, int K, const float* cent, float* centroids,
                  int32_t* labels, const Layout& L, int max_iter, float threshold, int ref_shift,
-                 int32_t* d_iter, cudaStream_t st) {
+                 int32_t* d_iter, const StageHeaders& own, cudaStream_t st) {
   DeviceInfo di;
   SG_TRY(device_info(&di));
   int per_sm = 0;
@@ -663,7 +664,7 @@ static int queue(bool cluster, const Points& P, int K, const float* cent, float*
   int64_t sb = ((int64_t)K * DIM + 255) / 256;
   if (sb > di.sm_count * 4) sb = di.sm_count * 4;
   SG_CUDA_TRY(launch_pdl(setup_kernel, dim3((unsigned)sb), dim3(256), 0, st, L, K, DIM, cent,
-                         d_iter, max_iter));
+                         d_iter, max_iter, own));
   SG_TRY(launch_status());
   FormArgs fa{};
   fa.L = L;
@@ -689,7 +690,7 @@ static int queue(bool cluster, const Points& P, int K, const float* cent, float*
 int run(bool cluster, const void* points, int layout, int dim, int64_t n, int width,
         float xy_scale, float* centroids, const float* cent_in, int K, int32_t* labels,
         void* ws, size_t ws_bytes, int max_iter, float threshold, int32_t* d_iter,
-        cudaStream_t st) {
+        cudaStream_t st, const StageHeaders& own) {
   const int ref_shift = (layout & SPLIT_KMEANS_REFERENCE_SHIFT) ? 1 : 0;
   layout &= ~(SPLIT_FEATURES_UNIT_RANGE | SPLIT_KMEANS_REFERENCE_SHIFT);
   if (!points || !cent_in || !labels || n <= 0 || n > 0x7fffffffLL || width < 1)
@@ -711,7 +712,7 @@ int run(bool cluster, const void* points, int layout, int dim, int64_t n, int wi
 #define SG_KMW_CASE(LY, D)                                                                  \
   if (layout == LY && dim == D)                                                             \
     return queue<LY, D>(cluster, P, K, cent_in, centroids, labels, l, max_iter, threshold,  \
-                        ref_shift, d_iter, st);
+                        ref_shift, d_iter, own, st);
   SG_KMW_CASE(SPLIT_LAYOUT_PLANAR, 3)
   SG_KMW_CASE(SPLIT_LAYOUT_PLANAR, 5)
   SG_KMW_CASE(SPLIT_LAYOUT_FLOAT4, 3)

@@ -54,6 +54,15 @@ static Layout carve(void* ws, int W, int H, const split_pipeline_params& p) {
   return l;
 }
 
+// Names what carve() depends on.  Bit 62: no merge's stamp, nor kStampDirty.
+static unsigned long long stamp_of(int W, int H, const split_pipeline_params& p) {
+  const unsigned v[] = {(unsigned)W, (unsigned)H, (unsigned)p.nclusters, (unsigned)p.dim,
+                        (unsigned)p.features, p.merge_P > 0 ? 1u : 0u, (unsigned)p.merge_policy};
+  unsigned long long h = 14695981039346656037ull;   // FNV-1a over the words
+  for (unsigned x : v) h = (h ^ x) * 1099511628211ull;
+  return (h & ((1ull << 62) - 1)) | 1ull << 62;
+}
+
 static bool valid(const split_pipeline_params* p) {
   // K above 64 runs the many-cluster k-means (split_kmeans_cluster picks it)
   return p && p->nclusters >= 1 && p->nclusters <= (1 << 20) && (p->dim == 3 || p->dim == 5) &&
@@ -97,12 +106,17 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
   l = pipe::carve(workspace, width, height, p);
   cudaStream_t st = as_stream(stream);
   const int64_t n = (int64_t)width * height;
-  // the stages' own status words (sub-workspace headers), cleared first and
-  // folded into the pipeline's status word at the end
-  StatusSources ss{};
+  // the stages' headers: cleared first, by the clustering's first launch, if
+  // another call or another layout has used the workspace since; their status
+  // words folded into the pipeline's at the end
+  StageHeaders own{};
+  own.hdr = l.hdr;
+  own.stamp = pipe::stamp_of(width, height, p);
+  StatusSources& ss = own.status;
   ss.p[ss.n++] = &static_cast<WsHeader*>(l.km_ws)->status;
   ss.p[ss.n++] = &static_cast<WsHeader*>(l.ccl_ws)->status;
   if (l.mrg_ws) ss.p[ss.n++] = &static_cast<WsHeader*>(l.mrg_ws)->status;
+  own.keeps = static_cast<WsHeader*>(l.mrg_ws);
   auto mark = [&](int i) -> int {
     if (stage_events)
       SG_CUDA_TRY(cudaEventRecord(reinterpret_cast<cudaEvent_t>(stage_events[i]), st));
@@ -110,11 +124,6 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
   };
   // 0: features
   SG_TRY(mark(0));
-  const unsigned long long layout_key =
-      ((unsigned long long)(unsigned)width << 32 | (unsigned)height) ^
-      ((unsigned long long)l.bytes << 7) ^ ((unsigned long long)p.features << 3) ^
-      (unsigned long long)(p.merge_P > 0) ^ ((unsigned long long)p.merge_policy << 1);
-  if (!layout_unchanged(workspace, layout_key)) SG_TRY(clear_status(ss, st));
   // with SPLIT_LAYOUT_FLOAT4 the normals come first (the normals stage below is
   // then empty)
   const bool first = p.features == SPLIT_LAYOUT_FLOAT4 && p.compute_normals;
@@ -126,17 +135,11 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
   SG_TRY(mark(1));
   // 1: k-means
   SG_TRY(mark(2));
-  if (p.features == SPLIT_LAYOUT_FLOAT4)
-    SG_TRY(kmeans_cluster_bytes(rgb, p.dim, n, width, p.xy_scale, centroids, p.nclusters,
-                                cluster_labels, l.km_ws, l.km_bytes, p.kmeans_iters,
-                                p.kmeans_threshold, st));
-  else
-    SG_TRY(split_kmeans_cluster(pipe::packs(p) ? static_cast<const void*>(l.features4)
-                                               : static_cast<const void*>(rgb),
-                                pipe::packs(p) ? SPLIT_LAYOUT_FLOAT4 : SPLIT_LAYOUT_RGB8, p.dim,
-                                n, width, p.xy_scale, centroids, p.nclusters, cluster_labels,
-                                l.km_ws, l.km_bytes, p.kmeans_iters, p.kmeans_threshold, nullptr,
-                                stream));
+  SG_TRY(kmeans_cluster_stage(
+      pipe::packs(p) ? static_cast<const void*>(l.features4) : static_cast<const void*>(rgb),
+      pipe::packs(p) ? SPLIT_LAYOUT_FLOAT4 : SPLIT_LAYOUT_RGB8, p.features == SPLIT_LAYOUT_FLOAT4,
+      p.dim, n, width, p.xy_scale, centroids, p.nclusters, cluster_labels, l.km_ws, l.km_bytes,
+      p.kmeans_iters, p.kmeans_threshold, own, st));
   SG_TRY(mark(3));
   // 2: connected components (+ component sizes for the merge)
   SG_TRY(mark(4));
@@ -175,7 +178,7 @@ extern "C" int split_pipeline_run(const uint8_t* rgb, int width, int height,
     SG_TRY(split_sobel_normals_rgb8(rgb, width, height, p.depth, normals, stream));
   // errors the stages recorded in their own workspace headers, into the
   // pipeline's status word
-  SG_TRY(fold_status(l.hdr, ss, st));
+  SG_TRY(fold_status(l.hdr, ss, st, own.stamp));
   SG_TRY(mark(11));
   return SPLIT_OK;
 }

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 W, H = 160, 96
 OTHERS = ["adjacency", "edges", "compress", "label", "cluster", "cluster_wide", "assign", "update",
-          "update_wide", "shading", "lab_beta", "smooth", "small", "smooth_size", "small_size"]
+          "update_wide", "shading", "lab_beta", "pipeline", "smooth", "small", "smooth_size", "small_size"]
 
 
 class Shared:
