@@ -430,15 +430,19 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
     if constexpr (ACC) {
       // Features in [0, 2^14) whose clusters fit the tile's sums (the common
       // case by far); below 2^32, the narrow fixed-point form straight into
-      // the global sums; otherwise the general form.
+      // the global sums; otherwise the general form.  A pixel that no distance
+      // named (all infinite or NaN) belongs to cluster 0, which the list may
+      // not hold: not for the tile's sums either.
       bool tiled = nchunks == 1 && nlist <= kSlots, small = true;
 #pragma unroll
-      for (int j = 0; j < kPix; ++j)
+      for (int j = 0; j < kPix; ++j) {
+        tiled = tiled && (j >= valid || bk[j] >= 0);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
           tiled = tiled && (j >= valid || (f[j][d] >= 0.0f && f[j][d] < 16384.0f));
           small = small && (j >= valid || fabsf(f[j][d]) < 4294967296.0f);
         }
+      }
       if (__all_sync(full, tiled)) {
         int at[kPix];
 #pragma unroll

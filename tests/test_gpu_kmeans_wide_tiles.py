@@ -35,3 +35,34 @@ def test_tiles(cuda, w, h, k, scale, shift, dim):
     want = want[0] if isinstance(want, tuple) else want
     got = cent.cpu().numpy().astype(np.float64)
     assert (np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1e-3)).all()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 1e25])
+@pytest.mark.parametrize("k", [64, 65, 128, 129, 1500])
+@pytest.mark.parametrize("dim", [3, 5])
+def test_no_distance_below_infinity(cuda, bad, k, dim):
+    """Centroids from which every distance is infinite or NaN: all pixels carry
+    label 0 and count in cluster 0, whatever sums their tile takes."""
+    import torch
+    from split_gb300 import kmeans
+    w, h = 70, 45
+    rng = np.random.default_rng(k + dim)
+    feats = rng.random((dim, w * h)).astype(np.float32)
+    c0 = np.full((dim, k), bad, dtype=np.float32)
+    for one in (False, True):
+        if one:   # and one finite centroid, which then gets every pixel
+            c0[:, k // 2] = 0.5
+        cent = torch.from_numpy(c0).to(cuda)
+        labels = torch.full((w * h,), -7, dtype=torch.int32, device=cuda)
+        ws = kmeans.cluster(torch.from_numpy(feats).to(cuda), cent, labels, None, 1, -1.0, dim=dim,
+                            width=w)
+        torch.cuda.synchronize()
+        lab = labels.cpu().numpy()
+        assert (lab == (k // 2 if one else 0)).all()
+        got = cent.cpu().numpy()
+        if k > 64:   # (the persistent kernel's update starts from the old centroid)
+            ws.check("cluster")
+            want = feats.astype(np.float64).mean(1)
+            assert np.allclose(got[:, lab[0]], want, rtol=1e-5, atol=0)
+        keep = np.arange(k) != lab[0]
+        assert np.array_equal(got[:, keep], c0[:, keep], equal_nan=True)
