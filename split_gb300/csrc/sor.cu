@@ -24,9 +24,11 @@
 // one the FP64 restatement in the oracle follows.  The residual test runs
 // before every sweep as in the reference's monitor; its sums are per-block
 // partials added in one fixed order by every block, so every block takes the
-// same decision and the result does not depend on timing.
+// same decision and the result does not depend on timing.  The decision is the
+// one of FP64 sums: the sums in two floats decide only where they are clear of
+// the limit, anywhere near it (or not finite) the residual is summed again in
+// FP64.
 #include <algorithm>
-#include <cfloat>
 #include <cmath>
 
 #include "common.cuh"
@@ -62,11 +64,12 @@ __device__ __forceinline__ int valence(int r, int c, int H, int W) {
   return 4 - ((r == 0 || r == H - 1) ? 1 : 0) - ((c == 0 || c == W - 1) ? 1 : 0);
 }
 
-// A sum of squares in two floats (about 48 bits): each square's product is
-// exact as p + pe, and so is each sum's rounding error, so only the small
-// word rounds.  FP64 on this part runs at two lanes per clock and SM: summing
-// the three squares of a pixel and the warp trees in FP64 took 5.6 us of a
-// VGA sweep, more than everything else in it.
+// A sum of squares in two floats (relative error below 2^-40): each square's
+// product is exact as p + pe (the fma's rest), and so is each sum's rounding
+// error (Knuth's two-sum), so only the small word rounds.  FP64 on this part
+// runs at two lanes per clock and SM: summing the three squares of a pixel and
+// the warp trees in FP64 takes 5.6 us of a VGA sweep, more than everything else
+// in it.
 struct Sum2 {
   float hi = 0.0f, lo = 0.0f;
   __device__ __forceinline__ void add(float v, float small) {
@@ -109,20 +112,18 @@ __device__ __forceinline__ void neighbour_sum(const Problem& P, const float4* y,
   }
 }
 
-// adds the squared residual of a pixel (scaled by the power of two `scale`)
-// whose unknowns are x and whose neighbours sum to S
+// the residual of a pixel whose unknowns are x and whose neighbours sum to S:
+// f(e) for each component
+template <class F>
 __device__ __forceinline__ void residual(const Problem& P, const float (&x)[3], float si, float v,
-                                         const float (&S)[3], float scale, Sum2& sum,
-                                         bool& nonzero) {
+                                         const float (&S)[3], F&& f) {
   const float lx = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], x[0]), __fmul_rn(P.L[1], x[1])),
                              __fmul_rn(P.L[2], x[2]));
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const float lap = __fsub_rn(__fmul_rn(v, x[d]), S[d]);
     const float ax = __fadd_rn(__fmul_rn(P.L[d], lx), __fmul_rn(P.lam2, lap));
-    const float e = __fsub_rn(__fmul_rn(si, P.L[d]), ax);
-    nonzero |= e != 0.0f;
-    sum.add_square(__fmul_rn(e, scale));
+    f(__fsub_rn(__fmul_rn(si, P.L[d]), ax));
   }
 }
 
@@ -210,6 +211,38 @@ struct Walk {
   }
 };
 
+// The thread's part of the squared residual of the iterate (red, blk), in FP64.
+__device__ __noinline__ double residual_fp64(Problem P, const float4* red, const float4* blk,
+                                             int chunk) {
+  double sum = 0.0;
+  for (int colour = 0; colour < 2; ++colour)
+    for (Walk w(P, chunk); w.more(); w.next()) {
+      const int c = 2 * w.k + ((w.r + colour) & 1);
+      if (c >= P.W) continue;
+      const float4 o = (colour ? blk : red)[w.i];
+      const float x[3] = {o.x, o.y, o.z};
+      float S[3];
+      neighbour_sum(P, colour ? red : blk, w.r, w.k, c, S);
+      residual(P, x, o.w, (float)valence(w.r, c, P.H, P.W), S,
+               [&](float e) { sum += (double)e * (double)e; });
+    }
+  return sum;
+}
+
+__device__ __forceinline__ Problem problem_of(const Args& a) {
+  Problem P;
+  P.L[0] = a.L0;
+  P.L[1] = a.L1;
+  P.L[2] = a.L2;
+  P.LL = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], P.L[0]), __fmul_rn(P.L[1], P.L[1])),
+                   __fmul_rn(P.L[2], P.L[2]));
+  P.lam2 = a.lam2;
+  P.W = a.W;
+  P.H = a.H;
+  P.wh = a.wh;
+  return P;
+}
+
 // One persistent cooperative launch, one block per SM at most, every block
 // owning the same contiguous packed pixels of both colours.
 //
@@ -226,16 +259,7 @@ struct Walk {
 // FP64 sums, one thread adding all blocks' partials and 760 blocks it took
 // 94 us.
 __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
-  Problem P;
-  P.L[0] = a.L0;
-  P.L[1] = a.L1;
-  P.L[2] = a.L2;
-  P.LL = __fadd_rn(__fadd_rn(__fmul_rn(P.L[0], P.L[0]), __fmul_rn(P.L[1], P.L[1])),
-                   __fmul_rn(P.L[2], P.L[2]));
-  P.lam2 = a.lam2;
-  P.W = a.W;
-  P.H = a.H;
-  P.wh = a.wh;
+  const Problem P = problem_of(a);
   unsigned nbar = 0;
   float4 *red = a.red, *red_next = a.red_next, *blk = a.black, *blk_next = a.black_next;
   // x0 = (0, 0, 1) and |b|^2 = sum s_i^2 |L|^2
@@ -256,15 +280,17 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
       block_total(has ? __ldcg(a.partial + kMaxBlocks + threadIdx.x) : 0.0, (int)gridDim.x) *
       (double)P.LL;
   // the residual is summed scaled by a power of two near 1 / |b|, so that its
-  // squares neither overflow nor vanish in FP32 at any intensity
+  // squares neither overflow nor vanish in FP32 at ordinary intensities
   int ex = 0;
   if (bnorm2 > 0.0 && bnorm2 < INFINITY) ex = -(ilogb(bnorm2) / 2);
   ex = max(-120, min(120, ex));
   const float scale = ldexpf(1.0f, ex);
   const double limit2 = (double)a.tol * (double)a.tol * bnorm2 * ldexp(1.0, 2 * ex);
+  // The scaled sum's error: below 2^-40 of it, and what its squares lose below
+  // FP32's range, under 2^-110 in all.  Within 2^-20 and 2^-90 FP64 decides.
+  const double band = limit2 * 0x1p-20 + 0x1p-90;
   // the black pixels' residual at x0
   Sum2 black;
-  bool black_nz = false;
   for (Walk w(P, chunk); w.more(); w.next()) {
     const int c = 2 * w.k + ((w.r + 1) & 1);
     if (c >= P.W) continue;
@@ -272,14 +298,14 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
     const float x[3] = {o.x, o.y, o.z};
     float S[3];
     neighbour_sum(P, red, w.r, w.k, c, S);
-    residual(P, x, o.w, (float)valence(w.r, c, P.H, P.W), S, scale, black, black_nz);
+    residual(P, x, o.w, (float)valence(w.r, c, P.H, P.W), S,
+             [&](float e) { black.add_square(__fmul_rn(e, scale)); });
   }
   int it = 0;
   for (; it < a.max_iter; ++it) {
     double* part = a.partial + (size_t)(it & 1) * kMaxBlocks;
     // red: the residual of the current iterate and the next one's values
     Sum2 sum = black;
-    bool nz = black_nz;
     for (Walk w(P, chunk); w.more(); w.next()) {
       const int c = 2 * w.k + (w.r & 1);
       if (c >= P.W) continue;
@@ -287,19 +313,16 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
       float x[3] = {o.x, o.y, o.z}, S[3];
       const float v = (float)valence(w.r, c, P.H, P.W);
       neighbour_sum(P, blk, w.r, w.k, c, S);
-      residual(P, x, o.w, v, S, scale, sum, nz);
+      residual(P, x, o.w, v, S, [&](float e) { sum.add_square(__fmul_rn(e, scale)); });
       solve(P, o.w, v, S, x);
       red_next[w.i] = make_float4(x[0], x[1], x[2], o.w);
     }
-    // a residual too small to square in FP32 still is not zero
-    if (nz) sum.hi = fmaxf(sum.hi, FLT_MIN);
     const double r2 = block_sum(sum);
     if (threadIdx.x == 0) __stcg(part + blockIdx.x, r2);
     if (!grid_barrier_counted(a.hdr, ++nbar)) return;
     const double mine = has ? __ldcg(part + threadIdx.x) : 0.0;
     // black: the next iterate's values and their residual
     black = Sum2();
-    black_nz = false;
     for (Walk w(P, chunk); w.more(); w.next()) {
       const int c = 2 * w.k + ((w.r + 1) & 1);
       if (c >= P.W) continue;
@@ -308,10 +331,21 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
       const float v = (float)valence(w.r, c, P.H, P.W);
       neighbour_sum(P, red_next, w.r, w.k, c, S);
       solve(P, si, v, S, x);
-      residual(P, x, si, v, S, scale, black, black_nz);
+      residual(P, x, si, v, S, [&](float e) { black.add_square(__fmul_rn(e, scale)); });
       blk_next[w.i] = make_float4(x[0], x[1], x[2], si);
     }
-    if (block_total(mine, (int)gridDim.x) <= limit2) break;   // iterate `it` is the result
+    const double sum2 = block_total(mine, (int)gridDim.x);
+    if (sum2 < limit2 - band) break;   // iterate `it` is the result
+    if (!(sum2 > limit2 + band && sum2 < INFINITY)) {
+      // (the same in every block; the other iteration's partials have been read)
+      double* exact = a.partial + (size_t)(~it & 1) * kMaxBlocks;
+      const double e2 = block_total(residual_fp64(P, red, blk, chunk), kThreads);
+      if (threadIdx.x == 0) __stcg(exact + blockIdx.x, e2);
+      if (!grid_barrier_counted(a.hdr, ++nbar)) return;
+      if (block_total(has ? __ldcg(exact + threadIdx.x) : 0.0, (int)gridDim.x) <=
+          (double)a.tol * (double)a.tol * bnorm2)
+        break;
+    }
     if (!grid_barrier_counted(a.hdr, ++nbar)) return;
     float4* r = red;
     red = red_next;
