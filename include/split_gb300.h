@@ -340,7 +340,10 @@ int split_sobel_normals(const float* heights, int width, int height,
  * normalised with z >= 0.  smoothness > 0.  *d_iterations (device int,
  * optional) receives the sweeps performed.  The reference's cuSPARSE
  * assembly no longer builds with CUDA 12; the system is applied matrix-free
- * here. */
+ * here.  The workspace size (66 KB and 32 bytes per pixel) is that of the image:
+ * query it for the largest one.  A smaller workspace of at least 65 792 bytes is
+ * accepted for any image: the unknowns then stay in `normals`, with the same
+ * results in several times the time. */
 size_t split_estimate_normals_workspace_size(int width, int height);
 int split_estimate_normals(const float* intensity, int width, int height, float lx,
                            float ly, float lz, float smoothness, int max_iter,

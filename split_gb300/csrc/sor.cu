@@ -211,6 +211,16 @@ struct Walk {
   }
 };
 
+// unit normal with z >= 0 of pixel i
+__device__ __forceinline__ void store_normal(float* normals, long long n, long long i, float x,
+                                             float y, float z) {
+  const float m = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+  const float rmag = __fdiv_rn(1.0f, __fsqrt_rn(m));
+  normals[i] = __fmul_rn(x, rmag);
+  normals[n + i] = __fmul_rn(y, rmag);
+  normals[2 * n + i] = __fmul_rn(fabsf(z), rmag);
+}
+
 // The thread's part of the squared residual of the iterate (red, blk), in FP64.
 __device__ __noinline__ double residual_fp64(Problem P, const float4* red, const float4* blk,
                                              int chunk) {
@@ -363,28 +373,103 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
       if (c >= P.W) continue;
       const long long i = (long long)w.r * P.W + c;
       const float4 x = (colour ? blk : red)[w.i];
-      const float m =
-          __fadd_rn(__fadd_rn(__fmul_rn(x.x, x.x), __fmul_rn(x.y, x.y)), __fmul_rn(x.z, x.z));
-      const float rmag = __fdiv_rn(1.0f, __fsqrt_rn(m));
-      a.normals[i] = __fmul_rn(x.x, rmag);
-      a.normals[n + i] = __fmul_rn(x.y, rmag);
-      a.normals[2 * n + i] = __fmul_rn(fabsf(x.z), rmag);
+      store_normal(a.normals, n, i, x.x, x.y, x.z);
     }
+}
+
+// The same relaxation with the unknowns in `normals`, for a workspace that holds
+// the sums alone.  A sweep is a residual pass in FP64, a red and a black pass,
+// each behind a barrier: the packed form above is several times faster and is
+// taken wherever the workspace has room for it.
+__global__ void __launch_bounds__(kThreads) sor_in_place_kernel(Args a) {
+  const Problem P = problem_of(a);
+  const long long n = (long long)P.W * P.H;
+  const long long first = (long long)blockIdx.x * kThreads + threadIdx.x;
+  const long long step = (long long)gridDim.x * kThreads;
+  float* const x = a.normals;   // (written and read by every block: no read-only loads)
+  const bool has = threadIdx.x < gridDim.x;
+  unsigned nbar = 0;
+  // FP64 sum over the grid, every block's result the same (slot: two in turn)
+  auto grid_sum = [&](double v, int slot, double* total) {
+    double* part = a.partial + (size_t)slot * kMaxBlocks;
+    v = block_total(v, kThreads);
+    if (threadIdx.x == 0) __stcg(part + blockIdx.x, v);
+    if (!grid_barrier_counted(a.hdr, ++nbar)) return false;
+    *total = block_total(has ? __ldcg(part + threadIdx.x) : 0.0, (int)gridDim.x);
+    return true;
+  };
+  auto sums = [&](int r, int c, float (&S)[3]) {
+    const long long i = (long long)r * P.W + c;
+    const long long at[4] = {i - P.W, i - 1, i + 1, i + P.W};
+    const bool in[4] = {r > 0, c > 0, c + 1 < P.W, r + 1 < P.H};
+    S[0] = S[1] = S[2] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (!in[q]) continue;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) S[d] = __fadd_rn(S[d], __ldcg(x + d * n + at[q]));
+    }
+  };
+  // x0 = (0, 0, 1) and |b|^2 = sum s_i^2 |L|^2
+  double acc = 0.0, total = 0.0;
+  for (long long i = first; i < n; i += step) {
+    __stcg(x + i, 0.0f);
+    __stcg(x + n + i, 0.0f);
+    __stcg(x + 2 * n + i, 1.0f);
+    const double si = (double)__ldg(a.s + i);
+    acc += si * si;
+  }
+  if (!grid_sum(acc, 1, &total)) return;
+  const double limit2 = (double)a.tol * (double)a.tol * (total * (double)P.LL);
+  int it = 0;
+  for (;; ++it) {
+    acc = 0.0;
+    for (long long i = first; i < n; i += step) {
+      const int r = (int)(i / P.W), c = (int)(i - (long long)r * P.W);
+      const float xi[3] = {__ldcg(x + i), __ldcg(x + n + i), __ldcg(x + 2 * n + i)};
+      float S[3];
+      sums(r, c, S);
+      residual(P, xi, __ldg(a.s + i), (float)valence(r, c, P.H, P.W), S,
+               [&](float e) { acc += (double)e * (double)e; });
+    }
+    if (!grid_sum(acc, it & 1, &total)) return;
+    if (total <= limit2 || it >= a.max_iter) break;
+    for (int colour = 0; colour < 2; ++colour) {
+      for (long long k = first; k < (long long)P.H * P.wh; k += step) {
+        const int r = (int)(k / P.wh);
+        const int c = 2 * (int)(k - (long long)r * P.wh) + ((r + colour) & 1);
+        if (c >= P.W) continue;
+        const long long i = (long long)r * P.W + c;
+        float S[3], v[3];
+        sums(r, c, S);
+        solve(P, __ldg(a.s + i), (float)valence(r, c, P.H, P.W), S, v);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) __stcg(x + d * n + i, v[d]);
+      }
+      if (!grid_barrier_counted(a.hdr, ++nbar)) return;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.d_iters) *a.d_iters = it;
+  for (long long i = first; i < n; i += step)
+    store_normal(x, n, i, __ldcg(x + i), __ldcg(x + n + i), __ldcg(x + 2 * n + i));
 }
 
 struct Layout {
   WsHeader* hdr;
   double* partial;
-  float4* x[2][2];
+  float4* x[2][2];     // the packed unknowns (null: they stay in the normals)
   size_t bytes;
 };
 
-inline Layout carve(void* ws, int W, int H) {
+constexpr int kPartials = 4096;   // words of a slot: 65 792 bytes without the unknowns
+static_assert(kMaxBlocks <= kPartials, "a word per block");
+
+inline Layout carve(void* ws, int W, int H, bool packed) {
   Carver c(ws);
-  Layout l;
+  Layout l{};
   l.hdr = c.take<WsHeader>(1);
-  l.partial = c.take<double>((size_t)2 * kMaxBlocks);
-  for (int colour = 0; colour < 2; ++colour)
+  l.partial = c.take<double>((size_t)2 * kPartials);
+  for (int colour = 0; colour < 2 && packed; ++colour)
     for (int i = 0; i < 2; ++i) l.x[colour][i] = c.take<float4>((size_t)H * ((W + 1) / 2));
   l.bytes = c.size();
   return l;
@@ -397,7 +482,7 @@ using namespace sg;
 
 extern "C" size_t split_estimate_normals_workspace_size(int width, int height) {
   if (width < 1 || height < 1) return 0;
-  return sor::carve(nullptr, width, height).bytes;
+  return sor::carve(nullptr, width, height, true).bytes;
 }
 
 extern "C" int split_estimate_normals(const float* intensity, int width, int height, float lx,
@@ -411,10 +496,11 @@ extern "C" int split_estimate_normals(const float* intensity, int width, int hei
   if ((int64_t)width * height > 0x7fffffffLL / 3) return SPLIT_ERR_INVALID;
   const float mag2 = lx * lx + ly * ly + lz * lz;
   if (!(mag2 > 0.0f)) return SPLIT_ERR_INVALID;
-  Layout l = carve(nullptr, width, height);
-  if (!workspace || workspace_bytes < l.bytes || (reinterpret_cast<uintptr_t>(workspace) & 255))
+  if (!workspace || workspace_bytes < carve(nullptr, width, height, false).bytes ||
+      (reinterpret_cast<uintptr_t>(workspace) & 255))
     return SPLIT_ERR_WORKSPACE;
-  l = carve(workspace, width, height);
+  const bool packed_x = workspace_bytes >= carve(nullptr, width, height, true).bytes;
+  const Layout l = carve(workspace, width, height, packed_x);
   cudaStream_t st = as_stream(stream);
   SG_CUDA_TRY(cudaMemsetAsync(l.hdr, 0, sizeof(WsHeader), st));
   DeviceInfo di;
@@ -432,8 +518,9 @@ extern "C" int split_estimate_normals(const float* intensity, int width, int hei
   Args a{intensity, normals, l.x[0][0], l.x[0][1], l.x[1][0], l.x[1][1], width, height, wh,
          lx * rmag, ly * rmag, lz * rmag, 2.0f * smoothness, max_iter, tol, l.partial,
          d_iterations, l.hdr};
-  void* args[] = {&a, &chunk};
-  SG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)sor_kernel, dim3(grid), dim3(kThreads),
-                                          args, 0, st));
+  void* args[] = {&a, &chunk};   // (the in-place kernel takes the first)
+  SG_CUDA_TRY(cudaLaunchCooperativeKernel(
+      packed_x ? (const void*)sor_kernel : (const void*)sor_in_place_kernel, dim3(grid),
+      dim3(kThreads), args, 0, st));
   return launch_status();
 }

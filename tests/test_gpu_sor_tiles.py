@@ -119,3 +119,28 @@ def test_intensities_that_are_not_finite(cuda):
     assert its == 0 and (out[2] == 1).all() and (out[:2] == 0).all()
     s[7, 9] = np.nan
     assert _sweeps(cuda, s, (1.0, 2.0, 2.0), 9, 1e-5)[0] == 9
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 700), (40, 50), (33, 65), (480, 640)])
+def test_workspace_without_the_unknowns(cuda, shape):
+    """A workspace of one size for every image: the same normals and sweeps, bit
+    for bit; a smaller one is refused."""
+    import torch
+    from split_gb300 import _native as N
+    from split_gb300._util import Workspace, ptr, stream_handle
+    s = np.random.default_rng(sum(shape)).random(shape).astype(np.float32)
+    dev, its = torch.from_numpy(s).to(cuda), torch.zeros(2, dtype=torch.int32, device=cuda)
+    out = torch.zeros((2, 3, s.size), dtype=torch.float32, device=cuda)
+    lib = N.load()
+    sizes = (lib.split_estimate_normals_workspace_size(shape[1], shape[0]), 65792)
+    for tol in (0.0, 1e-2):
+        for k, nbytes in enumerate(sizes):
+            ws = Workspace(nbytes, cuda)
+            N.check(lib.split_estimate_normals(
+                ptr(dev), shape[1], shape[0], 0.3, -0.2, 1.0, 1.0, 40, tol, ptr(out[k]),
+                ptr(its[k:]), ws.ptr, nbytes, stream_handle()), "estimate_normals")
+            ws.check("estimate_normals")
+        assert torch.equal(its[0], its[1]) and torch.equal(out[0], out[1])
+    assert lib.split_estimate_normals(
+        ptr(dev), shape[1], shape[0], 0.3, -0.2, 1.0, 1.0, 40, 0.0, ptr(out[0]), ptr(its), ws.ptr,
+        65792 - 256, stream_handle()) != N.OK
