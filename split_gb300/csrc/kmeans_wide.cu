@@ -39,10 +39,10 @@ constexpr int kMinK = 65;                 // smaller K runs in the persistent ke
 constexpr int kMaxClusters = 1 << 20;
 constexpr int kThreads = 256;
 constexpr int kPix = kPx;                 // pixels per thread (two pairs)
-constexpr int kTilePxLog2 = 10;           // a block's pixels, whole rows of lanes' four
-constexpr int kTileWLog2 = 6;             // 64 x 16 of them, see tile_width_log2
+constexpr int kTileW = 64, kTileH = 16;   // a block's pixels
+constexpr int kSubW = 32, kSubH = 4;      // a warp's
 constexpr int kWarps = kThreads / 32;
-static_assert(1 << kTilePxLog2 == kThreads * kPix && kPix == 4, "one lane each");
+static_assert(kTileW * kTileH == kThreads * kPix && kSubW * kSubH == 32 * kPix, "one lane each");
 constexpr int kSlots = 128;               // clusters of a tile summed in shared memory
 constexpr int kChunkF4 = 2048;            // float4 slots of one centroid chunk (32 KB)
 constexpr int kFormSlots = 1024;          // strided partials of the shift
@@ -129,7 +129,6 @@ struct AssignArgs {
   unsigned long long* hi;
   unsigned* cnt;
   int* status;
-  int tile_w_log2;          // a tile is 2^tile_w_log2 pixels wide
 };
 
 // Order-preserving float -> int key (warp min / max of the box).
@@ -291,14 +290,8 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
   float* csf = reinterpret_cast<float*>(cs);
   const int W = a.P.width;
   const int H = (int)((a.P.n + W - 1) / W);
-  const int tw = a.tile_w_log2, th = kTilePxLog2 - tw;
-  const int tiles_x = (W + (1 << tw) - 1) >> tw;
-  const int tiles = tiles_x * ((H + (1 << th) - 1) >> th);
-  // a warp's 128 pixels, 32 x 4 where the tile allows it: its place in the tile
-  // and the lane's four pixels in it
-  const int sw = tw > 8 ? tw - 3 : min(tw, 5);
-  const int wrow = (warp >> (tw - sw) << (7 - sw)) + (lane >> (sw - 2));
-  const int wcol = ((warp & ((1 << (tw - sw)) - 1)) << sw) + ((lane & ((1 << (sw - 2)) - 1)) << 2);
+  const int tiles_x = (W + kTileW - 1) / kTileW;
+  const int tiles = tiles_x * ((H + kTileH - 1) / kTileH);
 
   auto load_chunk = [&](int ch) {
     const int k0 = ch * kChunk;
@@ -318,7 +311,8 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
 
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
-    const int row = (ty << th) + wrow, col = (tx << tw) + wcol;
+    const int row = ty * kTileH + (warp >> 1) * kSubH + lane / (kSubW / kPix);
+    const int col = tx * kTileW + (warp & 1) * kSubW + (lane % (kSubW / kPix)) * kPix;
     const int64_t px0 = (int64_t)row * W + col;
     const int valid =
         row < H ? (int)max((int64_t)0, min((int64_t)min(kPix, W - col), a.P.n - px0)) : 0;
@@ -455,31 +449,14 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
         for (int j = 0; j < kPix; ++j) at[j] = j < valid ? bk[j] : -1;
         warp_to_tile<LAYOUT, DIM>(sums, f, at);
       } else if (__all_sync(full, small)) {
-        // where every lane's four pixels carry one label (or lie outside), the
-        // lane adds them first
-        bool one = valid == kPix;
 #pragma unroll
-        for (int j = 1; j < kPix; ++j) one = one && lab[j] == lab[0];
-        if (__all_sync(full, one || valid == 0)) {
+        for (int j = 0; j < kPix; ++j) {
+          const int l = j < valid ? lab[j] : -1;
           long long q[DIM];
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            q[d] = 0;
-#pragma unroll
-            for (int j = 0; j < kPix; ++j)
-              if (valid) q[d] += __float2ll_rn(__fmul_rn(f[j][d], fix::kScale));
-          }
-          fix::warp_add_narrow<DIM>(valid ? lab[0] : -1, q, kPix, a.lo, a.hi, a.cnt);
-        } else {
-#pragma unroll
-          for (int j = 0; j < kPix; ++j) {
-            const int l = j < valid ? lab[j] : -1;
-            long long q[DIM];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-              q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
-            fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
-          }
+          for (int d = 0; d < DIM; ++d)
+            q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
+          fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
         }
       } else {
 #pragma unroll
@@ -660,37 +637,8 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
 
 size_t workspace_bytes(int K, int dim) { return carve(nullptr, K, dim).bytes; }
 
-// The width of the tiles (as a power of two) and their number.  64 x 16 pixels
-// keep the candidates of an image few; where that shape leaves much of its tiles
-// outside the image (rows or columns shorter than a tile's), the shape with the
-// fewest tiles is taken instead, and features that do not depend on the place
-// (`xy`) are taken as one long row.  400 thousand points in one row, K = 1500,
-// 3-D: 64 x 16 tiles 3.4 ms an iteration, 1024 x 1 0.24.
-static int tile_width_log2(Points& P, bool xy, int64_t* tiles) {
-  auto count = [&](int tw) {
-    const int64_t w = 1 << tw, h = 1 << (kTilePxLog2 - tw);
-    const int64_t rows = (P.n + P.width - 1) / P.width;
-    return (P.width + w - 1) / w * ((rows + h - 1) / h);
-  };
-  int best = kTileWLog2;
-  *tiles = count(best);
-  const int64_t least = (P.n + (1 << kTilePxLog2) - 1) >> kTilePxLog2;
-  if (*tiles * 8 <= least * 9) return best;
-  if (!xy) {
-    P.width = (int)P.n;
-    *tiles = least;
-    return kTilePxLog2;
-  }
-  for (int tw = 2; tw <= kTilePxLog2; ++tw)
-    if (count(tw) < *tiles) {
-      best = tw;
-      *tiles = count(tw);
-    }
-  return best;
-}
-
 template <int LAYOUT, int DIM>
-static int queue(bool cluster, Points P, int K, const float* cent, float* centroids,
+static int queue(bool cluster, const Points& P, int K, const float* cent, float* centroids,
                  int32_t* labels, const Layout& L, int max_iter, float threshold, int ref_shift,
                  int32_t* d_iter, const StageHeaders& own, cudaStream_t st) {
   DeviceInfo di;
@@ -699,13 +647,12 @@ static int queue(bool cluster, Points P, int K, const float* cent, float* centro
   auto ak = cluster ? assign_kernel<LAYOUT, DIM, true> : assign_kernel<LAYOUT, DIM, false>;
   SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ak, kThreads, 0));
   if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-  int64_t blocks;
-  const int tw = tile_width_log2(P, LAYOUT != SPLIT_LAYOUT_PLANAR && DIM == 5, &blocks);
+  const int64_t rows = (P.n + P.width - 1) / P.width;
+  int64_t blocks = ((P.width + kTileW - 1) / kTileW) * ((rows + kTileH - 1) / kTileH);
   const int64_t cap = (int64_t)di.sm_count * per_sm;
   if (blocks > cap) blocks = cap;
   AssignArgs aa{};
   aa.P = P;
-  aa.tile_w_log2 = tw;
   aa.K = K;
   aa.labels = labels;
   aa.state = L.state;
