@@ -449,14 +449,31 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
         for (int j = 0; j < kPix; ++j) at[j] = j < valid ? bk[j] : -1;
         warp_to_tile<LAYOUT, DIM>(sums, f, at);
       } else if (__all_sync(full, small)) {
+        // where every lane's four pixels carry one label (or lie outside), the
+        // lane adds them first
+        bool one = valid == kPix;
 #pragma unroll
-        for (int j = 0; j < kPix; ++j) {
-          const int l = j < valid ? lab[j] : -1;
+        for (int j = 1; j < kPix; ++j) one = one && lab[j] == lab[0];
+        if (__all_sync(full, one || valid == 0)) {
           long long q[DIM];
 #pragma unroll
-          for (int d = 0; d < DIM; ++d)
-            q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
-          fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
+          for (int d = 0; d < DIM; ++d) {
+            q[d] = 0;
+#pragma unroll
+            for (int j = 0; j < kPix; ++j)
+              if (valid) q[d] += __float2ll_rn(__fmul_rn(f[j][d], fix::kScale));
+          }
+          fix::warp_add_narrow<DIM>(valid ? lab[0] : -1, q, kPix, a.lo, a.hi, a.cnt);
+        } else {
+#pragma unroll
+          for (int j = 0; j < kPix; ++j) {
+            const int l = j < valid ? lab[j] : -1;
+            long long q[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+              q[d] = l >= 0 ? __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)) : 0ll;
+            fix::warp_add_narrow<DIM>(l, q, 1u, a.lo, a.hi, a.cnt);
+          }
         }
       } else {
 #pragma unroll
