@@ -27,6 +27,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "fixsum.cuh"
@@ -39,10 +41,10 @@ constexpr int kMinK = 65;                 // smaller K runs in the persistent ke
 constexpr int kMaxClusters = 1 << 20;
 constexpr int kThreads = 256;
 constexpr int kPix = kPx;                 // pixels per thread (two pairs)
-constexpr int kTileW = 64, kTileH = 16;   // a block's pixels
-constexpr int kSubW = 32, kSubH = 4;      // a warp's
+constexpr int kTilePxLog2 = 10;           // a block's pixels, whole rows of lanes' four
+constexpr int kTileWLog2 = 6;             // 64 x 16 of them, see tile_width_log2
 constexpr int kWarps = kThreads / 32;
-static_assert(kTileW * kTileH == kThreads * kPix && kSubW * kSubH == 32 * kPix, "one lane each");
+static_assert(1 << kTilePxLog2 == kThreads * kPix && kPix == 4, "one lane each");
 constexpr int kSlots = 128;               // clusters of a tile summed in shared memory
 constexpr int kChunkF4 = 2048;            // float4 slots of one centroid chunk (32 KB)
 constexpr int kFormSlots = 1024;          // strided partials of the shift
@@ -129,6 +131,7 @@ struct AssignArgs {
   unsigned long long* hi;
   unsigned* cnt;
   int* status;
+  int tile_w_log2;          // a tile is 2^tile_w_log2 pixels wide
 };
 
 // Order-preserving float -> int key (warp min / max of the box).
@@ -267,7 +270,9 @@ __device__ __forceinline__ void warp_to_tile(TileSums<DIM>& ts, const float (&f)
 // warp's sums to global memory took 120 us an iteration at 2560 x 1440, K =
 // 256, 5-D (75 without the sums); with the tile's list and sums in shared
 // memory 56 (54 for the labels alone).
-template <int LAYOUT, int DIM, bool ACC>
+//
+// TW: log2 of the tile's width; 0: as given at run time (tile_w_log2).
+template <int LAYOUT, int DIM, bool ACC, int TW>
 __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
   constexpr int CS = DIM == 5 ? 2 : 1;          // float4 slots per centroid
   constexpr int kChunk = kChunkF4 / CS;         // centroids per chunk
@@ -290,8 +295,14 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
   float* csf = reinterpret_cast<float*>(cs);
   const int W = a.P.width;
   const int H = (int)((a.P.n + W - 1) / W);
-  const int tiles_x = (W + kTileW - 1) / kTileW;
-  const int tiles = tiles_x * ((H + kTileH - 1) / kTileH);
+  const int tw = TW ? TW : a.tile_w_log2, th = kTilePxLog2 - tw;
+  const int tiles_x = ((W - 1) >> tw) + 1;
+  const int tiles = tiles_x * (((H - 1) >> th) + 1);
+  // a warp's 128 pixels, 32 x 4 where the tile allows it: its place in the tile
+  // and the lane's four pixels in it
+  const int sw = tw > 8 ? tw - 3 : min(tw, 5);
+  const int wrow = (warp >> (tw - sw) << (7 - sw)) + (lane >> (sw - 2));
+  const int wcol = ((warp & ((1 << (tw - sw)) - 1)) << sw) + ((lane & ((1 << (sw - 2)) - 1)) << 2);
 
   auto load_chunk = [&](int ch) {
     const int k0 = ch * kChunk;
@@ -311,15 +322,16 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
 
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
-    const int row = ty * kTileH + (warp >> 1) * kSubH + lane / (kSubW / kPix);
-    const int col = tx * kTileW + (warp & 1) * kSubW + (lane % (kSubW / kPix)) * kPix;
+    // (64 bits where the last tile of a long row or column may reach past 2^31)
+    using Coord = std::conditional_t<TW == kTileWLog2, int, int64_t>;
+    const Coord row = ((Coord)ty << th) + wrow, col = ((Coord)tx << tw) + wcol;
     const int64_t px0 = (int64_t)row * W + col;
     const int valid =
-        row < H ? (int)max((int64_t)0, min((int64_t)min(kPix, W - col), a.P.n - px0)) : 0;
+        row < H ? (int)max((int64_t)0, min((int64_t)min((Coord)kPix, W - col), a.P.n - px0)) : 0;
     RawPx<LAYOUT, DIM> raw;
     raw.load(a.P.pts, a.P.n, px0, valid);
     float f[kPix][DIM];
-    raw.features(a.P.xy, row, col, f);
+    raw.features(a.P.xy, (int)row, (int)col, f);
     // box of the warp's pixels; fminf / fmaxf skip NaN (a NaN pixel's
     // distances all compare false, so it keeps label 0 whatever is skipped)
     float lo[DIM], hi[DIM];
@@ -654,22 +666,60 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
 
 size_t workspace_bytes(int K, int dim) { return carve(nullptr, K, dim).bytes; }
 
+// The width of the tiles (as a power of two) and their number.  64 x 16 pixels
+// keep the candidates of an image few; where that shape leaves much of its tiles
+// outside the image (rows or columns shorter than a tile's), the shape with the
+// fewest tiles is taken instead, and features that do not depend on the place
+// (`xy` false) are taken as one long row.  400 thousand points in one row, K =
+// 1500, 3-D: 64 x 16 tiles 3.4 ms an iteration, 1024 x 1 0.26.  From 1024
+// clusters on a place-independent tile prunes less, and the line lies lower (641
+// x 479, a tenth more tiles: K = 1500 218 against 194 us, K = 512 96 against 112).
+static int tile_width_log2(Points& P, int K, bool xy, int64_t* tiles) {
+  auto count = [&](int tw) {
+    const int64_t w = 1 << tw, h = 1 << (kTilePxLog2 - tw);
+    const int64_t rows = (P.n + P.width - 1) / P.width;
+    return (P.width + w - 1) / w * ((rows + h - 1) / h);
+  };
+  int best = kTileWLog2;
+  *tiles = count(best);
+  const int64_t least = (P.n + (1 << kTilePxLog2) - 1) >> kTilePxLog2;
+  const int64_t over = xy || K < 1024 ? 8 : 16;   // an eighth, or a sixteenth, more
+  if (*tiles * over <= least * (over + 1)) return best;
+  if (!xy) {
+    P.width = (int)P.n;
+    *tiles = least;
+    return kTilePxLog2;
+  }
+  for (int tw = 2; tw <= kTilePxLog2; ++tw)
+    if (count(tw) < *tiles) {
+      best = tw;
+      *tiles = count(tw);
+    }
+  return best;
+}
+
 template <int LAYOUT, int DIM>
-static int queue(bool cluster, const Points& P, int K, const float* cent, float* centroids,
+static int queue(bool cluster, Points P, int K, const float* cent, float* centroids,
                  int32_t* labels, const Layout& L, int max_iter, float threshold, int ref_shift,
                  int32_t* d_iter, const StageHeaders& own, cudaStream_t st) {
   DeviceInfo di;
   SG_TRY(device_info(&di));
   int per_sm = 0;
-  auto ak = cluster ? assign_kernel<LAYOUT, DIM, true> : assign_kernel<LAYOUT, DIM, false>;
+  constexpr bool kXY = LAYOUT != SPLIT_LAYOUT_PLANAR && DIM == 5;
+  constexpr int kOther = kXY ? 0 : kTilePxLog2;
+  int64_t blocks;
+  const int tw = tile_width_log2(P, K, kXY, &blocks);
+  auto ak = tw == kTileWLog2 ? cluster ? assign_kernel<LAYOUT, DIM, true, kTileWLog2>
+                                       : assign_kernel<LAYOUT, DIM, false, kTileWLog2>
+            : cluster        ? assign_kernel<LAYOUT, DIM, true, kOther>
+                             : assign_kernel<LAYOUT, DIM, false, kOther>;
   SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ak, kThreads, 0));
   if (per_sm < 1) return SPLIT_ERR_UNSUPPORTED;
-  const int64_t rows = (P.n + P.width - 1) / P.width;
-  int64_t blocks = ((P.width + kTileW - 1) / kTileW) * ((rows + kTileH - 1) / kTileH);
   const int64_t cap = (int64_t)di.sm_count * per_sm;
   if (blocks > cap) blocks = cap;
   AssignArgs aa{};
   aa.P = P;
+  aa.tile_w_log2 = tw;
   aa.K = K;
   aa.labels = labels;
   aa.state = L.state;
