@@ -416,15 +416,22 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
         const int i = g + lane;
         const bool in = i < nlist && lower_bound<DIM>(csf + list[i] * (4 * CS), lo, hi) <= thr;
         unsigned m = __ballot_sync(full, in);
+        // two at a time: both are read before the first is measured
         while (m) {
           const int p = g + __ffs(m) - 1;
           m &= m - 1;
-          const int kk = list[p];
-          const int name = nchunks == 1 ? p : k0 + kk;
-          const float4 c = cs[kk * CS];
-          const float c4 = DIM == 5 ? cs[kk * CS + (CS - 1)].x : 0.0f;
-          closer<DIM>(f[0], f[1], c, c4, name, best[0], best[1], bk[0], bk[1]);
-          closer<DIM>(f[2], f[3], c, c4, name, best[2], best[3], bk[2], bk[3]);
+          const int q = m ? g + __ffs(m) - 1 : p;
+          const int kp = list[p], kq = list[q];
+          const float4 c = cs[kp * CS], e = cs[kq * CS];
+          const float c4 = DIM == 5 ? cs[kp * CS + (CS - 1)].x : 0.0f;
+          const float e4 = DIM == 5 ? cs[kq * CS + (CS - 1)].x : 0.0f;
+          const int np = nchunks == 1 ? p : k0 + kp, nq = nchunks == 1 ? q : k0 + kq;
+          closer<DIM>(f[0], f[1], c, c4, np, best[0], best[1], bk[0], bk[1]);
+          closer<DIM>(f[2], f[3], c, c4, np, best[2], best[3], bk[2], bk[3]);
+          if (!m) break;
+          m &= m - 1;
+          closer<DIM>(f[0], f[1], e, e4, nq, best[0], best[1], bk[0], bk[1]);
+          closer<DIM>(f[2], f[3], e, e4, nq, best[2], best[3], bk[2], bk[3]);
         }
       }
     }
