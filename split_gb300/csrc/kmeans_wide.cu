@@ -46,10 +46,12 @@ constexpr int kTileWLog2 = 6;             // 64 x 16 of them, see tile_width_log
 constexpr int kWarps = kThreads / 32;
 static_assert(1 << kTilePxLog2 == kThreads * kPix && kPix == 4, "one lane each");
 constexpr int kSlots = 128;               // clusters of a tile summed in shared memory
+constexpr int kDirectTiles = 32;          // up to this many tiles add to the global sums
 constexpr int kChunkF4 = 2048;            // float4 slots of one centroid chunk (32 KB)
 constexpr int kFormSlots = 1024;          // strided partials of the shift
-constexpr int kFormThreads = 256;
-constexpr int kFormBlocks = 16;
+constexpr int kFormThreads = 256, kFormBlocks = 16;
+constexpr int kFormMaxThreads = 1024;     // one block, up to kFormFew values
+constexpr int kFormFew = 512;
 
 struct State {
   float delta;   // shift of the last formed iteration (0 before the first)
@@ -315,7 +317,11 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
     __syncthreads();
   };
   if (nchunks == 1) load_chunk(0);
-  if constexpr (ACC) {
+  // A few tiles hardly meet at the global sums, and a way through shared memory
+  // only adds to the one tile that their blocks wait for: 100 x 80, K = 128, 3-D,
+  // 35 us an iteration through the tile's sums, 29 without.
+  const bool tile_sums = ACC && nchunks == 1 && tiles > kDirectTiles;
+  if (ACC && tile_sums) {
     for (int i = threadIdx.x; i < kSlots * DIM; i += kThreads) sums.lo[i] = sums.hi[i] = 0u;
     for (int i = threadIdx.x; i < kSlots; i += kThreads) sums.cnt[i] = 0u;
   }
@@ -452,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
       // the global sums; otherwise the general form.  A pixel that no distance
       // named (all infinite or NaN) belongs to cluster 0, which the list may
       // not hold: not for the tile's sums either.
-      bool tiled = nchunks == 1 && nlist <= kSlots, small = true;
+      bool tiled = tile_sums && nlist <= kSlots, small = true;
 #pragma unroll
       for (int j = 0; j < kPix; ++j) {
         tiled = tiled && (j >= valid || bk[j] >= 0);
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, 3) assign_kernel(AssignArgs a) {
       // the tile's sums into the global ones (a block has few tiles: the list
       // changes with the tile)
       __syncthreads();
-      const int used = nchunks == 1 ? min(nlist, kSlots) : 0;
+      const int used = tile_sums ? min(nlist, kSlots) : 0;
       for (int i = threadIdx.x; i < used * DIM; i += kThreads) {
         const unsigned wl = sums.lo[i], wh = sums.hi[i];
         if ((wl | wh) == 0u) continue;
@@ -581,7 +587,7 @@ struct FormArgs {
 //           matrix from offset 0), sum of squares in dimension order;
 // and sums (c_new[j] - word[j])^2 in FP32 in j order.
 template <int LAYOUT, int DIM>
-__global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
+__global__ void __launch_bounds__(kFormMaxThreads) form_kernel(FormArgs a) {
   __shared__ float part[kFormSlots];
   __shared__ int stop, last, more;
   pdl_wait();
@@ -592,8 +598,9 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
   const int64_t kd = (int64_t)K * DIM;
   const float* c_old = a.L.cur + (size_t)((a.i - 1) & 1) * kd;
   float* c_new = a.L.cur + (size_t)(a.i & 1) * kd;
-  for (int slot = (int)blockIdx.x + (int)threadIdx.x * kFormBlocks; slot < kFormSlots;
-       slot += kFormBlocks * kFormThreads) {
+  const int nt = (int)blockDim.x;
+  for (int slot = (int)(blockIdx.x + threadIdx.x * gridDim.x); slot < kFormSlots;
+       slot += (int)gridDim.x * nt) {
     float acc = 0.0f;
     for (int64_t idx = slot; idx < kd; idx += kFormSlots) {
       const int d = (int)(idx / K), k = (int)(idx - (int64_t)d * K);
@@ -607,19 +614,24 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
       const float df = __fsub_rn(cn, c);
       acc = __fadd_rn(acc, __fmul_rn(df, df));
     }
-    __stcg(a.L.part + slot, acc);
+    if (gridDim.x == 1) part[slot] = acc;
+    else __stcg(a.L.part + slot, acc);
   }
-  // the block that finishes last has every block's words
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&a.L.state->arrived, 1u) + 1u == gridDim.x;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int i = threadIdx.x; i < kFormSlots; i += kFormThreads) part[i] = __ldcg(a.L.part + i);
+  if (gridDim.x > 1) {
+    // the block that finishes last has every block's words
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&a.L.state->arrived, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < kFormSlots; i += nt) part[i] = __ldcg(a.L.part + i);
+  } else {
+    __syncthreads();   // (the shift's words read other threads' centroids)
+  }
   if (DIM == 3 && a.ref_shift) {
     const int64_t base = 2 * a.P.n;
-    for (int64_t j = threadIdx.x; j < 3 * (int64_t)K; j += kFormThreads) {
+    for (int64_t j = threadIdx.x; j < 3 * (int64_t)K; j += nt) {
       float word;
       if (j < K) {
         word = __fdiv_rn(1.0f, (float)__ldcg(a.L.cnt + j));
@@ -643,7 +655,7 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
   }
   __syncthreads();
   for (int s = kFormSlots / 2; s > 0; s >>= 1) {
-    for (int i = threadIdx.x; i < s; i += kFormThreads) part[i] = __fadd_rn(part[i], part[i + s]);
+    for (int i = threadIdx.x; i < s; i += nt) part[i] = __fadd_rn(part[i], part[i + s]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -666,9 +678,9 @@ __global__ void __launch_bounds__(kFormThreads) form_kernel(FormArgs a) {
   }
   __syncthreads();
   if (!more)
-    for (int64_t idx = threadIdx.x; idx < kd; idx += kFormThreads)
+    for (int64_t idx = threadIdx.x; idx < kd; idx += nt)
       a.centroids[idx] = __ldcg(c_new + idx);
-  for (int k = threadIdx.x; k < K; k += kFormThreads) a.L.cnt[k] = 0u;
+  for (int k = threadIdx.x; k < K; k += nt) a.L.cnt[k] = 0u;
 }
 
 size_t workspace_bytes(int K, int dim) { return carve(nullptr, K, dim).bytes; }
@@ -754,12 +766,15 @@ static int queue(bool cluster, Points P, int K, const float* cent, float* centro
   fa.centroids = centroids;
   fa.d_iter = d_iter;
   const size_t kd = (size_t)K * DIM;
+  // few values: one block's divisions take less than the blocks' meeting
+  const bool few = kd <= kFormFew;
   for (int i = 1; i <= max_iter; ++i) {
     aa.cent = L.cur + (size_t)((i - 1) & 1) * kd;
     SG_CUDA_TRY(launch_pdl(ak, dim3((unsigned)blocks), dim3(kThreads), 0, st, aa));
     SG_TRY(launch_status());
     fa.i = i;
-    SG_CUDA_TRY(launch_pdl(form_kernel<LAYOUT, DIM>, dim3(kFormBlocks), dim3(kFormThreads), 0, st, fa));
+    SG_CUDA_TRY(launch_pdl(form_kernel<LAYOUT, DIM>, dim3(few ? 1 : kFormBlocks),
+                           dim3(few ? kFormMaxThreads : kFormThreads), 0, st, fa));
     SG_TRY(launch_status());
   }
   return SPLIT_OK;
