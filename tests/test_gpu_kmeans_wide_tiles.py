@@ -66,3 +66,41 @@ def test_no_distance_below_infinity(cuda, bad, k, dim):
             assert np.allclose(got[:, lab[0]], want, rtol=1e-5, atol=0)
         keep = np.arange(k) != lab[0]
         assert np.array_equal(got[:, keep], c0[:, keep], equal_nan=True)
+
+
+@pytest.mark.parametrize("w,h,k", [
+    (2000, 1, 70), (1, 2000, 70), (3000, 2, 200), (2, 3000, 200), (900, 5, 70), (5, 900, 1500),
+    (33, 40, 70), (100, 9, 70), (1025, 1, 70),
+    (64 * 32, 16, 70), (64 * 33, 16, 70),     # as many tiles as add directly, and one more
+    (128, 64, 1500)])                         # two chunks of centroids in five dimensions
+@pytest.mark.parametrize("layout", ["planar3", "planar5", "rgb3", "rgb5", "float5"])
+def test_tile_shapes(cuda, w, h, k, layout):
+    """Images whose rows or columns are shorter than a tile's, as flat as four
+    pixels' runs and as noise, with features that depend on the place or not."""
+    import torch
+    from split_gb300 import kmeans
+    rng = np.random.default_rng(w + h + k)
+    n, dim = w * h, int(layout[-1])
+    rgb = rng.integers(0, 256, (n, 3)).astype(np.uint8)
+    rgb[n // 2:] = rgb[n // 2:n // 2 + 1]      # lanes and warps of one label
+    c3 = (rgb.astype(np.float32) / np.float32(255)).T
+    xy = np.stack([np.arange(n) % w, np.arange(n) // w]).astype(np.float32) * np.float32(0.02)
+    feats = np.ascontiguousarray(np.concatenate([c3, xy])[:dim])
+    c0 = feats[:, rng.choice(n, size=k, replace=n < k)].copy()
+    if layout.startswith("planar"):
+        pts, ly = torch.from_numpy(feats), kmeans.PLANAR
+    elif layout.startswith("rgb"):
+        pts, ly = torch.from_numpy(rgb), kmeans.RGB8
+    else:
+        pts, ly = torch.from_numpy(np.concatenate([c3.T, np.zeros((n, 1), np.float32)], 1)), \
+            kmeans.FLOAT4
+    cent = torch.from_numpy(c0).to(cuda)
+    labels = torch.full((n,), -7, dtype=torch.int32, device=cuda)
+    ws = kmeans.cluster(pts.contiguous().to(cuda), cent, labels, None, 1, -1.0, layout=ly, dim=dim,
+                        width=w, xy_scale=0.02)
+    ws.check("cluster")
+    lab = labels.cpu().numpy()
+    assert np.array_equal(lab, oracle.kmeans_assign_f32(feats, c0))
+    want = oracle.kmeans_update_f64(lab, feats, c0)[0]
+    got = cent.cpu().numpy().astype(np.float64)
+    assert (np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1e-3)).all()
