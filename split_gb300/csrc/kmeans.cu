@@ -2467,25 +2467,82 @@ __device__ __forceinline__ void pixel_features(const void* points, int64_t n, in
   }
 }
 
-// Adds a run of pixels of one label, its words as 32-bit sums.
-template <int DIM>
-__device__ __forceinline__ void add_run(const Layout& L, int l, const unsigned (&q)[DIM],
+// A run's word of one dimension into the sums: below 2^32, or any 64-bit one.
+__device__ __forceinline__ void add_word(const Layout& L, size_t s, unsigned q) {
+  atomicAdd(L.lo + s, (unsigned long long)q);
+}
+__device__ __forceinline__ void add_word(const Layout& L, size_t s, long long q) {
+  atomicAdd(L.lo + s, (unsigned long long)q & 0xffffffffull);
+  if (q >> 32) atomicAdd(L.hi + s, (unsigned long long)(q >> 32));
+}
+__device__ __forceinline__ unsigned shfl_down(unsigned v, int o) {
+  return __shfl_down_sync(0xffffffffu, v, o);
+}
+__device__ __forceinline__ long long shfl_down(long long v, int o) {
+  return (long long)fix::shfl_down_u64((unsigned long long)v, o);
+}
+
+// Adds a run of pixels of one label.
+template <int DIM, typename W>
+__device__ __forceinline__ void add_run(const Layout& L, int l, const W (&q)[DIM],
                                         unsigned count) {
 #pragma unroll
-  for (int d = 0; d < DIM; ++d)
-    atomicAdd(L.lo + (size_t)l * DIM + d, (unsigned long long)q[d]);
+  for (int d = 0; d < DIM; ++d) add_word(L, (size_t)l * DIM + d, q[d]);
   atomicAdd(L.cnt + l, count);
 }
 
 // Bound by the reductions of runs and the atomics that they end in.  Four
-// consecutive pixels per thread.  A warp whose features all lie in [0, 1]
-// (colours do) has words of at most 2^24, so the sums of its 128 pixels fit 32
-// bits and their high words are zero: a thread adds the runs that end inside
-// its four pixels as they are, and its last run takes part in a segmented
-// reduction over the lanes, whose run heads add.  Other warps add the 96-bit
-// words, a pixel of every lane at a time.  2 Mpx in 24 thousand segments,
-// planar colours: 27.4 us with the 96-bit words throughout, 15.4 us.
+// consecutive pixels per thread: it adds the runs that end inside them as they
+// are, and its last run takes part in a segmented reduction over the lanes, whose
+// run heads add.  A warp whose features all lie in [0, 1] (colours do) has words
+// of at most 2^24, so the sums of its 128 pixels fit 32 bits; one with features
+// below 2^32 has 64-bit sums; others add 96-bit words, a pixel of every lane at a
+// time.  2 Mpx in 24 thousand segments, planar colours: 15.4 us.
 constexpr int kPer = 4;
+
+// the runs of the warp's pixels, words as W; `word` gives pixel j's
+template <int DIM, typename W, class F>
+__device__ __forceinline__ void add_runs(const Layout& L, const int (&l)[kPer], F&& word) {
+  const int lane = threadIdx.x & 31;
+  W q[DIM];
+  unsigned c = 0u;
+  int cur = l[0];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) q[d] = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (j > 0 && l[j] != cur) {
+      if (cur >= 0) add_run<DIM, W>(L, cur, q, c);
+      cur = l[j];
+      c = 0u;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) q[d] = 0;
+    }
+    ++c;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) q[d] += word(j, d);
+  }
+  // the lanes' last runs: a lane adds from lane + o while that lane is in its
+  // run; a lane that began its run with fewer than four pixels is a head, its
+  // label not the lane's before (or cut off by the runs already added)
+  const int before = __shfl_up_sync(0xffffffffu, cur, 1);
+  const unsigned heads =
+      __ballot_sync(0xffffffffu, lane == 0 || cur != before || c != (unsigned)kPer);
+  const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
+  const int run_end = after ? __ffs(after) - 1 : 32;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const bool in_run = lane + o < run_end;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const W a = shfl_down(q[d], o);
+      if (in_run) q[d] += a;
+    }
+    const unsigned a = __shfl_down_sync(0xffffffffu, c, o);
+    if (in_run) c += a;
+  }
+  if (cur >= 0 && (heads >> lane & 1u)) add_run<DIM, W>(L, cur, q, c);
+}
 
 template <int LAYOUT, int DIM>
 __global__ void __launch_bounds__(kThreads)
@@ -2521,58 +2578,37 @@ accumulate_kernel(const int32_t* __restrict__ labels, const void* __restrict__ p
       if (l[j] >= 0) pixel_features<LAYOUT, DIM>(points, n, i0 + j, width, xy_scale, f[j]);
     }
   }
-  bool unit = true;   // false for NaN
+  // (false for NaN)
+  bool unit = true, small = true;
 #pragma unroll
   for (int j = 0; j < kPer; ++j)
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) unit &= l[j] < 0 || (f[j][d] >= 0.0f && f[j][d] <= 1.0f);
-  if (!__all_sync(0xffffffffu, unit)) {
-#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      unit &= l[j] < 0 || (f[j][d] >= 0.0f && f[j][d] <= 1.0f);
+      small &= l[j] < 0 || fabsf(f[j][d]) < 4294967296.0f;
+    }
+  if (__all_sync(0xffffffffu, unit)) {
+    add_runs<DIM, unsigned>(
+        L, l, [&](int j, int d) { return __float2uint_rn(__fmul_rn(f[j][d], fix::kScale)); });
+  } else if (__all_sync(0xffffffffu, small)) {
+    add_runs<DIM, long long>(
+        L, l, [&](int j, int d) { return __float2ll_rn(__fmul_rn(f[j][d], fix::kScale)); });
+  } else {
+    // neighbouring pixels in neighbouring lanes again
+    const int64_t w0 = i0 - (int64_t)lane * kPer;
     for (int j = 0; j < kPer; ++j) {
-      const int lj = l[j] < 0 ? -1 : l[j];
+      const int64_t i = w0 + 32 * j + lane;
+      int lj = i < n ? __ldg(labels + i) : -1;
+      if (lj < 0 || lj >= K) lj = -1;
+      float g[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) g[d] = 0.0f;
+      if (lj >= 0) pixel_features<LAYOUT, DIM>(points, n, i, width, xy_scale, g);
       unsigned long long qlo[DIM], qhi[DIM];
-      fix::quantize<DIM>(f[j], lj, &L.hdr->status, qlo, qhi);
+      fix::quantize<DIM>(g, lj, &L.hdr->status, qlo, qhi);
       fix::warp_add<DIM>(lj, qlo, qhi, L.lo, L.hi, L.cnt);
     }
-    return;
   }
-  unsigned q[DIM], c = 0u;
-  int cur = l[0];
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) q[d] = 0u;
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    if (j > 0 && l[j] != cur) {
-      if (cur >= 0) add_run<DIM>(L, cur, q, c);
-      cur = l[j];
-      c = 0u;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) q[d] = 0u;
-    }
-    ++c;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) q[d] += __float2uint_rn(__fmul_rn(f[j][d], fix::kScale));
-  }
-  // the lanes' last runs: a lane adds from lane + o while that lane is in its
-  // run; a lane that began its run with fewer than four pixels is a head, its
-  // label not the lane's before (or cut off by the runs already added)
-  const int before = __shfl_up_sync(0xffffffffu, cur, 1);
-  const unsigned heads =
-      __ballot_sync(0xffffffffu, lane == 0 || cur != before || c != (unsigned)kPer);
-  const unsigned after = heads & ~(0xffffffffu >> (31 - lane));
-  const int run_end = after ? __ffs(after) - 1 : 32;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const bool in_run = lane + o < run_end;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      const unsigned a = __shfl_down_sync(0xffffffffu, q[d], o);
-      if (in_run) q[d] += a;
-    }
-    const unsigned a = __shfl_down_sync(0xffffffffu, c, o);
-    if (in_run) c += a;
-  }
-  if (cur >= 0 && (heads >> lane & 1u)) add_run<DIM>(L, cur, q, c);
 }
 
 __global__ void __launch_bounds__(kThreads)

@@ -69,3 +69,28 @@ def test_means_and_paint(cuda, n, offset, k, wide):
     kmeans.propagate_centroids(dev_lab, cent, out)
     assert np.array_equal(out.cpu().numpy(),
                           np.where(inside, want[:, np.where(inside, lab, 0)], np.float32(0)))
+
+
+@pytest.mark.parametrize("scale", [100.0, -1e6, 1e10, 2.0e11])
+@pytest.mark.parametrize("n,offset", [(5, 0), (127, 1), (4096, 0), (4098, 2), (33333, 3)])
+def test_means_of_large_features(cuda, n, offset, scale):
+    """Features outside [0, 1] everywhere: 64-bit sums of runs below 2^32, 96-bit
+    words above, in runs shorter and longer than a thread's four pixels."""
+    import torch
+    from split_gb300 import kmeans
+    k = 70
+    rng = np.random.default_rng(n)
+    lab = np.repeat(rng.integers(-1, k + 1, size=n), rng.integers(1, 9, size=n))[:n].astype(np.int32)
+    pts = ((rng.random((3, n)) - 0.25) * scale).astype(np.float32)
+    q = np.rint(pts.astype(np.float64) * 2.0**24).astype(np.int64)   # exact: floats have 24 bits
+    inside = (lab >= 0) & (lab < k)
+    old = rng.random((3, k), dtype=np.float32)
+    want = old.copy()
+    for c in np.unique(lab[inside]):
+        for d in range(3):
+            total = sum(int(v) for v in q[d, lab == c])
+            want[d, c] = np.float32(float(total) / 2.0**24 / int((lab == c).sum()))
+    cent = torch.from_numpy(old).to(cuda)
+    ws = kmeans.calculate_centroids(_at(lab, offset, cuda), _at(pts, offset, cuda), cent)
+    ws.check("calculate_centroids")
+    assert np.array_equal(cent.cpu().numpy(), want)
