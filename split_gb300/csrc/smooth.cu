@@ -48,6 +48,7 @@ struct Layout {
   unsigned* maxsq;              // bits of the largest |x|^2 (non-negative float)
   unsigned* list_count;
   unsigned* call;               // the call's number: marks this call's entries of fin
+  unsigned* full;               // a pair found no slot: the rest is not looked for
   unsigned long long* best;     // [n] winning bid per segment, 0 = none
   unsigned long long* fin;      // [n] (call number, final label)
   Slot* slots;                  // [cap]
@@ -69,6 +70,7 @@ inline Layout carve(void* ws, int64_t n) {
   l.maxsq = l.hdr ? l.hdr->counter : nullptr;
   l.list_count = l.hdr ? l.hdr->counter + 1 : nullptr;
   l.call = l.hdr ? reinterpret_cast<unsigned*>(l.hdr->pad) : nullptr;
+  l.full = l.hdr ? reinterpret_cast<unsigned*>(l.hdr->pad) + 1 : nullptr;
   l.best = c.take<unsigned long long>((size_t)n);
   l.fin = c.take<unsigned long long>((size_t)n);
   l.cap_log2 = cap_log2_for(n);
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(kThreads)
 guard_kernel(Layout L, unsigned long long stamp, long long n) {
   pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    L.hdr->barrier_count = *L.maxsq = *L.list_count = 0u;
+    L.hdr->barrier_count = *L.maxsq = *L.list_count = *L.full = 0u;
   if (L.hdr->stamp == stamp && *L.call != ~0u) return;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,6 +141,7 @@ __device__ void insert(const Layout& L, unsigned long long key, unsigned m, unsi
     }
   }
   set_status(status, SPLIT_ERR_OVERFLOW);
+  *(volatile unsigned*)L.full = 1u;
 }
 
 // One block per 32 x 64 tile: the largest feature norm, and the statistics of
@@ -151,8 +154,9 @@ __device__ void insert(const Layout& L, unsigned long long key, unsigned m, unsi
 // down the columns of one warp; the edges of a pair meet in a shared-memory
 // table and reach the global one as one entry per tile and pair.  The norms'
 // 62-bit values are added as four 16-bit pieces: a tile has at most 2^13
-// edges, so a piece's sum stays below 2^29.  A pair that the tile's table has
-// no room for within a short probe goes to the global one directly.  1080p, 400
+// edges, so a piece's sum stays below 2^29.  Pairs that the tile's table has no
+// room for within a short probe take another round in it: one by one into the
+// global table they cost a 64 x 48 image of 3 x 3 pixel segments 150 us.  1080p, 400
 // segments and 4000 single pixels: 81 us for a norm kernel and a kernel that
 // pushed every directed edge into the global table, 24 us; seven blocks per SM
 // hold the 1020 tiles at once (six: 33 us).
@@ -168,7 +172,7 @@ edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geom
   __shared__ unsigned long long key[kPairs];
   __shared__ unsigned count[kPairs], piece[4][kPairs];
   __shared__ unsigned short todo[kTilePx];   // local pixel, then its edges in 4 bits
-  __shared__ unsigned ntodo, maxsq;
+  __shared__ unsigned ntodo, maxsq, stopped;
   pdl_wait();
   const long long n = gs.total_px;
   const TileRef tr = tile_ref(gs, blockIdx.x);
@@ -178,7 +182,10 @@ edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geom
     *L.call = last == ~0u ? 1u : last + 1u;   // never 0, the mark of a cleared entry
     L.hdr->stamp = kStampDirty;               // until the call has cleared its words
   }
-  if (threadIdx.x == 0) ntodo = maxsq = 0u;
+  if (threadIdx.x == 0) {
+    ntodo = maxsq = 0u;
+    stopped = *(volatile unsigned*)L.full;
+  }
   // -1: outside the image, or no label
   bool bad = false;
   for (int q = threadIdx.x; q < kHaloH * kHaloW; q += kThreads) {
@@ -235,57 +242,75 @@ edge_kernel(const int32_t* __restrict__ lab, const float* __restrict__ pts, Geom
   __syncthreads();
   if (threadIdx.x == 0) atomicMax(L.maxsq, maxsq);
   const unsigned nt = ntodo;
-  if (nt == 0u) return;
-  for (unsigned q = threadIdx.x; q < nt; q += kThreads) {
-    const unsigned item = todo[q], m = item & 15u, px = item >> 4;
-    const int* c = tile + (px / kTileW) * kHaloW + px % kTileW + 1;
-    const int v = c[0];
-    const long long i =
-        tr.off + (long long)(tr.ty0 + (int)(px / kTileW)) * W + tr.tx0 + (int)(px % kTileW);
-    const int t[4] = {c[1], c[kHaloW - 1], c[kHaloW], c[kHaloW + 1]};
-    const long long j[4] = {i + 1, i + W - 1, i + W, i + W + 1};
-    float f[3], g[4][3];
+  if (nt == 0u || stopped) return;
+  // Edges whose pair finds no room stay in the list for another round with an
+  // emptied table.
+  for (bool again = true; again;) {
+    unsigned left = 0u;
+    for (unsigned q = threadIdx.x; q < nt; q += kThreads) {
+      const unsigned item = todo[q], m = item & 15u, px = item >> 4;
+      if (m == 0u) continue;
+      const int* c = tile + (px / kTileW) * kHaloW + px % kTileW + 1;
+      const int v = c[0];
+      const long long i =
+          tr.off + (long long)(tr.ty0 + (int)(px / kTileW)) * W + tr.tx0 + (int)(px % kTileW);
+      const int t[4] = {c[1], c[kHaloW - 1], c[kHaloW], c[kHaloW + 1]};
+      const long long j[4] = {i + 1, i + W - 1, i + W, i + W + 1};
+      float f[3], g[4][3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      f[d] = __ldg(pts + d * n + i);
+      for (int d = 0; d < 3; ++d) {
+        f[d] = __ldg(pts + d * n + i);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) g[k][d] = m >> k & 1u ? __ldg(pts + d * n + j[k]) : 0.0f;
+        for (int k = 0; k < 4; ++k) g[k][d] = m >> k & 1u ? __ldg(pts + d * n + j[k]) : 0.0f;
+      }
+      unsigned rest = 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!(m >> k & 1u)) continue;
+        const float e = edge_norm(f, g[k]);
+        const long long w = __float2ll_rn(__fmul_rn(e, 4294967296.0f));
+        const unsigned long long kk = pair_key(v, t[k]);
+        if (!(e < 1073741824.0f)) {   // 2^30, or NaN: too large for the pieces
+          set_status(status, SPLIT_ERR_OVERFLOW);
+          insert(L, kk, 1u, (unsigned long long)w & 0xffffffffull, (unsigned long long)(w >> 32),
+                 status);
+          continue;
+        }
+        unsigned h = key_hash(kk, kPairBits);
+        bool in = false;
+        for (int probe = 0; probe < kPairProbes; ++probe, h = (h + 1) & (kPairs - 1)) {
+          unsigned long long o = *(volatile unsigned long long*)&key[h];
+          if (o == 0ull) o = atomicCAS(&key[h], 0ull, kk);
+          in = o == 0ull || o == kk;
+          if (in) break;
+        }
+        if (!in) {
+          rest |= 1u << k;
+          continue;
+        }
+        atomicAdd(&count[h], 1u);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const unsigned p = (unsigned)(w >> (16 * a)) & 0xffffu;
+          if (p) atomicAdd(&piece[a][h], p);
+        }
+      }
+      if (rest != m) todo[q] = (unsigned short)(px << 4 | rest);
+      left |= rest;
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!(m >> k & 1u)) continue;
-      const float e = edge_norm(f, g[k]);
-      const bool large = !(e < 1073741824.0f);   // 2^30, or NaN
-      if (large) set_status(status, SPLIT_ERR_OVERFLOW);
-      const long long w = __float2ll_rn(__fmul_rn(e, 4294967296.0f));
-      const unsigned long long kk = pair_key(v, t[k]);
-      unsigned h = key_hash(kk, kPairBits);
-      bool in = false;
-      for (int probe = large ? kPairProbes : 0; probe < kPairProbes;
-           ++probe, h = (h + 1) & (kPairs - 1)) {
-        unsigned long long o = *(volatile unsigned long long*)&key[h];
-        if (o == 0ull) o = atomicCAS(&key[h], 0ull, kk);
-        in = o == 0ull || o == kk;
-        if (in) break;
-      }
-      if (!in) {
-        insert(L, kk, 1u, (unsigned long long)w & 0xffffffffull, (unsigned long long)(w >> 32),
-               status);
-        continue;
-      }
-      atomicAdd(&count[h], 1u);
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const unsigned p = (unsigned)(w >> (16 * a)) & 0xffffu;
-        if (p) atomicAdd(&piece[a][h], p);
-      }
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kPairs; i += kThreads)
-    if (key[i])
+    again = __syncthreads_or(left != 0u);
+    for (int i = threadIdx.x; i < kPairs; i += kThreads) {
+      if (!key[i]) continue;
       insert(L, key[i], count[i], piece[0][i] + ((unsigned long long)piece[1][i] << 16),
              piece[2][i] + ((unsigned long long)piece[3][i] << 16), status);
+      if (again) {
+        key[i] = 0ull;
+        count[i] = piece[0][i] = piece[1][i] = piece[2][i] = piece[3][i] = 0u;
+      }
+    }
+    // (a full global table: the call has failed, whatever else is tried)
+    if (again && __syncthreads_or(*(volatile unsigned*)L.full != 0u)) return;
+  }
 }
 
 // mean edge norm of a slot, rounded to FP32 (the reference keeps it as real);

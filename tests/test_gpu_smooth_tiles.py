@@ -54,3 +54,40 @@ def test_workspace_across_sizes(cuda):
         ccl.merge_smooth_boundaries(torch.from_numpy(pts).to(cuda), 0, got, ws, 0.05)
         ws.check("merge_smooth")
         assert np.array_equal(got.cpu().numpy(), oracle.merge_smooth(seg, pts, 0.05)), (w, h)
+
+
+@pytest.mark.parametrize("shape,block", [((20, 20), 1), ((48, 64), 3), ((33, 130), 2)])
+def test_more_pairs_than_a_tile_holds(cuda, shape, block):
+    """Tiles that fill their table several times over."""
+    import torch
+    from split_gb300 import ccl
+    h, w = shape
+    rng = np.random.default_rng(h + w)
+    y, x = np.mgrid[0:h, 0:w]
+    seg = (y // block * block * w + x // block * block).astype(np.int32)
+    seg[:, : w // 4] = 0     # and one large segment with many neighbours
+    pts = rng.random((3, h * w)).astype(np.float32)
+    got = torch.from_numpy(seg).to(cuda)
+    ws = ccl.merge_smooth_boundaries(torch.from_numpy(pts).to(cuda), 0, got, None, 2.0)
+    ws.check("merge_smooth")
+    assert np.array_equal(got.cpu().numpy(), oracle.merge_smooth(seg, pts, 2.0))
+
+
+def test_after_a_refused_call(cuda):
+    """More pairs than the global table holds is an error; the workspace is then as
+    good as new."""
+    import torch
+    from split_gb300 import ccl
+    from split_gb300._native import SplitError
+    h, w = 48, 64
+    pts = torch.rand((3, h * w), device=cuda)
+    seg = torch.arange(h * w, dtype=torch.int32, device=cuda).view(h, w)
+    ws = ccl.merge_smooth_boundaries(pts, 0, seg.clone(), None, 0.5)
+    with pytest.raises(SplitError):
+        ws.check("merge_smooth")
+    y, x = np.mgrid[0:h, 0:w]
+    lab = (y // 8 * 8 * w + x // 8 * 8).astype(np.int32)
+    got = torch.from_numpy(lab).to(cuda)
+    ccl.merge_smooth_boundaries(pts, 0, got, ws, 2.0)
+    ws.check("merge_smooth")
+    assert np.array_equal(got.cpu().numpy(), oracle.merge_smooth(lab, pts.cpu().numpy(), 2.0))
