@@ -229,24 +229,26 @@ __global__ void reset_kernel(const Layout l, int* d_count) {
 // order.  A pair borders both ways, so four of the eight neighbours (east,
 // south-west, south, south-east) find it and both its keys are appended; a
 // pair that the set has no room for within a short probe is appended as it is
-// (the sort brings the copies together).  A key is never 0: its two labels
+// (the sort brings the copies together), after a shorter one from then on: in
+// noise nearly every pair fails, and a failed probe takes as long as 16 loads.  A key is never 0: its two labels
 // differ.  Every pair appended has an edge of its own, at most 4 n there are,
 // so 8 n keys hold all.  The pixels that have an edge go to a list first, which
 // the block walks densely.  1080p, 400 segments and 4000 single pixels: 23 us
 // with all eight neighbours at every pixel, 14 us.
 constexpr int kPixH = 32, kPixW = 64, kHaloW = kPixW + 2, kHaloH = kPixH + 1;
 constexpr int kSetBits = 10, kSetProbes = 16;
+constexpr int kFullProbes = 4;   // once a pair has found no room
 static_assert(kPixH * kPixW <= 1 << 11 && kThreads % kPixW == 0, "list entries; whole rows");
 __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restrict__ lab, int w,
                                                          int h, const Layout l) {
   __shared__ int tile[kHaloH * kHaloW];
   __shared__ unsigned long long set[1 << kSetBits];
   __shared__ unsigned short todo[kPixH * kPixW];   // local pixel, then its edges in 4 bits
-  __shared__ int ntodo, found, base;
+  __shared__ int ntodo, found, base, full;
   pdl_wait();
   const int tiles_x = (w + kPixW - 1) / kPixW;
   const int x0 = (int)(blockIdx.x % tiles_x) * kPixW, y0 = (int)(blockIdx.x / tiles_x) * kPixH;
-  if (threadIdx.x == 0) ntodo = found = 0;
+  if (threadIdx.x == 0) ntodo = found = full = 0;
   // pixels outside the image take the nearest inside: the pixel itself or
   // another of its neighbours, so no pair is added
   for (int q = threadIdx.x; q < kHaloH * kHaloW; q += kThreads) {
@@ -284,11 +286,14 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
     o_or |= key | back;
     o_and &= key & back;
   };
-  for (int q = threadIdx.x; q < nt; q += kThreads) {
-    const unsigned item = todo[q], m = item & 15u, px = item >> 4;
+  for (int q0 = (int)threadIdx.x - lane; q0 < nt; q0 += kThreads) {   // whole warps
+    const int q = q0 + lane;
+    const unsigned item = q < nt ? todo[q] : 0u, m = item & 15u, px = item >> 4;
     const int* c = tile + (px / kPixW) * kHaloW + px % kPixW + 1;
     const int v = *c;
     const int t[4] = {c[1], c[kHaloW - 1], c[kHaloW], c[kHaloW + 1]};
+    const int probes = *(volatile int*)&full ? kFullProbes : kSetProbes;
+    unsigned out = 0u;   // pairs that found no room
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       bool add = m >> a & 1u;
@@ -298,13 +303,33 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
       const unsigned long long key = pair_key(min(v, t[a]), max(v, t[a]));
       unsigned s = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kSetBits));
       bool in = false;
-      for (int probe = 0; probe < kSetProbes && !in; ++probe, s = (s + 1) & ((1 << kSetBits) - 1)) {
+      for (int probe = 0; probe < probes && !in; ++probe, s = (s + 1) & ((1 << kSetBits) - 1)) {
         unsigned long long k = *(volatile unsigned long long*)&set[s];
         if (k == 0ull) k = atomicCAS(&set[s], 0ull, key);
         in = k == 0ull || k == key;
       }
-      if (!in) append(key, atomicAdd(l.total, 2));
+      if (!in) out |= 1u << a;
     }
+    __syncwarp();
+    if (!__any_sync(0xffffffffu, out != 0u)) continue;
+    *(volatile int*)&full = 1;
+    // one place in the list per warp
+    const int mine = 2 * __popc(out);
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += u;
+    }
+    int first = lane == 31 ? atomicAdd(l.total, at) : 0;
+    first = __shfl_sync(0xffffffffu, first, 31);
+    at += first - mine;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (out >> a & 1u) {
+        append(pair_key(min(v, t[a]), max(v, t[a])), at);
+        at += 2;
+      }
   }
   __syncthreads();
   // the set's keys, with one place in the list per block
