@@ -163,11 +163,13 @@ __device__ double block_sum(Sum2 v) {
   return t;
 }
 
-// FP64 sum of one value per thread, every thread's result the same; warps
-// whose lanes hold no value skip their tree
-__device__ double block_total(double v, int nvalues) {
+// What `of` makes of the FP64 sum of one value per thread, the same in every
+// thread: warps whose lanes hold no value skip their tree, and one thread calls
+// `of` (an FP64 operation of every warp takes the block's unit 16 clocks each).
+template <class F>
+__device__ __forceinline__ auto block_reduce(double v, int nvalues, F&& of) {
   __shared__ double w[kWarps];
-  __shared__ double tot;
+  __shared__ decltype(of(0.0)) result;
   const int warp = threadIdx.x >> 5;
   __syncthreads();
   if (warp * 32 < nvalues) {
@@ -179,11 +181,17 @@ __device__ double block_total(double v, int nvalues) {
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int i = 0; i * 32 < nvalues; ++i) t += w[i];
-    tot = t;
+    result = of(t);
   }
   __syncthreads();
-  return tot;
+  return result;
 }
+__device__ double block_total(double v, int nvalues) {
+  return block_reduce(v, nvalues, [](double t) { return t; });
+}
+
+// a sum in two floats against the limit -/+ what it may be off
+enum Test { kBelow, kNear, kAbove };
 
 // The pixels of one colour that a thread owns: packed indices first + j *
 // kThreads below `end`, row and place stepped without divisions.
@@ -221,24 +229,6 @@ __device__ __forceinline__ void store_normal(float* normals, long long n, long l
   normals[2 * n + i] = __fmul_rn(fabsf(z), rmag);
 }
 
-// The thread's part of the squared residual of the iterate (red, blk), in FP64.
-__device__ __noinline__ double residual_fp64(Problem P, const float4* red, const float4* blk,
-                                             int chunk) {
-  double sum = 0.0;
-  for (int colour = 0; colour < 2; ++colour)
-    for (Walk w(P, chunk); w.more(); w.next()) {
-      const int c = 2 * w.k + ((w.r + colour) & 1);
-      if (c >= P.W) continue;
-      const float4 o = (colour ? blk : red)[w.i];
-      const float x[3] = {o.x, o.y, o.z};
-      float S[3];
-      neighbour_sum(P, colour ? red : blk, w.r, w.k, c, S);
-      residual(P, x, o.w, (float)valence(w.r, c, P.H, P.W), S,
-               [&](float e) { sum += (double)e * (double)e; });
-    }
-  return sum;
-}
-
 __device__ __forceinline__ Problem problem_of(const Args& a) {
   Problem P;
   P.L[0] = a.L0;
@@ -251,6 +241,57 @@ __device__ __forceinline__ Problem problem_of(const Args& a) {
   P.H = a.H;
   P.wh = a.wh;
   return P;
+}
+
+// The sweeps from iterate `it` on with the residual summed in FP64 before each,
+// where sums in two floats do not tell it from the limit (or are not finite).
+struct Iterate {
+  int it;   // below 0: a barrier wait gave up
+  float4 *red, *blk;
+};
+__device__ __noinline__ Iterate sweeps_fp64(Args a, int chunk, double limit2, Iterate x,
+                                            float4* red_next, float4* blk_next, unsigned nbar) {
+  const Problem P = problem_of(a);
+  for (;; ++x.it) {
+    double sum = 0.0;
+    for (int colour = 0; colour < 2; ++colour)
+      for (Walk w(P, chunk); w.more(); w.next()) {
+        const int c = 2 * w.k + ((w.r + colour) & 1);
+        if (c >= P.W) continue;
+        const float4 o = (colour ? x.blk : x.red)[w.i];
+        const float v[3] = {o.x, o.y, o.z};
+        float S[3];
+        neighbour_sum(P, colour ? x.red : x.blk, w.r, w.k, c, S);
+        residual(P, v, o.w, (float)valence(w.r, c, P.H, P.W), S,
+                 [&](float e) { sum += (double)e * (double)e; });
+      }
+    // (the partials of the other parity were read before the last barrier)
+    double* part = a.partial + (size_t)(~x.it & 1) * kMaxBlocks;
+    sum = block_total(sum, kThreads);
+    if (threadIdx.x == 0) __stcg(part + blockIdx.x, sum);
+    if (!grid_barrier_counted(a.hdr, ++nbar)) return Iterate{-1, nullptr, nullptr};
+    const double e2 = block_total(threadIdx.x < gridDim.x ? __ldcg(part + threadIdx.x) : 0.0,
+                                  (int)gridDim.x);
+    if (e2 <= limit2 || x.it >= a.max_iter) return x;
+    for (int colour = 0; colour < 2; ++colour) {
+      for (Walk w(P, chunk); w.more(); w.next()) {
+        const int c = 2 * w.k + ((w.r + colour) & 1);
+        if (c >= P.W) continue;
+        const float si = (colour ? x.blk : x.red)[w.i].w;
+        float S[3], v[3];
+        neighbour_sum(P, colour ? red_next : x.blk, w.r, w.k, c, S);
+        solve(P, si, (float)valence(w.r, c, P.H, P.W), S, v);
+        (colour ? blk_next : red_next)[w.i] = make_float4(v[0], v[1], v[2], si);
+      }
+      if (!grid_barrier_counted(a.hdr, ++nbar)) return Iterate{-1, nullptr, nullptr};
+    }
+    float4* r = x.red;
+    x.red = red_next;
+    red_next = r;
+    r = x.blk;
+    x.blk = blk_next;
+    blk_next = r;
+  }
 }
 
 // One persistent cooperative launch, one block per SM at most, every block
@@ -299,6 +340,7 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
   // The scaled sum's error: below 2^-40 of it, and what its squares lose below
   // FP32's range, under 2^-110 in all.  Within 2^-20 and 2^-90 FP64 decides.
   const double band = limit2 * 0x1p-20 + 0x1p-90;
+  const double below = limit2 - band, above = limit2 + band;
   // the black pixels' residual at x0
   Sum2 black;
   for (Walk w(P, chunk); w.more(); w.next()) {
@@ -312,6 +354,7 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
              [&](float e) { black.add_square(__fmul_rn(e, scale)); });
   }
   int it = 0;
+  bool near = false;
   for (; it < a.max_iter; ++it) {
     double* part = a.partial + (size_t)(it & 1) * kMaxBlocks;
     // red: the residual of the current iterate and the next one's values
@@ -344,17 +387,13 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
       residual(P, x, si, v, S, [&](float e) { black.add_square(__fmul_rn(e, scale)); });
       blk_next[w.i] = make_float4(x[0], x[1], x[2], si);
     }
-    const double sum2 = block_total(mine, (int)gridDim.x);
-    if (sum2 < limit2 - band) break;   // iterate `it` is the result
-    if (!(sum2 > limit2 + band && sum2 < INFINITY)) {
-      // (the same in every block; the other iteration's partials have been read)
-      double* exact = a.partial + (size_t)(~it & 1) * kMaxBlocks;
-      const double e2 = block_total(residual_fp64(P, red, blk, chunk), kThreads);
-      if (threadIdx.x == 0) __stcg(exact + blockIdx.x, e2);
-      if (!grid_barrier_counted(a.hdr, ++nbar)) return;
-      if (block_total(has ? __ldcg(exact + threadIdx.x) : 0.0, (int)gridDim.x) <=
-          (double)a.tol * (double)a.tol * bnorm2)
-        break;
+    const Test test = block_reduce(mine, (int)gridDim.x, [&](double t) {
+      return t < below ? kBelow : t > above && t < INFINITY ? kAbove : kNear;
+    });
+    if (test == kBelow) break;   // iterate `it` is the result
+    if (test == kNear) {
+      near = true;               // (the same in every block)
+      break;
     }
     if (!grid_barrier_counted(a.hdr, ++nbar)) return;
     float4* r = red;
@@ -363,6 +402,14 @@ __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
     r = blk;
     blk = blk_next;
     blk_next = r;
+  }
+  if (near) {
+    const Iterate x = sweeps_fp64(a, chunk, (double)a.tol * (double)a.tol * bnorm2,
+                                  Iterate{it, red, blk}, red_next, blk_next, nbar);
+    if (x.it < 0) return;
+    it = x.it;
+    red = x.red;
+    blk = x.blk;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && a.d_iters) *a.d_iters = it;
   // unit normals with z >= 0, each thread from the pixels it wrote itself
