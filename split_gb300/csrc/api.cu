@@ -84,7 +84,7 @@ __global__ void clear_stages_kernel(StageHeaders s) {
   pdl_wait();
   if (threadIdx.x != 0) return;
   enter_stages(s);
-  s.hdr->stamp = kStampDirty;
+  s.hdr->stamp = s.stamp;
 }
 
 int clear_stages(const StageHeaders& s, cudaStream_t st) {

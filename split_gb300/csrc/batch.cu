@@ -94,6 +94,13 @@ Layout carve(void* ws, const split_batch& b) {
   return l;
 }
 
+// Names what carve() depends on.
+unsigned long long stamp_of(const split_batch& b) {
+  return layout_stamp({2ull, (unsigned long long)b.arena_px, b.images.size(), b.km_bytes,
+                       b.ccl_bytes, b.mrg_bytes, (unsigned)b.params.features,
+                       b.params.merge_P > 0 ? 1u : 0u});
+}
+
 std::vector<KmBatchImage> km_images(const split_batch& b, const Layout& l) {
   std::vector<KmBatchImage> v(b.images.size());
   for (size_t i = 0; i < b.images.size(); ++i) {
@@ -237,11 +244,12 @@ extern "C" int split_batch_bind(split_batch* b, const uint8_t* rgb, float* centr
                               cudaMemcpyHostToDevice, st));
   SG_CUDA_TRY(cudaMemcpyAsync(l.rgb_maps, rgb_maps.data(), sizeof(CUtensorMap) * ni,
                               cudaMemcpyHostToDevice, st));
-  // a rebound arena may hold anything where this layout's stage headers lie
+  // an arena that another layout has used may hold anything where the stages'
+  // headers lie
   {
     StageHeaders sh{};
     sh.hdr = l.hdr;
-    sh.stamp = kStampNone;
+    sh.stamp = stamp_of(*b);
     StatusSources& ss = sh.status;
     ss.p[ss.n++] = &static_cast<WsHeader*>(l.km_ws)->status;
     ss.p[ss.n++] = &static_cast<WsHeader*>(l.ccl_ws)->status;
@@ -317,6 +325,6 @@ extern "C" int split_batch_run_events(split_batch* b, void* const* stage_events,
     SG_TRY(normals_rgb8_geoms(b->rgb, device_geoms(*b, l, l.rgb_maps), p.depth, b->normals, st));
   // errors the stages recorded in their own workspace headers, into the
   // batch's status word
-  SG_TRY(fold_status(l.hdr, ss, st));
+  SG_TRY(fold_status(l.hdr, ss, st, stamp_of(*b)));
   return mark(11);
 }

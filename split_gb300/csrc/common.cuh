@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <initializer_list>
 #include <utility>
 
 #include <cuda/atomic>
@@ -95,7 +96,6 @@ static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 // way or has failed, or an entry point that keeps none has used the workspace
 // (each writes this, or a zero, before it returns).
 constexpr unsigned long long kStampDirty = ~0ull;
-constexpr unsigned long long kStampNone = ~0ull - 1;   // recorded by nobody
 
 // Bump allocator over a caller workspace; with base == nullptr it only
 // measures, so size queries and carving share one code path.
@@ -131,7 +131,7 @@ struct StatusSources {
   int n;
 };
 int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st,
-                unsigned long long stamp = kStampDirty);
+                unsigned long long stamp);
 // What a composite call finds where its stages' headers lie: the stages' as its
 // last run left them, or, when another call or another layout has used the
 // workspace since, anything.  Then the status words go to zero and the stage
@@ -148,8 +148,15 @@ __device__ __forceinline__ void enter_stages(const StageHeaders& s) {
   for (int i = 0; i < s.status.n; ++i) *s.status.p[i] = 0;
   if (s.keeps) s.keeps->stamp = kStampDirty;
 }
-// The same in a launch of its own.
+// The same in a launch of its own, which records the layout.
 int clear_stages(const StageHeaders& s, cudaStream_t st);
+// A composite's stamp from the values that its layout depends on.  Bit 62: no
+// merge's stamp, nor kStampDirty.
+inline unsigned long long layout_stamp(std::initializer_list<unsigned long long> values) {
+  unsigned long long h = 14695981039346656037ull;   // FNV-1a, a word at a time
+  for (unsigned long long v : values) h = (h ^ v) * 1099511628211ull;
+  return (h & ((1ull << 62) - 1)) | 1ull << 62;
+}
 
 // Iteration limit of every spin wait (about a second with the back-off below).
 constexpr unsigned kSpinLimit = 1u << 24;

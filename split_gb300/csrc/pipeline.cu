@@ -54,13 +54,10 @@ static Layout carve(void* ws, int W, int H, const split_pipeline_params& p) {
   return l;
 }
 
-// Names what carve() depends on.  Bit 62: no merge's stamp, nor kStampDirty.
+// Names what carve() depends on.
 static unsigned long long stamp_of(int W, int H, const split_pipeline_params& p) {
-  const unsigned v[] = {(unsigned)W, (unsigned)H, (unsigned)p.nclusters, (unsigned)p.dim,
-                        (unsigned)p.features, p.merge_P > 0 ? 1u : 0u, (unsigned)p.merge_policy};
-  unsigned long long h = 14695981039346656037ull;   // FNV-1a over the words
-  for (unsigned x : v) h = (h ^ x) * 1099511628211ull;
-  return (h & ((1ull << 62) - 1)) | 1ull << 62;
+  return layout_stamp({1ull, (unsigned)W, (unsigned)H, (unsigned)p.nclusters, (unsigned)p.dim,
+                       (unsigned)p.features, p.merge_P > 0 ? 1u : 0u, (unsigned)p.merge_policy});
 }
 
 static bool valid(const split_pipeline_params* p) {
