@@ -86,15 +86,15 @@ struct WsHeader {
   unsigned barrier_gen;
   unsigned counter[2];   // per call, cleared by its first launch
   int result;            // a call's count, for callers that read it with the status
-  // layout the workspace's persistent state is clean for (no layout's: 0, never
-  // used, and kStampDirty)
+  // layout the workspace's persistent state is clean for (no layout's: 0, a
+  // zero-filled workspace that was never used, and kStampDirty)
   unsigned long long stamp;
   int pad[56];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 // The body holds something else: a call that keeps state between calls is under
 // way or has failed, or an entry point that keeps none has used the workspace
-// (each writes this, or a zero, before it returns).
+// (each writes this, and none writes a zero).
 constexpr unsigned long long kStampDirty = ~0ull;
 
 // Bump allocator over a caller workspace; with base == nullptr it only

@@ -2548,6 +2548,7 @@ template <int LAYOUT, int DIM>
 __global__ void __launch_bounds__(kThreads)
 accumulate_kernel(const int32_t* __restrict__ labels, const void* __restrict__ points,
                   int64_t n, int width, float xy_scale, int K, Layout L, bool vec) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) L.hdr->stamp = kStampDirty;
   const int lane = threadIdx.x & 31;
   const int64_t i0 = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * kPer;
   int l[kPer];
@@ -2637,8 +2638,7 @@ int run(const int32_t* labels, const void* points, int layout, int dim, int64_t 
   if (!ws || ws_bytes < l.bytes || (reinterpret_cast<uintptr_t>(ws) & 255))
     return SPLIT_ERR_WORKSPACE;
   l = carve(ws, K, dim);
-  SG_CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(l.hdr) + sizeof(int), 0,
-                              l.bytes - sizeof(int), st));
+  SG_CUDA_TRY(cudaMemsetAsync(l.lo, 0, l.bytes - sizeof(WsHeader), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
   // whole vectors of labels and, planar, of every feature row

@@ -91,16 +91,17 @@ __device__ __forceinline__ unsigned key_hash(unsigned long long key, int bits) {
 }
 
 // The call's words of the header to zero; and, unless the workspace was last
-// used for this layout and left clean (another image size moves the pieces over
-// each other, another entry point writes over them), the pieces that every call
-// leaves clean.  relabel_kernel records the layout.  The call numbers start
-// again when they run out: the entries of fin go with them.
+// used for this layout and left clean, or never used (another image size moves
+// the pieces over each other, another entry point writes over them), the pieces
+// that every call leaves clean.  relabel_kernel records the layout.  The call
+// numbers start again when they run out: the entries of fin go with them.
 __global__ void __launch_bounds__(kThreads)
 guard_kernel(Layout L, unsigned long long stamp, long long n) {
   pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0)
     L.hdr->barrier_count = *L.maxsq = *L.list_count = *L.full = 0u;
-  if (L.hdr->stamp == stamp && *L.call != ~0u) return;
+  const unsigned long long last = L.hdr->stamp;
+  if ((last == stamp || last == 0ull) && *L.call != ~0u) return;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = first; i < n; i += step) L.best[i] = L.fin[i] = 0ull;

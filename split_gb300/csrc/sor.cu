@@ -311,6 +311,7 @@ __device__ __noinline__ Iterate sweeps_fp64(Args a, int chunk, double limit2, It
 // 94 us.
 __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
   const Problem P = problem_of(a);
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.hdr->stamp = kStampDirty;
   unsigned nbar = 0;
   float4 *red = a.red, *red_next = a.red_next, *blk = a.black, *blk_next = a.black_next;
   // x0 = (0, 0, 1) and |b|^2 = sum s_i^2 |L|^2
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(kThreads) sor_in_place_kernel(Args a) {
   const long long n = (long long)P.W * P.H;
   const long long first = (long long)blockIdx.x * kThreads + threadIdx.x;
   const long long step = (long long)gridDim.x * kThreads;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.hdr->stamp = kStampDirty;
   float* const x = a.normals;   // (written and read by every block: no read-only loads)
   const bool has = threadIdx.x < gridDim.x;
   unsigned nbar = 0;
@@ -549,7 +551,7 @@ extern "C" int split_estimate_normals(const float* intensity, int width, int hei
   const bool packed_x = workspace_bytes >= carve(nullptr, width, height, true).bytes;
   const Layout l = carve(workspace, width, height, packed_x);
   cudaStream_t st = as_stream(stream);
-  SG_CUDA_TRY(cudaMemsetAsync(l.hdr, 0, sizeof(WsHeader), st));
+  SG_CUDA_TRY(cudaMemsetAsync(l.hdr, 0, offsetof(WsHeader, stamp), st));
   DeviceInfo di;
   SG_TRY(device_info(&di));
   // One block per SM at most, and one pixel of a colour per thread at least:
