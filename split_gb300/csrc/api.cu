@@ -83,7 +83,7 @@ int fold_status(WsHeader* hdr, const StatusSources& s, cudaStream_t st,
 __global__ void clear_stages_kernel(StageHeaders s) {
   pdl_wait();
   if (threadIdx.x != 0) return;
-  enter_stages(s);
+  enter_stages(s, s.hdr->stamp);
   s.hdr->stamp = s.stamp;
 }
 

@@ -142,9 +142,10 @@ struct StageHeaders {
   StatusSources status;
   WsHeader* keeps;            // may be null
 };
-// By one thread of the first launch that writes to a stage's workspace.
-__device__ __forceinline__ void enter_stages(const StageHeaders& s) {
-  if (!s.hdr || s.hdr->stamp == s.stamp) return;
+// By one thread of the first launch that writes to a stage's workspace; `last`:
+// the stamp found.
+__device__ __forceinline__ void enter_stages(const StageHeaders& s, unsigned long long last) {
+  if (!s.hdr || last == s.stamp) return;
   for (int i = 0; i < s.status.n; ++i) *s.status.p[i] = 0;
   if (s.keeps) s.keeps->stamp = kStampDirty;
 }

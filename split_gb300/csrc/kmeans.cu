@@ -1773,8 +1773,9 @@ template <int DIM>
 __global__ void setup_kernel(Params p, unsigned* zero, int zero_words, StageHeaders own) {
   pdl_wait();
   const Image& im = p.img0;
+  // (read at once, used at the end: nothing here waits for it)
+  const unsigned long long last = threadIdx.x == 0 && own.hdr ? own.hdr->stamp : own.stamp;
   if (threadIdx.x == 0) {
-    enter_stages(own);
     p.hdr->barrier_count = 0u;
     p.hdr->barrier_gen = 0u;
     p.hdr->stamp = kStampDirty;
@@ -1785,6 +1786,7 @@ __global__ void setup_kernel(Params p, unsigned* zero, int zero_words, StageHead
     const int k = idx / DIM, d = idx % DIM;
     p.cur[k * 8 + d] = im.centroids[d * im.K + k];
   }
+  if (threadIdx.x == 0) enter_stages(own, last);
 }
 
 template <int DIM>

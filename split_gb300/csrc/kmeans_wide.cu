@@ -539,7 +539,7 @@ __global__ void setup_kernel(Layout L, int K, int dim, const float* __restrict__
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nt = (int64_t)gridDim.x * blockDim.x;
   if (t == 0) {
-    enter_stages(own);
+    enter_stages(own, own.hdr ? own.hdr->stamp : 0ull);
     State s;
     s.delta = 0.0f;
     s.iters = 0;
