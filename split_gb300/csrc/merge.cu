@@ -46,7 +46,7 @@ constexpr int kThreads = 256;
 constexpr int kPairThreads = 256, kPairBlocks = 6;
 constexpr int kListThreads = 512;   // the decision launch (1024: the 4K frame 4 us more)
 constexpr int kProbeCap = 1 << 16;
-constexpr int kNearProbes = 9;   // from one of eight starts: sixteen slots of a segment
+constexpr int kNearProbes = 4;   // from one of eight starts: eleven slots of a segment
 constexpr unsigned kChainCap = 1u << 24;
 // overflow path: pending classes (level, class) on a stack, and a bound on rounds
 constexpr int kStackCap = 64;
@@ -108,7 +108,7 @@ __device__ __forceinline__ int key_t(unsigned long long k) { return (int)(unsign
 __device__ __forceinline__ int claim(const Layout& L, int s, int t, unsigned m) {
   const unsigned long long key = pair_key(s, t);
   const unsigned mask = (1u << L.cap_log2) - 1u;
-  // A segment's first pairs share sixteen slots, so that its claims, counts and
+  // A segment's first pairs share eleven slots, so that its claims, counts and
   // bids meet in a cache line or two; a pair that finds no room there goes on at
   // a hash of both ids.  Without that a segment of d neighbours probes a run of
   // its own pairs d long.
