@@ -836,7 +836,7 @@ __device__ __forceinline__ void span_batches(const Image& im, Smem& sm, int warp
 
 
 // A warp span that lies wholly inside the image, with packed features (float4,
-// or RGB8 read as three 32-bit words per 4 pixels) and a candidate mask known
+// or RGB8 read as the up to four 32-bit words that hold 4 pixels) and a candidate mask known
 // for the whole span: no per-pixel bounds checks, one pointer step per batch,
 // the column feature hoisted.  Results equal the general path's labels; the
 // sums are the same pixels' in a fixed, data-dependent order.  Returns whether
@@ -891,16 +891,24 @@ __device__ __forceinline__ bool fast_span(const Image& im, Smem& sm, int warp, i
   return MODE == kCluster && kind != kSpanAny;
 }
 
-// Whether a warp span takes the fast path: xy features with colour known to
-// lie in [0, 1], the whole span inside the image, and (RGB8) 4-pixel-aligned
-// rows.  It depends only on the geometry and the layout, so a span is fast in
-// every iteration or in none.
-template <int LAYOUT, int DIM, int MODE>
+// Whether the features are xy ones with colour known to lie in [0, 1].  A batch
+// reads byte / 255 features from the bytes, and its float4 ones (Lab + beta) do
+// not lie there.
+template <int LAYOUT, int DIM, bool BATCH>
+__device__ __forceinline__ bool unit_features(const Image& im) {
+  return DIM == 5 && (LAYOUT == SPLIT_LAYOUT_RGB8 ||
+                      (LAYOUT == SPLIT_LAYOUT_FLOAT4 && !BATCH && im.unit_range));
+}
+
+// Whether a warp span takes the fast path: unit features and the whole span inside
+// the image.  Plain RGB8 asks for 4-pixel-aligned rows too: the loads take any
+// alignment, but which spans are summed exactly decides that layout's last bits.
+// It depends only on the geometry and the layout, so a span is fast in every
+// iteration or in none.
+template <int LAYOUT, int DIM, int MODE, bool BATCH>
 __device__ __forceinline__ bool fast_geometry(const Image& im, int row0, int col0, int wrows,
                                               bool vec_labels) {
-  constexpr bool kXY = DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR;
-  const bool unit_box = kXY && (LAYOUT == SPLIT_LAYOUT_RGB8 || im.unit_range);
-  return MODE != kUpdateOnly && unit_box && row0 + wrows <= im.height &&
+  return MODE != kUpdateOnly && unit_features<LAYOUT, DIM, BATCH>(im) && row0 + wrows <= im.height &&
          col0 + kTile <= im.width &&
          (LAYOUT == SPLIT_LAYOUT_FLOAT4 ||
           (LAYOUT == SPLIT_LAYOUT_RGB8 &&
@@ -947,7 +955,7 @@ __device__ __forceinline__ unsigned long long unit_box_mask(const Image& im, con
 // Returns whether the span needs its pixels in later iterations too (as long
 // as its candidates stay the same).
 // listed: span_mask is the span's candidate mask already (list_spans).
-template <int LAYOUT, int DIM, int MODE, bool FIRST>
+template <int LAYOUT, int DIM, int MODE, bool FIRST, bool BATCH>
 __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, Smem& sm,
                                              bool write_labels, int* status,
                                              unsigned long long span_mask, bool listed) {
@@ -962,14 +970,12 @@ __device__ __forceinline__ bool process_span(const Image& im, int srow, int tx, 
   const int lrow = lane / kLanesPerRow, lcol = (lane % kLanesPerRow) * kPx;
   const int rows_in = min(wrows, im.height - row0);
   const int cols_in = min(kTile, im.width - col0);
-  const bool unit_box = kXY && (LAYOUT == SPLIT_LAYOUT_RGB8 || im.unit_range);
+  const bool unit_box = unit_features<LAYOUT, DIM, BATCH>(im);
   const bool vec_labels =
       (reinterpret_cast<uintptr_t>(MODE == kUpdateOnly ? im.labels_in : im.labels) & 15) == 0 &&
       (im.width % kPx) == 0;
-  // float4 features: any width (labels stored one by one where a row's
-  // start is not 16-byte aligned); RGB8 read as 32-bit words needs
-  // 4-pixel-aligned rows
-  const bool fast = fast_geometry<LAYOUT, DIM, MODE>(im, row0, col0, wrows, vec_labels);
+  // (labels are stored one by one where a row's start is not 16-byte aligned)
+  const bool fast = fast_geometry<LAYOUT, DIM, MODE, BATCH>(im, row0, col0, wrows, vec_labels);
   // slot (srow, tx) of a fast span's kept sums
   long long* entry = (fast && MODE == kCluster && im.span_sum)
                          ? im.span_sum + ((size_t)srow * im.span_cols + tx) * kSpanSums
@@ -1390,7 +1396,7 @@ __device__ __forceinline__ void list_spans(Smem& sm, const Image& im,
         if (__fmaf_rn(g4, g4, __fmaf_rn(g3, g3, c.x)) <= thr) mask |= 1ull << q;
       }
       if (mask != 0ull && (mask & (mask - 1ull)) == 0ull &&
-          fast_geometry<LAYOUT, DIM, MODE>(im, row0, col0, wrows, vec_labels))
+          fast_geometry<LAYOUT, DIM, MODE, BATCH>(im, row0, col0, wrows, vec_labels))
         k = __ffsll((long long)mask) - 1;
     }
     if (k >= 0) {
@@ -1445,7 +1451,8 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
     for (int j = warp; j < share.count; j += kWarps) {
       int sr, tx;
       share.at(j, sr, tx);
-      counted += process_span<LAYOUT, DIM, MODE, true>(im, sr, tx, sm, wl, status, 0ull, false);
+      counted += process_span<LAYOUT, DIM, MODE, true, BATCH>(im, sr, tx, sm, wl, status, 0ull,
+                                                              false);
     }
     if (BATCH) {
       // what the next iteration may cost: spans, and those that need pixels
@@ -1458,9 +1465,8 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
     }
   } else {
     // (with at most one span per warp nothing is gained by listing)
-    constexpr bool kXY = DIM == 5 && LAYOUT != SPLIT_LAYOUT_PLANAR;
-    const bool light = kXY && (LAYOUT == SPLIT_LAYOUT_RGB8 || im.unit_range) && im.span_sum &&
-                       share.count > kWarps;
+    const bool light =
+        unit_features<LAYOUT, DIM, BATCH>(im) && im.span_sum && share.count > kWarps;
     for (int w0 = 0; w0 < share.count;) {
       const int w1 = light ? min(share.count, w0 + kHeavyCap) : share.count;
       if (light) {
@@ -1483,7 +1489,7 @@ __device__ __forceinline__ void span_pass(const Params& p, Smem& sm, const Image
         } else {
           share.at(idx, sr, tx);
         }
-        process_span<LAYOUT, DIM, MODE, false>(im, sr, tx, sm, wl, status,
+        process_span<LAYOUT, DIM, MODE, false, BATCH>(im, sr, tx, sm, wl, status,
                                                light ? sm.heavy_mask[idx] : 0ull, light);
       }
       w0 = w1;
@@ -1824,8 +1830,8 @@ split_tune_entry tuned(int64_t npix) {
 
 // The float4 kernels stage features in kStageBytes of dynamic shared memory,
 // above the default 48 KB limit with their static part: the attribute is set
-// once per device, before any launch (and outside any graph capture: batch
-// preparation calls this too).
+// once per device, before any launch (no stream work, so a graph capture may be
+// under way).  A batch stages nothing (unit_features).
 static int stage_attributes() {
   static std::mutex mu;
   static bool done[64] = {false};
@@ -1836,8 +1842,7 @@ static int stage_attributes() {
   if (done[dev]) return SPLIT_OK;
   const void* kerns[] = {
       (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kCluster>,
-      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kAssignOnly>,
-      (const void*)kmeans_batch_kernel<SPLIT_LAYOUT_FLOAT4, 5>};
+      (const void*)kmeans_kernel<SPLIT_LAYOUT_FLOAT4, 5, kAssignOnly>};
   for (const void* k : kerns)
     SG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kStageBytes));
@@ -1852,9 +1857,10 @@ static int launch(Params& p, cudaStream_t st) {
   auto kern = kmeans_kernel<LAYOUT, DIM, MODE>;
   if constexpr (MODE == kCluster)
     if (p.images) kern = kmeans_batch_kernel<LAYOUT, DIM>;
-  // (3-D features never take the fast path)
+  // (3-D features never take the fast path, a batch's float4 ones neither)
   const size_t dyn =
-      LAYOUT == SPLIT_LAYOUT_FLOAT4 && DIM == 5 && MODE != kUpdateOnly ? kStageBytes : 0;
+      LAYOUT == SPLIT_LAYOUT_FLOAT4 && DIM == 5 && MODE != kUpdateOnly && !p.images ? kStageBytes
+                                                                                    : 0;
   if (dyn) SG_TRY(stage_attributes());
   int per_sm = 0;
   SG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, dyn));
@@ -2279,11 +2285,8 @@ int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int 
                          cudaStream_t st, KmBatchPlan* plan) {
   using namespace km;
   if (!imgs || nimages < 1 || (dim != 3 && dim != 5)) return SPLIT_ERR_INVALID;
-  // kernel attributes now: the batch's launches may be captured into a graph
-  SG_TRY(stage_attributes());
-  const int unit_range = (layout & SPLIT_FEATURES_UNIT_RANGE) ? 1 : 0;
-  if (layout & SPLIT_KMEANS_REFERENCE_SHIFT) return SPLIT_ERR_INVALID;   // single images only
-  layout &= ~SPLIT_FEATURES_UNIT_RANGE;
+  // single images only (see unit_features)
+  if (layout & (SPLIT_KMEANS_REFERENCE_SHIFT | SPLIT_FEATURES_UNIT_RANGE)) return SPLIT_ERR_INVALID;
   const int slots = nimages > 1 ? nimages : 2;
   Layout l = carve(nullptr, slots);
   if (!ws || ws_bytes < l.bytes || (reinterpret_cast<uintptr_t>(ws) & 255))
@@ -2304,7 +2307,6 @@ int kmeans_batch_prepare(const KmBatchImage* imgs, int nimages, int layout, int 
     Image& im = host[i];
     memset(&im, 0, sizeof(im));
     im.points = b.points;
-    im.unit_range = unit_range;
     im.any_width = any_width;
     im.npoints = b.npoints;
     im.width = b.width;
