@@ -326,7 +326,7 @@ def run_batched(dev, nimages, steps, seed=SEED + 1000):
                                         for r in range(reps))
                 for i, name in enumerate(N.PIPELINE_STAGES)}
     peak, peak_kind = peaks()
-    km_bytes = sum(w * h * (16 * it + 4) for w, h, _, it in shapes)
+    km_bytes = 7 * total_px   # the bytes in, the labels out
     bpp = {"pack": 15 * total_px, "kmeans": km_bytes, "ccl": 8 * total_px,
            "merge": 4 * total_px, "erode": 8 * total_px}
     stages = {}
@@ -406,7 +406,7 @@ def run_batched(dev, nimages, steps, seed=SEED + 1000):
             "stages": stages,
             "stages_note": "CUDA-event time of each stage of the batch launched call by call "
                            "(median of runs, L2 flushed before each); frac = algorithmic bytes "
-                           "(normals 15 B/px, k-means 16 B/px per iteration + 4, "
+                           "(normals 15 B/px, k-means 7: bytes in once, labels out, "
                            f"labelling 8, merge pair pass 4, erosion 8) / time / {peak_kind} "
                            "HBM peak",
             "launches_per_run": {"batched": int(batch_launches), "plain": int(plain_launches)}}
@@ -869,7 +869,7 @@ def main():
 
     # ---- roofline of the dominant kernel (k-means, one cooperative launch)
     iters = params.kmeans_iters
-    km_bytes = npx * (16 * iters + 4)  # float4 features per iteration + final labels
+    km_bytes = npx * (3 + 4)   # the bytes in once, the labels out
     km_ms = stage_ms["kmeans"]
     peak, peak_kind = peaks()
     achieved = km_bytes / (km_ms * 1e-3) / 1e9
@@ -877,11 +877,9 @@ def main():
                 "frac": round(achieved / peak, 4), "traffic": profiled_traffic(),
                 "kernel": "kmeans_kernel (cooperative, 20 iterations)",
                 "algorithmic_bytes_per_launch": km_bytes, "peak_source": peak_kind,
-                "bytes_note": "algorithmic bytes of the reference's algorithm (every pixel's "
-                              "16 B features in every iteration, plus the labels); after the "
-                              "first iteration the kernel reads only the pixels of spans with "
-                              "more than one candidate cluster, so its DRAM traffic (ncu) is "
-                              "far below them"}
+                "bytes_note": f"RGB8 in once and labels out, for all {iters} iterations: the "
+                              "kernel is bound by its iterations' barriers and latencies, not by "
+                              "bytes"}
 
     batched = None
     if not args.no_batch and args.batch_images > 0:

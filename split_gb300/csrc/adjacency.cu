@@ -367,9 +367,7 @@ __global__ void __launch_bounds__(kThreads) pair_kernel(const int32_t* __restric
 // number of such keys below it in all tiles: one binary search per tile, whose
 // loads meet in the caches, the keys of a warp being neighbours in order.
 // Bound by the barriers and the searches' latency, kWide tiles in flight.
-// 12 thousand keys (12 tiles): 28 us, of which the three barriers are 7; with
-// four searches in flight and the tiles sorted in shared memory 50; the 27
-// launches of a digit sort and compaction took 158 us.
+// 12 thousand keys (12 tiles): 28 us, of which the three barriers are 7.
 
 // places of `key` in the kWide tiles from t0 on (tiles past the last repeat it)
 constexpr int kWide = 16;

@@ -51,8 +51,7 @@ namespace km {
 
 // Resident blocks per SM the register budget is set for: 2 (up to 128
 // registers a thread) keeps the span passes free of spills; at 3 (80
-// registers) they spill (512 x 512 alone: 0.323 against 0.287 ms in the unit
-// loop; the 48-image batch 3.67 against 3.58 ms in the span loop).
+// registers) they spill.
 #ifndef SG_KM_MINBLOCKS
 #define SG_KM_MINBLOCKS 2
 #endif
@@ -1558,10 +1557,9 @@ __global__ void __launch_bounds__(kThreads, SG_KM_MINBLOCKS) kmeans_kernel(Param
 // the image (steps of about 0.618 nspans), so that it gets its share of the
 // busy regions.
 //
-// What this replaces: 64-row units drawn from a work counter, each with its
-// own block barriers, image switch, flush of the block's sums and fetch, and a
-// second grid barrier to publish the centroids (48 images, 54.7 Mpix, with
-// the other stages: 3.97 ms, now 3.55).
+// What bounds it: an iteration waits for the block with the most spans that need
+// their pixels, each one warp's pass (48 images, 54.7 Mpix, with the other
+// stages: 3.0 ms).
 constexpr int kSegCap = 128;   // images of a range listed at a time
 struct RangeList {
   int n;

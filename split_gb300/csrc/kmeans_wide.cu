@@ -2,9 +2,9 @@
 // memory (64 < K <= 2^20): label_points (split/src/split/device/kmeans/
 // label.cu:74-106) and cluster (cluster.cu:27-93), which set no limit on K.
 //
-// Assignment (assign_kernel): a block takes 64 x 16 pixels at a time, a warp
-// 32 x 4 of them (4 consecutive ones per lane, measured as two packed FP32x2
-// pairs).  The centroids come in shared-memory chunks of 32 KB (1024
+// Assignment (assign_kernel): a block takes a tile of 1024 pixels at a time (64 x
+// 16 of most images), a warp 128 of them (4 consecutive ones per lane, measured as
+// two packed FP32x2 pairs).  The centroids come in shared-memory chunks of 32 KB (1024
 // centroids of 5 dimensions, 2048 of 3).  The block prunes a chunk exactly
 // with bounds over its tile's feature box to a list, each warp the list over
 // its own pixels' box, and measures the survivors.  The squared distance is
@@ -13,7 +13,8 @@
 // < in ascending k, as the reference's argmin over the distance row,
 // label.cu:98-105).  In a clustering the same pass adds every pixel's
 // features to its cluster's fixed-point sums (fixsum.cuh), so the update reads
-// no pixel again; a tile's sums are added up in shared memory first.
+// no pixel again; a tile's sums are added up in shared memory first where the
+// image has many tiles.
 //
 // Clustering: per iteration one assignment launch and one forming launch
 // (form_kernel), all max_iter pairs queued at once, each launch a

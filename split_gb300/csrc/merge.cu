@@ -170,7 +170,9 @@ __device__ __forceinline__ unsigned seg_class(int s, int lev) {
 }
 
 // Sum of x over the lanes of `peers` (the lanes that hold this lane's value),
-// left in the lowest of them: pairs of peers add up in log2 steps.
+// left in the lowest of them: pairs of peers add up in log2 steps (the peer
+// reduction by rank parity of E. Westphal, "Voting and Shuffling to Optimize
+// Atomic Operations", 2015).
 __device__ __forceinline__ double sum_peers(unsigned peers, double x) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -385,15 +387,11 @@ __device__ __forceinline__ bool tile_add_pair(T& tab, int slot, int t, unsigned 
 // more pixels than decided segments).
 //
 // What bounds it: the latency of global atomics where segments are small and
-// many.  Inserting pixel by pixel, up to eight dependent rounds of a table
-// probe, a compare-and-swap and two adds, took 237 us for a 512 x 512 frame
-// of 128 tiles and 4.2 ms for an 8192 x 8192 maze with 1.4 M segments.
-// The shared tables take one round per distinct pair and tile, segments inside
-// the tile (most segments below a few dozen pixels) none at all, and segments
-// of one pixel are decided from registers; list places are taken with one
-// atomic per block.  Maze: this pass 4.2 to 1.15 ms, with the labelling 6.67
-// to 2.61 ms; 512 x 512 speckle (which took the decision twice) 496 to 252 us
-// a frame.
+// many: an insert is a table probe, a compare-and-swap and two adds in turn.
+// So the shared tables take one round of them per distinct pair and tile,
+// segments inside the tile (most segments below a few dozen pixels) none at all,
+// and segments of one pixel are decided from registers; list places are taken
+// with one atomic per block.  8192 x 8192 maze, 1.4 M segments: 1.15 ms.
 template <bool CLASSES, bool DEFER, class T>
 __device__ __forceinline__ void pair_tile(const int32_t* __restrict__ lab, const Geoms& gs,
                                           const Layout& L, const int32_t* sizes, int P, int policy,

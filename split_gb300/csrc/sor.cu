@@ -306,9 +306,7 @@ __device__ __noinline__ Iterate sweeps_fp64(Args a, int chunk, double limit2, It
 // iterate.  The test's total is known after the barrier that ends the red
 // pass and is added up beside the black pass, so both passes write a second
 // buffer and the iterate before them is the result when the test holds.
-// VGA: 8.2 us a sweep; with a separate residual pass over planar unknowns,
-// FP64 sums, one thread adding all blocks' partials and 760 blocks it took
-// 94 us.
+// VGA: 8.2 us a sweep.
 __global__ void __launch_bounds__(kThreads) sor_kernel(Args a, int chunk) {
   const Problem P = problem_of(a);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.hdr->stamp = kStampDirty;
