@@ -111,3 +111,36 @@ def test_smooth_call_numbers_run_out(cuda):
     s.ws.view[:256].view(torch.int32)[8] = -3
     for _ in range(4):
         s.smooth()
+
+
+def test_batches_in_turn_in_one_arena(cuda):
+    """Two layouts, one of them twice in a row, and another call in between, in one
+    arena: every batch's segments are those of fresh buffers."""
+    import torch
+    from split_gb300 import batch, ccl, pipeline
+    params = pipeline.Params(merge_P=40, xy_scale=0.01)
+    shapes = [[(200, 150, 8, 3), (90, 70, 4, 2)], [(120, 110, 8, 3)]]
+    rng = np.random.default_rng(9)
+    imgs = [[rng.integers(0, 256, (h, w, 3)).astype(np.uint8) for w, h, _, _ in s] for s in shapes]
+    cents = [[rng.random((5, k)).astype(np.float32) for _, _, k, _ in s] for s in shapes]
+
+    def run(i, arena):
+        b = batch.Batch(shapes[i], params, cuda, arena=arena)
+        b.load(imgs[i], cents[i])
+        b.run()
+        torch.cuda.synchronize()
+        b.ws.check("batch")
+        return [b.segment_labels_of(k).clone() for k in range(len(shapes[i]))]
+
+    want = [run(i, None) for i in range(2)]
+    arena = batch.Arena(cuda)
+    run(0, arena)
+    lab = torch.arange(60 * 60, dtype=torch.int32, device=cuda).view(60, 60)
+    out = [torch.empty(8 * 3600, dtype=torch.int32, device=cuda) for _ in range(2)]
+    for i in (0, 1, 0, 0, -1, 0, 1, -1, 1, 1, 0):
+        if i < 0:
+            need = ccl.segment_adjacency_workspace(60, 60)
+            ccl.segment_adjacency(lab, *out, ccl.Workspace.over(arena.ws_buf, need))
+            continue
+        for got, ref in zip(run(i, arena), want[i]):
+            assert torch.equal(got, ref)
